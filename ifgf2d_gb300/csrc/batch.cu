@@ -110,8 +110,8 @@ int ensure_apply(ifgf2d_ctx* ctx, int B, bool mixed) {
             CK(W.rho32.alloc((size_t)N * W.cap)); CK(W.coef32.alloc(ncoef * W.cap)); CK(W.xt32.alloc((size_t)N * W.cap));
         }
         if (!W.pb32.p) {
-            CK(W.pb32.alloc(ctx->pp.n));
-            launch_sort_plan<float>(ctx->pp_ptr.p, ctx->T.total_cones, ctx->pp.p, ctx->T.P, W.pb32.p, ctx->stream);
+            CK(W.pb32.alloc(ctx->pp.child.n));
+            launch_sort_plan<float>(ctx->pp_ptr.p, ctx->T.total_cones, ctx->pp.view(), ctx->pp32.p, ctx->T.P, W.pb32.p, ctx->stream);
             CK(cudaGetLastError());
         }
         if (!W.t5err.p) {
@@ -140,11 +140,11 @@ int ensure_apply(ifgf2d_ctx* ctx, int B, bool mixed) {
     } else {
         if (!W.rho64.p) { CK(W.rho64.alloc((size_t)N * W.cap)); CK(W.coef64.alloc(ncoef * W.cap)); }
         if (!W.pb64.p) {
-            CK(W.pb64.alloc(ctx->pp.n));
-            launch_sort_plan<double>(ctx->pp_ptr.p, ctx->T.total_cones, ctx->pp.p, ctx->T.P, W.pb64.p, ctx->stream);
+            CK(W.pb64.alloc(ctx->pp.child.n));
+            launch_sort_plan<double>(ctx->pp_ptr.p, ctx->T.total_cones, ctx->pp.view(), ctx->pp32.p, ctx->T.P, W.pb64.p, ctx->stream);
             CK(cudaGetLastError());
-            CK(W.rows64.alloc(ctx->pp.n * (size_t)(ctx->T.Ps + ctx->T.Pang)));
-            launch_plan_rows<double>(W.pb64.p, (long long)ctx->pp.n, ctx->T.Ps, ctx->T.Pang, W.rows64.p, ctx->stream);
+            CK(W.rows64.alloc(ctx->pp.child.n * (size_t)(ctx->T.Ps + ctx->T.Pang)));
+            launch_plan_rows<double>(W.pb64.p, (long long)ctx->pp.child.n, ctx->T.Ps, ctx->T.Pang, W.rows64.p, ctx->stream);
             CK(cudaGetLastError());
         }
     }

@@ -95,6 +95,46 @@ struct DBuf {
     cudaError_t upload(const std::vector<T>& v) { return upload(v.data(), v.size()); }
 };
 
+// the arrays of a PlanX
+struct PlanBuf {
+    DBuf<int> child;
+    DBuf<unsigned short> slot;
+    DBuf<longlong2> st;
+    DBuf<double2> w;
+    cudaError_t alloc(size_t cnt) {
+        cudaError_t e = child.alloc(cnt);
+        if (e == cudaSuccess) e = slot.alloc(cnt);
+        if (e == cudaSuccess) e = st.alloc(cnt);
+        if (e == cudaSuccess) e = w.alloc(cnt);
+        return e;
+    }
+    PlanX view() const { return PlanX{child.p, slot.p, st.p, w.p}; }
+    size_t bytes() const { return child.n * (sizeof(int) + sizeof(short) + sizeof(longlong2) + sizeof(double2)); }
+};
+inline PlanX plan_at(PlanX p, long long e) { return PlanX{p.child + e, p.slot + e, p.st + e, p.w + e}; }
+// the staged groups of a tree's FP64 propagation (launch_stage_plan): level l's, parents at level
+// l - 1, from at[l]
+struct PlanStage {
+    DBuf<int> list;
+    std::vector<size_t> at;
+    const int* level(int l) const { return list.p + at[l]; }
+    cudaError_t build(const Tree& T, const long long* pp_ptr, PlanX pp, cudaStream_t s) {
+        at.assign(T.nlevels + 1, 0);
+        size_t total = 0;
+        for (int l = T.nlevels - 1; l >= 3; --l) {
+            at[l] = total;
+            total += stage_plan_size((int)T.L[l - 1].cone_nonrel.size(), T.Ps, T.Pang);
+        }
+        cudaError_t e = list.alloc(total);
+        for (int l = T.nlevels - 1; l >= 3 && e == cudaSuccess; --l) {
+            const TreeLevel& Lp = T.L[l - 1];
+            launch_stage_plan(Lp.cone_base, Lp.cone_base + (int)Lp.cone_nonrel.size(), pp_ptr, pp, T.Ps, T.Pang, list.p + at[l], s);
+            e = cudaGetLastError();
+        }
+        return e;
+    }
+};
+
 }  // namespace ifgf
 
 using namespace ifgf;
@@ -182,10 +222,14 @@ struct ifgf2d_ctx {
     DBuf<double2> leafL;
     DBuf<long long> pp_ptr;
     DBuf<int> pp_nchild;
-    DBuf<PropEntryD> pp;
+    PlanBuf pp;
+    PlanStage pp_stage;
     DBuf<int> ip_ptr;
-    DBuf<InterpEntryD> ip;
-    DBuf<double2> coef;
+    DBuf<InterpEntryD> ip;          // the batched FP64 form's
+    DBuf<InterpX> ipx;              // the single-vector FP64 form's
+    DBuf<int4> coef;                // FP64 form: fixed-point limbs, with
+    DBuf<int> cexp;                 // one exponent per cone
+    DBuf<int2> GsepX;               // Gsep as limbs
     DBuf<double> Gm, Gsep;          // full and separable values->coefficients maps
     DBuf<int> near_rowlen;          // per leaf box: sources in its 3x3 neighbourhood
     DBuf<int> near_src_off, near_src;   // per leaf box: the Morton indices of those sources, in row order
@@ -198,7 +242,7 @@ struct ifgf2d_ctx {
     // precisions, and the pieces' sums per target
     DBuf<int4> ib_items;
     DBuf<int2> nb_items;            // near field by leaf box (k_near_box): (box, first of up to 32 targets)
-    DBuf<InterpE<double>> ipT;
+    DBuf<InterpX> ipT;
     DBuf<InterpE<float>> ip32T;
     DBuf<double2> ib_part;
     DBuf<float2> ib_part32;
@@ -253,7 +297,7 @@ struct SetupExtra {
     const double2* keta_leafbox = nullptr;
     const double2* keta_leafcone = nullptr;
     std::function<cudaError_t(LeafNode*, cudaStream_t)> build_nodes;
-    std::function<cudaError_t(PropE<double>*, PropE<float>*, int*, cudaStream_t)> build_plan;
+    std::function<cudaError_t(PlanX, PropE<float>*, int*, cudaStream_t)> build_plan;
 };
 // the host tables of a context built from ctx->D: near-singular patches per point, the
 // rectangular-polar columns and rows (ifgf2d_capi.cu)
@@ -292,7 +336,7 @@ int net_prepare_single(ifgf2d_net* net, long long N, const double* geom_host, do
 // queued on `s`; otherwise the stream is synchronised before returning.  For a member of a group
 // of obstacles, level_cone_base[l] replaces level l's first global cone id and
 // level_entry_base[l] the first entry of the slots with children at level l.
-cudaError_t build_prop_plan(const Tree& T, PropE<double>* pp64, PropE<float>* pp32, int* err, cudaStream_t s,
+cudaError_t build_prop_plan(const Tree& T, PlanX pp64, PropE<float>* pp32, int* err, cudaStream_t s,
                             const int* level_cone_base = nullptr, const long long* level_entry_base = nullptr);
 // The propagation plan computed level by level while the host builds the tree's cones: after
 // each level's cones and slots exist, add() uploads them and launches that level's entries into
@@ -307,7 +351,7 @@ public:
     PropPlanByLevel(const PropPlanByLevel&) = delete;
     PropPlanByLevel& operator=(const PropPlanByLevel&) = delete;
     void add(const Tree& T, int level);
-    cudaError_t gather(PropE<double>* pp64, PropE<float>* pp32, int* err, cudaStream_t s);
+    cudaError_t gather(PlanX pp64, PropE<float>* pp32, int* err, cudaStream_t s);
 private:
     struct Impl;
     Impl* d;
@@ -318,7 +362,7 @@ cudaError_t build_leaf_nodes(const Tree& T, LeafNode* out, cudaStream_t s);
 // a parent's propagation terms sorted by child cone (stable), with the parent node recorded, for
 // the batched propagation
 template <typename R>
-void launch_sort_plan(const long long* pp_ptr, int ncones, const PropE<double>* pp, int P, PropB<R>* out, cudaStream_t s);
+void launch_sort_plan(const long long* pp_ptr, int ncones, PlanX px, const PropE<float>* pp32, int P, PropB<R>* out, cudaStream_t s);
 // the complex64 copy of the interpolation plan
 void launch_interp_to_c64(const InterpE<double>* in, long long n, InterpE<float>* out, cudaStream_t s);
 void net_precondition_launch(ifgf2d_net* net, const double2* r, double2* z, cudaStream_t s);

@@ -285,7 +285,7 @@ extern "C" int ifgf2d_group_create(ifgf2d_ctx* const* members, int n, ifgf2d_gro
         }
         return cudaSuccess;
     };
-    ex.build_plan = [&](PropE<double>* pp64, PropE<float>* pp32, int* err, cudaStream_t s) -> cudaError_t {
+    ex.build_plan = [&](PlanX pp64, PropE<float>* pp32, int* err, cudaStream_t s) -> cudaError_t {
         for (int o = 0; o < n; ++o) {
             const cudaError_t e = build_prop_plan(members[o]->T, pp64, pp32, err, s, cbase[o].data(), ebase[o].data());
             if (e != cudaSuccess) return e;

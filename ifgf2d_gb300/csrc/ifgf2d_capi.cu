@@ -494,8 +494,11 @@ static int setup_cones(ifgf2d_ctx* ctx, double k, int nlevels, const SetupExtra*
         for (int n = 0; n < Pa; ++n)
             for (int l = 0; l < Pa; ++l) Gs[(size_t)Ps * Ps + (size_t)n * Pa + l] = Tn(n, xa[l]) * ((n == 0 ? 1.0 : 2.0) / Pa);
         CK(ctx->Gsep.upload(Gs));
+        CK(ctx->GsepX.alloc(Gs.size()));
         std::vector<float> Gs32(Gs.begin(), Gs.end());
         CK(ctx->Gsep32.upload(Gs32));
+        launch_fx_weights(ctx->Gsep.p, (int)Gs.size(), ctx->GsepX.p, ctx->stream);
+        CK(cudaGetLastError());
     }
     // The uploads come before the kernels that follow them: a copy from pageable host memory
     // queued behind a running kernel holds the host until the kernel ends.  The leaf-cone nodes'
@@ -516,9 +519,10 @@ static int setup_cones(ifgf2d_ctx* ctx, double k, int nlevels, const SetupExtra*
     else CK(build_leaf_nodes(T, ctx->leaf_nodes_d.p, ctx->stream));
     // propagation plan: the entries are computed on the device from the tree's slot form (or
     // were, level by level, while the host built the cones)
-    if (ex) CK(ex->build_plan(ctx->pp.p, ctx->pp32.p, perr.p, ctx->stream));
-    else if (by_level) CK(by_level->gather(ctx->pp.p, ctx->pp32.p, perr.p, ctx->stream));
-    else CK(build_prop_plan(T, ctx->pp.p, ctx->pp32.p, perr.p, ctx->stream));
+    if (ex) CK(ex->build_plan(ctx->pp.view(), ctx->pp32.p, perr.p, ctx->stream));
+    else if (by_level) CK(by_level->gather(ctx->pp.view(), ctx->pp32.p, perr.p, ctx->stream));
+    else CK(build_prop_plan(T, ctx->pp.view(), ctx->pp32.p, perr.p, ctx->stream));
+    CK(ctx->pp_stage.build(T, ctx->pp_ptr.p, ctx->pp.view(), ctx->stream));
     // leaf-cone tables
     launch_leaf_setup(ctx->leaf_cone_box.p, ncl, ctx->leaf_start.p, ctx->leaf_count.p, ctx->leaf_off.p, ctx->leaf_nodes_d.p,
                       ctx->xs_s.p, ctx->ys_s.p, ctx->nxs_s.p, ctx->nys_s.p, T.Ps, T.Pang, k, ctx->form, ctx->eta, ctx->Gsep.p,
@@ -538,7 +542,9 @@ static int setup_interp(ifgf2d_ctx* ctx, int nlevels, DBuf<int>& perr) {
         CK(ctx->ip.upload(reinterpret_cast<const InterpEntryD*>(T.ip.data()), T.ip.size()));
         CK(ctx->ip_ptr.upload(T.ip_ptr));
         CK(ctx->ip32.alloc(T.ip.size()));
+        CK(ctx->ipx.alloc(T.ip.size()));
         launch_interp_to_c64(ctx->ip.p, (long long)T.ip.size(), ctx->ip32.p, ctx->stream);
+        launch_interp_fx(ctx->ip.p, (long long)T.ip.size(), ctx->ipx.p, ctx->stream);
         CK(cudaGetLastError());
     }
     {   // interpolation by leaf box: per box, chunks of 32 targets x pieces of kIbPiece terms
@@ -566,6 +572,7 @@ static int setup_interp(ifgf2d_ctx* ctx, int nlevels, DBuf<int>& perr) {
         CK(ctx->ib_part.alloc((size_t)std::max(maxpc, 1) * N)); CK(ctx->ib_part32.alloc((size_t)std::max(maxpc, 1) * N));
     }
     CK(ctx->coef.alloc((size_t)T.total_cones * P));
+    CK(ctx->cexp.alloc((size_t)T.total_cones));
     CK(ctx->coef32.alloc((size_t)T.total_cones * P));
     CK(ctx->rho32.alloc(N + 2));   // + padding: the TMA leaf kernel copies from 16-byte boundaries
     CK(ctx->near32.alloc(ctx->near.n));
@@ -582,7 +589,7 @@ static int setup_interp(ifgf2d_ctx* ctx, int nlevels, DBuf<int>& perr) {
     if (bad) return fail(ctx, IFGF2D_ERR_GEOMETRY, "internal: a propagation node's child cone is missing");
     ctx->counts[0] = T.near_pairs; ctx->counts[1] = T.leaf_evals; ctx->counts[2] = T.prop_evals;
     ctx->counts[3] = T.interp_evals; ctx->counts[4] = T.total_cones; ctx->counts[5] = nlevels;
-    ctx->counts[7] = (long long)(ctx->near.n + ctx->leafL.n + ctx->coef.n + ctx->W.n) * 16 + (long long)ctx->pp.n * sizeof(PropEntryD) +
+    ctx->counts[7] = (long long)(ctx->near.n + ctx->leafL.n + ctx->coef.n + ctx->W.n) * 16 + (long long)ctx->pp.bytes() +
                      (long long)ctx->ip.n * sizeof(InterpEntryD);
     ctx->ifgf_ready = true;
     if (ctx->gw) ctx->gw->drop_graphs();
@@ -625,23 +632,23 @@ static int check_kerr(ifgf2d_ctx* ctx) {
 // k_final_t, a warp per target.  By leaf box: the interpolation by k_interp_box (pieces per
 // target), then the near field by k_near_box, which adds the pieces in order.
 template <typename R>
-static void launch_interp_final(ifgf2d_ctx* ctx, const V2<R>* rho, const V2<R>* near, const InterpE<R>* ip, const V2<R>* coef,
+static void launch_interp_final(ifgf2d_ctx* ctx, const V2<R>* rho, const V2<R>* near, const InterpT<R>* ip, const CoefT<R>* coef,
                                 double2* y, bool by_box) {
     const Tree& T = ctx->T;
     const int N = (int)ctx->D.N;
     if (!by_box || ctx->nb_items.n == 0) {
         launch_final_t<R>(N, ctx->point_leaf.p, ctx->leaf_start.p, ctx->near_src_off.p, ctx->near_src.p, ctx->near_rowlen.p,
-                          ctx->near_off.p, near, rho, ctx->ip_ptr.p, ip, coef, T.Ps, T.Pang, ctx->sorting.p, y, ctx->stream);
+                          ctx->near_off.p, near, rho, ctx->ip_ptr.p, ip, coef, ctx->cexp.p, T.Ps, T.Pang, ctx->sorting.p, y, ctx->stream);
         return;
     }
     const V2<R>* part = nullptr;
     if (ctx->ib_items.n > 0) {
         V2<R>* pp;
-        const InterpE<R>* ipT;
+        const InterpT<R>* ipT;
         if constexpr (sizeof(R) == 4) { pp = ctx->ib_part32.p; ipT = ctx->ip32T.p; }
         else { pp = ctx->ib_part.p; ipT = ctx->ipT.p; }
         launch_interp_box<R>(ctx->ib_items.p, (int)ctx->ib_items.n, N, ctx->leaf_start.p, ctx->leaf_count.p, ctx->ip_ptr.p, ipT,
-                             coef, T.Ps, T.Pang, pp, ctx->stream);
+                             coef, ctx->cexp.p, T.Ps, T.Pang, pp, ctx->stream);
         part = pp;
     }
     launch_near_box<R>(ctx->nb_items.p, (int)ctx->nb_items.n, ctx->leaf_start.p, ctx->leaf_count.p, ctx->near_src_off.p,
@@ -649,10 +656,24 @@ static void launch_interp_final(ifgf2d_ctx* ctx, const V2<R>* rho, const V2<R>* 
                        ctx->stream);
 }
 
+// children at level l -> parents at level l - 1; `shape`: the complex64 kernel's launch shape (the
+// FP64 kernel has one)
+template <typename R>
+static void launch_prop_level(ifgf2d_ctx* ctx, int l, CoefT<R>* coef, int shape) {
+    const Tree& T = ctx->T;
+    const TreeLevel& Lp = T.L[l - 1];
+    const int p0 = Lp.cone_base, p1 = Lp.cone_base + (int)Lp.cone_nonrel.size();
+    if constexpr (sizeof(R) == 4)
+        launch_propagate_t(p0, p1, ctx->pp_ptr.p, ctx->pp_nchild.p, ctx->pp32.p, T.Ps, T.Pang, ctx->Gsep32.p, coef, ctx->stream, shape);
+    else
+        launch_propagate_fx(p0, p1, ctx->pp.view(), ctx->pp_stage.level(l), T.Ps, T.Pang, ctx->GsepX.p, coef, ctx->cexp.p,
+                            ctx->stream);
+}
+
 // y += far field of the Morton-ordered intensities (rho / rho32), BoxTree.h:1037-1061
 template <typename R>
-static void far_ifgf_t(ifgf2d_ctx* ctx, const V2<R>* rho, const V2<R>* near, const V2<R>* leafL, const PropE<R>* pp,
-                       const InterpE<R>* ip, const R* Gsep, V2<R>* coef, double2* y, cudaEvent_t* ev) {
+static void far_ifgf_t(ifgf2d_ctx* ctx, const V2<R>* rho, const V2<R>* near, const V2<R>* leafL, const InterpT<R>* ip,
+                       CoefT<R>* coef, double2* y, cudaEvent_t* ev) {
     const Tree& T = ctx->T;
     const int Dl = ctx->nlevels - 1, P = T.P;
     const TreeLevel& LD = T.L[Dl];
@@ -666,12 +687,10 @@ static void far_ifgf_t(ifgf2d_ctx* ctx, const V2<R>* rho, const V2<R>* near, con
     }
     if (!leaf_done)
         launch_leaf_apply_t<R>(ctx->leaf_cone_box.p, (int)LD.cone_nonrel.size(), LD.cone_base, ctx->leaf_start.p, ctx->leaf_count.p,
-                               ctx->leaf_off.p, leafL, rho, P, coef, s, ctx->tune_leaf[pr]);
+                               ctx->leaf_off.p, leafL, rho, P, T.Ps, coef, ctx->cexp.p, s, ctx->tune_leaf[pr]);
     if (ev) cudaEventRecord(ev[0], s);
     for (int l = Dl; l >= 3; --l) {
-        const TreeLevel& Lp = T.L[l - 1];
-        launch_propagate_t<R>(Lp.cone_base, Lp.cone_base + (int)Lp.cone_nonrel.size(), ctx->pp_ptr.p, ctx->pp_nchild.p, pp,
-                              T.Ps, T.Pang, Gsep, coef, s, l < kTuneLevels ? ctx->tune_prop[pr][l] : 0);
+        launch_prop_level<R>(ctx, l, coef, l < kTuneLevels ? ctx->tune_prop[pr][l] : 0);
     }
     if (ev) cudaEventRecord(ev[1], s);
     launch_interp_final<R>(ctx, rho, near, ip, coef, y, (ctx->tune_batch_tc & (pr ? kSingleInterpBox32 : kSingleInterpBox64)) != 0);
@@ -685,13 +704,11 @@ static int far_apply(ifgf2d_ctx* ctx, const double2* x, const double* wq, double
     if (mode == IFGF2D_APPLY_IFGF_MIXED) {
         if (!rho_ready) launch_intensities_t<float>(x, wq, ctx->sorting.p, N, ctx->rho32.p, ctx->stream);
         if (ev) cudaEventRecord(ev[0], ctx->stream);
-        far_ifgf_t<float>(ctx, ctx->rho32.p, ctx->near32.p, ctx->leafL32.p, ctx->pp32.p, ctx->ip32.p, ctx->Gsep32.p,
-                          ctx->coef32.p, y, ev ? ev + 1 : nullptr);
+        far_ifgf_t<float>(ctx, ctx->rho32.p, ctx->near32.p, ctx->leafL32.p, ctx->ip32.p, ctx->coef32.p, y, ev ? ev + 1 : nullptr);
     } else {
         if (!rho_ready) launch_intensities_t<double>(x, wq, ctx->sorting.p, N, ctx->rho.p, ctx->stream);
         if (ev) cudaEventRecord(ev[0], ctx->stream);
-        far_ifgf_t<double>(ctx, ctx->rho.p, ctx->near.p, ctx->leafL.p, ctx->pp.p, ctx->ip.p, ctx->Gsep.p, ctx->coef.p, y,
-                           ev ? ev + 1 : nullptr);
+        far_ifgf_t<double>(ctx, ctx->rho.p, ctx->near.p, ctx->leafL.p, ctx->ipx.p, ctx->coef.p, y, ev ? ev + 1 : nullptr);
     }
     CK(cudaGetLastError());
     return IFGF2D_OK;
@@ -789,8 +806,7 @@ extern "C" int ifgf2d_set_tuning(ifgf2d_ctx* ctx, const int* c) {
     return IFGF2D_OK;
 }
 template <typename R>
-static int tune_precision(ifgf2d_ctx* ctx, int reps, const V2<R>* rho, const V2<R>* leafL, const PropE<R>* pp, const R* Gsep,
-                          V2<R>* coef) {
+static int tune_precision(ifgf2d_ctx* ctx, int reps, const V2<R>* rho, const V2<R>* leafL, CoefT<R>* coef) {
     const Tree& T = ctx->T;
     const int Dl = ctx->nlevels - 1, P = T.P, pr = sizeof(R) == 4 ? 1 : 0;
     const TreeLevel& LD = T.L[Dl];
@@ -820,19 +836,15 @@ static int tune_precision(ifgf2d_ctx* ctx, int reps, const V2<R>* rho, const V2<
             }
             if (!done)
                 launch_leaf_apply_t<R>(ctx->leaf_cone_box.p, (int)LD.cone_nonrel.size(), LD.cone_base, ctx->leaf_start.p,
-                                       ctx->leaf_count.p, ctx->leaf_off.p, leafL, rho, P, coef, s, ch);
+                                       ctx->leaf_count.p, ctx->leaf_off.p, leafL, rho, P, T.Ps, coef, ctx->cexp.p, s, ch);
         });
         if (ms < best) { best = ms; bestc = ch; }
     }
     ctx->tune_leaf[pr] = bestc;
-    for (int l = Dl; l >= 3 && l < kTuneLevels; --l) {
-        const TreeLevel& Lp = T.L[l - 1];
+    for (int l = Dl; l >= 3 && l < kTuneLevels && sizeof(R) == 4; --l) {   // the FP64 kernel has one shape
         best = 1e30f; int bestp = 0;
         for (int cpb : {2, 4, 0, kPropStaged}) {
-            const float ms = time_it([&] {
-                launch_propagate_t<R>(Lp.cone_base, Lp.cone_base + (int)Lp.cone_nonrel.size(), ctx->pp_ptr.p, ctx->pp_nchild.p, pp,
-                                      T.Ps, T.Pang, Gsep, coef, s, cpb);
-            });
+            const float ms = time_it([&] { launch_prop_level<R>(ctx, l, coef, cpb); });
             if (ms < best) { best = ms; bestp = cpb; }
         }
         ctx->tune_prop[pr][l] = bestp;
@@ -840,9 +852,9 @@ static int tune_precision(ifgf2d_ctx* ctx, int reps, const V2<R>* rho, const V2<
     {   // the interpolation by leaf box or by target (y: the context's output vector, overwritten later)
         const int bit = pr ? kSingleInterpBox32 : kSingleInterpBox64;
         const V2<R>* near;
-        const InterpE<R>* ip;
+        const InterpT<R>* ip;
         if constexpr (sizeof(R) == 4) { near = ctx->near32.p; ip = ctx->ip32.p; }
-        else { near = ctx->near.p; ip = ctx->ip.p; }
+        else { near = ctx->near.p; ip = ctx->ipx.p; }
         const float tb = time_it([&] { launch_interp_final<R>(ctx, rho, near, ip, coef, ctx->vout.p, true); });
         const float tt = time_it([&] { launch_interp_final<R>(ctx, rho, near, ip, coef, ctx->vout.p, false); });
         if (tb < tt) ctx->tune_batch_tc |= bit;
@@ -861,8 +873,8 @@ extern "C" int ifgf2d_autotune(ifgf2d_ctx* ctx, int reps, int* choices) {
     int rc;
     if ((rc = apply_dev(ctx, ctx->vin.p, ctx->vout.p, IFGF2D_APPLY_IFGF))) return rc;
     if ((rc = apply_dev(ctx, ctx->vin.p, ctx->vout.p, IFGF2D_APPLY_IFGF_MIXED))) return rc;
-    if ((rc = tune_precision<double>(ctx, reps, ctx->rho.p, ctx->leafL.p, ctx->pp.p, ctx->Gsep.p, ctx->coef.p))) return rc;
-    if ((rc = tune_precision<float>(ctx, reps, ctx->rho32.p, ctx->leafL32.p, ctx->pp32.p, ctx->Gsep32.p, ctx->coef32.p))) return rc;
+    if ((rc = tune_precision<double>(ctx, reps, ctx->rho.p, ctx->leafL.p, ctx->coef.p))) return rc;
+    if ((rc = tune_precision<float>(ctx, reps, ctx->rho32.p, ctx->leafL32.p, ctx->coef32.p))) return rc;
     CK(cudaStreamSynchronize(ctx->stream));
     if (ctx->gw) ctx->gw->drop_graphs();
     if (choices) write_tuning(ctx, choices);

@@ -43,9 +43,20 @@ template <> struct InterpE<float> { int cone; float s, th, fr, fi; };
 // batched complex64 interpolation term, grouped by leaf box and cone: cone id, Morton target,
 // (s, theta), factor
 struct InterpG { int cone; int t; float s, th, fr, fi; };
+// the FP64 form of the same, (s, theta) as fixed-point weights (fixpoint.cuh)
+struct InterpX { int cone; int pad; long long s, th; double fr, fi; };
+// cone coefficients of the single-vector apply: complex64, or fixed-point limbs (re.h, re.l, im.h,
+// im.l) with one exponent per cone (fixpoint.cuh) in the FP64 form; and the terms that read them
+template <typename R> struct CoefOf;
+template <> struct CoefOf<double> { using T = int4; };
+template <> struct CoefOf<float> { using T = float2; };
+template <typename R> using CoefT = typename CoefOf<R>::T;
+template <typename R> struct InterpOf;
+template <> struct InterpOf<double> { using T = InterpX; };
+template <> struct InterpOf<float> { using T = InterpE<float>; };
+template <typename R> using InterpT = typename InterpOf<R>::T;
 // one (parent cone, child, node) propagation term: child cone id, (s, theta), factor ratio
 template <typename R> struct PropE;
-template <> struct PropE<double> { int child_cone; int pad; double s, th, wr, wi; };
 template <> struct PropE<float> { int child_cone; float s, th, wr, wi; };
 // batched propagation term: the parent node pt it feeds, then as PropE.  A parent's terms are
 // sorted by child cone, so a warp loads each child cone's coefficients once per parent.
@@ -53,7 +64,10 @@ template <typename R> struct PropB;
 template <> struct PropB<double> { int child_cone; int pt; double s, th, wr, wi; };
 template <> struct PropB<float> { int child_cone; int pt; float s, th, wr, wi; };
 using InterpEntryD = InterpE<double>;
-using PropEntryD = PropE<double>;
+// the FP64 propagation plan, array by array (each lane's loads are whole vectors, coalesced): child
+// cone, its slot in its group's staged list (launch_stage_plan), (s, theta) as fixed-point weights,
+// factor ratio
+struct PlanX { int* child; unsigned short* slot; longlong2* st; double2* w; };
 
 constexpr int kMaxP = 64;          // Ps * Pang limit of the device interpolator
 
@@ -97,8 +111,8 @@ template <typename R>
 void launch_intensities_t(const double2* x, const double* wq, const long long* perm, int N, V2<R>* rho, cudaStream_t s);
 template <typename R>
 void launch_leaf_apply_t(const int* cone_box, int ncones, int cone_base, const int* leaf_start, const int* leaf_count,
-                         const long long* leaf_off, const V2<R>* L, const V2<R>* rho, int P, V2<R>* coef, cudaStream_t s,
-                         int chunks = 5);
+                         const long long* leaf_off, const V2<R>* L, const V2<R>* rho, int P, int Ps, CoefT<R>* coef, int* cexp,
+                         cudaStream_t s, int chunks = 5);
 // complex64 leaf cones with the table streamed through shared memory by TMA bulk copies
 // (P = 25); false when not launched (other P, or leaf_tma_init not run).  *err is set when a
 // completion wait runs out.  leaf_tma_init sets the kernel's shared-memory attribute (outside
@@ -110,22 +124,31 @@ cudaError_t leaf_tma_init();
 // the propagation variant that stages child coefficient blocks in shared memory (k_propagate_st);
 // other values of cones_per_block: 2, 4, or 0 for the most that fit 256 threads
 constexpr int kPropStaged = 1;
-template <typename R>
-void launch_propagate_t(int pbegin, int pend, const long long* pp_ptr, const int* pp_nchild, const PropE<R>* pp, int Ps,
-                        int Pang, const R* Gsep, V2<R>* coef, cudaStream_t s, int cones_per_block = 0);
+void launch_propagate_t(int pbegin, int pend, const long long* pp_ptr, const int* pp_nchild, const PropE<float>* pp, int Ps,
+                        int Pang, const float* Gsep, float2* coef, cudaStream_t s, int cones_per_block = 0);
+// the FP64 form in fixed point: GsepX the separable map's entries as limbs, cexp the cones' exponents,
+// stage the records of the level's groups of parents (stage_plan_size ints for ncones parents), which
+// launch_stage_plan fills together with pp.slot
+size_t stage_plan_size(int ncones, int Ps, int Pang);
+void launch_stage_plan(int pbegin, int pend, const long long* pp_ptr, PlanX pp, int Ps, int Pang, int* stage, cudaStream_t s);
+void launch_propagate_fx(int pbegin, int pend, PlanX pp, const int* stage, int Ps, int Pang, const int2* GsepX, int4* coef, int* cexp,
+                         cudaStream_t s);
+// n doubles in [-1, 1] as fixed-point limbs; the interpolation plan with (s, theta) as weights
+void launch_fx_weights(const double* in, int n, int2* out, cudaStream_t s);
+void launch_interp_fx(const InterpE<double>* in, long long n, InterpX* out, cudaStream_t s);
 // with `part`, the interpolation terms were summed by launch_interp_box: the near field plus each
 // target's pieces in order
 template <typename R>
 void launch_final_t(int N, const int* point_leaf, const int* leaf_start, const int* near_src_off, const int* near_src,
                     const int* near_rowlen, const long long* near_off, const V2<R>* near,
-                    const V2<R>* rho, const int* ip_ptr, const InterpE<R>* ip, const V2<R>* coef, int Ps, int Pang,
-                    const long long* sorting, double2* y, cudaStream_t s, const V2<R>* part = nullptr);
+                    const V2<R>* rho, const int* ip_ptr, const InterpT<R>* ip, const CoefT<R>* coef, const int* cexp, int Ps,
+                    int Pang, const long long* sorting, double2* y, cudaStream_t s, const V2<R>* part = nullptr);
 // interpolation by leaf box (k_interp_box): items[w] = (leaf box, first target, first term, end
 // term), pieces of kIbPiece terms; part[piece * N + target] receives each piece's sum
 constexpr int kIbPiece = 8;
 template <typename R>
 void launch_interp_box(const int4* items, int nitems, int N, const int* leaf_start, const int* leaf_count, const int* ip_ptr,
-                       const InterpE<R>* ipT, const V2<R>* coef, int Ps, int Pang, V2<R>* part, cudaStream_t s);
+                       const InterpT<R>* ipT, const CoefT<R>* coef, const int* cexp, int Ps, int Pang, V2<R>* part, cudaStream_t s);
 // near field by leaf box (k_near_box): items[w] = (leaf box, first of up to 32 targets); adds the
 // near field, then the target's interpolation pieces (when part is not null), into y
 constexpr int kNearChunk = 1024, kNearTargets = 32;
@@ -136,7 +159,7 @@ void launch_near_box(const int2* items, int nitems, const int* leaf_start, const
 // the interpolation plan box-transposed (term j of box target t at the box's first entry + j n + t)
 template <typename R>
 void launch_interp_transpose(int N, const int* point_leaf, const int* leaf_start, const int* leaf_count, const int* ip_ptr,
-                             const InterpE<double>* in, InterpE<R>* out, cudaStream_t s);
+                             const InterpE<double>* in, InterpT<R>* out, cudaStream_t s);
 void launch_d2f(const double2* a, long long n, float2* b, cudaStream_t s);
 // Load the direct map's kernels (singular correction, FP64 intensities, both far-sum shapes) into
 // the current device's context now.  Under lazy module loading a kernel is otherwise loaded,

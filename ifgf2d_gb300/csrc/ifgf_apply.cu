@@ -1,6 +1,7 @@
 // ifgf_apply.cu -- per-apply IFGF kernels, templated on the arithmetic type.
 //
-// R = double: the plain form (complex128 tables, FP64 arithmetic).
+// R = double: the plain form (complex128 tables; cone coefficients and interpolation in block fixed
+//             point of FP64 accuracy, fixpoint.cuh, the rest FP64 arithmetic).
 // R = float : the mixed form (complex64 copies of the same FP64-computed tables, FP32
 //             arithmetic; the rectangular-polar correction stays FP64).
 //
@@ -10,7 +11,7 @@
 //                  separable values->coefficients map                             BoxTree.h:767-868, Interpolator.h:81-120
 //   k_final        near field + every level's cousin interpolants, one warp per target,
 //                  result added to y at the target's original index               BoxTree.h:614-683, 876-937, 1063-1069
-#include "ifgf_device.cuh"
+#include "fixpoint.cuh"
 #include "tcgen05.cuh"
 #include <type_traits>
 #include <algorithm>
@@ -38,8 +39,11 @@ template <typename R, int CH>
 __global__ void __launch_bounds__(256) k_leaf_apply_t(const int* __restrict__ cone_box, int ncones, int cone_base,
                                                       const int* __restrict__ leaf_start, const int* __restrict__ leaf_count,
                                                       const long long* __restrict__ leaf_off, const V2<R>* __restrict__ L,
-                                                      const V2<R>* __restrict__ rho, int P, V2<R>* __restrict__ coef) {
+                                                      const V2<R>* __restrict__ rho, int P, int Ps, CoefT<R>* __restrict__ coef,
+                                                      int* __restrict__ cexp) {
     __shared__ V2<R> part[256];
+    __shared__ int smax[256];               // FP64: per cone, the largest high word of its coefficients
+    if constexpr (sizeof(R) == 8) smax[threadIdx.x] = 0;
     const int per_cone = P * CH;
     const int cpb = blockDim.x / per_cone;
     const int local = threadIdx.x / per_cone, r = threadIdx.x - local * per_cone;
@@ -64,10 +68,20 @@ __global__ void __launch_bounds__(256) k_leaf_apply_t(const int* __restrict__ co
     }
     part[threadIdx.x] = a0;
     __syncthreads();
-    if (active && ch == 0) {
-        V2<R> acc = a0;
+    V2<R> acc = a0;
+    if (active && ch == 0)
         for (int q = 1; q < CH; ++q) { const V2<R> v = part[local * per_cone + q * P + m]; acc.x += v.x; acc.y += v.y; }
-        coef[(long long)(cone_base + c) * P + m] = acc;
+    if constexpr (sizeof(R) == 8) {
+        if (active && ch == 0) atomicMax(&smax[local], fx_absmax_hi(acc.x, acc.y));
+        __syncthreads();
+        if (active && ch == 0) {
+            const int E = fx_expo(smax[local]), T = fx_top(P);
+            const long long xr = E == kFxBad ? 0 : fx_from(acc.x, E, T), xi = E == kFxBad ? 0 : fx_from(acc.y, E, T);
+            coef[(long long)(cone_base + c) * P + m] = m % Ps ? fx_pack(xr, xi) : fx_pack_raw(xr, xi);
+            if (m == 0) cexp[cone_base + c] = E;
+        }
+    } else {
+        if (active && ch == 0) coef[(long long)(cone_base + c) * P + m] = acc;
     }
 }
 
@@ -169,12 +183,13 @@ __global__ void __launch_bounds__(kLtThreads) k_leaf_tma(const int* __restrict__
     }
 }
 
-// thread = (parent cone, interpolation node); CPB cones per block.  Gsep = [PS x PS radial
+// complex64: thread = (parent cone, interpolation node); CPB cones per block.  Gsep = [PS x PS radial
 // map | PA x PA angular map] of the values->coefficients transform, normalisation included.
-template <typename R, int PS, int PA, int CPB>
+template <int PS, int PA, int CPB>
 __global__ void __launch_bounds__(256) k_propagate_t(int pbegin, int pend, const long long* __restrict__ pp_ptr,
-                                                     const int* __restrict__ pp_nchild, const PropE<R>* __restrict__ pp,
-                                                     const R* __restrict__ Gsep, V2<R>* __restrict__ coef) {
+                                                     const int* __restrict__ pp_nchild, const PropE<float>* __restrict__ pp,
+                                                     const float* __restrict__ Gsep, float2* __restrict__ coef) {
+    using R = float;
     constexpr int P = PS * PA;
     __shared__ V2<R> sv[CPB][P];
     __shared__ V2<R> su[CPB][P];
@@ -188,34 +203,25 @@ __global__ void __launch_bounds__(256) k_propagate_t(int pbegin, int pend, const
         const long long e0 = pp_ptr[pc];
         const int nch = pp_nchild[pc];
         V2<R> v; v.x = R(0); v.y = R(0);
-        if (sizeof(R) == 4) {
-            // all plan entries first, then two children's coefficient gathers before any arithmetic
-            PropE<R> E[4];
+        // all plan entries first, then two children's coefficient gathers before any arithmetic
+        PropE<R> E[4];
 #pragma unroll
-            for (int ch = 0; ch < 4; ++ch) if (ch < nch) E[ch] = pp[e0 + (long long)ch * P + pt];
+        for (int ch = 0; ch < 4; ++ch) if (ch < nch) E[ch] = pp[e0 + (long long)ch * P + pt];
 #pragma unroll
-            for (int c0 = 0; c0 < 4; c0 += 2) {
-                if (c0 >= nch) break;
-                V2<R> ca[P], cb[P];
-                const V2<R>* pa = coef + (long long)E[c0].child_cone * P;
-                const bool two = c0 + 1 < nch;
-                const int cb_cone = two ? E[c0 + 1].child_cone : E[c0].child_cone;
-                const V2<R>* pb = coef + (long long)cb_cone * P;
+        for (int c0 = 0; c0 < 4; c0 += 2) {
+            if (c0 >= nch) break;
+            V2<R> ca[P], cb[P];
+            const V2<R>* pa = coef + (long long)E[c0].child_cone * P;
+            const bool two = c0 + 1 < nch;
+            const int cb_cone = two ? E[c0 + 1].child_cone : E[c0].child_cone;
+            const V2<R>* pb = coef + (long long)cb_cone * P;
 #pragma unroll
-                for (int q = 0; q < P; ++q) { ca[q] = pa[q]; cb[q] = pb[q]; }
-                V2<R> w; w.x = E[c0].wr; w.y = E[c0].wi;
-                cmac<R>(v, interp_eval<R, PS, PA>(ca, E[c0].s, E[c0].th), w);
-                if (two) {
-                    w.x = E[c0 + 1].wr; w.y = E[c0 + 1].wi;
-                    cmac<R>(v, interp_eval<R, PS, PA>(cb, E[c0 + 1].s, E[c0 + 1].th), w);
-                }
-            }
-        } else {
-            for (int ch = 0; ch < nch; ++ch) {
-                const PropE<R> E = pp[e0 + (long long)ch * P + pt];
-                const V2<R> it = interp_eval<R, PS, PA>(coef + (long long)E.child_cone * P, E.s, E.th);
-                V2<R> w; w.x = E.wr; w.y = E.wi;
-                cmac<R>(v, it, w);
+            for (int q = 0; q < P; ++q) { ca[q] = pa[q]; cb[q] = pb[q]; }
+            V2<R> w; w.x = E[c0].wr; w.y = E[c0].wi;
+            cmac<R>(v, interp_eval<R, PS, PA>(ca, E[c0].s, E[c0].th), w);
+            if (two) {
+                w.x = E[c0 + 1].wr; w.y = E[c0 + 1].wi;
+                cmac<R>(v, interp_eval<R, PS, PA>(cb, E[c0 + 1].s, E[c0 + 1].th), w);
             }
         }
         sv[local][pt] = v;
@@ -246,6 +252,163 @@ __global__ void __launch_bounds__(256) k_propagate_t(int pbegin, int pend, const
     }
 }
 
+// k_propagate_fx's blocks: parent cones (a thread per node), child blocks held in shared memory, and
+// the block's record: first plan entry (two ints), staged children, the cones' first entries from it
+// (cones + 1), the children
+constexpr int kPropFxThreads = 128;
+template <int P>
+struct PropFx {
+    static constexpr int cones = kPropFxThreads / P;
+    static constexpr int slots = 12000 / (16 * P);
+    static constexpr int list = 4 + cones;
+    static constexpr int record = list + slots;
+    static constexpr int terms = cones * 4 * P;
+};
+__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// FP64 in fixed point (fixpoint.cuh).  A block takes a group of PropFx::cones parent cones.  The group's
+// terms are one contiguous range of the plan; the range and the distinct child blocks it reads (listed
+// at set-up, k_stage_plan; about four per parent cone, each read by some 14 terms) are copied into
+// shared memory, all copies in flight together behind the group's one record.  Every term gets a thread
+// (no lane waits for a cone with more children); then a thread per node sums its children in order.  A
+// term interpolates in integers (about 160 wide multiply-adds) and takes 6 FP64 operations for its
+// conversion and factor ratio, against 60 with FP64 interpolation.  The node values get their cone's
+// common exponent, the values->coefficients map runs in integers again, and the coefficients are
+// normalised to the top bits of the cone's largest.  Kite, all levels: k = 500 290 -> 100 us, k = 2000
+// 1287 -> 399 us (the FP64 kernel before it ran at 91-95 % of the FP64 pipe).  What bounds it: the wide
+// multiply-adds and 64-bit shifts take two issue slots each; some 45 % of the slots issue.  Measured
+// slower: a thread per node gathering from L1 (110 us), a warp per parent cone (131 us: 25 of 32
+// lanes), persistent blocks that fetch ahead (111-125 us).
+template <int PS, int PA>
+__global__ void __launch_bounds__(kPropFxThreads) k_propagate_fx(int pbegin, int pend, PlanX pp, const int* __restrict__ stage,
+                                                                 const int2* __restrict__ Gsep, int4* __restrict__ coef,
+                                                                 int* __restrict__ cexp) {
+    constexpr int P = PS * PA, T = fx_top(P), NT = kPropFxThreads;
+    using F = PropFx<P>;
+    constexpr int CPB = F::cones, CAP = F::slots;
+    static_assert(CPB * P <= NT && F::terms <= 4 * NT, "a thread per node, at most four terms a thread");
+    __shared__ int4 blk[CAP * P];
+    __shared__ longlong2 sst[F::terms];
+    __shared__ double2 val[F::terms];          // the terms' factor ratios, then their values
+    __shared__ int4 sv[CPB * P];
+    __shared__ int2 sGs[PS * PS], sGa[PA * PA];
+    __shared__ int rec[F::record], sE[CAP], smax[CPB], slz[CPB];
+    const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
+    for (int i = tid; i < F::record; i += NT) rec[i] = stage[(long long)blockIdx.x * F::record + i];
+    for (int i = tid; i < PS * PS; i += NT) sGs[i] = Gsep[i];
+    for (int i = tid; i < PA * PA; i += NT) sGa[i] = Gsep[PS * PS + i];
+    if (tid < CPB) { smax[tid] = 0; slz[tid] = 64; }
+    __syncthreads();
+    const long long e0 = ((long long)rec[1] << 32) | (unsigned)rec[0];
+    const int ns = rec[2], nt = rec[3 + CPB];
+    for (int k = wp; k < ns; k += NT / 32) {
+        const int4* src = coef + (long long)rec[F::list + k] * P;
+#pragma unroll
+        for (int i = 0; i < P; i += 32) if (lane + i < P) cp_async16(&blk[k * P + lane + i], src + lane + i);
+    }
+    int slot[4] = {0, 0, 0, 0};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const int t = tid + k * NT;
+        if (t < nt) {
+            cp_async16(&sst[t], pp.st + e0 + t);
+            cp_async16(&val[t], pp.w + e0 + t);
+            slot[k] = pp.slot[e0 + t];
+        }
+    }
+    for (int i = tid; i < ns; i += NT) sE[i] = cexp[rec[F::list + i]];
+    cp_async_wait_all();
+    __syncthreads();
+#pragma unroll 1
+    for (int k = 0; k < 4; ++k) {
+        const int t = tid + k * NT, sl = k == 0 ? slot[0] : (k == 1 ? slot[1] : (k == 2 ? slot[2] : slot[3]));
+        if (t >= nt) break;
+        double2 it;
+        if (sl < CAP) {
+            it = fx_interp_value<PS, PA>([&](int i) { return blk[sl * P + i]; }, sE[sl], sst[t]);
+        } else {   // more distinct children than slots
+            const int c = pp.child[e0 + t];
+            const int4* src = coef + (long long)c * P;
+            it = fx_interp_value<PS, PA>([&](int i) { return src[i]; }, cexp[c], sst[t]);
+        }
+        const double2 w = val[t];
+        val[t] = make_double2(it.x * w.x - it.y * w.y, it.x * w.y + it.y * w.x);
+    }
+    __syncthreads();
+    const int local = tid / P, pt = tid - local * P, m = pt % PS, l = pt / PS;
+    const int pc = pbegin + blockIdx.x * CPB + local;
+    const bool active = local < CPB && pc < pend;
+    double2 v = make_double2(0.0, 0.0);
+    if (active) {
+        for (int t = rec[3 + local] + pt; t < rec[4 + local]; t += P) { v.x += val[t].x; v.y += val[t].y; }
+        atomicMax(&smax[local], fx_absmax_hi(v.x, v.y));
+    }
+    __syncthreads();
+    const int E = active ? fx_expo(smax[local]) : 0;
+    if (active) sv[tid] = E == kFxBad ? make_int4(0, 0, 0, 0) : fx_pack(fx_from(v.x, E, T), fx_from(v.y, E, T));
+    __syncthreads();
+    int4* su = blk;          // the child blocks have been read
+    if (active) {            // u[l][m] = sum_k Gs[m][k] v[l*PS + k]
+        long long ur, ui;
+        fx_map<PS>([&](int k) { return sGs[m * PS + k]; }, [&](int k) { return sv[local * P + l * PS + k]; }, ur, ui);
+        su[tid] = fx_pack(ur, ui);
+    }
+    __syncthreads();
+    long long cr = 0, ci = 0;
+    if (active) {            // c[n][m] = sum_l Ga[n][l] u[l][m], stored at n*PS + m
+        fx_map<PA>([&](int q) { return sGa[l * PA + q]; }, [&](int q) { return su[local * P + q * PS + m]; }, cr, ci);
+        atomicMin(&slz[local], min(__clzll(cr < 0 ? -cr : cr), __clzll(ci < 0 ? -ci : ci)));
+    }
+    __syncthreads();
+    if (active) {
+        int sh = slz[local] - (63 - T);      // left shift that brings the largest to [2^(T-1), 2^T)
+        sh = E == kFxBad ? 0 : min(sh, E - kFxMinExp);
+        cr = fx_shift(cr, sh); ci = fx_shift(ci, sh);
+        coef[(long long)pc * P + pt] = m ? fx_pack(cr, ci) : fx_pack_raw(cr, ci);
+        if (pt == 0) cexp[pc] = E == kFxBad ? kFxBad : E - sh;
+    }
+}
+
+// set-up of k_propagate_fx: a group's record with the first PropFx::slots of its distinct child cones
+// in ascending order, and per term its slot (PropFx::slots: not staged)
+template <int P>
+__global__ void __launch_bounds__(kPropFxThreads) k_stage_plan(int pbegin, int pend, const long long* __restrict__ pp_ptr, PlanX pp,
+                                                               int* __restrict__ stage) {
+    using F = PropFx<P>;
+    constexpr int CPB = F::cones, CAP = F::slots, NT = kPropFxThreads;
+    __shared__ int kid[F::terms], uniq[F::terms];
+    __shared__ int nu;
+    const int tid = threadIdx.x;
+    const int c0 = pbegin + blockIdx.x * CPB, nc = min(CPB, pend - c0);
+    const long long e0 = pp_ptr[c0];
+    const int nt = min((int)(pp_ptr[c0 + nc] - e0), F::terms);
+    if (tid == 0) nu = 0;
+    for (int t = tid; t < nt; t += NT) kid[t] = pp.child[e0 + t];
+    __syncthreads();
+    for (int t = tid; t < nt; t += NT) {       // a child's first term lists it (neighbouring terms mostly share a child)
+        const int c = kid[t];
+        bool first = true;
+        for (int q = t - 1; q >= 0 && first; --q) first = kid[q] != c;
+        if (first) uniq[atomicAdd(&nu, 1)] = c;
+    }
+    __syncthreads();
+    int* rec = stage + (long long)blockIdx.x * F::record;
+    const int n = nu;
+    if (tid == 0) { rec[0] = (int)e0; rec[1] = (int)(e0 >> 32); rec[2] = min(n, CAP); }
+    if (tid <= CPB) rec[3 + tid] = (int)(pp_ptr[c0 + min(tid, nc)] - e0);
+    for (int i = n + tid; i < CAP; i += NT) rec[F::list + i] = 0;
+    for (int t = tid; t < nt; t += NT) {
+        const int c = kid[t];
+        int r = 0;
+        for (int q = 0; q < n; ++q) r += uniq[q] < c;
+        pp.slot[e0 + t] = (unsigned short)min(r, CAP);
+        if (r < CAP) rec[F::list + r] = c;
+    }
+}
+
 // k_propagate_t with the child coefficient blocks staged in shared memory.  A parent cone's 25
 // nodes read 1-4 children's blocks each, but the block's ten parent cones touch only about 40
 // distinct child cones (3.4-4.3 per parent cone on the kite trees), so the per-thread gathers
@@ -254,17 +417,17 @@ __global__ void __launch_bounds__(256) k_propagate_t(int pbegin, int pend, const
 // copies each one's block once with coalesced loads, and evaluates from shared memory.  A child
 // cone that finds no free key or no data slot is read from global memory.  Each thread's
 // arithmetic is that of k_propagate_t in the same order, so the results are bit-identical.
-// FP64 gains a few per cent from it (the autotuner takes it on the finer levels); in complex64
-// the 25 shared-memory reads per term cost as much as the L1 hits they replace.
+// On the kite trees the 25 shared-memory reads per term cost as much as the L1 hits they replace.
 constexpr int kStageKeys = 128;
 template <typename R, int P>
 struct PropStage {
     static constexpr int cap = (size_t)P * sizeof(V2<R>) * 64 <= 26000 ? 64 : (int)(26000 / ((size_t)P * sizeof(V2<R>)));
 };
-template <typename R, int PS, int PA, int CPB>
+template <int PS, int PA, int CPB>
 __global__ void __launch_bounds__(256) k_propagate_st(int pbegin, int pend, const long long* __restrict__ pp_ptr,
-                                                      const int* __restrict__ pp_nchild, const PropE<R>* __restrict__ pp,
-                                                      const R* __restrict__ Gsep, V2<R>* __restrict__ coef) {
+                                                      const int* __restrict__ pp_nchild, const PropE<float>* __restrict__ pp,
+                                                      const float* __restrict__ Gsep, float2* __restrict__ coef) {
+    using R = float;
     constexpr int P = PS * PA;
     constexpr int CAP = PropStage<R, P>::cap;
     __shared__ int key[kStageKeys], slot_of[kStageKeys], ulist[CAP];
@@ -376,6 +539,18 @@ __global__ void __launch_bounds__(256) k_propagate_st(int pbegin, int pend, cons
     }
 }
 
+// one interpolation term in the arithmetic type: the interpolant at the term's point times its factor
+template <int PS, int PA>
+__device__ __forceinline__ void add_term(double2& acc, const InterpX& E, const int4* __restrict__ coef, const int* __restrict__ cexp) {
+    const int4* c = coef + (long long)E.cone * (PS * PA);
+    cmac<double>(acc, fx_interp_value<PS, PA>([&](int i) { return c[i]; }, cexp[E.cone], make_longlong2(E.s, E.th)),
+                 make_double2(E.fr, E.fi));
+}
+template <int PS, int PA>
+__device__ __forceinline__ void add_term(float2& acc, const InterpE<float>& E, const float2* __restrict__ coef, const int*) {
+    cmac<float>(acc, interp_eval<float, PS, PA>(coef + (long long)E.cone * (PS * PA), E.s, E.th), make_float2(E.fr, E.fi));
+}
+
 // one warp per (leaf box, up to 32 of its targets, kIbPiece of their interpolation terms), one
 // lane per target.  The targets of a leaf box share their ancestors, hence the same cousin lists
 // in the same order: their j-th terms read the same cousin box, mostly the same cone (2.5-3
@@ -386,9 +561,9 @@ __global__ void __launch_bounds__(256) k_propagate_st(int pbegin, int pend, cons
 template <typename R, int PS, int PA>
 __global__ void __launch_bounds__(256) k_interp_box(const int4* __restrict__ items, int nitems, int N,
                                                     const int* __restrict__ leaf_start, const int* __restrict__ leaf_count,
-                                                    const int* __restrict__ ip_ptr, const InterpE<R>* __restrict__ ipT,
-                                                    const V2<R>* __restrict__ coef, V2<R>* __restrict__ part) {
-    constexpr int P = PS * PA;
+                                                    const int* __restrict__ ip_ptr, const InterpT<R>* __restrict__ ipT,
+                                                    const CoefT<R>* __restrict__ coef, const int* __restrict__ cexp,
+                                                    V2<R>* __restrict__ part) {
     const int w = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     if (w >= nitems) return;
     const int lane = threadIdx.x & 31;
@@ -396,10 +571,11 @@ __global__ void __launch_bounds__(256) k_interp_box(const int4* __restrict__ ite
     const int s = leaf_start[I.x], n = leaf_count[I.x];
     const int t = I.y + lane;
     if (t >= n) return;
-    const InterpE<R>* e = ipT + ip_ptr[s] + t;
+    const InterpT<R>* e = ipT + ip_ptr[s] + t;
     V2<R> acc; acc.x = R(0); acc.y = R(0);
     int j = I.z;
     if constexpr (sizeof(R) == 4) {   // two terms' loads in flight before either is evaluated
+        constexpr int P = PS * PA;
         for (; j + 1 < I.w; j += 2) {
             const InterpE<R> E0 = e[(long long)j * n], E1 = e[(long long)(j + 1) * n];
             V2<R> c0[P], c1[P];
@@ -414,13 +590,8 @@ __global__ void __launch_bounds__(256) k_interp_box(const int4* __restrict__ ite
         }
     }
     for (; j < I.w; ++j) {
-        const InterpE<R> E = e[(long long)j * n];
-        V2<R> c[P];
-        const V2<R>* cb = coef + (long long)E.cone * P;
-#pragma unroll
-        for (int q = 0; q < P; ++q) c[q] = cb[q];
-        V2<R> f; f.x = E.fr; f.y = E.fi;
-        cmac<R>(acc, interp_eval<R, PS, PA>(c, E.s, E.th), f);
+        const InterpT<R> E = e[(long long)j * n];
+        add_term<PS, PA>(acc, E, coef, cexp);
     }
     part[(long long)(I.z / kIbPiece) * N + s + t] = acc;
 }
@@ -489,22 +660,34 @@ __global__ void __launch_bounds__(256) k_near_box(const int2* __restrict__ items
     }
 }
 
+__device__ __forceinline__ InterpX interp_fx(const InterpE<double>& E) {
+    return InterpX{E.cone, E.pad, fx_weight(E.s), fx_weight(E.th), E.fr, E.fi};
+}
 // the interpolation plan of each leaf box transposed: term j of the box's target t moves from
 // ip_ptr[i] + j to ip_ptr[box's first target] + j n + t (every target of a box has as many terms)
 template <typename R>
 __global__ void k_interp_transpose(int N, const int* __restrict__ point_leaf, const int* __restrict__ leaf_start,
                                    const int* __restrict__ leaf_count, const int* __restrict__ ip_ptr,
-                                   const InterpE<double>* __restrict__ in, InterpE<R>* __restrict__ out) {
+                                   const InterpE<double>* __restrict__ in, InterpT<R>* __restrict__ out) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= N) return;
     const int b = point_leaf[i], s = leaf_start[b], n = leaf_count[b], t = i - s;
     const int base = ip_ptr[s], nt = ip_ptr[i + 1] - ip_ptr[i];
     for (int j = 0; j < nt; ++j) {
         const InterpE<double> E = in[ip_ptr[i] + j];
-        InterpE<R> o{};
-        o.cone = E.cone; o.s = (R)E.s; o.th = (R)E.th; o.fr = (R)E.fr; o.fi = (R)E.fi;
+        InterpT<R> o{};
+        if constexpr (sizeof(R) == 8) o = interp_fx(E);
+        else { o.cone = E.cone; o.s = (R)E.s; o.th = (R)E.th; o.fr = (R)E.fr; o.fi = (R)E.fi; }
         out[base + (long long)j * n + t] = o;
     }
+}
+__global__ void k_interp_fx(const InterpE<double>* __restrict__ in, long long n, InterpX* __restrict__ out) {
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) out[i] = interp_fx(in[i]);
+}
+__global__ void k_fx_weights(const double* __restrict__ in, int n, int2* __restrict__ out) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) { const FxLimb t = fx_split(fx_weight(in[i])); out[i] = make_int2(t.h, t.l); }
 }
 
 // one warp per Morton-sorted target; near row layout [target][neighbour sources], and
@@ -517,10 +700,9 @@ __global__ void __launch_bounds__(256) k_final_t(int N, const int* __restrict__ 
                                                  const int* __restrict__ near_rowlen,
                                                  const long long* __restrict__ near_off, const V2<R>* __restrict__ near,
                                                  const V2<R>* __restrict__ rho, const int* __restrict__ ip_ptr,
-                                                 const InterpE<R>* __restrict__ ip, const V2<R>* __restrict__ coef,
-                                                 const long long* __restrict__ sorting, double2* __restrict__ y,
-                                                 const V2<R>* __restrict__ part) {
-    constexpr int P = PS * PA;
+                                                 const InterpT<R>* __restrict__ ip, const CoefT<R>* __restrict__ coef,
+                                                 const int* __restrict__ cexp, const long long* __restrict__ sorting,
+                                                 double2* __restrict__ y, const V2<R>* __restrict__ part) {
     const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (i >= N) return;
@@ -534,10 +716,8 @@ __global__ void __launch_bounds__(256) k_final_t(int N, const int* __restrict__ 
     for (int e = lane; e < rl; e += 32) cmac<R>(acc, row[e], rho[src[e]]);
     if (!part) {
         for (int e = ip_ptr[i] + lane; e < ip_ptr[i + 1]; e += 32) {
-            const InterpE<R> E = ip[e];
-            const V2<R> it = interp_eval<R, PS, PA>(coef + (long long)E.cone * P, E.s, E.th);
-            V2<R> f; f.x = E.fr; f.y = E.fi;
-            cmac<R>(acc, it, f);
+            const InterpT<R> E = ip[e];
+            add_term<PS, PA>(acc, E, coef, cexp);
         }
     }
     acc.x = warp_sum_r<R>(acc.x);
@@ -572,15 +752,15 @@ cudaError_t preload_intensities_kernel() {
 }
 template <typename R>
 void launch_leaf_apply_t(const int* cone_box, int ncones, int cone_base, const int* leaf_start, const int* leaf_count,
-                         const long long* leaf_off, const V2<R>* L, const V2<R>* rho, int P, V2<R>* coef, cudaStream_t s,
-                         int chunks) {
+                         const long long* leaf_off, const V2<R>* L, const V2<R>* rho, int P, int Ps, CoefT<R>* coef, int* cexp,
+                         cudaStream_t s, int chunks) {
     if (ncones <= 0) return;
     // chunks per coefficient (the tuning variant): 1, 2, 5 or 10; a block holds 256 / (P * CH) cones
     auto go = [&](auto ch_tag) {
         constexpr int CH = decltype(ch_tag)::value;
         const int cpb = 256 / (P * CH);
         k_leaf_apply_t<R, CH><<<nblk_a(ncones, cpb), cpb * P * CH, 0, s>>>(cone_box, ncones, cone_base, leaf_start, leaf_count,
-                                                                          leaf_off, L, rho, P, coef);
+                                                                          leaf_off, L, rho, P, Ps, coef, cexp);
     };
     if (chunks == 10 && 256 / (P * 10) >= 1) go(std::integral_constant<int, 10>{});
     else if (chunks == 2 && 256 / (P * 2) >= 1) go(std::integral_constant<int, 2>{});
@@ -605,41 +785,62 @@ bool launch_leaf_tma(const int* cone_box, int ncones, int cone_base, const int* 
                                                               rho, coef, err);
     return true;
 }
-template <typename R>
-void launch_propagate_t(int pbegin, int pend, const long long* pp_ptr, const int* pp_nchild, const PropE<R>* pp, int Ps, int Pang,
-                        const R* Gsep, V2<R>* coef, cudaStream_t s, int cones_per_block) {
+void launch_propagate_t(int pbegin, int pend, const long long* pp_ptr, const int* pp_nchild, const PropE<float>* pp, int Ps, int Pang,
+                        const float* Gsep, float2* coef, cudaStream_t s, int cones_per_block) {
     if (pend <= pbegin) return;
     // cones per block (the tuning variant): 2, 4 or the most that fit 256 threads; kPropStaged:
     // the most that fit, child blocks staged in shared memory
     IFGF_DISPATCH_P(Ps, Pang, {
         constexpr int CPBMAX = 256 / (PS * PA);
         if (cones_per_block == kPropStaged)
-            k_propagate_st<R, PS, PA, CPBMAX><<<nblk_a(pend - pbegin, CPBMAX), CPBMAX * PS * PA, 0, s>>>(pbegin, pend, pp_ptr,
+            k_propagate_st<PS, PA, CPBMAX><<<nblk_a(pend - pbegin, CPBMAX), CPBMAX * PS * PA, 0, s>>>(pbegin, pend, pp_ptr,
                                                                                                       pp_nchild, pp, Gsep, coef);
         else if (cones_per_block == 2 && CPBMAX >= 2)
-            k_propagate_t<R, PS, PA, 2><<<nblk_a(pend - pbegin, 2), 2 * PS * PA, 0, s>>>(pbegin, pend, pp_ptr, pp_nchild, pp, Gsep, coef);
+            k_propagate_t<PS, PA, 2><<<nblk_a(pend - pbegin, 2), 2 * PS * PA, 0, s>>>(pbegin, pend, pp_ptr, pp_nchild, pp, Gsep, coef);
         else if (cones_per_block == 4 && CPBMAX >= 4)
-            k_propagate_t<R, PS, PA, 4><<<nblk_a(pend - pbegin, 4), 4 * PS * PA, 0, s>>>(pbegin, pend, pp_ptr, pp_nchild, pp, Gsep, coef);
+            k_propagate_t<PS, PA, 4><<<nblk_a(pend - pbegin, 4), 4 * PS * PA, 0, s>>>(pbegin, pend, pp_ptr, pp_nchild, pp, Gsep, coef);
         else
-            k_propagate_t<R, PS, PA, CPBMAX><<<nblk_a(pend - pbegin, CPBMAX), CPBMAX * PS * PA, 0, s>>>(pbegin, pend, pp_ptr,
+            k_propagate_t<PS, PA, CPBMAX><<<nblk_a(pend - pbegin, CPBMAX), CPBMAX * PS * PA, 0, s>>>(pbegin, pend, pp_ptr,
                                                                                                      pp_nchild, pp, Gsep, coef);
     });
+}
+size_t stage_plan_size(int ncones, int Ps, int Pang) {
+    size_t n = 0;
+    IFGF_DISPATCH_P(Ps, Pang, n = (size_t)((ncones + PropFx<PS * PA>::cones - 1) / PropFx<PS * PA>::cones) * PropFx<PS * PA>::record;);
+    return n;
+}
+void launch_stage_plan(int pbegin, int pend, const long long* pp_ptr, PlanX pp, int Ps, int Pang, int* stage, cudaStream_t s) {
+    if (pend <= pbegin) return;
+    IFGF_DISPATCH_P(Ps, Pang, (k_stage_plan<PS * PA><<<nblk_a(pend - pbegin, PropFx<PS * PA>::cones), kPropFxThreads, 0, s>>>(
+                                   pbegin, pend, pp_ptr, pp, stage)));
+}
+void launch_propagate_fx(int pbegin, int pend, PlanX pp, const int* stage, int Ps, int Pang, const int2* GsepX, int4* coef, int* cexp,
+                         cudaStream_t s) {
+    if (pend <= pbegin) return;
+    IFGF_DISPATCH_P(Ps, Pang, (k_propagate_fx<PS, PA><<<nblk_a(pend - pbegin, PropFx<PS * PA>::cones), kPropFxThreads, 0, s>>>(
+                                   pbegin, pend, pp, stage, GsepX, coef, cexp)));
+}
+void launch_fx_weights(const double* in, int n, int2* out, cudaStream_t s) {
+    if (n > 0) k_fx_weights<<<nblk_a(n, 128), 128, 0, s>>>(in, n, out);
+}
+void launch_interp_fx(const InterpE<double>* in, long long n, InterpX* out, cudaStream_t s) {
+    if (n > 0) k_interp_fx<<<nblk_a(n, 256), 256, 0, s>>>(in, n, out);
 }
 template <typename R>
 void launch_final_t(int N, const int* point_leaf, const int* leaf_start, const int* near_src_off, const int* near_src,
                     const int* near_rowlen, const long long* near_off, const V2<R>* near, const V2<R>* rho,
-                    const int* ip_ptr, const InterpE<R>* ip, const V2<R>* coef, int Ps, int Pang, const long long* sorting,
-                    double2* y, cudaStream_t s, const V2<R>* part) {
+                    const int* ip_ptr, const InterpT<R>* ip, const CoefT<R>* coef, const int* cexp, int Ps, int Pang,
+                    const long long* sorting, double2* y, cudaStream_t s, const V2<R>* part) {
     IFGF_DISPATCH_P(Ps, Pang, (k_final_t<R, PS, PA><<<nblk_a((long long)N * 32, 256), 256, 0, s>>>(
                                    N, point_leaf, leaf_start, near_src_off, near_src, near_rowlen, near_off, near, rho,
-                                   ip_ptr, ip, coef, sorting, y, part)));
+                                   ip_ptr, ip, coef, cexp, sorting, y, part)));
 }
 template <typename R>
 void launch_interp_box(const int4* items, int nitems, int N, const int* leaf_start, const int* leaf_count, const int* ip_ptr,
-                       const InterpE<R>* ipT, const V2<R>* coef, int Ps, int Pang, V2<R>* part, cudaStream_t s) {
+                       const InterpT<R>* ipT, const CoefT<R>* coef, const int* cexp, int Ps, int Pang, V2<R>* part, cudaStream_t s) {
     if (nitems <= 0) return;
     IFGF_DISPATCH_P(Ps, Pang, (k_interp_box<R, PS, PA><<<nblk_a((long long)nitems * 32, 256), 256, 0, s>>>(
-                                   items, nitems, N, leaf_start, leaf_count, ip_ptr, ipT, coef, part)));
+                                   items, nitems, N, leaf_start, leaf_count, ip_ptr, ipT, coef, cexp, part)));
 }
 template <typename R>
 void launch_near_box(const int2* items, int nitems, const int* leaf_start, const int* leaf_count, const int* near_src_off,
@@ -651,7 +852,7 @@ void launch_near_box(const int2* items, int nitems, const int* leaf_start, const
 }
 template <typename R>
 void launch_interp_transpose(int N, const int* point_leaf, const int* leaf_start, const int* leaf_count, const int* ip_ptr,
-                             const InterpE<double>* in, InterpE<R>* out, cudaStream_t s) {
+                             const InterpE<double>* in, InterpT<R>* out, cudaStream_t s) {
     if (N > 0) k_interp_transpose<R><<<nblk_a(N, 256), 256, 0, s>>>(N, point_leaf, leaf_start, leaf_count, ip_ptr, in, out);
 }
 void launch_d2f(const double2* a, long long n, float2* b, cudaStream_t s) {
@@ -661,18 +862,17 @@ void launch_d2f(const double2* a, long long n, float2* b, cudaStream_t s) {
 #define IFGF_INSTANTIATE(R)                                                                                          \
     template void launch_intensities_t<R>(const double2*, const double*, const long long*, int, V2<R>*, cudaStream_t); \
     template void launch_leaf_apply_t<R>(const int*, int, int, const int*, const int*, const long long*, const V2<R>*,  \
-                                         const V2<R>*, int, V2<R>*, cudaStream_t, int);                               \
-    template void launch_propagate_t<R>(int, int, const long long*, const int*, const PropE<R>*, int, int, const R*,   \
-                                        V2<R>*, cudaStream_t, int);                                                    \
+                                         const V2<R>*, int, int, CoefT<R>*, int*, cudaStream_t, int);                       \
     template void launch_final_t<R>(int, const int*, const int*, const int*, const int*, const int*,                   \
-                                    const long long*, const V2<R>*, const V2<R>*, const int*, const InterpE<R>*,       \
-                                    const V2<R>*, int, int, const long long*, double2*, cudaStream_t, const V2<R>*);      \
-    template void launch_interp_box<R>(const int4*, int, int, const int*, const int*, const int*, const InterpE<R>*,     \
-                                       const V2<R>*, int, int, V2<R>*, cudaStream_t);                                    \
-    template void launch_interp_transpose<R>(int, const int*, const int*, const int*, const int*,                        \
-                                             const InterpE<double>*, InterpE<R>*, cudaStream_t);                          \
-    template void launch_near_box<R>(const int2*, int, const int*, const int*, const int*, const int*, const int*,       \
-                                     const long long*, const V2<R>*, const V2<R>*, const int*, const V2<R>*, int,        \
+                                    const long long*, const V2<R>*, const V2<R>*, const int*, const InterpT<R>*,       \
+                                    const CoefT<R>*, const int*, int, int, const long long*, double2*, cudaStream_t,   \
+                                    const V2<R>*);                                                                     \
+    template void launch_interp_box<R>(const int4*, int, int, const int*, const int*, const int*, const InterpT<R>*,   \
+                                       const CoefT<R>*, const int*, int, int, V2<R>*, cudaStream_t);                   \
+    template void launch_interp_transpose<R>(int, const int*, const int*, const int*, const int*,                      \
+                                             const InterpE<double>*, InterpT<R>*, cudaStream_t);                       \
+    template void launch_near_box<R>(const int2*, int, const int*, const int*, const int*, const int*, const int*,     \
+                                     const long long*, const V2<R>*, const V2<R>*, const int*, const V2<R>*, int,      \
                                      const long long*, double2*, cudaStream_t);
 IFGF_INSTANTIATE(double)
 IFGF_INSTANTIATE(float)

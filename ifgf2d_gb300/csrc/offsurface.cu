@@ -9,7 +9,7 @@
 // which covers every source once.  Targets may lie anywhere, also outside the root box.
 #include "context.hpp"
 #include "hankel.cuh"
-#include "ifgf_device.cuh"
+#include "fixpoint.cuh"
 
 struct EvalWork {
     Tree E;
@@ -21,10 +21,13 @@ struct EvalWork {
     DBuf<double2> leafL;
     DBuf<long long> pp_ptr;
     DBuf<int> pp_nchild;
-    DBuf<PropEntryD> pp;
+    PlanBuf pp;
+    PlanStage stage;
     DBuf<int> ip_ptr, nb_ptr, nb_box;
-    DBuf<InterpEntryD> ip;
-    DBuf<double2> coef, out;
+    DBuf<InterpX> ip;
+    DBuf<int4> coef;
+    DBuf<int> cexp;
+    DBuf<double2> out;
 };
 
 void ifgf::free_eval(ifgf2d_ctx* ctx) {
@@ -43,8 +46,9 @@ __global__ void __launch_bounds__(256) k_eval_targets(long long M, const double*
                                                       const double* __restrict__ xs, const double* __restrict__ ys,
                                                       const double* __restrict__ nxs, const double* __restrict__ nys,
                                                       const double2* __restrict__ rho, double k, int form, double eta,
-                                                      const int* __restrict__ ip_ptr, const InterpEntryD* __restrict__ ip,
-                                                      const double2* __restrict__ coef, double2* __restrict__ out) {
+                                                      const int* __restrict__ ip_ptr, const InterpX* __restrict__ ip,
+                                                      const int4* __restrict__ coef, const int* __restrict__ cexp,
+                                                      double2* __restrict__ out) {
     constexpr int P = PS * PA;
     const long long t = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
@@ -61,8 +65,9 @@ __global__ void __launch_bounds__(256) k_eval_targets(long long M, const double*
         }
     }
     for (int e = ip_ptr[t] + lane; e < ip_ptr[t + 1]; e += 32) {
-        const InterpEntryD E = ip[e];
-        const double2 it = interp_eval<double, PS, PA>(coef + (long long)E.cone * P, E.s, E.th);
+        const InterpX E = ip[e];
+        const int4* c = coef + (long long)E.cone * P;
+        const double2 it = fx_interp_value<PS, PA>([&](int i) { return c[i]; }, cexp[E.cone], make_longlong2(E.s, E.th));
         cmac<double>(acc, it, make_double2(E.fr, E.fi));
     }
     acc.x = warp_sum_r<double>(acc.x);
@@ -73,12 +78,12 @@ __global__ void __launch_bounds__(256) k_eval_targets(long long M, const double*
 void launch_eval_targets(long long M, const double* tx, const double* ty, const int* nb_ptr, const int* nb_box,
                          const int* leaf_start, const int* leaf_count, const double* xs, const double* ys, const double* nxs,
                          const double* nys, const double2* rho, double k, int form, double eta, const int* ip_ptr,
-                         const InterpEntryD* ip, const double2* coef, int Ps, int Pang, double2* out, cudaStream_t s) {
+                         const InterpX* ip, const int4* coef, const int* cexp, int Ps, int Pang, double2* out, cudaStream_t s) {
     if (M <= 0) return;
     const unsigned grid = (unsigned)((M * 32 + 255) / 256);
     IFGF_DISPATCH_P(Ps, Pang, (k_eval_targets<PS, PA><<<grid, 256, 0, s>>>(M, tx, ty, nb_ptr, nb_box, leaf_start, leaf_count, xs,
                                                                           ys, nxs, nys, rho, k, form, eta, ip_ptr, ip, coef,
-                                                                          out)));
+                                                                          cexp, out)));
 }
 
 }  // namespace
@@ -122,16 +127,24 @@ extern "C" int ifgf2d_eval_offsurface_setup(ifgf2d_ctx* ctx, long long m, const 
         DBuf<int> perr;
         CK(perr.alloc(1));
         CK(cudaMemsetAsync(perr.p, 0, sizeof(int), s));
-        CK(build_prop_plan(E, W.pp.p, nullptr, perr.p, s));
+        CK(build_prop_plan(E, W.pp.view(), nullptr, perr.p, s));
         int bad = 0;
         CK(cudaMemcpyAsync(&bad, perr.p, sizeof(int), cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
+        CK(W.stage.build(E, W.pp_ptr.p, W.pp.view(), s));
         if (bad) { free_eval(ctx); return fail(ctx, IFGF2D_ERR_GEOMETRY, "internal: a propagation node's child cone is missing"); }
     }
-    CK(W.ip.upload(reinterpret_cast<const InterpEntryD*>(E.ip.data()), E.ip.size()));
+    {
+        DBuf<InterpEntryD> ip;
+        CK(ip.upload(reinterpret_cast<const InterpEntryD*>(E.ip.data()), E.ip.size()));
+        CK(W.ip.alloc(E.ip.size()));
+        launch_interp_fx(ip.p, (long long)E.ip.size(), W.ip.p, s);
+        CK(cudaGetLastError());
+    }
     CK(W.ip_ptr.upload(E.ip_ptr));
     CK(W.nb_ptr.upload(E.nbr_ptr)); CK(W.nb_box.upload(E.nbr_box));
     CK(W.coef.alloc((size_t)std::max(1, E.total_cones) * P));
+    CK(W.cexp.alloc((size_t)std::max(1, E.total_cones)));
     CK(W.out.alloc(m));
     CK(cudaStreamSynchronize(s));
     return IFGF2D_OK;
@@ -152,15 +165,15 @@ extern "C" int ifgf2d_eval_offsurface(ifgf2d_ctx* ctx, const double* density, do
     launch_intensities(ctx->vin.p, ctx->wq.p, ctx->sorting.p, N, ctx->rho.p, s);
     const TreeLevel& LD = E.L[D];
     launch_leaf_apply_t<double>(W.leaf_cone_box.p, (int)LD.cone_nonrel.size(), LD.cone_base, ctx->leaf_start.p, ctx->leaf_count.p,
-                                W.leaf_off.p, W.leafL.p, ctx->rho.p, P, W.coef.p, s);
+                                W.leaf_off.p, W.leafL.p, ctx->rho.p, P, E.Ps, W.coef.p, W.cexp.p, s);
     for (int l = D; l >= 3; --l) {
         const TreeLevel& Lp = E.L[l - 1];
-        launch_propagate_t<double>(Lp.cone_base, Lp.cone_base + (int)Lp.cone_nonrel.size(), W.pp_ptr.p, W.pp_nchild.p, W.pp.p,
-                                   E.Ps, E.Pang, ctx->Gsep.p, W.coef.p, s);
+        launch_propagate_fx(Lp.cone_base, Lp.cone_base + (int)Lp.cone_nonrel.size(), W.pp.view(), W.stage.level(l), E.Ps, E.Pang,
+                            ctx->GsepX.p, W.coef.p, W.cexp.p, s);
     }
     launch_eval_targets(W.M, W.tx.p, W.ty.p, W.nb_ptr.p, W.nb_box.p, ctx->leaf_start.p, ctx->leaf_count.p, ctx->xs_s.p,
                         ctx->ys_s.p, ctx->nxs_s.p, ctx->nys_s.p, ctx->rho.p, ctx->k, ctx->form, ctx->eta, W.ip_ptr.p, W.ip.p,
-                        W.coef.p, E.Ps, E.Pang, W.out.p, s);
+                        W.coef.p, W.cexp.p, E.Ps, E.Pang, W.out.p, s);
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(out, W.out.p, sizeof(double2) * W.M, cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));

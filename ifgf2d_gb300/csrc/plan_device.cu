@@ -13,6 +13,7 @@
 // is compiled without FMA contraction so the arithmetic rounds as the host's does, and only
 // the device's cos / sin / atan may differ from the host's by an ulp.
 #include "context.hpp"
+#include "fixpoint.cuh"
 #include <memory>
 
 namespace ifgf {
@@ -73,7 +74,7 @@ __device__ __forceinline__ double radius_to_cheb(const LevelDesc& L, long long p
 __global__ void k_prop_plan(LevelDesc Lp, LevelDesc Lc, double min_x, double min_y, double k, int Ps, ChebNodes cn, int P,
                             const int* __restrict__ slot_parent, const int* __restrict__ slot_child_box,
                             const int* __restrict__ slot_pos, const int* __restrict__ slot_route,
-                            const int* __restrict__ route_nonrel, long long nslots, PropE<double>* __restrict__ out64,
+                            const int* __restrict__ route_nonrel, long long nslots, PlanX out64,
                             PropE<float>* __restrict__ out32, int* __restrict__ err) {
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= nslots * P) return;
@@ -112,7 +113,7 @@ __global__ void k_prop_plan(LevelDesc Lp, LevelDesc Lc, double min_x, double min
     const long long e = idx;
     if (lo >= Lc.cone_ptr[cb + 1] || Lc.cone_nonrel[lo] != nonrel) {
         atomicExch(err, 1);
-        out64[e] = PropE<double>{0, it, 0.0, 0.0, 0.0, 0.0};
+        out64.child[e] = 0; out64.st[e] = make_longlong2(0, 0); out64.w[e] = make_double2(0.0, 0.0);
         if (out32) out32[e] = PropE<float>{0, 0.f, 0.f, 0.f, 0.f};
         return;
     }
@@ -125,7 +126,9 @@ __global__ void k_prop_plan(LevelDesc Lp, LevelDesc Lc, double min_x, double min
     const double den = gr * gr + gi * gi;
     const double wr = (fr * gr + fi * gi) / den, wi = (fi * gr - fr * gi) / den;
     const int child = Lc.cone_base + lo;
-    out64[e] = PropE<double>{child, it, ls, lt, wr, wi};
+    out64.child[e] = child;
+    out64.st[e] = make_longlong2(fx_weight(ls), fx_weight(lt));
+    out64.w[e] = make_double2(wr, wi);
     if (out32) out32[e] = PropE<float>{child, (float)ls, (float)lt, (float)wr, (float)wi};
 }
 
@@ -156,7 +159,7 @@ __global__ void k_leaf_nodes(LevelDesc L, double min_x, double min_y, double k, 
 constexpr int kSortWarps = 8;
 template <typename R>
 __global__ void __launch_bounds__(kSortWarps * 32) k_sort_plan(const long long* __restrict__ pp_ptr, int ncones,
-                                                               const PropE<double>* __restrict__ pp, int P,
+                                                               PlanX px, const PropE<float>* __restrict__ pp32, int P,
                                                                PropB<R>* __restrict__ out) {
     __shared__ int cc[kSortWarps][4 * kMaxP];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -164,7 +167,7 @@ __global__ void __launch_bounds__(kSortWarps * 32) k_sort_plan(const long long* 
     if (pc >= ncones) return;
     const long long e0 = pp_ptr[pc];
     const int ne = (int)(pp_ptr[pc + 1] - e0);
-    for (int i = lane; i < ne; i += 32) cc[warp][i] = pp[e0 + i].child_cone;
+    for (int i = lane; i < ne; i += 32) cc[warp][i] = px.child[e0 + i];
     __syncwarp();
     for (int i = lane; i < ne; i += 32) {
         const int c = cc[warp][i];
@@ -173,8 +176,14 @@ __global__ void __launch_bounds__(kSortWarps * 32) k_sort_plan(const long long* 
             const int d = cc[warp][j];
             rank += (d < c) || (d == c && j < i);
         }
-        const PropE<double> E = pp[e0 + i];
-        out[e0 + rank] = PropB<R>{E.child_cone, i % P, (R)E.s, (R)E.th, (R)E.wr, (R)E.wi};
+        if constexpr (sizeof(R) == 4) {
+            const PropE<float> E = pp32[e0 + i];
+            out[e0 + rank] = PropB<R>{E.child_cone, i % P, E.s, E.th, E.wr, E.wi};
+        } else {
+            const longlong2 t = px.st[e0 + i];
+            const double2 w = px.w[e0 + i];
+            out[e0 + rank] = PropB<R>{c, i % P, fx_weight_value(t.x), fx_weight_value(t.y), w.x, w.y};
+        }
     }
 }
 
@@ -205,7 +214,7 @@ cudaError_t upload_level(const TreeLevel& L, int cone_base, LevelBufs& B, LevelD
 
 }  // namespace
 
-cudaError_t build_prop_plan(const Tree& T, PropE<double>* pp64, PropE<float>* pp32, int* err, cudaStream_t s,
+cudaError_t build_prop_plan(const Tree& T, PlanX pp64, PropE<float>* pp32, int* err, cudaStream_t s,
                             const int* level_cone_base, const long long* level_entry_base) {
     if (T.Ps > 8 || T.Pang > 8) return cudaErrorInvalidValue;
     ChebNodes cn{};
@@ -244,7 +253,7 @@ cudaError_t build_prop_plan(const Tree& T, PropE<double>* pp64, PropE<float>* pp
         const long long eb = level_entry_base ? level_entry_base[S.level] : S.entry_base;
         k_prop_plan<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(ld[S.level - 1], ld[S.level], T.min_x, T.min_y, T.k, T.Ps, cn, T.P,
                                                                  sp[q].p, scb[q].p, spos[q].p, sr[q].p, rn[q].p, nslots,
-                                                                 pp64 + eb, pp32 ? pp32 + eb : nullptr, err);
+                                                                 plan_at(pp64, eb), pp32 ? pp32 + eb : nullptr, err);
         e = cudaGetLastError();
     }
     // stream-ordered buffers are freed in stream order after the kernels; plain ones need the
@@ -258,7 +267,7 @@ struct PropPlanByLevel::Impl {
     struct Level {
         long long entry_base = 0, n = 0;
         DBuf<int> sp, scb, spos, sr, rn;
-        DBuf<PropE<double>> o64;
+        PlanBuf o64;
         DBuf<PropE<float>> o32;
     };
     cudaStream_t st = nullptr;
@@ -324,7 +333,7 @@ void PropPlanByLevel::add(const Tree& T, int l) {
         if (e == cudaSuccess) {
             k_prop_plan<<<(unsigned)((v.n + 255) / 256), 256, 0, I.st>>>(I.ld[l - 1], I.ld[l], T.min_x, T.min_y, T.k, T.Ps, I.cn, T.P,
                                                                          v.sp.p, v.scb.p, v.spos.p, v.sr.p, v.rn.p,
-                                                                         (long long)S.slot_parent.size(), v.o64.p, v.o32.p, I.err.p);
+                                                                         (long long)S.slot_parent.size(), v.o64.view(), v.o32.p, I.err.p);
             e = cudaGetLastError();
         }
     }
@@ -332,7 +341,7 @@ void PropPlanByLevel::add(const Tree& T, int l) {
     I.lv.push_back(std::move(vp));
 }
 
-cudaError_t PropPlanByLevel::gather(PropE<double>* pp64, PropE<float>* pp32, int* err, cudaStream_t s) {
+cudaError_t PropPlanByLevel::gather(PlanX pp64, PropE<float>* pp32, int* err, cudaStream_t s) {
     Impl& I = *d;
     if (I.status != cudaSuccess) return I.status;
     AllocStream guard(I.st);
@@ -341,7 +350,10 @@ cudaError_t PropPlanByLevel::gather(PropE<double>* pp64, PropE<float>* pp32, int
     for (const auto& vp : I.lv) {
         const Impl::Level& v = *vp;
         if (v.n == 0 || e != cudaSuccess) continue;
-        e = cudaMemcpyAsync(pp64 + v.entry_base, v.o64.p, sizeof(PropE<double>) * (size_t)v.n, cudaMemcpyDeviceToDevice, I.st);
+        const PlanX to = plan_at(pp64, v.entry_base), from = v.o64.view();
+        e = cudaMemcpyAsync(to.child, from.child, sizeof(int) * (size_t)v.n, cudaMemcpyDeviceToDevice, I.st);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(to.st, from.st, sizeof(longlong2) * (size_t)v.n, cudaMemcpyDeviceToDevice, I.st);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(to.w, from.w, sizeof(double2) * (size_t)v.n, cudaMemcpyDeviceToDevice, I.st);
         if (e == cudaSuccess && pp32)
             e = cudaMemcpyAsync(pp32 + v.entry_base, v.o32.p, sizeof(PropE<float>) * (size_t)v.n, cudaMemcpyDeviceToDevice, I.st);
     }
@@ -373,12 +385,12 @@ cudaError_t build_leaf_nodes(const Tree& T, LeafNode* out, cudaStream_t s) {
 }
 
 template <typename R>
-void launch_sort_plan(const long long* pp_ptr, int ncones, const PropE<double>* pp, int P, PropB<R>* out, cudaStream_t s) {
+void launch_sort_plan(const long long* pp_ptr, int ncones, PlanX px, const PropE<float>* pp32, int P, PropB<R>* out, cudaStream_t s) {
     if (ncones <= 0) return;
-    k_sort_plan<R><<<(ncones + kSortWarps - 1) / kSortWarps, kSortWarps * 32, 0, s>>>(pp_ptr, ncones, pp, P, out);
+    k_sort_plan<R><<<(ncones + kSortWarps - 1) / kSortWarps, kSortWarps * 32, 0, s>>>(pp_ptr, ncones, px, pp32, P, out);
 }
-template void launch_sort_plan<double>(const long long*, int, const PropE<double>*, int, PropB<double>*, cudaStream_t);
-template void launch_sort_plan<float>(const long long*, int, const PropE<double>*, int, PropB<float>*, cudaStream_t);
+template void launch_sort_plan<double>(const long long*, int, PlanX, const PropE<float>*, int, PropB<double>*, cudaStream_t);
+template void launch_sort_plan<float>(const long long*, int, PlanX, const PropE<float>*, int, PropB<float>*, cudaStream_t);
 
 void launch_interp_to_c64(const InterpE<double>* in, long long n, InterpE<float>* out, cudaStream_t s) {
     if (n <= 0) return;
