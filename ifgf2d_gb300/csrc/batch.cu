@@ -14,13 +14,27 @@
 #include <complex>
 #include <vector>
 
+struct TermsXBuf {
+    DBuf<int2> id;
+    DBuf<double2> w;
+    DBuf<int4> rows;
+    cudaError_t alloc(size_t n, int Ps, int Pang) {
+        cudaError_t e = id.alloc(n);
+        if (e == cudaSuccess) e = w.alloc(n);
+        if (e == cudaSuccess) e = rows.alloc(n * batch_x_rows(Ps, Pang));
+        return e;
+    }
+    TermsX view() const { return TermsX{id.p, w.p, rows.p}; }
+};
+
 struct BatchWork {
     int cap = 0;                               // right-hand sides the apply buffers hold
     DBuf<double2> xt, yt;                      // interleaved [N][cap]
-    DBuf<double2> rho64, coef64;
+    DBuf<double2> rho64;
+    DBuf<int4> coef64;                         // fixed-point limbs (fixpoint.cuh), with
+    DBuf<int> cexp64;                          // one exponent per cone and right-hand side
     DBuf<float2> rho32, coef32;
-    DBuf<PropB<double>> pb64;
-    DBuf<double> rows64;                       // the FP64 plan terms' Chebyshev rows (FP64-pipe work the lanes share)
+    TermsXBuf px64, ig64;                      // the FP64 propagation's and interpolation's terms
     DBuf<PropB<float>> pb32;
     DBuf<float2> W32;                          // complex64 copy of the singular-correction weights
     DBuf<float2> xt32;                         // complex64 copy of the interleaved input (mixed form)
@@ -29,8 +43,8 @@ struct BatchWork {
     DBuf<int> t5err;
     int nsm = 0;
     DBuf<int4> leaf_items;                     // (leaf box, first cone, end cone, 0) of the tensor-core leaf kernel
-    // the complex64 interpolation grouped by cone: work items (terms, targets) and their terms
-    DBuf<int4> ig_items;
+    // the interpolation grouped by cone: work items (terms, targets) and their complex64 terms
+    DBuf<int4> ig_items, ig64_items;
     DBuf<InterpG> ig_terms;
     // GMRES
     int m = 0, scap = 0;
@@ -59,8 +73,10 @@ void ifgf::free_batch(ifgf2d_ctx* ctx) {
 namespace {
 
 // The interpolation terms of each leaf box's targets, kInterpGrpTargets targets per work item,
-// sorted by cone (stable) within an item: items (first term, end term, first target, targets).
-void grouped_interp_plan(const Tree& T, std::vector<int4>& items, std::vector<InterpG>& terms) {
+// sorted by cone (stable) within an item: items (first term, end term, first target, targets), and the
+// terms, make(plan entry, target, the item's first target).
+template <typename Term, typename Make>
+void grouped_interp_plan(const Tree& T, std::vector<int4>& items, std::vector<Term>& terms, Make&& make) {
     const int nleaf = (int)T.leaf_start.size();
     std::vector<long long> item_ptr(nleaf + 1, 0), term_ptr(nleaf + 1, 0);
     for (int b = 0; b < nleaf; ++b) {
@@ -85,8 +101,7 @@ void grouped_interp_plan(const Tree& T, std::vector<int4>& items, std::vector<In
                 for (int i : idx) {
                     int t = t0 + c0;
                     while (T.ip_ptr[t + 1] <= i) ++t;   // the target owning term i
-                    const InterpEntry& q = T.ip[i];
-                    terms[e++] = InterpG{q.cone, t, (float)q.s, (float)q.th, (float)q.fr, (float)q.fi};
+                    terms[e++] = make(i, t, t0 + c0);
                 }
                 items[it] = make_int4((int)first, (int)e, t0 + c0, nt);
             }
@@ -101,7 +116,7 @@ int ensure_apply(ifgf2d_ctx* ctx, int B, bool mixed) {
     const size_t ncoef = (size_t)ctx->T.total_cones * ctx->T.P;
     if (W.cap < B) {
         W.xt.release(); W.yt.release(); W.rho64.release(); W.coef64.release(); W.rho32.release(); W.coef32.release();
-        W.xt32.release();
+        W.xt32.release(); W.cexp64.release();
         CK(W.xt.alloc((size_t)N * B)); CK(W.yt.alloc((size_t)N * B));
         W.cap = B;
     }
@@ -111,7 +126,7 @@ int ensure_apply(ifgf2d_ctx* ctx, int B, bool mixed) {
         }
         if (!W.pb32.p) {
             CK(W.pb32.alloc(ctx->pp.child.n));
-            launch_sort_plan<float>(ctx->pp_ptr.p, ctx->T.total_cones, ctx->pp.view(), ctx->pp32.p, ctx->T.P, W.pb32.p, ctx->stream);
+            launch_sort_plan(ctx->pp_ptr.p, ctx->T.total_cones, ctx->pp32.p, ctx->T.P, W.pb32.p, ctx->stream);
             CK(cudaGetLastError());
         }
         if (!W.t5err.p) {
@@ -129,7 +144,10 @@ int ensure_apply(ifgf2d_ctx* ctx, int B, bool mixed) {
             CK(W.leaf_items.upload(items));
             std::vector<int4> gi;
             std::vector<InterpG> gt;
-            grouped_interp_plan(ctx->T, gi, gt);
+            grouped_interp_plan(ctx->T, gi, gt, [&](int i, int t, int) {
+                const InterpEntry& q = ctx->T.ip[i];
+                return InterpG{q.cone, t, (float)q.s, (float)q.th, (float)q.fr, (float)q.fi};
+            });
             CK(W.ig_items.upload(gi));
             CK(W.ig_terms.upload(gt));
         }
@@ -139,63 +157,79 @@ int ensure_apply(ifgf2d_ctx* ctx, int B, bool mixed) {
         }
     } else {
         if (!W.rho64.p) { CK(W.rho64.alloc((size_t)N * W.cap)); CK(W.coef64.alloc(ncoef * W.cap)); }
-        if (!W.pb64.p) {
-            CK(W.pb64.alloc(ctx->pp.child.n));
-            launch_sort_plan<double>(ctx->pp_ptr.p, ctx->T.total_cones, ctx->pp.view(), ctx->pp32.p, ctx->T.P, W.pb64.p, ctx->stream);
+        if (!W.cexp64.p) CK(W.cexp64.alloc((size_t)ctx->T.total_cones * W.cap));
+        if (!W.px64.id.p) {
+            const Tree& T = ctx->T;
+            std::vector<int4> gi;
+            std::vector<int2> gt;
+            grouped_interp_plan(T, gi, gt, [](int i, int t, int first) { return make_int2(i, t - first); });   // entry, target of the item
+            DBuf<int2> src;
+            CK(W.ig64_items.upload(gi));
+            CK(src.upload(gt));
+            CK(W.ig64.alloc(gt.size(), T.Ps, T.Pang));
+            CK(W.px64.alloc(ctx->pp.child.n, T.Ps, T.Pang));
+            launch_group_terms_x(ctx->ipx.p, src.p, (long long)gt.size(), T.Ps, T.Pang, W.ig64.view(), ctx->stream);
+            launch_sort_plan_x(ctx->pp_ptr.p, T.total_cones, ctx->pp.view(), T.Ps, T.Pang, W.px64.view(), ctx->stream);
             CK(cudaGetLastError());
-            CK(W.rows64.alloc(ctx->pp.child.n * (size_t)(ctx->T.Ps + ctx->T.Pang)));
-            launch_plan_rows<double>(W.pb64.p, (long long)ctx->pp.child.n, ctx->T.Ps, ctx->T.Pang, W.rows64.p, ctx->stream);
-            CK(cudaGetLastError());
+            if (!src.owner) CK(cudaStreamSynchronize(ctx->stream));   // src is freed at once
         }
     }
     return IFGF2D_OK;
 }
 
-template <typename R>
-void far_b(ifgf2d_ctx* ctx, const V2<R>* rho, const V2<R>* near, const V2<R>* leafL, const PropB<R>* pb,
-           const InterpE<R>* ip, const R* Gsep, V2<R>* coef, int B, double2* yt) {
+// yt += the far field: complex64
+void far_b(ifgf2d_ctx* ctx, int B, double2* yt) {
     const Tree& T = ctx->T;
     const int Dl = ctx->nlevels - 1;
     const TreeLevel& LD = T.L[Dl];
     cudaStream_t s = ctx->stream;
+    BatchWork& W = *ctx->bw;
+    const float2 *rho = W.rho32.p, *leafL = ctx->leafL32.p;
+    float2* coef = W.coef32.p;
+    const PropB<float>* pb = W.pb32.p;
     bool leaf_done = false;
-    if constexpr (sizeof(R) == 4) {
-        BatchWork& W = *ctx->bw;
-        if (ctx->tune_batch_tc & (kBatchTcLeaf | kBatchTcLeaf6))
-            leaf_done = launch_leaf_t5(W.leaf_items.p, (int)W.leaf_items.n, ctx->leaf_start.p, ctx->leaf_count.p, ctx->leaf_off.p,
-                                       leafL, rho, T.Ps, T.Pang, B, coef + (long long)LD.cone_base * T.P * B, W.t5err.p, W.nsm,
-                                       (ctx->tune_batch_tc & kBatchTcLeaf6) ? 3 : 2, s);
-    }
+    if (ctx->tune_batch_tc & (kBatchTcLeaf | kBatchTcLeaf6))
+        leaf_done = launch_leaf_t5(W.leaf_items.p, (int)W.leaf_items.n, ctx->leaf_start.p, ctx->leaf_count.p, ctx->leaf_off.p,
+                                   leafL, rho, T.Ps, T.Pang, B, coef + (long long)LD.cone_base * T.P * B, W.t5err.p, W.nsm,
+                                   (ctx->tune_batch_tc & kBatchTcLeaf6) ? 3 : 2, s);
     if (!leaf_done)
-        launch_leaf_b<R>(ctx->leaf_cone_box.p, (int)LD.cone_nonrel.size(), LD.cone_base, ctx->leaf_start.p, ctx->leaf_count.p,
-                         ctx->leaf_off.p, leafL, rho, T.Ps, T.Pang, B, coef, s);
+        launch_leaf_b<float>(ctx->leaf_cone_box.p, (int)LD.cone_nonrel.size(), LD.cone_base, ctx->leaf_start.p, ctx->leaf_count.p,
+                             ctx->leaf_off.p, leafL, rho, T.Ps, T.Pang, B, coef, nullptr, s);
     for (int l = Dl; l >= 3; --l) {
         const TreeLevel& Lp = T.L[l - 1];
         const int p0 = Lp.cone_base, p1 = Lp.cone_base + (int)Lp.cone_nonrel.size();
-        if constexpr (sizeof(R) == 4) {
-            BatchWork& W = *ctx->bw;
-            if ((ctx->tune_batch_tc & kBatchTcProp) && launch_prop_t5(p0, p1, ctx->pp_ptr.p, ctx->pp_nchild.p, pb, T.Ps, T.Pang, Gsep, B, coef,
-                                                     W.t5err.p, W.nsm, s))
-                continue;
-            if ((ctx->tune_batch_tc & kBatchBulkProp) &&
-                launch_prop_bk(p0, p1, ctx->pp_ptr.p, ctx->pp_nchild.p, pb, T.Ps, T.Pang, Gsep, B, coef, W.t5err.p, s))
-                continue;
-        }
-        const R* rows = nullptr;
-        if constexpr (sizeof(R) == 8) rows = ctx->bw->rows64.p;
-        launch_prop_b<R>(p0, p1, ctx->pp_ptr.p, ctx->pp_nchild.p, pb, T.Ps, T.Pang, Gsep, B, coef, s, rows);
+        if ((ctx->tune_batch_tc & kBatchTcProp) && launch_prop_t5(p0, p1, ctx->pp_ptr.p, ctx->pp_nchild.p, pb, T.Ps, T.Pang,
+                                                                  ctx->Gsep32.p, B, coef, W.t5err.p, W.nsm, s))
+            continue;
+        if ((ctx->tune_batch_tc & kBatchBulkProp) &&
+            launch_prop_bk(p0, p1, ctx->pp_ptr.p, ctx->pp_nchild.p, pb, T.Ps, T.Pang, ctx->Gsep32.p, B, coef, W.t5err.p, s))
+            continue;
+        launch_prop_b(p0, p1, ctx->pp_ptr.p, ctx->pp_nchild.p, pb, T.Ps, T.Pang, ctx->Gsep32.p, B, coef, s);
     }
-    bool grouped = false;
-    if constexpr (sizeof(R) == 4) grouped = (ctx->tune_batch_tc & kBatchGroupedInterp) && B <= 64 && T.Ps == 5 && T.Pang == 5;
-    launch_final_b<R>((int)ctx->D.N, ctx->point_leaf.p, ctx->leaf_start.p, ctx->leaf_count.p, ctx->nbr_ptr.p, ctx->nbr_box.p,
-                      ctx->near_rowlen.p, ctx->near_off.p, near, rho, ctx->ip_ptr.p, grouped ? nullptr : ip, coef, T.Ps, T.Pang,
-                      ctx->sorting.p, B, yt, s);
-    if constexpr (sizeof(R) == 4) {
-        if (grouped) {
-            BatchWork& W = *ctx->bw;
-            launch_interp_grp(W.ig_items.p, (int)W.ig_items.n, W.ig_terms.p, coef, T.Ps, T.Pang, ctx->sorting.p, B, yt, s);
-        }
+    const bool grouped = (ctx->tune_batch_tc & kBatchGroupedInterp) && B <= 64 && T.Ps == 5 && T.Pang == 5;
+    launch_final_b<float>((int)ctx->D.N, ctx->point_leaf.p, ctx->leaf_start.p, ctx->leaf_count.p, ctx->nbr_ptr.p, ctx->nbr_box.p,
+                          ctx->near_rowlen.p, ctx->near_off.p, ctx->near32.p, rho, ctx->ip_ptr.p, grouped ? nullptr : ctx->ip32.p, coef,
+                          T.Ps, T.Pang, ctx->sorting.p, B, yt, s);
+    if (grouped) launch_interp_grp(W.ig_items.p, (int)W.ig_items.n, W.ig_terms.p, coef, T.Ps, T.Pang, ctx->sorting.p, B, yt, s);
+}
+// the same in FP64: the cone sums in fixed point (fixpoint.cuh)
+void far_bx(ifgf2d_ctx* ctx, int B, double2* yt) {
+    const Tree& T = ctx->T;
+    const int Dl = ctx->nlevels - 1;
+    const TreeLevel& LD = T.L[Dl];
+    cudaStream_t s = ctx->stream;
+    BatchWork& W = *ctx->bw;
+    launch_leaf_b<double>(ctx->leaf_cone_box.p, (int)LD.cone_nonrel.size(), LD.cone_base, ctx->leaf_start.p, ctx->leaf_count.p,
+                          ctx->leaf_off.p, ctx->leafL.p, W.rho64.p, T.Ps, T.Pang, B, W.coef64.p, W.cexp64.p, s);
+    for (int l = Dl; l >= 3; --l) {
+        const TreeLevel& Lp = T.L[l - 1];
+        launch_prop_bx(Lp.cone_base, Lp.cone_base + (int)Lp.cone_nonrel.size(), ctx->pp_ptr.p, W.px64.view(), T.Ps, T.Pang, ctx->GsepX.p,
+                       B, W.coef64.p, W.cexp64.p, s);
     }
+    launch_final_b<double>((int)ctx->D.N, ctx->point_leaf.p, ctx->leaf_start.p, ctx->leaf_count.p, ctx->nbr_ptr.p, ctx->nbr_box.p,
+                           ctx->near_rowlen.p, ctx->near_off.p, ctx->near.p, W.rho64.p, ctx->ip_ptr.p, nullptr, nullptr, T.Ps, T.Pang,
+                           ctx->sorting.p, B, yt, s);
+    launch_interp_bx(W.ig64_items.p, (int)W.ig64_items.n, W.ig64.view(), W.coef64.p, W.cexp64.p, T.Ps, T.Pang, ctx->sorting.p, B, yt, s);
 }
 
 // yt = A xt for B <= kMaxBatch interleaved right-hand sides (IFGF modes)
@@ -210,9 +244,9 @@ int apply_il(ifgf2d_ctx* ctx, const double2* xt, double2* yt, int B, int mode) {
     launch_sing_b(xt, W.xt32.p, ctx->W.p, W.W32.p, ctx->srow_ptr.p, ctx->srow_col.p, ctx->cols.p, (int)D.N, D.Np, B, half, yt, ctx->wq.p,
                   ctx->inverse.p, mixed ? nullptr : W.rho64.p, mixed ? W.rho32.p : nullptr, ctx->stream);
     if (mixed)
-        far_b<float>(ctx, W.rho32.p, ctx->near32.p, ctx->leafL32.p, W.pb32.p, ctx->ip32.p, ctx->Gsep32.p, W.coef32.p, B, yt);
+        far_b(ctx, B, yt);
     else
-        far_b<double>(ctx, W.rho64.p, ctx->near.p, ctx->leafL.p, W.pb64.p, ctx->ip.p, ctx->Gsep.p, W.coef64.p, B, yt);
+        far_bx(ctx, B, yt);
     CK(cudaGetLastError());
     return IFGF2D_OK;
 }

@@ -225,8 +225,7 @@ struct ifgf2d_ctx {
     PlanBuf pp;
     PlanStage pp_stage;
     DBuf<int> ip_ptr;
-    DBuf<InterpEntryD> ip;          // the batched FP64 form's
-    DBuf<InterpX> ipx;              // the single-vector FP64 form's
+    DBuf<InterpX> ipx;
     DBuf<int4> coef;                // FP64 form: fixed-point limbs, with
     DBuf<int> cexp;                 // one exponent per cone
     DBuf<int2> GsepX;               // Gsep as limbs
@@ -361,8 +360,7 @@ private:
 cudaError_t build_leaf_nodes(const Tree& T, LeafNode* out, cudaStream_t s);
 // a parent's propagation terms sorted by child cone (stable), with the parent node recorded, for
 // the batched propagation
-template <typename R>
-void launch_sort_plan(const long long* pp_ptr, int ncones, PlanX px, const PropE<float>* pp32, int P, PropB<R>* out, cudaStream_t s);
+void launch_sort_plan(const long long* pp_ptr, int ncones, const PropE<float>* pp, int P, PropB<float>* out, cudaStream_t s);
 // the complex64 copy of the interpolation plan
 void launch_interp_to_c64(const InterpE<double>* in, long long n, InterpE<float>* out, cudaStream_t s);
 void net_precondition_launch(ifgf2d_net* net, const double2* r, double2* z, cudaStream_t s);

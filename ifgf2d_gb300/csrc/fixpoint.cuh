@@ -1,7 +1,7 @@
 // fixpoint.cuh -- block fixed-point arithmetic for the FP64 form of the IFGF sums.
 //
 // GB300 retires about 2 FP64 operations per SM and clock (FMA, add, multiply and every conversion
-// from or to a double alike), but 61 wide integer multiply-adds (32 x 32 + 64 bits), both measured.
+// from or to a double alike), but 29 wide integer multiply-adds (32 x 32 + 64 bits), both measured.
 // The cone interpolants are sums of products of known range, so the FP64 form evaluates them in
 // integers:
 //   * a block of coefficients (one cone, one right-hand side) shares one binary exponent E: the
@@ -38,10 +38,12 @@ __device__ __forceinline__ FxLimb fx_split(long long x) {
 __device__ __forceinline__ FxLimb fx_cut(long long x) {
     return FxLimb{(int)(x >> kFxLow), (int)((unsigned)x & ((1u << kFxLow) - 1u))};
 }
+// a b + c: one wide multiply-add (as mad.wide it becomes a multiply and a 64-bit add, 10 % slower here)
 __device__ __forceinline__ long long fx_wide(int a, int b, long long c) {
-    long long r;
-    asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(r) : "r"(a), "r"(b), "l"(c));
-    return r;
+    unsigned lo = (unsigned)c;
+    int hi = (int)(c >> 32);
+    asm("mad.lo.cc.s32 %0, %2, %3, %0; madc.hi.s32 %1, %2, %3, %1;" : "+r"(lo), "+r"(hi) : "r"(a), "r"(b));
+    return ((long long)hi << 32) | lo;
 }
 // the low-order half of a product sum: m += a b without their high limbs' product
 __device__ __forceinline__ long long fx_low(FxLimb a, FxLimb b, long long m) { return fx_wide(a.l, b.h, fx_wide(a.h, b.l, m)); }
@@ -50,6 +52,9 @@ constexpr long long kFxHalf = 1ll << (kFxLow - 1);   // start of m: its shift by
 // a weight in [-1, 1]
 __device__ __forceinline__ long long fx_weight(double t) { return __double2ll_rn(t * (double)(1ll << kFxOne)); }
 __device__ __forceinline__ double fx_weight_value(long long t) { return (double)t * (1.0 / (double)(1ll << kFxOne)); }
+
+// int4 that hold the Chebyshev values T_1.. of s and theta of a batched term
+__host__ __device__ constexpr int fx_rows4(int Ps, int Pang) { return (Ps + Pang - 1) / 2; }
 
 // a block's exponent from the largest high word of its values' magnitudes: |value| < 2^E
 __device__ __forceinline__ int fx_expo(int maxhi) {

@@ -537,14 +537,15 @@ static int setup_interp(ifgf2d_ctx* ctx, int nlevels, DBuf<int>& perr) {
     const long long N = D.N;
     const int P = T.P;
     const int nleaf = (int)T.leaf_start.size();
+    DBuf<InterpEntryD> ip;
     {   // interpolation plan: the entries come from the host tree
         static_assert(sizeof(InterpEntry) == sizeof(InterpEntryD), "host and device plan layouts differ");
-        CK(ctx->ip.upload(reinterpret_cast<const InterpEntryD*>(T.ip.data()), T.ip.size()));
+        CK(ip.upload(reinterpret_cast<const InterpEntryD*>(T.ip.data()), T.ip.size()));
         CK(ctx->ip_ptr.upload(T.ip_ptr));
         CK(ctx->ip32.alloc(T.ip.size()));
         CK(ctx->ipx.alloc(T.ip.size()));
-        launch_interp_to_c64(ctx->ip.p, (long long)T.ip.size(), ctx->ip32.p, ctx->stream);
-        launch_interp_fx(ctx->ip.p, (long long)T.ip.size(), ctx->ipx.p, ctx->stream);
+        launch_interp_to_c64(ip.p, (long long)T.ip.size(), ctx->ip32.p, ctx->stream);
+        launch_interp_fx(ip.p, (long long)T.ip.size(), ctx->ipx.p, ctx->stream);
         CK(cudaGetLastError());
     }
     {   // interpolation by leaf box: per box, chunks of 32 targets x pieces of kIbPiece terms
@@ -564,9 +565,9 @@ static int setup_interp(ifgf2d_ctx* ctx, int nlevels, DBuf<int>& perr) {
         CK(ctx->ib_items.upload(items));
         CK(ctx->nb_items.upload(nitems));
         CK(ctx->ipT.alloc(T.ip.size())); CK(ctx->ip32T.alloc(T.ip.size()));
-        launch_interp_transpose<double>((int)N, ctx->point_leaf.p, ctx->leaf_start.p, ctx->leaf_count.p, ctx->ip_ptr.p, ctx->ip.p,
+        launch_interp_transpose<double>((int)N, ctx->point_leaf.p, ctx->leaf_start.p, ctx->leaf_count.p, ctx->ip_ptr.p, ip.p,
                                         ctx->ipT.p, ctx->stream);
-        launch_interp_transpose<float>((int)N, ctx->point_leaf.p, ctx->leaf_start.p, ctx->leaf_count.p, ctx->ip_ptr.p, ctx->ip.p,
+        launch_interp_transpose<float>((int)N, ctx->point_leaf.p, ctx->leaf_start.p, ctx->leaf_count.p, ctx->ip_ptr.p, ip.p,
                                        ctx->ip32T.p, ctx->stream);
         CK(cudaGetLastError());
         CK(ctx->ib_part.alloc((size_t)std::max(maxpc, 1) * N)); CK(ctx->ib_part32.alloc((size_t)std::max(maxpc, 1) * N));
@@ -590,7 +591,7 @@ static int setup_interp(ifgf2d_ctx* ctx, int nlevels, DBuf<int>& perr) {
     ctx->counts[0] = T.near_pairs; ctx->counts[1] = T.leaf_evals; ctx->counts[2] = T.prop_evals;
     ctx->counts[3] = T.interp_evals; ctx->counts[4] = T.total_cones; ctx->counts[5] = nlevels;
     ctx->counts[7] = (long long)(ctx->near.n + ctx->leafL.n + ctx->coef.n + ctx->W.n) * 16 + (long long)ctx->pp.bytes() +
-                     (long long)ctx->ip.n * sizeof(InterpEntryD);
+                     (long long)ctx->ipx.n * sizeof(InterpX);
     ctx->ifgf_ready = true;
     if (ctx->gw) ctx->gw->drop_graphs();
     return IFGF2D_OK;

@@ -61,7 +61,6 @@ template <> struct PropE<float> { int child_cone; float s, th, wr, wi; };
 // batched propagation term: the parent node pt it feeds, then as PropE.  A parent's terms are
 // sorted by child cone, so a warp loads each child cone's coefficients once per parent.
 template <typename R> struct PropB;
-template <> struct PropB<double> { int child_cone; int pt; double s, th, wr, wi; };
 template <> struct PropB<float> { int child_cone; int pt; float s, th, wr, wi; };
 using InterpEntryD = InterpE<double>;
 // the FP64 propagation plan, array by array (each lane's loads are whole vectors, coalesced): child
@@ -171,6 +170,11 @@ inline void launch_intensities(const double2* x, const double* wq, const long lo
     launch_intensities_t<double>(x, wq, perm, N, rho, s);
 }
 
+// terms of the batched FP64 form, sorted by cone within a list: cone and node (or target of the work
+// item), factor, and the Chebyshev values T_1.. of s, then of theta, as fixed-point limbs
+// (batch_x_rows int4 per term)
+struct TermsX { int2* id; double2* w; int4* rows; };
+
 // ---------------- batched apply (ifgf_batch.cu) ----------------
 // A batch of B right-hand sides is held interleaved, [N][B] (RHS index fastest); cone
 // coefficients likewise [cone][P][B].  One warp serves 32 right-hand sides of one row, cone or
@@ -185,15 +189,22 @@ void launch_sing_b(const double2* xt, const float2* xt32, const double2* W, cons
                    const double* wq, const long long* inv, double2* rho64, float2* rho32, cudaStream_t s);
 template <typename R>
 void launch_leaf_b(const int* cone_box, int ncones, int cone_base, const int* leaf_start, const int* leaf_count,
-                   const long long* leaf_off, const V2<R>* L, const V2<R>* rho, int Ps, int Pang, int B, V2<R>* coef,
-                   cudaStream_t s);
-// rows (optional): the terms' Chebyshev rows from launch_plan_rows, read instead of computed
-template <typename R>
-void launch_prop_b(int pbegin, int pend, const long long* pp_ptr, const int* pp_nchild, const PropB<R>* pb, int Ps, int Pang,
-                   const R* Gsep, int B, V2<R>* coef, cudaStream_t s, const R* rows = nullptr);
-// the Chebyshev rows T_0..T_{Ps-1}(s), T_0..T_{Pang-1}(th) of n batched plan terms, [term][Ps + Pang]
-template <typename R>
-void launch_plan_rows(const PropB<R>* pb, long long n, int Ps, int Pang, R* rows, cudaStream_t s);
+                   const long long* leaf_off, const V2<R>* L, const V2<R>* rho, int Ps, int Pang, int B, CoefT<R>* coef,
+                   int* cexp, cudaStream_t s);
+void launch_prop_b(int pbegin, int pend, const long long* pp_ptr, const int* pp_nchild, const PropB<float>* pb, int Ps, int Pang,
+                   const float* Gsep, int B, float2* coef, cudaStream_t s);
+// the FP64 form in fixed point (fixpoint.cuh): coefficients [cone][P][B] as limbs with one exponent per
+// cone and right-hand side, cexp [cone][B].  launch_sort_plan_x fills the propagation's terms, sorted by
+// child cone within a parent; launch_group_terms_x the interpolation's from the plan ip: term i is
+// ip[src[i]] of target tgt[i] (within its work item)
+int batch_x_rows(int Ps, int Pang);
+void launch_sort_plan_x(const long long* pp_ptr, int ncones, PlanX px, int Ps, int Pang, TermsX out, cudaStream_t s);
+void launch_group_terms_x(const InterpX* ip, const int2* src_tgt, long long n, int Ps, int Pang, TermsX out, cudaStream_t s);
+void launch_prop_bx(int pbegin, int pend, const long long* pp_ptr, TermsX terms, int Ps, int Pang, const int2* GsepX, int B, int4* coef,
+                    int* cexp, cudaStream_t s);
+// yt[sorting[t]] += the interpolation of work items (first term, end term, first Morton target, targets)
+void launch_interp_bx(const int4* items, int nitems, TermsX terms, const int4* coef, const int* cexp, int Ps, int Pang,
+                      const long long* sorting, int B, double2* yt, cudaStream_t s);
 // the complex64 propagation on the tcgen05 tensor cores in 3xTF32 (batch_tcgen05.cu); false when
 // the shape is not supported (Ps x Pang other than 5 x 5, more than 64 right-hand sides) and
 // nothing was launched.  *err is set when a completion wait runs out.  The kernel's shared-memory

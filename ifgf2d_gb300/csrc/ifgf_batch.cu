@@ -14,10 +14,13 @@
 //   k_prop_b   child -> parent, per parent cone one warp; the
 //              parent's terms sorted by child cone so each child
 //              cone's coefficients are loaded once                 BoxTree.h:767-868, Interpolator.h:81-120
-//   k_final_b  near field + cousin interpolation per target       BoxTree.h:614-683, 876-937
+//   k_prop_bx, k_interp_bx  the FP64 propagation and interpolation
+//              in fixed point (fixpoint.cuh)
+//   k_final_b  near field (+ complex64 cousin interpolation) per
+//              target                                              BoxTree.h:614-683, 876-937
 //
 // plus the batched GMRES vector kernels (per-RHS dot products, CGS updates, scaling).
-#include "ifgf_device.cuh"
+#include "fixpoint.cuh"
 #include "tcgen05.cuh"
 
 namespace ifgf {
@@ -136,7 +139,7 @@ __global__ void __launch_bounds__(kLeafWarps * 32) k_leaf_b(const int* __restric
                                                             const int* __restrict__ leaf_count,
                                                             const long long* __restrict__ leaf_off,
                                                             const V2<R>* __restrict__ L, const V2<R>* __restrict__ rho, int B,
-                                                            V2<R>* __restrict__ coef) {
+                                                            int Ps, CoefT<R>* __restrict__ coef, int* __restrict__ cexp) {
     constexpr int TS = sizeof(R) == 4 ? 16 : 8;
     __shared__ V2<R> tile[kLeafWarps][2][TS * P];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -199,25 +202,38 @@ __global__ void __launch_bounds__(kLeafWarps * 32) k_leaf_b(const int* __restric
 #pragma unroll
     for (int k = 0; k < RPL; ++k) {
         if (!act[k]) continue;
-        V2<R>* out = coef + (long long)(cone_base + c) * P * B + rr[k];
+        CoefT<R>* out = coef + (long long)(cone_base + c) * P * B + rr[k];
+        if constexpr (sizeof(R) == 8) {      // the block's common exponent, and fixed-point limbs
+            int mx = 0;
 #pragma unroll
-        for (int m = 0; m < P; ++m) out[(long long)m * B] = acc[k][m];
+            for (int m = 0; m < P; ++m) mx = max(mx, fx_absmax_hi(acc[k][m].x, acc[k][m].y));
+            const int E = fx_expo(mx), T = fx_top(P);
+#pragma unroll
+            for (int m = 0; m < P; ++m) {
+                const long long a = E == kFxBad ? 0 : fx_from(acc[k][m].x, E, T), b = E == kFxBad ? 0 : fx_from(acc[k][m].y, E, T);
+                out[(long long)m * B] = m % Ps ? fx_pack(a, b) : fx_pack_raw(a, b);
+            }
+            cexp[(long long)(cone_base + c) * B + rr[k]] = E;
+        } else {
+#pragma unroll
+            for (int m = 0; m < P; ++m) out[(long long)m * B] = acc[k][m];
+        }
     }
 }
 
 // ------------------------------------------------------------------ propagation
-// warp = one parent cone x 32*RPL right-hand sides.  Node values accumulate in the lane's own
+// complex64: warp = one parent cone x 32*RPL right-hand sides.  Node values accumulate in the lane's own
 // shared-memory columns; the values -> coefficients map then runs in the lane's registers.
-template <typename R, int P, int RPL>
+template <int P, int RPL>
 struct PropBlock {
-    static constexpr int bytes_per_warp = P * 32 * RPL * (int)sizeof(V2<R>);
+    static constexpr int bytes_per_warp = P * 32 * RPL * (int)sizeof(float2);
     static constexpr int W = 32768 / bytes_per_warp >= 4 ? 4 : (32768 / bytes_per_warp >= 2 ? 2 : 1);
 };
-template <typename R, int PS, int PA, int WPB, int RPL, bool ROWS = false>
+template <int PS, int PA, int WPB, int RPL>
 __global__ void __launch_bounds__(WPB * 32) k_prop_b(int pbegin, int pend, const long long* __restrict__ pp_ptr,
-                                                     const int* __restrict__ pp_nchild, const PropB<R>* __restrict__ pb,
-                                                     const R* __restrict__ Gsep, int B, V2<R>* __restrict__ coef,
-                                                     const R* __restrict__ rows = nullptr) {
+                                                     const int* __restrict__ pp_nchild, const PropB<float>* __restrict__ pb,
+                                                     const float* __restrict__ Gsep, int B, float2* __restrict__ coef) {
+    using R = float;
     constexpr int P = PS * PA;
     __shared__ V2<R> sv[WPB][P][32 * RPL];
     __shared__ R sG[PS * PS + PA * PA];
@@ -256,16 +272,8 @@ __global__ void __launch_bounds__(WPB * 32) k_prop_b(int pbegin, int pend, const
                 for (int q = 0; q < P; ++q) cc[k][q] = src[(long long)q * B + rr[k]];
         }
         R Ts[PS], Tt[PA];
-        if constexpr (ROWS) {   // the same rows, computed once per term by k_plan_rows
-            const R* rw = rows + (e0 + e) * (PS + PA);
-#pragma unroll
-            for (int q = 0; q < PS; ++q) Ts[q] = rw[q];
-#pragma unroll
-            for (int q = 0; q < PA; ++q) Tt[q] = rw[PS + q];
-        } else {
-            cheb_row<R, PS>(E.s, Ts);
-            cheb_row<R, PA>(E.th, Tt);
-        }
+        cheb_row<R, PS>(E.s, Ts);
+        cheb_row<R, PA>(E.th, Tt);
         V2<R> wv; wv.x = E.wr; wv.y = E.wi;
 #pragma unroll
         for (int k = 0; k < RPL; ++k) {
@@ -309,22 +317,154 @@ __global__ void __launch_bounds__(WPB * 32) k_prop_b(int pbegin, int pend, const
     }
 }
 
-// the Chebyshev rows T_q(s), T_a(th) of every batched plan term, [term][PS + PA]: the propagation
-// reads them once per warp instead of computing them in every lane (they are the same for all
-// the warp's right-hand sides), with the same cheb_row arithmetic
-template <typename R, int PS, int PA>
-__global__ void k_plan_rows(const PropB<R>* __restrict__ pb, long long n, R* __restrict__ rows) {
-    const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= n) return;
-    const PropB<R> E = pb[e];
-    R Ts[PS], Tt[PA];
-    cheb_row<R, PS>(E.s, Ts);
-    cheb_row<R, PA>(E.th, Tt);
-    R* rw = rows + e * (PS + PA);
+// ------------------------------------------------------------------ FP64 cone sums in fixed point
+// fixpoint.cuh's arithmetic, one right-hand side per thread.  A block's threads share one list of terms
+// sorted by cone: the list is staged in shared memory kTermsChunk terms at a time, with the Chebyshev
+// values computed at set-up (they are the same for every right-hand side), and a cone's block stays in
+// registers for all its terms (about 14).  A term takes some 140 wide multiply-adds a thread, the bound,
+// and 6 FP64 operations (conversion and factor) beside them, against 56 FP64 operations before.  Kite
+// k = 500, 64 right-hand sides: propagation 11.0 -> 3.2 ms, interpolation 1.6 -> 0.48 ms.
+constexpr int kTermsChunk = 64;
+template <int PS, int PA>
+struct StageX {
+    int4 rows[kTermsChunk * fx_rows4(PS, PA)];
+    double2 w[kTermsChunk];
+    int2 id[kTermsChunk];
+};
+// add(node, value) for the terms [e0, e0 + n)
+template <int PS, int PA, int NT, typename Add>
+__device__ __forceinline__ void terms_x(StageX<PS, PA>& S, TermsX terms, long long e0, int n, const int4* __restrict__ coef,
+                                        const int* __restrict__ cexp, int B, int rr, Add&& add) {
+    constexpr int P = PS * PA, N4 = fx_rows4(PS, PA), T = fx_top(P);
+    int4 cc[P];
+    int cur = -1, E = 0;
+    for (int c0 = 0; c0 < n; c0 += kTermsChunk) {
+        const int cnt = min(kTermsChunk, n - c0);
+        __syncthreads();                       // the previous chunk has been read
+        for (int i = threadIdx.x; i < cnt * N4; i += NT) cp_async_el<16>(&S.rows[i], terms.rows + (e0 + c0) * N4 + i);
+        for (int i = threadIdx.x; i < cnt; i += NT) {
+            cp_async_el<16>(&S.w[i], terms.w + e0 + c0 + i);
+            cp_async_el<8>(&S.id[i], terms.id + e0 + c0 + i);
+        }
+        cp_async_commit();
+        cp_async_wait<0>();
+        __syncthreads();
+        for (int i = 0; i < cnt; ++i) {
+            const int2 id = S.id[i];
+            if (id.x != cur) {                 // uniform over the block
+                cur = id.x;
+                const int4* src = coef + (long long)cur * P * B + rr;
 #pragma unroll
-    for (int q = 0; q < PS; ++q) rw[q] = Ts[q];
+                for (int q = 0; q < P; ++q) cc[q] = src[(long long)q * B];
+                E = cexp[(long long)cur * B + rr];
+            }
+            FxLimb t[2 * N4];
 #pragma unroll
-    for (int q = 0; q < PA; ++q) rw[PS + q] = Tt[q];
+            for (int q = 0; q < N4; ++q) {
+                const int4 a = S.rows[i * N4 + q];
+                t[2 * q] = FxLimb{a.x, a.y}; t[2 * q + 1] = FxLimb{a.z, a.w};
+            }
+            long long re, im;
+            fx_interp<PS, PA>(t, t + PS - 1, [&](int q) { return cc[q]; }, re, im);
+            const double2 w = S.w[i];
+            add(id.y, make_double2(fx_value(re, E, T), fx_value(im, E, T)), w);
+        }
+    }
+}
+
+// block = one parent cone x NT right-hand sides.  Node values accumulate in the thread's own column of
+// shared memory; then the cone's exponent, the values->coefficients map and the normalisation, all
+// within the column.
+template <int PS, int PA, int NT>
+__global__ void __launch_bounds__(NT) k_prop_bx(int pbegin, const long long* __restrict__ pp_ptr, TermsX terms,
+                                                const int2* __restrict__ Gsep, int B, int4* __restrict__ coef, int* __restrict__ cexp) {
+    constexpr int P = PS * PA, T = fx_top(P);
+    __shared__ StageX<PS, PA> S;
+    __shared__ int4 sv[P][NT];                 // FP64 node values, then limbs
+    __shared__ int2 sG[PS * PS + PA * PA];
+    const int tid = threadIdx.x;
+    for (int i = tid; i < PS * PS + PA * PA; i += NT) sG[i] = Gsep[i];
+    const int pc = pbegin + blockIdx.x;
+    const int r = blockIdx.y * NT + tid;
+    const bool act = r < B;
+    const int rr = act ? r : 0;
+    auto node = [&](int q) -> double2& { return *reinterpret_cast<double2*>(&sv[q][tid]); };
+#pragma unroll
+    for (int q = 0; q < P; ++q) node(q) = make_double2(0.0, 0.0);
+    const long long e0 = pp_ptr[pc];
+    terms_x<PS, PA, NT>(S, terms, e0, (int)(pp_ptr[pc + 1] - e0), coef, cexp, B, rr, [&](int pt, double2 it, double2 w) {
+        double2 a = node(pt);
+        cmac<double>(a, it, w);
+        node(pt) = a;
+    });
+    __syncthreads();
+    if (!act) return;
+    int mx = 0;
+    for (int q = 0; q < P; ++q) { const double2 a = node(q); mx = max(mx, fx_absmax_hi(a.x, a.y)); }
+    const int E = fx_expo(mx);
+    for (int l = 0; l < PA; ++l) {             // u[l][m] = sum_k Gs[m][k] v[l][k]
+        int4 v[PS];
+#pragma unroll
+        for (int q = 0; q < PS; ++q) {
+            const double2 a = node(l * PS + q);
+            v[q] = E == kFxBad ? make_int4(0, 0, 0, 0) : fx_pack(fx_from(a.x, E, T), fx_from(a.y, E, T));
+        }
+#pragma unroll
+        for (int m = 0; m < PS; ++m) {
+            long long ur, ui;
+            fx_map<PS>([&](int k) { return sG[m * PS + k]; }, [&](int k) { return v[k]; }, ur, ui);
+            sv[l * PS + m][tid] = fx_pack(ur, ui);
+        }
+    }
+    int lz = 64;
+    for (int m = 0; m < PS; ++m) {             // c[n][m] = sum_l Ga[n][l] u[l][m], stored at n*PS + m
+        int4 u[PA];
+#pragma unroll
+        for (int l = 0; l < PA; ++l) u[l] = sv[l * PS + m][tid];
+#pragma unroll
+        for (int n = 0; n < PA; ++n) {
+            long long cr, ci;
+            fx_map<PA>([&](int l) { return sG[PS * PS + n * PA + l]; }, [&](int l) { return u[l]; }, cr, ci);
+            lz = min(lz, min(__clzll(cr < 0 ? -cr : cr), __clzll(ci < 0 ? -ci : ci)));
+            sv[n * PS + m][tid] = fx_pack_raw(cr, ci);
+        }
+    }
+    int sh = lz - (63 - T);                    // left shift that brings the largest to [2^(T-1), 2^T)
+    sh = E == kFxBad ? 0 : min(sh, E - kFxMinExp);
+    int4* out = coef + (long long)pc * P * B + r;
+    for (int q = 0; q < P; ++q) {
+        const int4 a = sv[q][tid];
+        const long long x = fx_shift(fx_raw(a.x, a.y), sh), y = fx_shift(fx_raw(a.z, a.w), sh);
+        out[(long long)q * B] = q % PS ? fx_pack(x, y) : fx_pack_raw(x, y);
+    }
+    cexp[(long long)pc * B + r] = E == kFxBad ? kFxBad : E - sh;
+}
+
+// block = one work item (up to kInterpGrpTargets targets of one leaf box) x NT right-hand sides; the
+// targets' sums accumulate in the thread's column of shared memory, then are added into yt
+template <int PS, int PA, int NT>
+__global__ void __launch_bounds__(NT) k_interp_bx(const int4* __restrict__ items, TermsX terms, const int4* __restrict__ coef,
+                                                  const int* __restrict__ cexp, const long long* __restrict__ sorting, int B,
+                                                  double2* __restrict__ yt) {
+    __shared__ StageX<PS, PA> S;
+    __shared__ double2 acc[kInterpGrpTargets][NT];
+    const int4 I = items[blockIdx.x];          // terms [x, y), targets [z, z + w)
+    const int r = blockIdx.y * NT + threadIdx.x;
+    const bool act = r < B;
+    for (int t = 0; t < I.w; ++t) acc[t][threadIdx.x] = make_double2(0.0, 0.0);
+    terms_x<PS, PA, NT>(S, terms, I.x, I.y - I.x, coef, cexp, B, act ? r : 0, [&](int t, double2 it, double2 f) {
+        double2 a = acc[t][threadIdx.x];
+        cmac<double>(a, it, f);
+        acc[t][threadIdx.x] = a;
+    });
+    if (!act) return;
+    for (int t = 0; t < I.w; ++t) {
+        double2* yo = yt + sorting[I.z + t] * B + r;
+        const double2 a = acc[t][threadIdx.x];
+        double2 v = *yo;
+        v.x += a.x; v.y += a.y;
+        *yo = v;
+    }
 }
 
 // ------------------------------------------------------------------ propagation, TMA-staged
@@ -682,32 +822,46 @@ void launch_sing_b(const double2* xt, const float2* xt32, const double2* W, cons
 }
 template <typename R>
 void launch_leaf_b(const int* cone_box, int ncones, int cone_base, const int* leaf_start, const int* leaf_count,
-                   const long long* leaf_off, const V2<R>* L, const V2<R>* rho, int Ps, int Pang, int B, V2<R>* coef,
-                   cudaStream_t s) {
+                   const long long* leaf_off, const V2<R>* L, const V2<R>* rho, int Ps, int Pang, int B, CoefT<R>* coef,
+                   int* cexp, cudaStream_t s) {
     if (ncones <= 0) return;
     constexpr int RPL = Rpl<R>::v;
     const dim3 grid(nblk_b(ncones, kLeafWarps), nblk_b(B, 32 * RPL));
     IFGF_DISPATCH_P(Ps, Pang, (k_leaf_b<R, PS * PA, RPL><<<grid, kLeafWarps * 32, 0, s>>>(
-                                   cone_box, ncones, cone_base, leaf_start, leaf_count, leaf_off, L, rho, B, coef)));
+                                   cone_box, ncones, cone_base, leaf_start, leaf_count, leaf_off, L, rho, B, PS, coef, cexp)));
 }
-template <typename R>
-void launch_prop_b(int pbegin, int pend, const long long* pp_ptr, const int* pp_nchild, const PropB<R>* pb, int Ps, int Pang,
-                   const R* Gsep, int B, V2<R>* coef, cudaStream_t s, const R* rows) {
+void launch_prop_b(int pbegin, int pend, const long long* pp_ptr, const int* pp_nchild, const PropB<float>* pb, int Ps, int Pang,
+                   const float* Gsep, int B, float2* coef, cudaStream_t s) {
     if (pend <= pbegin) return;
-    constexpr int RPL = Rpl<R>::v;
+    constexpr int RPL = Rpl<float>::v;
     IFGF_DISPATCH_P(Ps, Pang, {
-        constexpr int WPB = PropBlock<R, PS * PA, RPL>::W;
+        constexpr int WPB = PropBlock<PS * PA, RPL>::W;
         const dim3 grid(nblk_b(pend - pbegin, WPB), nblk_b(B, 32 * RPL));
-        if (rows)
-            k_prop_b<R, PS, PA, WPB, RPL, true><<<grid, WPB * 32, 0, s>>>(pbegin, pend, pp_ptr, pp_nchild, pb, Gsep, B, coef, rows);
-        else
-            k_prop_b<R, PS, PA, WPB, RPL><<<grid, WPB * 32, 0, s>>>(pbegin, pend, pp_ptr, pp_nchild, pb, Gsep, B, coef);
+        k_prop_b<PS, PA, WPB, RPL><<<grid, WPB * 32, 0, s>>>(pbegin, pend, pp_ptr, pp_nchild, pb, Gsep, B, coef);
     });
 }
-template <typename R>
-void launch_plan_rows(const PropB<R>* pb, long long n, int Ps, int Pang, R* rows, cudaStream_t s) {
-    if (n <= 0) return;
-    IFGF_DISPATCH_P(Ps, Pang, (k_plan_rows<R, PS, PA><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(pb, n, rows)));
+// threads (right-hand sides) of a block of the FP64 kernels: 64 share a list of terms where its shared
+// memory allows (up to 36 nodes); 32 for batches that fit one warp
+template <int P> struct BatchXThreads { static constexpr int v = P <= 36 ? 64 : 32; };
+void launch_prop_bx(int pbegin, int pend, const long long* pp_ptr, TermsX terms, int Ps, int Pang, const int2* GsepX, int B, int4* coef,
+                    int* cexp, cudaStream_t s) {
+    if (pend <= pbegin || B <= 0) return;
+    IFGF_DISPATCH_P(Ps, Pang, {
+        constexpr int NT = BatchXThreads<PS * PA>::v;
+        const dim3 grid(pend - pbegin, nblk_b(B, B <= 32 ? 32 : NT));
+        if (B <= 32) k_prop_bx<PS, PA, 32><<<grid, 32, 0, s>>>(pbegin, pp_ptr, terms, GsepX, B, coef, cexp);
+        else k_prop_bx<PS, PA, NT><<<grid, NT, 0, s>>>(pbegin, pp_ptr, terms, GsepX, B, coef, cexp);
+    });
+}
+void launch_interp_bx(const int4* items, int nitems, TermsX terms, const int4* coef, const int* cexp, int Ps, int Pang,
+                      const long long* sorting, int B, double2* yt, cudaStream_t s) {
+    if (nitems <= 0 || B <= 0) return;
+    IFGF_DISPATCH_P(Ps, Pang, {
+        constexpr int NT = BatchXThreads<PS * PA>::v;
+        const dim3 grid(nitems, nblk_b(B, B <= 32 ? 32 : NT));
+        if (B <= 32) k_interp_bx<PS, PA, 32><<<grid, 32, 0, s>>>(items, terms, coef, cexp, sorting, B, yt);
+        else k_interp_bx<PS, PA, NT><<<grid, NT, 0, s>>>(items, terms, coef, cexp, sorting, B, yt);
+    });
 }
 bool launch_interp_grp(const int4* items, int nitems, const InterpG* terms, const float2* coef, int Ps, int Pang,
                        const long long* sorting, int B, double2* yt, cudaStream_t s) {
@@ -752,10 +906,7 @@ void launch_bscale(const double2* w, const double2* hn, long long N, int B, doub
 
 #define IFGF_BATCH_INSTANTIATE(R)                                                                                       \
     template void launch_leaf_b<R>(const int*, int, int, const int*, const int*, const long long*, const V2<R>*,        \
-                                   const V2<R>*, int, int, int, V2<R>*, cudaStream_t);                                  \
-    template void launch_prop_b<R>(int, int, const long long*, const int*, const PropB<R>*, int, int, const R*, int,    \
-                                   V2<R>*, cudaStream_t, const R*);                                                     \
-    template void launch_plan_rows<R>(const PropB<R>*, long long, int, int, R*, cudaStream_t);                         \
+                                   const V2<R>*, int, int, int, CoefT<R>*, int*, cudaStream_t);                         \
     template void launch_final_b<R>(int, const int*, const int*, const int*, const int*, const int*, const int*,        \
                                     const long long*, const V2<R>*, const V2<R>*, const int*, const InterpE<R>*,        \
                                     const V2<R>*, int, int, const long long*, int, double2*, cudaStream_t);

@@ -155,19 +155,17 @@ __global__ void k_leaf_nodes(LevelDesc L, double min_x, double min_y, double k, 
 
 // a parent's terms sorted by child cone (stable), with the parent node (entry index mod P)
 // recorded: one warp per parent cone, each lane ranking its entries against the parent's
-// child-cone list in shared memory
+// child-cone list in shared memory; put(sorted entry, entry, entry of the parent, child cone)
 constexpr int kSortWarps = 8;
-template <typename R>
-__global__ void __launch_bounds__(kSortWarps * 32) k_sort_plan(const long long* __restrict__ pp_ptr, int ncones,
-                                                               PlanX px, const PropE<float>* __restrict__ pp32, int P,
-                                                               PropB<R>* __restrict__ out) {
+template <typename Child, typename Put>
+__device__ __forceinline__ void sort_parent(const long long* __restrict__ pp_ptr, int ncones, Child&& child, Put&& put) {
     __shared__ int cc[kSortWarps][4 * kMaxP];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int pc = blockIdx.x * kSortWarps + warp;
     if (pc >= ncones) return;
     const long long e0 = pp_ptr[pc];
     const int ne = (int)(pp_ptr[pc + 1] - e0);
-    for (int i = lane; i < ne; i += 32) cc[warp][i] = px.child[e0 + i];
+    for (int i = lane; i < ne; i += 32) cc[warp][i] = child(e0 + i);
     __syncwarp();
     for (int i = lane; i < ne; i += 32) {
         const int c = cc[warp][i];
@@ -176,15 +174,47 @@ __global__ void __launch_bounds__(kSortWarps * 32) k_sort_plan(const long long* 
             const int d = cc[warp][j];
             rank += (d < c) || (d == c && j < i);
         }
-        if constexpr (sizeof(R) == 4) {
-            const PropE<float> E = pp32[e0 + i];
-            out[e0 + rank] = PropB<R>{E.child_cone, i % P, E.s, E.th, E.wr, E.wi};
-        } else {
-            const longlong2 t = px.st[e0 + i];
-            const double2 w = px.w[e0 + i];
-            out[e0 + rank] = PropB<R>{c, i % P, fx_weight_value(t.x), fx_weight_value(t.y), w.x, w.y};
-        }
+        put(e0 + rank, e0 + i, i, c);
     }
+}
+__global__ void __launch_bounds__(kSortWarps * 32) k_sort_plan(const long long* __restrict__ pp_ptr, int ncones,
+                                                               const PropE<float>* __restrict__ pp, int P,
+                                                               PropB<float>* __restrict__ out) {
+    sort_parent(pp_ptr, ncones, [&](long long e) { return pp[e].child_cone; }, [&](long long to, long long from, int i, int c) {
+        const PropE<float> E = pp[from];
+        out[to] = PropB<float>{c, i % P, E.s, E.th, E.wr, E.wi};
+    });
+}
+// the Chebyshev values of a batched FP64 term
+template <int PS, int PA>
+__device__ __forceinline__ void put_rows(longlong2 st, int4* __restrict__ out) {
+    constexpr int N4 = fx_rows4(PS, PA);
+    FxLimb t[2 * N4];
+#pragma unroll
+    for (int i = PS + PA - 2; i < 2 * N4; ++i) t[i] = FxLimb{0, 0};
+    fx_cheb<PS>(st.x, t);
+    fx_cheb<PA>(st.y, t + PS - 1);
+#pragma unroll
+    for (int i = 0; i < N4; ++i) out[i] = make_int4(t[2 * i].h, t[2 * i].l, t[2 * i + 1].h, t[2 * i + 1].l);
+}
+template <int PS, int PA>
+__global__ void __launch_bounds__(kSortWarps * 32) k_sort_plan_x(const long long* __restrict__ pp_ptr, int ncones, PlanX px,
+                                                                 TermsX out) {
+    sort_parent(pp_ptr, ncones, [&](long long e) { return px.child[e]; }, [&](long long to, long long from, int i, int c) {
+        out.id[to] = make_int2(c, i % (PS * PA));
+        out.w[to] = px.w[from];
+        put_rows<PS, PA>(px.st[from], out.rows + to * fx_rows4(PS, PA));
+    });
+}
+template <int PS, int PA>
+__global__ void k_group_terms_x(const InterpX* __restrict__ ip, const int2* __restrict__ src_tgt, long long n, TermsX out) {
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int2 q = src_tgt[i];
+    const InterpX E = ip[q.x];
+    out.id[i] = make_int2(E.cone, q.y);
+    out.w[i] = make_double2(E.fr, E.fi);
+    put_rows<PS, PA>(make_longlong2(E.s, E.th), out.rows + i * fx_rows4(PS, PA));
 }
 
 __global__ void k_interp_to_c64(const InterpE<double>* __restrict__ in, long long n, InterpE<float>* __restrict__ out) {
@@ -384,13 +414,19 @@ cudaError_t build_leaf_nodes(const Tree& T, LeafNode* out, cudaStream_t s) {
     return e != cudaSuccess ? e : es;
 }
 
-template <typename R>
-void launch_sort_plan(const long long* pp_ptr, int ncones, PlanX px, const PropE<float>* pp32, int P, PropB<R>* out, cudaStream_t s) {
-    if (ncones <= 0) return;
-    k_sort_plan<R><<<(ncones + kSortWarps - 1) / kSortWarps, kSortWarps * 32, 0, s>>>(pp_ptr, ncones, px, pp32, P, out);
+void launch_sort_plan(const long long* pp_ptr, int ncones, const PropE<float>* pp, int P, PropB<float>* out, cudaStream_t s) {
+    if (ncones > 0) k_sort_plan<<<(ncones + kSortWarps - 1) / kSortWarps, kSortWarps * 32, 0, s>>>(pp_ptr, ncones, pp, P, out);
 }
-template void launch_sort_plan<double>(const long long*, int, PlanX, const PropE<float>*, int, PropB<double>*, cudaStream_t);
-template void launch_sort_plan<float>(const long long*, int, PlanX, const PropE<float>*, int, PropB<float>*, cudaStream_t);
+int batch_x_rows(int Ps, int Pang) { return fx_rows4(Ps, Pang); }
+void launch_sort_plan_x(const long long* pp_ptr, int ncones, PlanX px, int Ps, int Pang, TermsX out, cudaStream_t s) {
+    if (ncones <= 0) return;
+    IFGF_DISPATCH_P(Ps, Pang, (k_sort_plan_x<PS, PA><<<(ncones + kSortWarps - 1) / kSortWarps, kSortWarps * 32, 0, s>>>(pp_ptr, ncones,
+                                                                                                                    px, out)));
+}
+void launch_group_terms_x(const InterpX* ip, const int2* src_tgt, long long n, int Ps, int Pang, TermsX out, cudaStream_t s) {
+    if (n <= 0) return;
+    IFGF_DISPATCH_P(Ps, Pang, (k_group_terms_x<PS, PA><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(ip, src_tgt, n, out)));
+}
 
 void launch_interp_to_c64(const InterpE<double>* in, long long n, InterpE<float>* out, cudaStream_t s) {
     if (n <= 0) return;
