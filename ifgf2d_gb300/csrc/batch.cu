@@ -33,6 +33,8 @@ struct BatchWork {
     DBuf<double2> rho64;
     DBuf<int4> coef64;                         // fixed-point limbs (fixpoint.cuh), with
     DBuf<int> cexp64;                          // one exponent per cone and right-hand side
+    DBuf<int4> rhox;                           // the densities as limbs, with
+    DBuf<int> rexp;                            // one exponent per leaf box and right-hand side
     DBuf<float2> rho32, coef32;
     TermsXBuf px64, ig64;                      // the FP64 propagation's and interpolation's terms
     DBuf<PropB<float>> pb32;
@@ -116,7 +118,7 @@ int ensure_apply(ifgf2d_ctx* ctx, int B, bool mixed) {
     const size_t ncoef = (size_t)ctx->T.total_cones * ctx->T.P;
     if (W.cap < B) {
         W.xt.release(); W.yt.release(); W.rho64.release(); W.coef64.release(); W.rho32.release(); W.coef32.release();
-        W.xt32.release(); W.cexp64.release();
+        W.xt32.release(); W.cexp64.release(); W.rhox.release(); W.rexp.release();
         CK(W.xt.alloc((size_t)N * B)); CK(W.yt.alloc((size_t)N * B));
         W.cap = B;
     }
@@ -157,7 +159,10 @@ int ensure_apply(ifgf2d_ctx* ctx, int B, bool mixed) {
         }
     } else {
         if (!W.rho64.p) { CK(W.rho64.alloc((size_t)N * W.cap)); CK(W.coef64.alloc(ncoef * W.cap)); }
-        if (!W.cexp64.p) CK(W.cexp64.alloc((size_t)ctx->T.total_cones * W.cap));
+        if (!W.cexp64.p) {
+            CK(W.cexp64.alloc((size_t)ctx->T.total_cones * W.cap));
+            CK(W.rhox.alloc((size_t)N * W.cap)); CK(W.rexp.alloc(ctx->T.leaf_start.size() * W.cap));
+        }
         if (!W.px64.id.p) {
             const Tree& T = ctx->T;
             std::vector<int4> gi;
@@ -193,8 +198,8 @@ void far_b(ifgf2d_ctx* ctx, int B, double2* yt) {
                                    leafL, rho, T.Ps, T.Pang, B, coef + (long long)LD.cone_base * T.P * B, W.t5err.p, W.nsm,
                                    (ctx->tune_batch_tc & kBatchTcLeaf6) ? 3 : 2, s);
     if (!leaf_done)
-        launch_leaf_b<float>(ctx->leaf_cone_box.p, (int)LD.cone_nonrel.size(), LD.cone_base, ctx->leaf_start.p, ctx->leaf_count.p,
-                             ctx->leaf_off.p, leafL, rho, T.Ps, T.Pang, B, coef, nullptr, s);
+        launch_leaf_b(ctx->leaf_cone_box.p, (int)LD.cone_nonrel.size(), LD.cone_base, ctx->leaf_start.p, ctx->leaf_count.p,
+                      ctx->leaf_off.p, leafL, rho, T.Ps, T.Pang, B, coef, s);
     for (int l = Dl; l >= 3; --l) {
         const TreeLevel& Lp = T.L[l - 1];
         const int p0 = Lp.cone_base, p1 = Lp.cone_base + (int)Lp.cone_nonrel.size();
@@ -219,8 +224,9 @@ void far_bx(ifgf2d_ctx* ctx, int B, double2* yt) {
     const TreeLevel& LD = T.L[Dl];
     cudaStream_t s = ctx->stream;
     BatchWork& W = *ctx->bw;
-    launch_leaf_b<double>(ctx->leaf_cone_box.p, (int)LD.cone_nonrel.size(), LD.cone_base, ctx->leaf_start.p, ctx->leaf_count.p,
-                          ctx->leaf_off.p, ctx->leafL.p, W.rho64.p, T.Ps, T.Pang, B, W.coef64.p, W.cexp64.p, s);
+    launch_rho_bx(ctx->leaf_start.p, ctx->leaf_count.p, (int)T.leaf_start.size(), W.rho64.p, B, W.rhox.p, W.rexp.p, s);
+    launch_leaf_bx(ctx->leaf_cone_box.p, (int)LD.cone_nonrel.size(), LD.cone_base, ctx->leaf_start.p, ctx->leaf_count.p,
+                   ctx->leaf_off.p, ctx->leafL.p, ctx->lexp.p, W.rhox.p, W.rexp.p, T.Ps, T.Pang, B, W.coef64.p, W.cexp64.p, s);
     for (int l = Dl; l >= 3; --l) {
         const TreeLevel& Lp = T.L[l - 1];
         launch_prop_bx(Lp.cone_base, Lp.cone_base + (int)Lp.cone_nonrel.size(), ctx->pp_ptr.p, W.px64.view(), T.Ps, T.Pang, ctx->GsepX.p,

@@ -219,7 +219,8 @@ struct ifgf2d_ctx {
     DBuf<int> leaf_cone_box;
     DBuf<long long> leaf_off;
     DBuf<LeafNode> leaf_nodes_d;
-    DBuf<double2> leafL;
+    DBuf<int4> leafL;               // the FP64 form's leaf-cone tables: fixed-point limbs, with
+    DBuf<int> lexp;                 // one exponent per cone and coefficient (FP64 values until set-up fixes them)
     DBuf<long long> pp_ptr;
     DBuf<int> pp_nchild;
     PlanBuf pp;
@@ -246,6 +247,8 @@ struct ifgf2d_ctx {
     DBuf<double2> ib_part;
     DBuf<float2> ib_part32;
     // work vectors
+    DBuf<int4> rhox;                // the densities as limbs, with
+    DBuf<int> rexp;                 // one exponent per leaf box
     DBuf<double2> rho, vin, vout;
     std::unique_ptr<GmresWork> gw;
     BatchWork* bw = nullptr;        // batched apply / solve workspace (batch.cu), freed by destroy

@@ -146,6 +146,44 @@ __device__ __forceinline__ double2 fx_interp_value(Load&& c, int E, longlong2 st
     fx_interp<PS, PA>(Ts, Tt, c, re, im);
     return make_double2(fx_value(re, E, fx_top(PS * PA)), fx_value(im, E, fx_top(PS * PA)));
 }
+// ---- table sums (leaf cones): sum_s L[s] rho[s] of complex values, the table entries and the densities
+// both as integers of kFxSumTop bits in two 27-bit limbs, X = h 2^27 + l, |l| <= 2^26 (the left-out
+// products l l stay below 2^-56 of the largest).  The entries of one coefficient share an exponent, the
+// densities of one leaf box another; a box of more than 128 points gives its densities fewer bits, so
+// that no sum overflows.
+constexpr int kFxSumLow = 27, kFxSumTop = 54, kFxSumFold = 64;
+__device__ __forceinline__ int fx_rho_top(int n) { return kFxSumTop - max(0, 32 - __clz(max(n - 1, 0)) - 7); }
+__device__ __forceinline__ int4 fx_pack_sum(long long re, long long im) {
+    const int rh = (int)((re + (1ll << (kFxSumLow - 1))) >> kFxSumLow), ih = (int)((im + (1ll << (kFxSumLow - 1))) >> kFxSumLow);
+    return make_int4(rh, (int)((unsigned)re - ((unsigned)rh << kFxSumLow)), ih, (int)((unsigned)im - ((unsigned)ih << kFxSumLow)));
+}
+// a sum's value is (h + m 2^-27) 2^54 in units of the two blocks'; kFxSumFold terms after a fold at most
+struct FxSum { long long h, m; };
+__device__ __forceinline__ void fx_sum_mac(FxSum& s, int ah, int al, int bh, int bl) {
+    s.m = fx_wide(ah, bl, s.m);
+    s.m = fx_wide(al, bh, s.m);
+    s.h = fx_wide(ah, bh, s.h);
+}
+__device__ __forceinline__ void fx_sum_fold(FxSum& s) {
+    s.h += s.m >> kFxSumLow;
+    s.m &= (1ll << kFxSumLow) - 1;
+}
+// a folded sum of blocks with exponent E (table plus density, minus their bits) as y 2^e, |y| < 2^62 with
+// at most the sum's own bits lost
+__device__ __forceinline__ long long fx_sum_value(FxSum s, int E, int& e) {
+    const int lz = __clzll(s.h < 0 ? ~s.h : s.h);
+    const int sh = min(max(lz - 3, 0), kFxSumLow);
+    e = E + 2 * kFxSumLow - sh;
+    return (s.h << sh) + (s.m >> (kFxSumLow - sh));
+}
+// y 2^e as the integer of a block with exponent E and T bits, rounded
+__device__ __forceinline__ long long fx_align(long long y, int e, int E, int T) {
+    const int sh = e - E + T;
+    return sh >= 0 ? y << sh : (sh < -62 ? 0ll : (y + (1ll << (-sh - 1))) >> -sh);
+}
+// the exponent that y 2^e stays below
+__device__ __forceinline__ int fx_top_of(long long y, int e) { return y ? e + 64 - __clzll(y < 0 ? -y : y) : kFxMinExp; }
+
 // re + i im = sum_k g(k) v(k): a row of the values->coefficients map
 template <int N, typename G, typename V>
 __device__ __forceinline__ void fx_map(G&& g, V&& v, long long& re, long long& im) {

@@ -526,7 +526,7 @@ static int setup_cones(ifgf2d_ctx* ctx, double k, int nlevels, const SetupExtra*
     // leaf-cone tables
     launch_leaf_setup(ctx->leaf_cone_box.p, ncl, ctx->leaf_start.p, ctx->leaf_count.p, ctx->leaf_off.p, ctx->leaf_nodes_d.p,
                       ctx->xs_s.p, ctx->ys_s.p, ctx->nxs_s.p, ctx->nys_s.p, T.Ps, T.Pang, k, ctx->form, ctx->eta, ctx->Gsep.p,
-                      ctx->leafL.p, ctx->stream, ex ? ex->keta_leafcone : nullptr);
+                      reinterpret_cast<double2*>(ctx->leafL.p), ctx->stream, ex ? ex->keta_leafcone : nullptr);
     CK(cudaGetLastError());
     return IFGF2D_OK;
 }
@@ -582,7 +582,14 @@ static int setup_interp(ifgf2d_ctx* ctx, int nlevels, DBuf<int>& perr) {
     CK(cudaDeviceGetAttribute(&ctx->nsm, cudaDevAttrMultiProcessorCount, ctx->device));
     if (!ctx->kerr.p) { CK(ctx->kerr.alloc(1)); CK(cudaMemsetAsync(ctx->kerr.p, 0, sizeof(int), ctx->stream)); }
     launch_d2f(ctx->near.p, (long long)ctx->near.n, ctx->near32.p, ctx->stream);
-    launch_d2f(ctx->leafL.p, (long long)ctx->leafL.n, ctx->leafL32.p, ctx->stream);
+    {
+        const TreeLevel& LD = T.L[nlevels - 1];
+        const int ncl = (int)LD.cone_nonrel.size();
+        CK(ctx->lexp.alloc((size_t)ncl * P));
+        launch_leaf_fix(ctx->leaf_cone_box.p, ncl, ctx->leaf_count.p, ctx->leaf_off.p, P, ctx->leafL.p, ctx->lexp.p, ctx->leafL32.p,
+                        ctx->stream);
+    }
+    CK(ctx->rhox.alloc(N)); CK(ctx->rexp.alloc(nleaf));
     CK(cudaGetLastError());
     int bad = 0;
     CK(cudaMemcpyAsync(&bad, perr.p, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
@@ -657,6 +664,24 @@ static void launch_interp_final(ifgf2d_ctx* ctx, const V2<R>* rho, const V2<R>* 
                        ctx->stream);
 }
 
+// leaf-cone sums of the Morton-ordered intensities (rhox or rho32); `shape`: the threads that share a
+// coefficient's sum (1, 2, 5 or 10; complex64 also 0, the table streamed by TMA bulk copies)
+template <typename R>
+static void launch_leaf(ifgf2d_ctx* ctx, CoefT<R>* coef, int shape) {
+    const Tree& T = ctx->T;
+    const TreeLevel& LD = T.L[ctx->nlevels - 1];
+    const int ncl = (int)LD.cone_nonrel.size();
+    if constexpr (sizeof(R) == 4) {
+        if (shape == 0 && launch_leaf_tma(ctx->leaf_cone_box.p, ncl, LD.cone_base, ctx->leaf_start.p, ctx->leaf_count.p, ctx->leaf_off.p,
+                                          ctx->leafL32.p, ctx->rho32.p, T.P, coef, ctx->kerr.p, ctx->nsm, ctx->stream))
+            return;
+        launch_leaf_apply_t(ctx->leaf_cone_box.p, ncl, LD.cone_base, ctx->leaf_start.p, ctx->leaf_count.p, ctx->leaf_off.p,
+                            ctx->leafL32.p, ctx->rho32.p, T.P, coef, ctx->stream, shape);
+    } else {
+        launch_leaf_fx(ctx->leaf_cone_box.p, ncl, LD.cone_base, ctx->leaf_start.p, ctx->leaf_count.p, ctx->leaf_off.p, ctx->leafL.p,
+                       ctx->lexp.p, ctx->rhox.p, ctx->rexp.p, T.P, T.Ps, coef, ctx->cexp.p, ctx->stream, shape);
+    }
+}
 // children at level l -> parents at level l - 1; `shape`: the complex64 kernel's launch shape (the
 // FP64 kernel has one)
 template <typename R>
@@ -673,22 +698,12 @@ static void launch_prop_level(ifgf2d_ctx* ctx, int l, CoefT<R>* coef, int shape)
 
 // y += far field of the Morton-ordered intensities (rho / rho32), BoxTree.h:1037-1061
 template <typename R>
-static void far_ifgf_t(ifgf2d_ctx* ctx, const V2<R>* rho, const V2<R>* near, const V2<R>* leafL, const InterpT<R>* ip,
-                       CoefT<R>* coef, double2* y, cudaEvent_t* ev) {
-    const Tree& T = ctx->T;
-    const int Dl = ctx->nlevels - 1, P = T.P;
-    const TreeLevel& LD = T.L[Dl];
+static void far_ifgf_t(ifgf2d_ctx* ctx, const V2<R>* rho, const V2<R>* near, const InterpT<R>* ip, CoefT<R>* coef, double2* y,
+                       cudaEvent_t* ev) {
+    const int Dl = ctx->nlevels - 1;
     cudaStream_t s = ctx->stream;
     const int pr = sizeof(R) == 4 ? 1 : 0;
-    bool leaf_done = false;
-    if constexpr (sizeof(R) == 4) {
-        if (ctx->tune_leaf[1] == 0)
-            leaf_done = launch_leaf_tma(ctx->leaf_cone_box.p, (int)LD.cone_nonrel.size(), LD.cone_base, ctx->leaf_start.p,
-                                        ctx->leaf_count.p, ctx->leaf_off.p, leafL, rho, P, coef, ctx->kerr.p, ctx->nsm, s);
-    }
-    if (!leaf_done)
-        launch_leaf_apply_t<R>(ctx->leaf_cone_box.p, (int)LD.cone_nonrel.size(), LD.cone_base, ctx->leaf_start.p, ctx->leaf_count.p,
-                               ctx->leaf_off.p, leafL, rho, P, T.Ps, coef, ctx->cexp.p, s, ctx->tune_leaf[pr]);
+    launch_leaf<R>(ctx, coef, ctx->tune_leaf[pr]);
     if (ev) cudaEventRecord(ev[0], s);
     for (int l = Dl; l >= 3; --l) {
         launch_prop_level<R>(ctx, l, coef, l < kTuneLevels ? ctx->tune_prop[pr][l] : 0);
@@ -705,11 +720,15 @@ static int far_apply(ifgf2d_ctx* ctx, const double2* x, const double* wq, double
     if (mode == IFGF2D_APPLY_IFGF_MIXED) {
         if (!rho_ready) launch_intensities_t<float>(x, wq, ctx->sorting.p, N, ctx->rho32.p, ctx->stream);
         if (ev) cudaEventRecord(ev[0], ctx->stream);
-        far_ifgf_t<float>(ctx, ctx->rho32.p, ctx->near32.p, ctx->leafL32.p, ctx->ip32.p, ctx->coef32.p, y, ev ? ev + 1 : nullptr);
+        far_ifgf_t<float>(ctx, ctx->rho32.p, ctx->near32.p, ctx->ip32.p, ctx->coef32.p, y, ev ? ev + 1 : nullptr);
     } else {
-        if (!rho_ready) launch_intensities_t<double>(x, wq, ctx->sorting.p, N, ctx->rho.p, ctx->stream);
+        if (!rho_ready) {
+            launch_intensities_t<double>(x, wq, ctx->sorting.p, N, ctx->rho.p, ctx->stream);
+            launch_rho_fx(ctx->leaf_start.p, ctx->leaf_count.p, (int)ctx->T.leaf_start.size(), ctx->rho.p, ctx->rhox.p, ctx->rexp.p,
+                          ctx->stream);
+        }
         if (ev) cudaEventRecord(ev[0], ctx->stream);
-        far_ifgf_t<double>(ctx, ctx->rho.p, ctx->near.p, ctx->leafL.p, ctx->ipx.p, ctx->coef.p, y, ev ? ev + 1 : nullptr);
+        far_ifgf_t<double>(ctx, ctx->rho.p, ctx->near.p, ctx->ipx.p, ctx->coef.p, y, ev ? ev + 1 : nullptr);
     }
     CK(cudaGetLastError());
     return IFGF2D_OK;
@@ -724,9 +743,13 @@ static int apply_dev(ifgf2d_ctx* ctx, const double2* x, double2* y, int mode) {
     if (mode != IFGF2D_APPLY_DIRECT && !ctx->ifgf_ready) return fail(ctx, IFGF2D_ERR_STATE, "setup before an IFGF apply");
     const double half = ctx->form == IFGF2D_COMBINED ? 0.5 : 0.0;
     if (mode != IFGF2D_APPLY_DIRECT) {
-        launch_sing_intens(x, ctx->W.p, ctx->srow_ptr.p, ctx->srow_col.p, ctx->cols.p, N, D.Np, half, y, ctx->wq.p,
-                           ctx->inverse.p, mode == IFGF2D_APPLY_IFGF_MIXED ? nullptr : ctx->rho.p,
-                           mode == IFGF2D_APPLY_IFGF_MIXED ? ctx->rho32.p : nullptr, ctx->stream);
+        if (mode == IFGF2D_APPLY_IFGF_MIXED)
+            launch_sing_intens(x, ctx->W.p, ctx->srow_ptr.p, ctx->srow_col.p, ctx->cols.p, N, D.Np, half, y, ctx->wq.p,
+                               ctx->inverse.p, nullptr, ctx->rho32.p, ctx->stream);
+        else
+            launch_sing_box(x, ctx->W.p, ctx->srow_ptr.p, ctx->srow_col.p, ctx->cols.p, D.Np, half, y, ctx->wq.p, ctx->leaf_start.p,
+                            ctx->leaf_count.p, (int)ctx->T.leaf_start.size(), ctx->sorting.p, ctx->rho.p, ctx->rhox.p, ctx->rexp.p,
+                            ctx->stream);
         return far_apply(ctx, x, ctx->wq.p, y, mode, nullptr, true);
     }
     launch_sing_intens(x, ctx->W.p, ctx->srow_ptr.p, ctx->srow_col.p, ctx->cols.p, N, D.Np, half, y, ctx->wq.p, nullptr,
@@ -807,10 +830,8 @@ extern "C" int ifgf2d_set_tuning(ifgf2d_ctx* ctx, const int* c) {
     return IFGF2D_OK;
 }
 template <typename R>
-static int tune_precision(ifgf2d_ctx* ctx, int reps, const V2<R>* rho, const V2<R>* leafL, CoefT<R>* coef) {
-    const Tree& T = ctx->T;
-    const int Dl = ctx->nlevels - 1, P = T.P, pr = sizeof(R) == 4 ? 1 : 0;
-    const TreeLevel& LD = T.L[Dl];
+static int tune_precision(ifgf2d_ctx* ctx, int reps, const V2<R>* rho, CoefT<R>* coef) {
+    const int Dl = ctx->nlevels - 1, pr = sizeof(R) == 4 ? 1 : 0;
     cudaStream_t s = ctx->stream;
     cudaEvent_t e0, e1;
     CK(cudaEventCreate(&e0)); CK(cudaEventCreate(&e1));
@@ -828,17 +849,7 @@ static int tune_precision(ifgf2d_ctx* ctx, int reps, const V2<R>* rho, const V2<
     float best = 1e30f; int bestc = 5;
     for (int ch : {1, 2, 5, 10, 0}) {   // 0: complex64 only, the table streamed by TMA bulk copies
         if (ch == 0 && sizeof(R) != 4) continue;
-        const float ms = time_it([&] {
-            bool done = false;
-            if constexpr (sizeof(R) == 4) {
-                if (ch == 0)
-                    done = launch_leaf_tma(ctx->leaf_cone_box.p, (int)LD.cone_nonrel.size(), LD.cone_base, ctx->leaf_start.p,
-                                           ctx->leaf_count.p, ctx->leaf_off.p, leafL, rho, P, coef, ctx->kerr.p, ctx->nsm, s);
-            }
-            if (!done)
-                launch_leaf_apply_t<R>(ctx->leaf_cone_box.p, (int)LD.cone_nonrel.size(), LD.cone_base, ctx->leaf_start.p,
-                                       ctx->leaf_count.p, ctx->leaf_off.p, leafL, rho, P, T.Ps, coef, ctx->cexp.p, s, ch);
-        });
+        const float ms = time_it([&] { launch_leaf<R>(ctx, coef, ch); });
         if (ms < best) { best = ms; bestc = ch; }
     }
     ctx->tune_leaf[pr] = bestc;
@@ -874,8 +885,8 @@ extern "C" int ifgf2d_autotune(ifgf2d_ctx* ctx, int reps, int* choices) {
     int rc;
     if ((rc = apply_dev(ctx, ctx->vin.p, ctx->vout.p, IFGF2D_APPLY_IFGF))) return rc;
     if ((rc = apply_dev(ctx, ctx->vin.p, ctx->vout.p, IFGF2D_APPLY_IFGF_MIXED))) return rc;
-    if ((rc = tune_precision<double>(ctx, reps, ctx->rho.p, ctx->leafL.p, ctx->coef.p))) return rc;
-    if ((rc = tune_precision<float>(ctx, reps, ctx->rho32.p, ctx->leafL32.p, ctx->coef32.p))) return rc;
+    if ((rc = tune_precision<double>(ctx, reps, ctx->rho.p, ctx->coef.p))) return rc;
+    if ((rc = tune_precision<float>(ctx, reps, ctx->rho32.p, ctx->coef32.p))) return rc;
     CK(cudaStreamSynchronize(ctx->stream));
     if (ctx->gw) ctx->gw->drop_graphs();
     if (choices) write_tuning(ctx, choices);

@@ -99,6 +99,11 @@ void launch_sing_apply(const double2* x, const double2* W, const int* row_ptr, c
 void launch_sing_intens(const double2* x, const double2* W, const int* row_ptr, const int* row_col,
                         const RPColumn* cols, int N, int Np, double half, double2* y, const double* wq,
                         const long long* inv, double2* rho64, float2* rho32, cudaStream_t s);
+// the FP64 form leaf box by leaf box, which also writes the intensities in Morton order: rho in FP64,
+// rhox as fixed-point limbs with one exponent per box (fixpoint.cuh)
+void launch_sing_box(const double2* x, const double2* W, const int* row_ptr, const int* row_col, const RPColumn* cols, int Np,
+                     double half, double2* y, const double* wq, const int* leaf_start, const int* leaf_count, int nleaf,
+                     const long long* sorting, double2* rho, int4* rhox, int* rexp, cudaStream_t s);
 // sources with unit normals snx, sny (NULL for the single layer); form 0 single layer, 2 combined
 void launch_direct_far(const double* tx, const double* ty, int ntarget, const int* t_patch, const int* t_nsp_ptr,
                        const int* t_nsp, const double* sx, const double* sy, const double* snx, const double* sny,
@@ -108,10 +113,18 @@ void launch_direct_far(const double* tx, const double* ty, int ntarget, const in
 // precision-templated IFGF apply (ifgf_apply.cu); R = double (plain) or float (mixed)
 template <typename R>
 void launch_intensities_t(const double2* x, const double* wq, const long long* perm, int N, V2<R>* rho, cudaStream_t s);
-template <typename R>
 void launch_leaf_apply_t(const int* cone_box, int ncones, int cone_base, const int* leaf_start, const int* leaf_count,
-                         const long long* leaf_off, const V2<R>* L, const V2<R>* rho, int P, int Ps, CoefT<R>* coef, int* cexp,
-                         cudaStream_t s, int chunks = 5);
+                         const long long* leaf_off, const float2* L, const float2* rho, int P, float2* coef, cudaStream_t s,
+                         int chunks = 5);
+// the FP64 form in fixed point (fixpoint.cuh): the table and its exponents [cone][coefficient] from
+// launch_leaf_fix (in place of the FP64 table; l32, when not null, receives the complex64 copy), the
+// densities and their exponents per leaf box from launch_rho_fx or launch_sing_box
+void launch_leaf_fx(const int* cone_box, int ncones, int cone_base, const int* leaf_start, const int* leaf_count,
+                    const long long* leaf_off, const int4* L, const int* lexp, const int4* rho, const int* rexp, int P, int Ps,
+                    int4* coef, int* cexp, cudaStream_t s, int chunks = 5);
+void launch_leaf_fix(const int* cone_box, int ncones, const int* leaf_count, const long long* leaf_off, int P, int4* L, int* lexp,
+                     float2* l32, cudaStream_t s);
+void launch_rho_fx(const int* leaf_start, const int* leaf_count, int nleaf, const double2* rho, int4* out, int* rexp, cudaStream_t s);
 // complex64 leaf cones with the table streamed through shared memory by TMA bulk copies
 // (P = 25); false when not launched (other P, or leaf_tma_init not run).  *err is set when a
 // completion wait runs out.  leaf_tma_init sets the kernel's shared-memory attribute (outside
@@ -187,10 +200,15 @@ void launch_deinterleave(const double2* xt, long long N, int B, double2* x, cuda
 void launch_sing_b(const double2* xt, const float2* xt32, const double2* W, const float2* W32, const int* row_ptr,
                    const int* row_col, const RPColumn* cols, int N, int Np, int B, double half, double2* yt,
                    const double* wq, const long long* inv, double2* rho64, float2* rho32, cudaStream_t s);
-template <typename R>
 void launch_leaf_b(const int* cone_box, int ncones, int cone_base, const int* leaf_start, const int* leaf_count,
-                   const long long* leaf_off, const V2<R>* L, const V2<R>* rho, int Ps, int Pang, int B, CoefT<R>* coef,
-                   int* cexp, cudaStream_t s);
+                   const long long* leaf_off, const float2* L, const float2* rho, int Ps, int Pang, int B, float2* coef,
+                   cudaStream_t s);
+// the FP64 form in fixed point: table as launch_leaf_fx's, densities and exponents [box][B] from launch_rho_bx
+void launch_rho_bx(const int* leaf_start, const int* leaf_count, int nleaf, const double2* rho, int B, int4* out, int* rexp,
+                   cudaStream_t s);
+void launch_leaf_bx(const int* cone_box, int ncones, int cone_base, const int* leaf_start, const int* leaf_count,
+                    const long long* leaf_off, const int4* L, const int* lexp, const int4* rho, const int* rexp, int Ps, int Pang, int B,
+                    int4* coef, int* cexp, cudaStream_t s);
 void launch_prop_b(int pbegin, int pend, const long long* pp_ptr, const int* pp_nchild, const PropB<float>* pb, int Ps, int Pang,
                    const float* Gsep, int B, float2* coef, cudaStream_t s);
 // the FP64 form in fixed point (fixpoint.cuh): coefficients [cone][P][B] as limbs with one exponent per

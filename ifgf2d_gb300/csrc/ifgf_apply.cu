@@ -35,53 +35,149 @@ __global__ void k_intensities_t(const double2* __restrict__ x, const double* __r
 // chunk ch takes the sources s = ch, ch + CH, ...; the CH partial sums meet in shared memory.
 // Boxes hold 10-100 points, so splitting the source walk shortens the latency chain of the
 // longest boxes by CH.
-template <typename R, int CH>
+template <int CH>
 __global__ void __launch_bounds__(256) k_leaf_apply_t(const int* __restrict__ cone_box, int ncones, int cone_base,
                                                       const int* __restrict__ leaf_start, const int* __restrict__ leaf_count,
-                                                      const long long* __restrict__ leaf_off, const V2<R>* __restrict__ L,
-                                                      const V2<R>* __restrict__ rho, int P, int Ps, CoefT<R>* __restrict__ coef,
-                                                      int* __restrict__ cexp) {
-    __shared__ V2<R> part[256];
-    __shared__ int smax[256];               // FP64: per cone, the largest high word of its coefficients
-    if constexpr (sizeof(R) == 8) smax[threadIdx.x] = 0;
+                                                      const long long* __restrict__ leaf_off, const float2* __restrict__ L,
+                                                      const float2* __restrict__ rho, int P, float2* __restrict__ coef) {
+    __shared__ float2 part[256];
     const int per_cone = P * CH;
     const int cpb = blockDim.x / per_cone;
     const int local = threadIdx.x / per_cone, r = threadIdx.x - local * per_cone;
     const int ch = r / P, m = r - ch * P;
     const int c = blockIdx.x * cpb + local;
     const bool active = local < cpb && c < ncones;
-    V2<R> a0, a1;
-    a0.x = a0.y = a1.x = a1.y = R(0);
+    float2 a0 = make_float2(0.f, 0.f), a1 = a0;
     if (active) {
         const int b = cone_box[c];
         const int n = leaf_count[b], s0 = leaf_start[b];
-        const V2<R>* Lc = L + leaf_off[c] + m;
-        const V2<R>* rh = rho + s0;
+        const float2* Lc = L + leaf_off[c] + m;
+        const float2* rh = rho + s0;
         int s = ch;
         for (; s + CH < n; s += 2 * CH) {
-            const V2<R> l0 = Lc[(long long)s * P], l1 = Lc[(long long)(s + CH) * P];
-            const V2<R> r0 = rh[s], r1 = rh[s + CH];
-            cmac<R>(a0, l0, r0); cmac<R>(a1, l1, r1);
+            const float2 l0 = Lc[(long long)s * P], l1 = Lc[(long long)(s + CH) * P];
+            const float2 r0 = rh[s], r1 = rh[s + CH];
+            cmac<float>(a0, l0, r0); cmac<float>(a1, l1, r1);
         }
-        if (s < n) cmac<R>(a0, Lc[(long long)s * P], rh[s]);
+        if (s < n) cmac<float>(a0, Lc[(long long)s * P], rh[s]);
         a0.x += a1.x; a0.y += a1.y;
     }
     part[threadIdx.x] = a0;
     __syncthreads();
-    V2<R> acc = a0;
-    if (active && ch == 0)
-        for (int q = 1; q < CH; ++q) { const V2<R> v = part[local * per_cone + q * P + m]; acc.x += v.x; acc.y += v.y; }
-    if constexpr (sizeof(R) == 8) {
-        if (active && ch == 0) atomicMax(&smax[local], fx_absmax_hi(acc.x, acc.y));
-        __syncthreads();
-        if (active && ch == 0) {
-            const int E = fx_expo(smax[local]), T = fx_top(P);
-            const long long xr = E == kFxBad ? 0 : fx_from(acc.x, E, T), xi = E == kFxBad ? 0 : fx_from(acc.y, E, T);
-            coef[(long long)(cone_base + c) * P + m] = m % Ps ? fx_pack(xr, xi) : fx_pack_raw(xr, xi);
-            if (m == 0) cexp[cone_base + c] = E;
+    if (active && ch == 0) {
+        float2 acc = a0;
+        for (int q = 1; q < CH; ++q) { const float2 v = part[local * per_cone + q * P + m]; acc.x += v.x; acc.y += v.y; }
+        coef[(long long)(cone_base + c) * P + m] = acc;
+    }
+}
+
+// The FP64 form of the same in fixed point (fixpoint.cuh): table and densities as 27-bit limbs, 12 wide
+// multiply-adds an entry where FP64 took 4 of the FP64 pipe's operations.  The kernel streams the table
+// from HBM (16 bytes an entry); kite k = 500 91 -> 55 us, k = 2000 582 -> 291 us (4.1 TB/s; the FP64
+// kernel before it ran at 93 % of the FP64 pipe).  The chunks' integer sums meet in shared memory; then the cone's
+// coefficients, whose entries have an exponent per coefficient, are brought to the cone's exponent.
+template <int CH>
+__global__ void __launch_bounds__(256) k_leaf_fx(const int* __restrict__ cone_box, int ncones, int cone_base,
+                                                 const int* __restrict__ leaf_start, const int* __restrict__ leaf_count,
+                                                 const long long* __restrict__ leaf_off, const int4* __restrict__ L,
+                                                 const int* __restrict__ lexp, const int4* __restrict__ rho,
+                                                 const int* __restrict__ rexp, int P, int Ps, int4* __restrict__ coef,
+                                                 int* __restrict__ cexp) {
+    __shared__ FxSum part[CH > 1 ? 256 : 1][2];
+    __shared__ int stop[256];
+    stop[threadIdx.x] = kFxMinExp;
+    const int per_cone = P * CH;
+    const int cpb = blockDim.x / per_cone;
+    const int local = threadIdx.x / per_cone, r = threadIdx.x - local * per_cone;
+    const int ch = r / P, m = r - ch * P;
+    const int c = blockIdx.x * cpb + local;
+    const bool active = local < cpb && c < ncones;
+    FxSum rr{0, 0}, ii{0, 0}, im{0, 0};
+    int n = 0, Er = 0, El = 0;
+    if (active) {
+        const int b = cone_box[c];
+        n = leaf_count[b];
+        Er = rexp[b];
+        El = lexp[(long long)c * P + m];
+        const int4* Lc = L + leaf_off[c] + m;
+        const int4* rh = rho + leaf_start[b];
+        for (int f0 = ch; f0 < n; f0 += kFxSumFold * CH) {
+            const int f1 = min(n, f0 + kFxSumFold * CH);
+#pragma unroll 4
+            for (int s = f0; s < f1; s += CH) {
+                const int4 l = Lc[(long long)s * P], d = rh[s];
+                fx_sum_mac(rr, l.x, l.y, d.x, d.y);
+                fx_sum_mac(ii, l.z, l.w, d.z, d.w);
+                fx_sum_mac(im, l.x, l.y, d.z, d.w);
+                fx_sum_mac(im, l.z, l.w, d.x, d.y);
+            }
+            fx_sum_fold(rr); fx_sum_fold(ii); fx_sum_fold(im);
         }
-    } else {
-        if (active && ch == 0) coef[(long long)(cone_base + c) * P + m] = acc;
+    }
+    FxSum re{rr.h - ii.h, rr.m - ii.m};
+    if constexpr (CH > 1) {
+        part[threadIdx.x][0] = re; part[threadIdx.x][1] = im;
+        __syncthreads();
+        if (active && ch == 0)
+            for (int q = 1; q < CH; ++q) {
+                const FxSum a = part[local * per_cone + q * P + m][0], b = part[local * per_cone + q * P + m][1];
+                re.h += a.h; re.m += a.m; im.h += b.h; im.m += b.m;
+            }
+    }
+    fx_sum_fold(re); fx_sum_fold(im);
+    const bool bad = Er == kFxBad || El == kFxBad;
+    int er = 0, ei = 0;
+    const int E0 = bad ? 0 : El + Er - kFxSumTop - fx_rho_top(n);
+    const long long yr = fx_sum_value(re, E0, er), yi = fx_sum_value(im, E0, ei);
+    __syncthreads();
+    if (active && ch == 0) atomicMax(&stop[local], bad ? kFxBad : max(fx_top_of(yr, er), fx_top_of(yi, ei)));
+    __syncthreads();
+    if (active && ch == 0) {
+        const int E = stop[local] > kFxMaxExp ? kFxBad : stop[local], T = fx_top(P);
+        const long long xr = E == kFxBad ? 0 : fx_align(yr, er, E, T), xi = E == kFxBad ? 0 : fx_align(yi, ei, E, T);
+        coef[(long long)(cone_base + c) * P + m] = m % Ps ? fx_pack(xr, xi) : fx_pack_raw(xr, xi);
+        if (m == 0) cexp[cone_base + c] = E;
+    }
+}
+
+// set-up: a leaf cone's FP64 table in place as 27-bit limbs, an exponent per coefficient; l32 (may be
+// null) receives the complex64 copy
+__global__ void __launch_bounds__(256) k_leaf_fix(const int* __restrict__ cone_box, const int* __restrict__ leaf_count,
+                                                  const long long* __restrict__ leaf_off, int P, double2* __restrict__ L,
+                                                  int* __restrict__ lexp, float2* __restrict__ l32) {
+    __shared__ int smax[kMaxP];
+    const int c = blockIdx.x;
+    const long long o = leaf_off[c];
+    const int n = leaf_count[cone_box[c]] * P;
+    for (int m = threadIdx.x; m < P; m += blockDim.x) smax[m] = 0;
+    __syncthreads();
+    for (int i = threadIdx.x; i < n; i += blockDim.x) { const double2 v = L[o + i]; atomicMax(&smax[i % P], fx_absmax_hi(v.x, v.y)); }
+    __syncthreads();
+    for (int m = threadIdx.x; m < P; m += blockDim.x) lexp[(long long)c * P + m] = fx_expo(smax[m]);
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        const double2 v = L[o + i];
+        const int E = fx_expo(smax[i % P]);
+        if (l32) l32[o + i] = make_float2((float)v.x, (float)v.y);
+        reinterpret_cast<int4*>(L)[o + i] =
+            E == kFxBad ? make_int4(0, 0, 0, 0) : fx_pack_sum(fx_from(v.x, E, kFxSumTop), fx_from(v.y, E, kFxSumTop));
+    }
+}
+// the densities of a leaf box as limbs, one exponent per box (a block per box)
+__global__ void __launch_bounds__(64) k_rho_fx(const int* __restrict__ leaf_start, const int* __restrict__ leaf_count,
+                                               const double2* __restrict__ rho, int4* __restrict__ out, int* __restrict__ rexp) {
+    __shared__ int smax;
+    const int b = blockIdx.x, s0 = leaf_start[b], n = leaf_count[b], T = fx_rho_top(n);
+    if (threadIdx.x == 0) smax = 0;
+    __syncthreads();
+    int mx = 0;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) { const double2 v = rho[s0 + i]; mx = max(mx, fx_absmax_hi(v.x, v.y)); }
+    atomicMax(&smax, mx);
+    __syncthreads();
+    const int E = fx_expo(smax);
+    if (threadIdx.x == 0) rexp[b] = E;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        const double2 v = rho[s0 + i];
+        out[s0 + i] = E == kFxBad ? make_int4(0, 0, 0, 0) : fx_pack_sum(fx_from(v.x, E, T), fx_from(v.y, E, T));
     }
 }
 
@@ -750,22 +846,41 @@ cudaError_t preload_intensities_kernel() {
     cudaFuncAttributes a;
     return cudaFuncGetAttributes(&a, k_intensities_t<double>);
 }
-template <typename R>
-void launch_leaf_apply_t(const int* cone_box, int ncones, int cone_base, const int* leaf_start, const int* leaf_count,
-                         const long long* leaf_off, const V2<R>* L, const V2<R>* rho, int P, int Ps, CoefT<R>* coef, int* cexp,
-                         cudaStream_t s, int chunks) {
-    if (ncones <= 0) return;
-    // chunks per coefficient (the tuning variant): 1, 2, 5 or 10; a block holds 256 / (P * CH) cones
-    auto go = [&](auto ch_tag) {
-        constexpr int CH = decltype(ch_tag)::value;
-        const int cpb = 256 / (P * CH);
-        k_leaf_apply_t<R, CH><<<nblk_a(ncones, cpb), cpb * P * CH, 0, s>>>(cone_box, ncones, cone_base, leaf_start, leaf_count,
-                                                                          leaf_off, L, rho, P, Ps, coef, cexp);
-    };
+// chunks per coefficient (the tuning variant): 1, 2, 5 or 10; a block holds 256 / (P * CH) cones
+template <typename Go>
+static void leaf_chunks(int P, int chunks, Go&& go) {
     if (chunks == 10 && 256 / (P * 10) >= 1) go(std::integral_constant<int, 10>{});
     else if (chunks == 2 && 256 / (P * 2) >= 1) go(std::integral_constant<int, 2>{});
     else if (chunks == 1 || 256 / (P * 5) < 1) go(std::integral_constant<int, 1>{});
     else go(std::integral_constant<int, 5>{});
+}
+void launch_leaf_apply_t(const int* cone_box, int ncones, int cone_base, const int* leaf_start, const int* leaf_count,
+                         const long long* leaf_off, const float2* L, const float2* rho, int P, float2* coef, cudaStream_t s, int chunks) {
+    if (ncones <= 0) return;
+    leaf_chunks(P, chunks, [&](auto tag) {
+        constexpr int CH = decltype(tag)::value;
+        const int cpb = 256 / (P * CH);
+        k_leaf_apply_t<CH><<<nblk_a(ncones, cpb), cpb * P * CH, 0, s>>>(cone_box, ncones, cone_base, leaf_start, leaf_count, leaf_off, L,
+                                                                       rho, P, coef);
+    });
+}
+void launch_leaf_fx(const int* cone_box, int ncones, int cone_base, const int* leaf_start, const int* leaf_count,
+                    const long long* leaf_off, const int4* L, const int* lexp, const int4* rho, const int* rexp, int P, int Ps,
+                    int4* coef, int* cexp, cudaStream_t s, int chunks) {
+    if (ncones <= 0) return;
+    leaf_chunks(P, chunks, [&](auto tag) {
+        constexpr int CH = decltype(tag)::value;
+        const int cpb = 256 / (P * CH);
+        k_leaf_fx<CH><<<nblk_a(ncones, cpb), cpb * P * CH, 0, s>>>(cone_box, ncones, cone_base, leaf_start, leaf_count, leaf_off, L, lexp,
+                                                                  rho, rexp, P, Ps, coef, cexp);
+    });
+}
+void launch_leaf_fix(const int* cone_box, int ncones, const int* leaf_count, const long long* leaf_off, int P, int4* L, int* lexp,
+                     float2* l32, cudaStream_t s) {
+    if (ncones > 0) k_leaf_fix<<<ncones, 256, 0, s>>>(cone_box, leaf_count, leaf_off, P, reinterpret_cast<double2*>(L), lexp, l32);
+}
+void launch_rho_fx(const int* leaf_start, const int* leaf_count, int nleaf, const double2* rho, int4* out, int* rexp, cudaStream_t s) {
+    if (nleaf > 0) k_rho_fx<<<nleaf, 64, 0, s>>>(leaf_start, leaf_count, rho, out, rexp);
 }
 static std::atomic<int> g_leaf_tma_ready{0};
 cudaError_t leaf_tma_init() {
@@ -861,8 +976,6 @@ void launch_d2f(const double2* a, long long n, float2* b, cudaStream_t s) {
 
 #define IFGF_INSTANTIATE(R)                                                                                          \
     template void launch_intensities_t<R>(const double2*, const double*, const long long*, int, V2<R>*, cudaStream_t); \
-    template void launch_leaf_apply_t<R>(const int*, int, int, const int*, const int*, const long long*, const V2<R>*,  \
-                                         const V2<R>*, int, int, CoefT<R>*, int*, cudaStream_t, int);                       \
     template void launch_final_t<R>(int, const int*, const int*, const int*, const int*, const int*,                   \
                                     const long long*, const V2<R>*, const V2<R>*, const int*, const InterpT<R>*,       \
                                     const CoefT<R>*, const int*, int, int, const long long*, double2*, cudaStream_t,   \

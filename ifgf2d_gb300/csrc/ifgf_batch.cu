@@ -11,6 +11,7 @@
 //              (FP32 weights in the mixed form)
 //   k_leaf_b   leaf cone coefficients, table rows staged in shared
 //              memory by cp.async, 25 accumulators per RHS          BoxTree.h:685-762
+//   k_leaf_bx  the same in fixed point (FP64 form, fixpoint.cuh)
 //   k_prop_b   child -> parent, per parent cone one warp; the
 //              parent's terms sorted by child cone so each child
 //              cone's coefficients are loaded once                 BoxTree.h:767-868, Interpolator.h:81-120
@@ -129,18 +130,19 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 template <typename R> struct Rpl { static constexpr int v = sizeof(R) == 4 ? 2 : 1; };
 
 // ------------------------------------------------------------------ leaf cones
-// warp = one leaf cone x 32*RPL right-hand sides, P accumulators per (lane, RHS).  The cone's
+// complex64: warp = one leaf cone x 32*RPL right-hand sides, P accumulators per (lane, RHS).  The cone's
 // table rows stream through shared memory in tiles of TS sources (cp.async, double-buffered)
 // and every lane reads them as broadcasts; densities are prefetched one source ahead.
 constexpr int kLeafWarps = 4;
-template <typename R, int P, int RPL>
+template <int P, int RPL>
 __global__ void __launch_bounds__(kLeafWarps * 32) k_leaf_b(const int* __restrict__ cone_box, int ncones, int cone_base,
                                                             const int* __restrict__ leaf_start,
                                                             const int* __restrict__ leaf_count,
                                                             const long long* __restrict__ leaf_off,
-                                                            const V2<R>* __restrict__ L, const V2<R>* __restrict__ rho, int B,
-                                                            int Ps, CoefT<R>* __restrict__ coef, int* __restrict__ cexp) {
-    constexpr int TS = sizeof(R) == 4 ? 16 : 8;
+                                                            const float2* __restrict__ L, const float2* __restrict__ rho, int B,
+                                                            float2* __restrict__ coef) {
+    using R = float;
+    constexpr int TS = 16;
     __shared__ V2<R> tile[kLeafWarps][2][TS * P];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int c = blockIdx.x * kLeafWarps + w;
@@ -202,23 +204,119 @@ __global__ void __launch_bounds__(kLeafWarps * 32) k_leaf_b(const int* __restric
 #pragma unroll
     for (int k = 0; k < RPL; ++k) {
         if (!act[k]) continue;
-        CoefT<R>* out = coef + (long long)(cone_base + c) * P * B + rr[k];
-        if constexpr (sizeof(R) == 8) {      // the block's common exponent, and fixed-point limbs
-            int mx = 0;
+        float2* out = coef + (long long)(cone_base + c) * P * B + rr[k];
 #pragma unroll
-            for (int m = 0; m < P; ++m) mx = max(mx, fx_absmax_hi(acc[k][m].x, acc[k][m].y));
-            const int E = fx_expo(mx), T = fx_top(P);
-#pragma unroll
-            for (int m = 0; m < P; ++m) {
-                const long long a = E == kFxBad ? 0 : fx_from(acc[k][m].x, E, T), b = E == kFxBad ? 0 : fx_from(acc[k][m].y, E, T);
-                out[(long long)m * B] = m % Ps ? fx_pack(a, b) : fx_pack_raw(a, b);
-            }
-            cexp[(long long)(cone_base + c) * B + rr[k]] = E;
-        } else {
-#pragma unroll
-            for (int m = 0; m < P; ++m) out[(long long)m * B] = acc[k][m];
-        }
+        for (int m = 0; m < P; ++m) out[(long long)m * B] = acc[k][m];
     }
+}
+
+// FP64 in fixed point (fixpoint.cuh): the densities of a leaf box as limbs with one exponent per box and
+// right-hand side (a block per box, a thread per right-hand side)
+__global__ void k_rho_bx(const int* __restrict__ leaf_start, const int* __restrict__ leaf_count, const double2* __restrict__ rho, int B,
+                         int4* __restrict__ out, int* __restrict__ rexp) {
+    const int b = blockIdx.x, r = threadIdx.x;
+    if (r >= B) return;
+    const int n = leaf_count[b], T = fx_rho_top(n);
+    const long long s0 = leaf_start[b];
+    int mx = 0;
+    for (int i = 0; i < n; ++i) { const double2 v = rho[(s0 + i) * B + r]; mx = max(mx, fx_absmax_hi(v.x, v.y)); }
+    const int E = fx_expo(mx);
+    rexp[(long long)b * B + r] = E;
+    for (int i = 0; i < n; ++i) {
+        const double2 v = rho[(s0 + i) * B + r];
+        out[(s0 + i) * B + r] = E == kFxBad ? make_int4(0, 0, 0, 0) : fx_pack_sum(fx_from(v.x, E, T), fx_from(v.y, E, T));
+    }
+}
+// block = one leaf cone x NT right-hand sides x MS parts of the coefficients (blockDim.y), PM
+// coefficients a thread: their integer sums (eight registers each) stay in registers.  The table streams
+// through shared memory kLeafBxTile sources at a time (cp.async, double-buffered), read as broadcasts.
+// Bound by the wide multiply-adds (12 an entry); kite k = 500, 64 right-hand sides 4.0 -> 1.2 ms.
+constexpr int kLeafBxTile = 8;
+template <int P, int MS, int NT>
+__global__ void __launch_bounds__(NT * MS) k_leaf_bx(const int* __restrict__ cone_box, int cone_base, const int* __restrict__ leaf_start,
+                                                     const int* __restrict__ leaf_count, const long long* __restrict__ leaf_off,
+                                                     const int4* __restrict__ L, const int* __restrict__ lexp,
+                                                     const int4* __restrict__ rho, const int* __restrict__ rexp, int B, int Ps,
+                                                     int4* __restrict__ coef, int* __restrict__ cexp) {
+    constexpr int PM = (P + MS - 1) / MS, TS = kLeafBxTile;
+    static_assert(kFxSumFold % TS == 0, "folds between tiles");
+    __shared__ int4 tile[2][TS * P];
+    __shared__ int stop[NT];
+    const int c = blockIdx.x, lt = threadIdx.x, part = threadIdx.y, tid = part * NT + lt;
+    const int r = blockIdx.y * NT + lt;
+    const bool act = r < B;
+    const int rr = act ? r : 0;
+    const int b = cone_box[c], n = leaf_count[b];
+    const int4* Lc = L + leaf_off[c];
+    if (part == 0) stop[lt] = kFxMinExp;
+    auto load_tile = [&](int t) {
+        const int cnt = min(TS, n - t * TS) * P;
+        for (int q = tid; q < cnt; q += NT * MS) cp_async_el<16>(&tile[t & 1][q], Lc + (long long)t * TS * P + q);
+        cp_async_commit();
+    };
+    FxSum re[PM], im[PM];
+#pragma unroll
+    for (int m = 0; m < PM; ++m) re[m] = im[m] = FxSum{0, 0};
+    const int4* rh = rho + (long long)leaf_start[b] * B + rr;
+    const int nt = (n + TS - 1) / TS;
+    int4 dn = n > 0 ? rh[0] : make_int4(0, 0, 0, 0);
+    if (nt > 0) load_tile(0);
+    for (int t = 0; t < nt; ++t) {
+        if (t + 1 < nt) { load_tile(t + 1); cp_async_wait<1>(); }
+        else cp_async_wait<0>();
+        __syncthreads();
+        const int4* Lt = tile[t & 1] + part * PM;
+        const int cnt = min(TS, n - t * TS);
+        for (int s = 0; s < cnt; ++s) {
+            const int4 d = dn;
+            if (t * TS + s + 1 < n) dn = rh[(long long)(t * TS + s + 1) * B];
+            const int nh = -d.z, nl = -d.w;
+#pragma unroll
+            for (int m = 0; m < PM; ++m) {
+                if (P % MS && part * PM + m >= P) break;
+                const int4 l = Lt[s * P + m];
+                fx_sum_mac(re[m], l.x, l.y, d.x, d.y);
+                fx_sum_mac(re[m], l.z, l.w, nh, nl);
+                fx_sum_mac(im[m], l.x, l.y, d.z, d.w);
+                fx_sum_mac(im[m], l.z, l.w, d.x, d.y);
+            }
+        }
+        if ((t + 1) % (kFxSumFold / TS) == 0 || t + 1 == nt)
+#pragma unroll
+            for (int m = 0; m < PM; ++m) { fx_sum_fold(re[m]); fx_sum_fold(im[m]); }
+        __syncthreads();                        // the buffer is refilled two tiles later
+    }
+    const int Er = rexp[(long long)b * B + rr], T = fx_top(P);
+    int top = kFxMinExp;                        // the sums in place as y = .h, e = .m of y 2^e
+#pragma unroll
+    for (int m = 0; m < PM; ++m) {
+        const int q = part * PM + m;
+        if (q >= P) continue;
+        const int El = lexp[(long long)c * P + q];
+        if (Er == kFxBad || El == kFxBad) { top = kFxBad; continue; }
+        const int E0 = El + Er - kFxSumTop - fx_rho_top(n);
+        int ea, eb;
+        const long long ya = fx_sum_value(re[m], E0, ea), yb = fx_sum_value(im[m], E0, eb);
+        re[m].h = ya; im[m].h = yb; re[m].m = ea; im[m].m = eb;
+        top = max(top, max(fx_top_of(ya, ea), fx_top_of(yb, eb)));
+    }
+    if (MS > 1) {
+        if (nt == 0) __syncthreads();
+        atomicMax(&stop[lt], top);
+        __syncthreads();
+        top = stop[lt];
+    }
+    if (!act) return;
+    const int E = top > kFxMaxExp ? kFxBad : top;
+    int4* out = coef + (long long)(cone_base + c) * P * B + r;
+#pragma unroll
+    for (int m = 0; m < PM; ++m) {
+        const int q = part * PM + m;
+        if (q >= P) continue;
+        const long long xr = E == kFxBad ? 0 : fx_align(re[m].h, (int)re[m].m, E, T), xi = E == kFxBad ? 0 : fx_align(im[m].h, (int)im[m].m, E, T);
+        out[(long long)q * B] = q % Ps ? fx_pack(xr, xi) : fx_pack_raw(xr, xi);
+    }
+    if (part == 0) cexp[(long long)(cone_base + c) * B + r] = E;
 }
 
 // ------------------------------------------------------------------ propagation
@@ -820,15 +918,32 @@ void launch_sing_b(const double2* xt, const float2* xt32, const double2* W, cons
     else
         k_sing_b<double2, double2><<<grid, 256, 0, s>>>(xt, xt, W, row_ptr, row_col, cols, N, Np, B, half, yt, wq, inv, rho64);
 }
-template <typename R>
 void launch_leaf_b(const int* cone_box, int ncones, int cone_base, const int* leaf_start, const int* leaf_count,
-                   const long long* leaf_off, const V2<R>* L, const V2<R>* rho, int Ps, int Pang, int B, CoefT<R>* coef,
-                   int* cexp, cudaStream_t s) {
+                   const long long* leaf_off, const float2* L, const float2* rho, int Ps, int Pang, int B, float2* coef,
+                   cudaStream_t s) {
     if (ncones <= 0) return;
-    constexpr int RPL = Rpl<R>::v;
+    constexpr int RPL = Rpl<float>::v;
     const dim3 grid(nblk_b(ncones, kLeafWarps), nblk_b(B, 32 * RPL));
-    IFGF_DISPATCH_P(Ps, Pang, (k_leaf_b<R, PS * PA, RPL><<<grid, kLeafWarps * 32, 0, s>>>(
-                                   cone_box, ncones, cone_base, leaf_start, leaf_count, leaf_off, L, rho, B, PS, coef, cexp)));
+    IFGF_DISPATCH_P(Ps, Pang, (k_leaf_b<PS * PA, RPL><<<grid, kLeafWarps * 32, 0, s>>>(
+                                   cone_box, ncones, cone_base, leaf_start, leaf_count, leaf_off, L, rho, B, coef)));
+}
+void launch_rho_bx(const int* leaf_start, const int* leaf_count, int nleaf, const double2* rho, int B, int4* out, int* rexp,
+                   cudaStream_t s) {
+    if (nleaf > 0 && B > 0) k_rho_bx<<<nleaf, (B + 31) / 32 * 32, 0, s>>>(leaf_start, leaf_count, rho, B, out, rexp);
+}
+void launch_leaf_bx(const int* cone_box, int ncones, int cone_base, const int* leaf_start, const int* leaf_count,
+                    const long long* leaf_off, const int4* L, const int* lexp, const int4* rho, const int* rexp, int Ps, int Pang, int B,
+                    int4* coef, int* cexp, cudaStream_t s) {
+    if (ncones <= 0 || B <= 0) return;
+    IFGF_DISPATCH_P(Ps, Pang, {
+        constexpr int P = PS * PA, MS = (P + 12) / 13;   // at most 13 coefficients (104 registers of sums) a thread
+        if (B <= 32)
+            k_leaf_bx<P, MS, 32><<<dim3(ncones, 1), dim3(32, MS), 0, s>>>(cone_box, cone_base, leaf_start, leaf_count, leaf_off, L, lexp,
+                                                                         rho, rexp, B, Ps, coef, cexp);
+        else
+            k_leaf_bx<P, MS, 64><<<dim3(ncones, nblk_b(B, 64)), dim3(64, MS), 0, s>>>(cone_box, cone_base, leaf_start, leaf_count, leaf_off,
+                                                                                     L, lexp, rho, rexp, B, Ps, coef, cexp);
+    });
 }
 void launch_prop_b(int pbegin, int pend, const long long* pp_ptr, const int* pp_nchild, const PropB<float>* pb, int Ps, int Pang,
                    const float* Gsep, int B, float2* coef, cudaStream_t s) {
@@ -905,8 +1020,6 @@ void launch_bscale(const double2* w, const double2* hn, long long N, int B, doub
 }
 
 #define IFGF_BATCH_INSTANTIATE(R)                                                                                       \
-    template void launch_leaf_b<R>(const int*, int, int, const int*, const int*, const long long*, const V2<R>*,        \
-                                   const V2<R>*, int, int, int, CoefT<R>*, int*, cudaStream_t);                         \
     template void launch_final_b<R>(int, const int*, const int*, const int*, const int*, const int*, const int*,        \
                                     const long long*, const V2<R>*, const V2<R>*, const int*, const InterpE<R>*,        \
                                     const V2<R>*, int, int, const long long*, int, double2*, cudaStream_t);

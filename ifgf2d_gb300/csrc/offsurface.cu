@@ -18,7 +18,8 @@ struct EvalWork {
     DBuf<int> leaf_cone_box;
     DBuf<long long> leaf_off;
     DBuf<LeafNode> nodes;
-    DBuf<double2> leafL;
+    DBuf<int4> leafL;
+    DBuf<int> lexp;
     DBuf<long long> pp_ptr;
     DBuf<int> pp_nchild;
     PlanBuf pp;
@@ -117,7 +118,9 @@ extern "C" int ifgf2d_eval_offsurface_setup(ifgf2d_ctx* ctx, long long m, const 
         CK(W.leafL.alloc(loff[ncl]));
         launch_leaf_setup(W.leaf_cone_box.p, ncl, ctx->leaf_start.p, ctx->leaf_count.p, W.leaf_off.p, W.nodes.p, ctx->xs_s.p,
                           ctx->ys_s.p, ctx->nxs_s.p, ctx->nys_s.p, ctx->T.Ps, ctx->T.Pang, ctx->k, ctx->form, ctx->eta, ctx->Gsep.p,
-                          W.leafL.p, s);
+                          reinterpret_cast<double2*>(W.leafL.p), s);
+        CK(W.lexp.alloc((size_t)ncl * P));
+        launch_leaf_fix(W.leaf_cone_box.p, ncl, ctx->leaf_count.p, W.leaf_off.p, P, W.leafL.p, W.lexp.p, nullptr, s);
         CK(cudaGetLastError());
     }
     static_assert(sizeof(InterpEntry) == sizeof(InterpEntryD), "host and device plan layouts differ");
@@ -164,8 +167,9 @@ extern "C" int ifgf2d_eval_offsurface(ifgf2d_ctx* ctx, const double* density, do
     CK(cudaMemcpyAsync(ctx->vin.p, density, sizeof(double2) * N, cudaMemcpyHostToDevice, s));
     launch_intensities(ctx->vin.p, ctx->wq.p, ctx->sorting.p, N, ctx->rho.p, s);
     const TreeLevel& LD = E.L[D];
-    launch_leaf_apply_t<double>(W.leaf_cone_box.p, (int)LD.cone_nonrel.size(), LD.cone_base, ctx->leaf_start.p, ctx->leaf_count.p,
-                                W.leaf_off.p, W.leafL.p, ctx->rho.p, P, E.Ps, W.coef.p, W.cexp.p, s);
+    launch_rho_fx(ctx->leaf_start.p, ctx->leaf_count.p, (int)ctx->T.leaf_start.size(), ctx->rho.p, ctx->rhox.p, ctx->rexp.p, s);
+    launch_leaf_fx(W.leaf_cone_box.p, (int)LD.cone_nonrel.size(), LD.cone_base, ctx->leaf_start.p, ctx->leaf_count.p, W.leaf_off.p,
+                   W.leafL.p, W.lexp.p, ctx->rhox.p, ctx->rexp.p, P, E.Ps, W.coef.p, W.cexp.p, s);
     for (int l = D; l >= 3; --l) {
         const TreeLevel& Lp = E.L[l - 1];
         launch_propagate_fx(Lp.cone_base, Lp.cone_base + (int)Lp.cone_nonrel.size(), W.pp.view(), W.stage.level(l), E.Ps, E.Pang,
