@@ -212,8 +212,8 @@ void far_b(ifgf2d_ctx* ctx, int B, double2* yt) {
         launch_prop_b(p0, p1, ctx->pp_ptr.p, ctx->pp_nchild.p, pb, T.Ps, T.Pang, ctx->Gsep32.p, B, coef, s);
     }
     const bool grouped = (ctx->tune_batch_tc & kBatchGroupedInterp) && B <= 64 && T.Ps == 5 && T.Pang == 5;
-    launch_final_b<float>((int)ctx->D.N, ctx->point_leaf.p, ctx->leaf_start.p, ctx->leaf_count.p, ctx->nbr_ptr.p, ctx->nbr_box.p,
-                          ctx->near_rowlen.p, ctx->near_off.p, ctx->near32.p, rho, ctx->ip_ptr.p, grouped ? nullptr : ctx->ip32.p, coef,
+    launch_final_b((int)ctx->D.N, ctx->point_leaf.p, ctx->leaf_start.p, ctx->leaf_count.p, ctx->nbr_ptr.p, ctx->nbr_box.p,
+                   ctx->near_rowlen.p, ctx->near_off.p, ctx->near32.p, rho, ctx->ip_ptr.p, grouped ? nullptr : ctx->ip32.p, coef,
                           T.Ps, T.Pang, ctx->sorting.p, B, yt, s);
     if (grouped) launch_interp_grp(W.ig_items.p, (int)W.ig_items.n, W.ig_terms.p, coef, T.Ps, T.Pang, ctx->sorting.p, B, yt, s);
 }
@@ -232,9 +232,8 @@ void far_bx(ifgf2d_ctx* ctx, int B, double2* yt) {
         launch_prop_bx(Lp.cone_base, Lp.cone_base + (int)Lp.cone_nonrel.size(), ctx->pp_ptr.p, W.px64.view(), T.Ps, T.Pang, ctx->GsepX.p,
                        B, W.coef64.p, W.cexp64.p, s);
     }
-    launch_final_b<double>((int)ctx->D.N, ctx->point_leaf.p, ctx->leaf_start.p, ctx->leaf_count.p, ctx->nbr_ptr.p, ctx->nbr_box.p,
-                           ctx->near_rowlen.p, ctx->near_off.p, ctx->near.p, W.rho64.p, ctx->ip_ptr.p, nullptr, nullptr, T.Ps, T.Pang,
-                           ctx->sorting.p, B, yt, s);
+    launch_near_bx((int)ctx->D.N, ctx->point_leaf.p, ctx->leaf_start.p, ctx->leaf_count.p, ctx->nbr_ptr.p, ctx->nbr_box.p,
+                   ctx->near_rowlen.p, ctx->near_off.p, ctx->near.p, ctx->nexp.p, W.rhox.p, W.rexp.p, ctx->sorting.p, B, yt, s);
     launch_interp_bx(W.ig64_items.p, (int)W.ig64_items.n, W.ig64.view(), W.coef64.p, W.cexp64.p, T.Ps, T.Pang, ctx->sorting.p, B, yt, s);
 }
 

@@ -26,7 +26,7 @@ constexpr int kBatchTcProp = 2;   // propagation (k_prop_t5)
 constexpr int kBatchTcLeaf6 = 4;  // leaf-cone sums with three TF32 terms per operand (6 products)
 constexpr int kBatchBulkProp = 8; // FP32 FMA propagation with TMA-staged child coefficients (k_prop_bk)
 constexpr int kBatchGroupedInterp = 16;   // interpolation grouped by cone per leaf box (k_interp_grp)
-constexpr int kSingleInterpBox64 = 32;    // single vector, FP64: interpolation by leaf box (k_interp_box)
+constexpr int kSingleInterpBox64 = 32;    // single vector, FP64: accepted (its one kernel works by leaf box)
 constexpr int kSingleInterpBox32 = 64;    // single vector, complex64: interpolation by leaf box
 constexpr int kKernelBits = kBatchTcLeaf | kBatchTcProp | kBatchTcLeaf6 | kBatchBulkProp | kBatchGroupedInterp |
                             kSingleInterpBox64 | kSingleInterpBox32;
@@ -184,7 +184,7 @@ struct ifgf2d_ctx {
     // launch shapes per precision (0 FP64, 1 complex64): leaf-kernel source chunks, and cones
     // per block of each level's propagation (0 = the most that fit 256 threads); set by
     // ifgf2d_autotune / ifgf2d_set_tuning
-    int tune_leaf[2] = {5, 5};      // complex64 also 0: the table streamed by TMA bulk copies (k_leaf_tma)
+    int tune_leaf[2] = {2, 5};      // complex64 also 0: the table streamed by TMA bulk copies (k_leaf_tma)
     int tune_prop[2][kTuneLevels] = {};
     // kernel choices (bit mask): batched complex64 kernels on the tcgen05 tensor cores in 3xTF32
     // (else FP32 FMA), the batched grouped interpolation, the single-vector interpolation by box
@@ -215,9 +215,11 @@ struct ifgf2d_ctx {
     DBuf<int> patch_s, nsp_ptr_s, nsp_s;
     DBuf<int> leaf_start, leaf_count, point_leaf, nbr_ptr, nbr_box;
     DBuf<long long> near_off;
-    DBuf<double2> near;
+    DBuf<int4> near;                // the FP64 form's near-field blocks: fixed-point limbs, with
+    DBuf<int> nexp;                 // one exponent per Morton-sorted target (FP64 values until set-up fixes them)
     DBuf<int> leaf_cone_box;
     DBuf<long long> leaf_off;
+    DBuf<LeafItem> leaf_items;      // work items of the FP64 leaf sums
     DBuf<LeafNode> leaf_nodes_d;
     DBuf<int4> leafL;               // the FP64 form's leaf-cone tables: fixed-point limbs, with
     DBuf<int> lexp;                 // one exponent per cone and coefficient (FP64 values until set-up fixes them)
@@ -238,17 +240,15 @@ struct ifgf2d_ctx {
     DBuf<PropE<float>> pp32;
     DBuf<InterpE<float>> ip32;
     DBuf<float> Gsep32;
-    // interpolation by leaf box (k_interp_box): work items, the plan box-transposed in both
-    // precisions, and the pieces' sums per target
+    // interpolation by leaf box: work items, the plan box-transposed in both precisions, and the
+    // complex64 pieces' sums per target
     DBuf<int4> ib_items;
     DBuf<int2> nb_items;            // near field by leaf box (k_near_box): (box, first of up to 32 targets)
-    DBuf<InterpX> ipT;
+    PlanBuf ipT;
+    DBuf<FinItem> fx_items;         // work items of k_final_fx
     DBuf<InterpE<float>> ip32T;
-    DBuf<double2> ib_part;
     DBuf<float2> ib_part32;
     // work vectors
-    DBuf<int4> rhox;                // the densities as limbs, with
-    DBuf<int> rexp;                 // one exponent per leaf box
     DBuf<double2> rho, vin, vout;
     std::unique_ptr<GmresWork> gw;
     BatchWork* bw = nullptr;        // batched apply / solve workspace (batch.cu), freed by destroy
@@ -292,6 +292,19 @@ static inline bool all_finite(const double* v, long long n) {
 }
 
 namespace ifgf {
+// the work items of launch_leaf_fx: runs of up to leaf_fx_cones cones of one box
+inline std::vector<LeafItem> leaf_fx_items(const std::vector<int>& cone_box, const std::vector<int>& start, const std::vector<int>& count,
+                                           const std::vector<long long>& off, int P) {
+    std::vector<LeafItem> items;
+    const int nc = (int)cone_box.size(), most = leaf_fx_cones(P);
+    for (int c = 0; c < nc;) {
+        int e = c + 1;
+        while (e < nc && e - c < most && cone_box[e] == cone_box[c]) ++e;
+        items.push_back(LeafItem{off[c], c, e - c, start[cone_box[c]], count[cone_box[c]]});
+        c = e;
+    }
+    return items;
+}
 // What a group of obstacles (group.cu) changes in the device part of the IFGF set-up: (k, eta)
 // per leaf box and per leaf cone (device arrays), and the leaf-cone nodes and the propagation
 // plan, both built member by member.

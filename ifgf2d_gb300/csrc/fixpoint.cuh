@@ -181,6 +181,14 @@ __device__ __forceinline__ long long fx_align(long long y, int e, int E, int T) 
     const int sh = e - E + T;
     return sh >= 0 ? y << sh : (sh < -62 ? 0ll : (y + (1ll << (-sh - 1))) >> -sh);
 }
+// y 2^e as a double, 0 or infinity outside its range
+__device__ __forceinline__ double fx_scaled(long long y, int e) {
+    const double d = (double)y;
+    const int hi = __double2hiint(d), x = ((hi >> 20) & 0x7ff) + e;
+    if (y == 0 || x <= 0) return 0.0;
+    return x >= 0x7ff ? __hiloint2double((hi & 0x80000000) | 0x7ff00000, 0)
+                      : __hiloint2double((hi & 0x800fffff) | (x << 20), __double2loint(d));
+}
 // the exponent that y 2^e stays below
 __device__ __forceinline__ int fx_top_of(long long y, int e) { return y ? e + 64 - __clzll(y < 0 ? -y : y) : kFxMinExp; }
 

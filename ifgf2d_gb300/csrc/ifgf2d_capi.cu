@@ -462,7 +462,7 @@ static int setup_boxes(ifgf2d_ctx* ctx, double k, int nlevels, const SetupExtra*
     CK(ctx->near.alloc(noff[nleaf]));
     launch_near_setup(ctx->leaf_start.p, ctx->leaf_count.p, ctx->nbr_ptr.p, ctx->nbr_box.p, ctx->near_off.p, nleaf,
                       ctx->xs_s.p, ctx->ys_s.p, ctx->nxs_s.p, ctx->nys_s.p, ctx->patch_s.p, ctx->nsp_ptr_s.p, ctx->nsp_s.p, k,
-                      ctx->form, ctx->eta, ctx->near.p, ctx->stream, ex ? ex->keta_leafbox : nullptr);
+                      ctx->form, ctx->eta, reinterpret_cast<double2*>(ctx->near.p), ctx->stream, ex ? ex->keta_leafbox : nullptr);
     CK(cudaGetLastError());
     return IFGF2D_OK;
 }
@@ -508,6 +508,7 @@ static int setup_cones(ifgf2d_ctx* ctx, double k, int nlevels, const SetupExtra*
     std::vector<long long> loff(ncl + 1, 0);
     for (int c = 0; c < ncl; ++c) loff[c + 1] = loff[c] + (long long)P * T.leaf_count[LD.cone_box[c]];
     CK(ctx->leaf_cone_box.upload(LD.cone_box)); CK(ctx->leaf_off.upload(loff));
+    CK(ctx->leaf_items.upload(leaf_fx_items(LD.cone_box, T.leaf_start, T.leaf_count, loff, P)));
     CK(ctx->leafL.alloc(loff[ncl]));
     CK(ctx->leaf_nodes_d.alloc((size_t)ncl * P));
     CK(ctx->pp.alloc((size_t)T.pp_total)); CK(ctx->pp32.alloc((size_t)T.pp_total));
@@ -551,11 +552,28 @@ static int setup_interp(ifgf2d_ctx* ctx, int nlevels, DBuf<int>& perr) {
     {   // interpolation by leaf box: per box, chunks of 32 targets x pieces of kIbPiece terms
         std::vector<int4> items;
         std::vector<int2> nitems;
+        std::vector<FinItem> fitems;
+        long long near_at = 0;      // the box's near-field block, and its list of sources
+        int src_at = 0;
         int maxpc = 0;
         for (int b = 0; b < nleaf; ++b) {
             const int s0 = T.leaf_start[b], n = T.leaf_count[b];
-            if (n <= 0) continue;
+            int rl = 0;
+            for (int q = T.nbr_ptr[b]; q < T.nbr_ptr[b + 1]; ++q) rl += T.leaf_count[T.nbr_box[q]];
+            if (n <= 0) { src_at += rl; continue; }
             for (int c0 = 0; c0 < n; c0 += kNearTargets) nitems.push_back(make_int2(b, c0));
+            const int nf = (n + kFinTargets - 1) / kFinTargets;      // equal shares
+            for (int q = 0; q < nf; ++q) {
+                const int c0 = (int)((long long)n * q / nf);
+                FinItem it{};
+                it.near = near_at + (long long)c0 * rl;
+                it.first = s0 + c0; it.cnt = (int)((long long)n * (q + 1) / nf) - c0; it.n = n;
+                it.ip = T.ip_ptr[s0] + c0; it.nt = T.ip_ptr[s0 + 1] - T.ip_ptr[s0];
+                it.rl = rl; it.src = src_at;
+                fitems.push_back(it);
+            }
+            near_at += (long long)n * rl;
+            src_at += rl;
             const int nt = T.ip_ptr[s0 + 1] - T.ip_ptr[s0];   // the same for every target of the box
             const int npc = (nt + kIbPiece - 1) / kIbPiece;
             maxpc = std::max(maxpc, npc);
@@ -564,13 +582,12 @@ static int setup_interp(ifgf2d_ctx* ctx, int nlevels, DBuf<int>& perr) {
         }
         CK(ctx->ib_items.upload(items));
         CK(ctx->nb_items.upload(nitems));
+        CK(ctx->fx_items.upload(fitems));
         CK(ctx->ipT.alloc(T.ip.size())); CK(ctx->ip32T.alloc(T.ip.size()));
-        launch_interp_transpose<double>((int)N, ctx->point_leaf.p, ctx->leaf_start.p, ctx->leaf_count.p, ctx->ip_ptr.p, ip.p,
-                                        ctx->ipT.p, ctx->stream);
-        launch_interp_transpose<float>((int)N, ctx->point_leaf.p, ctx->leaf_start.p, ctx->leaf_count.p, ctx->ip_ptr.p, ip.p,
-                                       ctx->ip32T.p, ctx->stream);
+        launch_interp_transpose((int)N, ctx->point_leaf.p, ctx->leaf_start.p, ctx->leaf_count.p, ctx->ip_ptr.p, ip.p, ctx->ip32T.p,
+                                ctx->ipT.view(), ctx->stream);
         CK(cudaGetLastError());
-        CK(ctx->ib_part.alloc((size_t)std::max(maxpc, 1) * N)); CK(ctx->ib_part32.alloc((size_t)std::max(maxpc, 1) * N));
+        CK(ctx->ib_part32.alloc((size_t)std::max(maxpc, 1) * N));
     }
     CK(ctx->coef.alloc((size_t)T.total_cones * P));
     CK(ctx->cexp.alloc((size_t)T.total_cones));
@@ -581,7 +598,9 @@ static int setup_interp(ifgf2d_ctx* ctx, int nlevels, DBuf<int>& perr) {
     CK(leaf_tma_init());
     CK(cudaDeviceGetAttribute(&ctx->nsm, cudaDevAttrMultiProcessorCount, ctx->device));
     if (!ctx->kerr.p) { CK(ctx->kerr.alloc(1)); CK(cudaMemsetAsync(ctx->kerr.p, 0, sizeof(int), ctx->stream)); }
-    launch_d2f(ctx->near.p, (long long)ctx->near.n, ctx->near32.p, ctx->stream);
+    CK(ctx->nexp.alloc(N));
+    launch_near_fix((int)N, ctx->point_leaf.p, ctx->leaf_start.p, ctx->near_rowlen.p, ctx->near_off.p, ctx->near.p, ctx->nexp.p,
+                    ctx->near32.p, ctx->stream);
     {
         const TreeLevel& LD = T.L[nlevels - 1];
         const int ncl = (int)LD.cone_nonrel.size();
@@ -589,7 +608,6 @@ static int setup_interp(ifgf2d_ctx* ctx, int nlevels, DBuf<int>& perr) {
         launch_leaf_fix(ctx->leaf_cone_box.p, ncl, ctx->leaf_count.p, ctx->leaf_off.p, P, ctx->leafL.p, ctx->lexp.p, ctx->leafL32.p,
                         ctx->stream);
     }
-    CK(ctx->rhox.alloc(N)); CK(ctx->rexp.alloc(nleaf));
     CK(cudaGetLastError());
     int bad = 0;
     CK(cudaMemcpyAsync(&bad, perr.p, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
@@ -636,35 +654,35 @@ static int check_kerr(ifgf2d_ctx* ctx) {
 }
 
 // ------------------------------------------------------------------ apply
-// y += near field + cousin interpolants of every target (BoxTree.h:1049-1069).  By target:
-// k_final_t, a warp per target.  By leaf box: the interpolation by k_interp_box (pieces per
-// target), then the near field by k_near_box, which adds the pieces in order.
+// y += near field + cousin interpolants of every target (BoxTree.h:1049-1069), from the Morton-ordered
+// intensities.  FP64: k_final_fx, by leaf box.  complex64, by target: k_final_t, a warp per target; by
+// leaf box: the interpolation by k_interp_box (pieces per target), then the near field by k_near_box,
+// which adds the pieces in order.
 template <typename R>
-static void launch_interp_final(ifgf2d_ctx* ctx, const V2<R>* rho, const V2<R>* near, const InterpT<R>* ip, const CoefT<R>* coef,
-                                double2* y, bool by_box) {
+static void launch_interp_final(ifgf2d_ctx* ctx, const CoefT<R>* coef, double2* y, bool by_box) {
     const Tree& T = ctx->T;
     const int N = (int)ctx->D.N;
-    if (!by_box || ctx->nb_items.n == 0) {
-        launch_final_t<R>(N, ctx->point_leaf.p, ctx->leaf_start.p, ctx->near_src_off.p, ctx->near_src.p, ctx->near_rowlen.p,
-                          ctx->near_off.p, near, rho, ctx->ip_ptr.p, ip, coef, ctx->cexp.p, T.Ps, T.Pang, ctx->sorting.p, y, ctx->stream);
-        return;
-    }
-    const V2<R>* part = nullptr;
-    if (ctx->ib_items.n > 0) {
-        V2<R>* pp;
-        const InterpT<R>* ipT;
-        if constexpr (sizeof(R) == 4) { pp = ctx->ib_part32.p; ipT = ctx->ip32T.p; }
-        else { pp = ctx->ib_part.p; ipT = ctx->ipT.p; }
-        launch_interp_box<R>(ctx->ib_items.p, (int)ctx->ib_items.n, N, ctx->leaf_start.p, ctx->leaf_count.p, ctx->ip_ptr.p, ipT,
-                             coef, ctx->cexp.p, T.Ps, T.Pang, pp, ctx->stream);
-        part = pp;
-    }
-    launch_near_box<R>(ctx->nb_items.p, (int)ctx->nb_items.n, ctx->leaf_start.p, ctx->leaf_count.p, ctx->near_src_off.p,
-                       ctx->near_src.p, ctx->near_rowlen.p, ctx->near_off.p, near, rho, ctx->ip_ptr.p, part, N, ctx->sorting.p, y,
+    if constexpr (sizeof(R) == 8) {
+        launch_final_fx(ctx->fx_items.p, (int)ctx->fx_items.n, ctx->near_src.p, ctx->near.p, ctx->nexp.p, ctx->rho.p, ctx->ipT.view(),
+                        coef, ctx->cexp.p, T.Ps, T.Pang, ctx->sorting.p, y, ctx->stream);
+    } else if (!by_box || ctx->nb_items.n == 0) {
+        launch_final_t(N, ctx->point_leaf.p, ctx->leaf_start.p, ctx->near_src_off.p, ctx->near_src.p, ctx->near_rowlen.p,
+                       ctx->near_off.p, ctx->near32.p, ctx->rho32.p, ctx->ip_ptr.p, ctx->ip32.p, coef, T.Ps, T.Pang, ctx->sorting.p, y,
                        ctx->stream);
+    } else {
+        const float2* part = nullptr;
+        if (ctx->ib_items.n > 0) {
+            launch_interp_box(ctx->ib_items.p, (int)ctx->ib_items.n, N, ctx->leaf_start.p, ctx->leaf_count.p, ctx->ip_ptr.p,
+                              ctx->ip32T.p, coef, T.Ps, T.Pang, ctx->ib_part32.p, ctx->stream);
+            part = ctx->ib_part32.p;
+        }
+        launch_near_box(ctx->nb_items.p, (int)ctx->nb_items.n, ctx->leaf_start.p, ctx->leaf_count.p, ctx->near_src_off.p,
+                        ctx->near_src.p, ctx->near_rowlen.p, ctx->near_off.p, ctx->near32.p, ctx->rho32.p, ctx->ip_ptr.p, part, N,
+                        ctx->sorting.p, y, ctx->stream);
+    }
 }
 
-// leaf-cone sums of the Morton-ordered intensities (rhox or rho32); `shape`: the threads that share a
+// leaf-cone sums of the Morton-ordered intensities (rho or rho32); `shape`: the threads that share a
 // coefficient's sum (1, 2, 5 or 10; complex64 also 0, the table streamed by TMA bulk copies)
 template <typename R>
 static void launch_leaf(ifgf2d_ctx* ctx, CoefT<R>* coef, int shape) {
@@ -678,8 +696,8 @@ static void launch_leaf(ifgf2d_ctx* ctx, CoefT<R>* coef, int shape) {
         launch_leaf_apply_t(ctx->leaf_cone_box.p, ncl, LD.cone_base, ctx->leaf_start.p, ctx->leaf_count.p, ctx->leaf_off.p,
                             ctx->leafL32.p, ctx->rho32.p, T.P, coef, ctx->stream, shape);
     } else {
-        launch_leaf_fx(ctx->leaf_cone_box.p, ncl, LD.cone_base, ctx->leaf_start.p, ctx->leaf_count.p, ctx->leaf_off.p, ctx->leafL.p,
-                       ctx->lexp.p, ctx->rhox.p, ctx->rexp.p, T.P, T.Ps, coef, ctx->cexp.p, ctx->stream, shape);
+        launch_leaf_fx(ctx->leaf_items.p, (int)ctx->leaf_items.n, LD.cone_base, ctx->leafL.p, ctx->lexp.p, ctx->rho.p, T.P, T.Ps, coef, ctx->cexp.p,
+                       ctx->stream, shape);
     }
 }
 // children at level l -> parents at level l - 1; `shape`: the complex64 kernel's launch shape (the
@@ -698,8 +716,7 @@ static void launch_prop_level(ifgf2d_ctx* ctx, int l, CoefT<R>* coef, int shape)
 
 // y += far field of the Morton-ordered intensities (rho / rho32), BoxTree.h:1037-1061
 template <typename R>
-static void far_ifgf_t(ifgf2d_ctx* ctx, const V2<R>* rho, const V2<R>* near, const InterpT<R>* ip, CoefT<R>* coef, double2* y,
-                       cudaEvent_t* ev) {
+static void far_ifgf_t(ifgf2d_ctx* ctx, CoefT<R>* coef, double2* y, cudaEvent_t* ev) {
     const int Dl = ctx->nlevels - 1;
     cudaStream_t s = ctx->stream;
     const int pr = sizeof(R) == 4 ? 1 : 0;
@@ -709,7 +726,7 @@ static void far_ifgf_t(ifgf2d_ctx* ctx, const V2<R>* rho, const V2<R>* near, con
         launch_prop_level<R>(ctx, l, coef, l < kTuneLevels ? ctx->tune_prop[pr][l] : 0);
     }
     if (ev) cudaEventRecord(ev[1], s);
-    launch_interp_final<R>(ctx, rho, near, ip, coef, y, (ctx->tune_batch_tc & (pr ? kSingleInterpBox32 : kSingleInterpBox64)) != 0);
+    launch_interp_final<R>(ctx, coef, y, (ctx->tune_batch_tc & kSingleInterpBox32) != 0);
 }
 
 // the IFGF far field in the precision of `mode`; x in original order, y += result.  With
@@ -720,15 +737,11 @@ static int far_apply(ifgf2d_ctx* ctx, const double2* x, const double* wq, double
     if (mode == IFGF2D_APPLY_IFGF_MIXED) {
         if (!rho_ready) launch_intensities_t<float>(x, wq, ctx->sorting.p, N, ctx->rho32.p, ctx->stream);
         if (ev) cudaEventRecord(ev[0], ctx->stream);
-        far_ifgf_t<float>(ctx, ctx->rho32.p, ctx->near32.p, ctx->ip32.p, ctx->coef32.p, y, ev ? ev + 1 : nullptr);
+        far_ifgf_t<float>(ctx, ctx->coef32.p, y, ev ? ev + 1 : nullptr);
     } else {
-        if (!rho_ready) {
-            launch_intensities_t<double>(x, wq, ctx->sorting.p, N, ctx->rho.p, ctx->stream);
-            launch_rho_fx(ctx->leaf_start.p, ctx->leaf_count.p, (int)ctx->T.leaf_start.size(), ctx->rho.p, ctx->rhox.p, ctx->rexp.p,
-                          ctx->stream);
-        }
+        if (!rho_ready) launch_intensities_t<double>(x, wq, ctx->sorting.p, N, ctx->rho.p, ctx->stream);
         if (ev) cudaEventRecord(ev[0], ctx->stream);
-        far_ifgf_t<double>(ctx, ctx->rho.p, ctx->near.p, ctx->ipx.p, ctx->coef.p, y, ev ? ev + 1 : nullptr);
+        far_ifgf_t<double>(ctx, ctx->coef.p, y, ev ? ev + 1 : nullptr);
     }
     CK(cudaGetLastError());
     return IFGF2D_OK;
@@ -743,13 +756,9 @@ static int apply_dev(ifgf2d_ctx* ctx, const double2* x, double2* y, int mode) {
     if (mode != IFGF2D_APPLY_DIRECT && !ctx->ifgf_ready) return fail(ctx, IFGF2D_ERR_STATE, "setup before an IFGF apply");
     const double half = ctx->form == IFGF2D_COMBINED ? 0.5 : 0.0;
     if (mode != IFGF2D_APPLY_DIRECT) {
-        if (mode == IFGF2D_APPLY_IFGF_MIXED)
-            launch_sing_intens(x, ctx->W.p, ctx->srow_ptr.p, ctx->srow_col.p, ctx->cols.p, N, D.Np, half, y, ctx->wq.p,
-                               ctx->inverse.p, nullptr, ctx->rho32.p, ctx->stream);
-        else
-            launch_sing_box(x, ctx->W.p, ctx->srow_ptr.p, ctx->srow_col.p, ctx->cols.p, D.Np, half, y, ctx->wq.p, ctx->leaf_start.p,
-                            ctx->leaf_count.p, (int)ctx->T.leaf_start.size(), ctx->sorting.p, ctx->rho.p, ctx->rhox.p, ctx->rexp.p,
-                            ctx->stream);
+        launch_sing_intens(x, ctx->W.p, ctx->srow_ptr.p, ctx->srow_col.p, ctx->cols.p, N, D.Np, half, y, ctx->wq.p,
+                           ctx->inverse.p, mode == IFGF2D_APPLY_IFGF_MIXED ? nullptr : ctx->rho.p,
+                           mode == IFGF2D_APPLY_IFGF_MIXED ? ctx->rho32.p : nullptr, ctx->stream);
         return far_apply(ctx, x, ctx->wq.p, y, mode, nullptr, true);
     }
     launch_sing_intens(x, ctx->W.p, ctx->srow_ptr.p, ctx->srow_col.p, ctx->cols.p, N, D.Np, half, y, ctx->wq.p, nullptr,
@@ -830,7 +839,7 @@ extern "C" int ifgf2d_set_tuning(ifgf2d_ctx* ctx, const int* c) {
     return IFGF2D_OK;
 }
 template <typename R>
-static int tune_precision(ifgf2d_ctx* ctx, int reps, const V2<R>* rho, CoefT<R>* coef) {
+static int tune_precision(ifgf2d_ctx* ctx, int reps, CoefT<R>* coef) {
     const int Dl = ctx->nlevels - 1, pr = sizeof(R) == 4 ? 1 : 0;
     cudaStream_t s = ctx->stream;
     cudaEvent_t e0, e1;
@@ -861,16 +870,11 @@ static int tune_precision(ifgf2d_ctx* ctx, int reps, const V2<R>* rho, CoefT<R>*
         }
         ctx->tune_prop[pr][l] = bestp;
     }
-    {   // the interpolation by leaf box or by target (y: the context's output vector, overwritten later)
-        const int bit = pr ? kSingleInterpBox32 : kSingleInterpBox64;
-        const V2<R>* near;
-        const InterpT<R>* ip;
-        if constexpr (sizeof(R) == 4) { near = ctx->near32.p; ip = ctx->ip32.p; }
-        else { near = ctx->near.p; ip = ctx->ipx.p; }
-        const float tb = time_it([&] { launch_interp_final<R>(ctx, rho, near, ip, coef, ctx->vout.p, true); });
-        const float tt = time_it([&] { launch_interp_final<R>(ctx, rho, near, ip, coef, ctx->vout.p, false); });
-        if (tb < tt) ctx->tune_batch_tc |= bit;
-        else ctx->tune_batch_tc &= ~bit;
+    if constexpr (sizeof(R) == 4) {   // the interpolation by leaf box or by target (y: the context's output vector, overwritten later)
+        const float tb = time_it([&] { launch_interp_final<R>(ctx, coef, ctx->vout.p, true); });
+        const float tt = time_it([&] { launch_interp_final<R>(ctx, coef, ctx->vout.p, false); });
+        if (tb < tt) ctx->tune_batch_tc |= kSingleInterpBox32;
+        else ctx->tune_batch_tc &= ~kSingleInterpBox32;
     }
     cudaEventDestroy(e0); cudaEventDestroy(e1);
     CK(cudaGetLastError());
@@ -885,8 +889,8 @@ extern "C" int ifgf2d_autotune(ifgf2d_ctx* ctx, int reps, int* choices) {
     int rc;
     if ((rc = apply_dev(ctx, ctx->vin.p, ctx->vout.p, IFGF2D_APPLY_IFGF))) return rc;
     if ((rc = apply_dev(ctx, ctx->vin.p, ctx->vout.p, IFGF2D_APPLY_IFGF_MIXED))) return rc;
-    if ((rc = tune_precision<double>(ctx, reps, ctx->rho.p, ctx->coef.p))) return rc;
-    if ((rc = tune_precision<float>(ctx, reps, ctx->rho32.p, ctx->coef32.p))) return rc;
+    if ((rc = tune_precision<double>(ctx, reps, ctx->coef.p))) return rc;
+    if ((rc = tune_precision<float>(ctx, reps, ctx->coef32.p))) return rc;
     CK(cudaStreamSynchronize(ctx->stream));
     if (ctx->gw) ctx->gw->drop_graphs();
     if (choices) write_tuning(ctx, choices);

@@ -12,7 +12,6 @@
 //                                                             BoxTree.h:614-683, 876-937, 1063-1069
 #include "ifgf2d_kernels.cuh"
 #include "hankel.cuh"
-#include "fixpoint.cuh"
 
 namespace ifgf {
 
@@ -179,56 +178,6 @@ __global__ void k_sing_apply(const double2* __restrict__ x, const double2* __res
             RhoT r; r.x = v.x * wv; r.y = v.y * wv;
             rho[inv ? inv[o] : o] = r;
         }
-    }
-}
-
-// The same with a block per leaf box, whose points' intensities it writes in Morton order, in FP64 and as
-// fixed-point limbs with the box's exponent (fixpoint.cuh).
-__global__ void __launch_bounds__(256) k_sing_box(const double2* __restrict__ x, const double2* __restrict__ W,
-                                                  const int* __restrict__ row_ptr, const int* __restrict__ row_col,
-                                                  const RPColumn* __restrict__ cols, int Np, double half, double2* __restrict__ y,
-                                                  const double* __restrict__ wq, const int* __restrict__ leaf_start,
-                                                  const int* __restrict__ leaf_count, const long long* __restrict__ sorting,
-                                                  double2* __restrict__ rho, int4* __restrict__ rhox, int* __restrict__ rexp) {
-    __shared__ int smax;
-    const int b = blockIdx.x, s0 = leaf_start[b], n = leaf_count[b];
-    const int k8 = threadIdx.x & 7;
-    if (threadIdx.x == 0) smax = 0;
-    __syncthreads();
-    for (int i0 = 0; i0 < n; i0 += 32) {
-        const int i = i0 + (threadIdx.x >> 3);
-        double2 acc = make_double2(0.0, 0.0);
-        int o = 0;
-        if (i < n) {
-            o = (int)sorting[s0 + i];
-            for (int q = row_ptr[o]; q < row_ptr[o + 1]; ++q) {
-                const int col = row_col[q];
-                const double2* w = W + (long long)col * Np;
-                const double2* d = x + (long long)cols[col].patch * Np;
-                for (int kk = k8; kk < Np; kk += 8) cfma(acc, d[kk], w[kk]);
-            }
-        }
-#pragma unroll
-        for (int off = 4; off > 0; off >>= 1) {
-            acc.x += __shfl_xor_sync(0xffffffffu, acc.x, off);
-            acc.y += __shfl_xor_sync(0xffffffffu, acc.y, off);
-        }
-        if (i < n && k8 == 0) {
-            const double2 v = x[o];
-            if (half != 0.0) { acc.x += half * v.x; acc.y += half * v.y; }   // jump term
-            y[o] = acc;
-            const double wv = wq[o];
-            const double2 r = make_double2(v.x * wv, v.y * wv);
-            rho[s0 + i] = r;
-            atomicMax(&smax, fx_absmax_hi(r.x, r.y));
-        }
-    }
-    __syncthreads();
-    const int E = fx_expo(smax), T = fx_rho_top(n);
-    if (threadIdx.x == 0) rexp[b] = E;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const double2 v = rho[s0 + i];       // written by this block before the barrier
-        rhox[s0 + i] = E == kFxBad ? make_int4(0, 0, 0, 0) : fx_pack_sum(fx_from(v.x, E, T), fx_from(v.y, E, T));
     }
 }
 
@@ -548,12 +497,6 @@ void launch_sing_intens(const double2* x, const double2* W, const int* row_ptr, 
         k_sing_apply<float2><<<nblk((long long)N * 8, 256), 256, 0, s>>>(x, W, row_ptr, row_col, cols, N, Np, half, y, wq, inv, rho32);
     else
         k_sing_apply<double2><<<nblk((long long)N * 8, 256), 256, 0, s>>>(x, W, row_ptr, row_col, cols, N, Np, half, y, wq, inv, rho64);
-}
-void launch_sing_box(const double2* x, const double2* W, const int* row_ptr, const int* row_col, const RPColumn* cols, int Np,
-                     double half, double2* y, const double* wq, const int* leaf_start, const int* leaf_count, int nleaf,
-                     const long long* sorting, double2* rho, int4* rhox, int* rexp, cudaStream_t s) {
-    if (nleaf > 0)
-        k_sing_box<<<nleaf, 256, 0, s>>>(x, W, row_ptr, row_col, cols, Np, half, y, wq, leaf_start, leaf_count, sorting, rho, rhox, rexp);
 }
 void launch_direct_far(const double* tx, const double* ty, int nt, const int* t_patch, const int* t_nsp_ptr, const int* t_nsp,
                        const double* sx, const double* sy, const double* snx, const double* sny, const int* s_patch,

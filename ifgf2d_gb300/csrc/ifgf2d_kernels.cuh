@@ -51,10 +51,6 @@ template <typename R> struct CoefOf;
 template <> struct CoefOf<double> { using T = int4; };
 template <> struct CoefOf<float> { using T = float2; };
 template <typename R> using CoefT = typename CoefOf<R>::T;
-template <typename R> struct InterpOf;
-template <> struct InterpOf<double> { using T = InterpX; };
-template <> struct InterpOf<float> { using T = InterpE<float>; };
-template <typename R> using InterpT = typename InterpOf<R>::T;
 // one (parent cone, child, node) propagation term: child cone id, (s, theta), factor ratio
 template <typename R> struct PropE;
 template <> struct PropE<float> { int child_cone; float s, th, wr, wi; };
@@ -99,11 +95,6 @@ void launch_sing_apply(const double2* x, const double2* W, const int* row_ptr, c
 void launch_sing_intens(const double2* x, const double2* W, const int* row_ptr, const int* row_col,
                         const RPColumn* cols, int N, int Np, double half, double2* y, const double* wq,
                         const long long* inv, double2* rho64, float2* rho32, cudaStream_t s);
-// the FP64 form leaf box by leaf box, which also writes the intensities in Morton order: rho in FP64,
-// rhox as fixed-point limbs with one exponent per box (fixpoint.cuh)
-void launch_sing_box(const double2* x, const double2* W, const int* row_ptr, const int* row_col, const RPColumn* cols, int Np,
-                     double half, double2* y, const double* wq, const int* leaf_start, const int* leaf_count, int nleaf,
-                     const long long* sorting, double2* rho, int4* rhox, int* rexp, cudaStream_t s);
 // sources with unit normals snx, sny (NULL for the single layer); form 0 single layer, 2 combined
 void launch_direct_far(const double* tx, const double* ty, int ntarget, const int* t_patch, const int* t_nsp_ptr,
                        const int* t_nsp, const double* sx, const double* sy, const double* snx, const double* sny,
@@ -117,14 +108,15 @@ void launch_leaf_apply_t(const int* cone_box, int ncones, int cone_base, const i
                          const long long* leaf_off, const float2* L, const float2* rho, int P, float2* coef, cudaStream_t s,
                          int chunks = 5);
 // the FP64 form in fixed point (fixpoint.cuh): the table and its exponents [cone][coefficient] from
-// launch_leaf_fix (in place of the FP64 table; l32, when not null, receives the complex64 copy), the
-// densities and their exponents per leaf box from launch_rho_fx or launch_sing_box
-void launch_leaf_fx(const int* cone_box, int ncones, int cone_base, const int* leaf_start, const int* leaf_count,
-                    const long long* leaf_off, const int4* L, const int* lexp, const int4* rho, const int* rexp, int P, int Ps,
-                    int4* coef, int* cexp, cudaStream_t s, int chunks = 5);
+// launch_leaf_fix (in place of the FP64 table; l32, when not null, receives the complex64 copy); an item
+// is up to leaf_fx_cones cones of one leaf box: the table offset of the first, its local index, how many,
+// and the box's sources
+struct LeafItem { long long off; int cone, cones, first, n; };
+int leaf_fx_cones(int P);
+void launch_leaf_fx(const LeafItem* items, int nitems, int cone_base, const int4* L, const int* lexp, const double2* rho, int P, int Ps,
+                    int4* coef, int* cexp, cudaStream_t s, int chunks = 2);
 void launch_leaf_fix(const int* cone_box, int ncones, const int* leaf_count, const long long* leaf_off, int P, int4* L, int* lexp,
                      float2* l32, cudaStream_t s);
-void launch_rho_fx(const int* leaf_start, const int* leaf_count, int nleaf, const double2* rho, int4* out, int* rexp, cudaStream_t s);
 // complex64 leaf cones with the table streamed through shared memory by TMA bulk copies
 // (P = 25); false when not launched (other P, or leaf_tma_init not run).  *err is set when a
 // completion wait runs out.  leaf_tma_init sets the kernel's shared-memory attribute (outside
@@ -148,30 +140,40 @@ void launch_propagate_fx(int pbegin, int pend, PlanX pp, const int* stage, int P
 // n doubles in [-1, 1] as fixed-point limbs; the interpolation plan with (s, theta) as weights
 void launch_fx_weights(const double* in, int n, int2* out, cudaStream_t s);
 void launch_interp_fx(const InterpE<double>* in, long long n, InterpX* out, cudaStream_t s);
-// with `part`, the interpolation terms were summed by launch_interp_box: the near field plus each
-// target's pieces in order
-template <typename R>
 void launch_final_t(int N, const int* point_leaf, const int* leaf_start, const int* near_src_off, const int* near_src,
-                    const int* near_rowlen, const long long* near_off, const V2<R>* near,
-                    const V2<R>* rho, const int* ip_ptr, const InterpT<R>* ip, const CoefT<R>* coef, const int* cexp, int Ps,
-                    int Pang, const long long* sorting, double2* y, cudaStream_t s, const V2<R>* part = nullptr);
-// interpolation by leaf box (k_interp_box): items[w] = (leaf box, first target, first term, end
+                    const int* near_rowlen, const long long* near_off, const float2* near, const float2* rho, const int* ip_ptr,
+                    const InterpE<float>* ip, const float2* coef, int Ps, int Pang, const long long* sorting, double2* y,
+                    cudaStream_t s);
+// the FP64 form in fixed point, near field and interpolation by leaf box: a record per box and up to
+// kFinTargets of its targets, the near table and its exponents per target from launch_near_fix (in place
+// of the FP64 table, with the complex64 copy n32), the plan box-transposed (launch_interp_transpose)
+constexpr int kFinTargets = 20;
+struct FinItem {
+    long long near;            // first near-field table entry of the item's first target
+    int first, cnt, n;         // first Morton target, targets, targets of the box
+    int ip, nt;                // plan: the box's first entry plus the first target's place in it; terms per target
+    int rl, src, pad;          // near-field row: sources, their list
+};
+void launch_final_fx(const FinItem* items, int nitems, const int* near_src, const int4* near, const int* nexp, const double2* rho,
+                     PlanX ip, const int4* coef, const int* cexp, int Ps, int Pang, const long long* sorting, double2* y,
+                     cudaStream_t s);
+void launch_near_fix(int N, const int* point_leaf, const int* leaf_start, const int* near_rowlen, const long long* near_off, int4* near,
+                     int* nexp, float2* n32, cudaStream_t s);
+// complex64 interpolation by leaf box (k_interp_box): items[w] = (leaf box, first target, first term, end
 // term), pieces of kIbPiece terms; part[piece * N + target] receives each piece's sum
 constexpr int kIbPiece = 8;
-template <typename R>
 void launch_interp_box(const int4* items, int nitems, int N, const int* leaf_start, const int* leaf_count, const int* ip_ptr,
-                       const InterpT<R>* ipT, const CoefT<R>* coef, const int* cexp, int Ps, int Pang, V2<R>* part, cudaStream_t s);
-// near field by leaf box (k_near_box): items[w] = (leaf box, first of up to 32 targets); adds the
-// near field, then the target's interpolation pieces (when part is not null), into y
+                       const InterpE<float>* ipT, const float2* coef, int Ps, int Pang, float2* part, cudaStream_t s);
+// complex64 near field by leaf box (k_near_box): items[w] = (leaf box, first of up to 32 targets); adds
+// the near field, then the target's interpolation pieces (when part is not null), into y
 constexpr int kNearChunk = 1024, kNearTargets = 32;
-template <typename R>
 void launch_near_box(const int2* items, int nitems, const int* leaf_start, const int* leaf_count, const int* near_src_off,
-                     const int* near_src, const int* near_rowlen, const long long* near_off, const V2<R>* near, const V2<R>* rho,
-                     const int* ip_ptr, const V2<R>* part, int N, const long long* sorting, double2* y, cudaStream_t s);
-// the interpolation plan box-transposed (term j of box target t at the box's first entry + j n + t)
-template <typename R>
+                     const int* near_src, const int* near_rowlen, const long long* near_off, const float2* near, const float2* rho,
+                     const int* ip_ptr, const float2* part, int N, const long long* sorting, double2* y, cudaStream_t s);
+// the interpolation plan box-transposed (term j of box target t at the box's first entry + j n + t), in
+// complex64 and as px (child the cone, w the factor)
 void launch_interp_transpose(int N, const int* point_leaf, const int* leaf_start, const int* leaf_count, const int* ip_ptr,
-                             const InterpE<double>* in, InterpT<R>* out, cudaStream_t s);
+                             const InterpE<double>* in, InterpE<float>* out, PlanX px, cudaStream_t s);
 void launch_d2f(const double2* a, long long n, float2* b, cudaStream_t s);
 // Load the direct map's kernels (singular correction, FP64 intensities, both far-sum shapes) into
 // the current device's context now.  Under lazy module loading a kernel is otherwise loaded,
@@ -250,11 +252,14 @@ bool launch_interp_grp(const int4* items, int nitems, const InterpG* terms, cons
                        const long long* sorting, int B, double2* yt, cudaStream_t s);
 bool launch_prop_bk(int pbegin, int pend, const long long* pp_ptr, const int* pp_nchild, const PropB<float>* pb, int Ps, int Pang,
                     const float* Gsep, int B, float2* coef, int* err, cudaStream_t s);
-template <typename R>
 void launch_final_b(int N, const int* point_leaf, const int* leaf_start, const int* leaf_count, const int* nbr_ptr,
-                    const int* nbr_box, const int* near_rowlen, const long long* near_off, const V2<R>* near,
-                    const V2<R>* rho, const int* ip_ptr, const InterpE<R>* ip, const V2<R>* coef, int Ps, int Pang,
+                    const int* nbr_box, const int* near_rowlen, const long long* near_off, const float2* near,
+                    const float2* rho, const int* ip_ptr, const InterpE<float>* ip, const float2* coef, int Ps, int Pang,
                     const long long* sorting, int B, double2* yt, cudaStream_t s);
+// the FP64 near field in fixed point (tables as launch_final_fx's, densities as launch_leaf_bx's)
+void launch_near_bx(int N, const int* point_leaf, const int* leaf_start, const int* leaf_count, const int* nbr_ptr, const int* nbr_box,
+                    const int* near_rowlen, const long long* near_off, const int4* near, const int* nexp, const int4* rho,
+                    const int* rexp, const long long* sorting, int B, double2* yt, cudaStream_t s);
 // batched GMRES helpers on interleaved [N][B] vectors; column c of a basis starts at V + c * ldc
 int bdot_chunks(long long N);
 // h[c][r] = sum_i conj(V_c[i][r]) w[i][r] for c < ncols; Hcol[c][r] = h (add: +=).  With

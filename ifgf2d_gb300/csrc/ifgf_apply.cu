@@ -72,69 +72,102 @@ __global__ void __launch_bounds__(256) k_leaf_apply_t(const int* __restrict__ co
 }
 
 // The FP64 form of the same in fixed point (fixpoint.cuh): table and densities as 27-bit limbs, 12 wide
-// multiply-adds an entry where FP64 took 4 of the FP64 pipe's operations.  The kernel streams the table
-// from HBM (16 bytes an entry); kite k = 500 91 -> 55 us, k = 2000 582 -> 291 us (4.1 TB/s; the FP64
-// kernel before it ran at 93 % of the FP64 pipe).  The chunks' integer sums meet in shared memory; then the cone's
+// multiply-adds an entry where FP64 took 4 of the FP64 pipe's operations.  A block takes up to
+// kLeafFxCones / CH cones of one leaf box (items: table offset, first cone, cones, first source,
+// sources): it brings the box's densities to their exponent in shared memory once, while its threads'
+// first table entries are in flight; the chunks' integer sums meet in shared memory; then the cone's
 // coefficients, whose entries have an exponent per coefficient, are brought to the cone's exponent.
+// Bound by the table's loads in flight (4 ahead of the barriers, then 4 a step, 3 blocks an SM).  Kite
+// k = 500 / 2000, 145 MB / 1.2 GB of table: 145 / 830 us with FP64 multiply-adds, 53 / 281 us so (2.9 / 4.3
+// TB/s).  CH = 2 keeps blocks of 5 cones, which amortises the conversion; 5 takes 67 / 350 us, 1 takes
+// 65 / 272; 8 loads ahead or 4 or 5 blocks an SM: within 3 % or slower.
+constexpr int kLeafFxAhead = 4, kLeafFxChunk = 256;
 template <int CH>
-__global__ void __launch_bounds__(256) k_leaf_fx(const int* __restrict__ cone_box, int ncones, int cone_base,
-                                                 const int* __restrict__ leaf_start, const int* __restrict__ leaf_count,
-                                                 const long long* __restrict__ leaf_off, const int4* __restrict__ L,
-                                                 const int* __restrict__ lexp, const int4* __restrict__ rho,
-                                                 const int* __restrict__ rexp, int P, int Ps, int4* __restrict__ coef,
+__global__ void __launch_bounds__(256) k_leaf_fx(const LeafItem* __restrict__ items, int split, int cone_base,
+                                                 const int4* __restrict__ L, const int* __restrict__ lexp,
+                                                 const double2* __restrict__ rho, int P, int Ps, int4* __restrict__ coef,
                                                  int* __restrict__ cexp) {
+    __shared__ int4 sr[kLeafFxChunk];
     __shared__ FxSum part[CH > 1 ? 256 : 1][2];
-    __shared__ int stop[256];
-    stop[threadIdx.x] = kFxMinExp;
-    const int per_cone = P * CH;
-    const int cpb = blockDim.x / per_cone;
-    const int local = threadIdx.x / per_cone, r = threadIdx.x - local * per_cone;
-    const int ch = r / P, m = r - ch * P;
-    const int c = blockIdx.x * cpb + local;
-    const bool active = local < cpb && c < ncones;
-    FxSum rr{0, 0}, ii{0, 0}, im{0, 0};
-    int n = 0, Er = 0, El = 0;
+    __shared__ int stop[256], smax;
+    const LeafItem I = items[blockIdx.x / split];
+    const int per_cone = P * CH, cpb = blockDim.x / per_cone, tid = threadIdx.x;
+    const int local = tid / per_cone, r = tid - local * per_cone;
+    const int ch = CH > 1 ? r / P : 0, m = r - ch * P;
+    const int q = (blockIdx.x % split) * cpb + local;         // cone of the item
+    const bool active = q < I.cones;
+    const int n = I.n, c = I.cone + q;
+    const int4* Lc = L + I.off + (long long)q * n * P + m;
+    const double2* rh = rho + I.first;
+    int4 ahead[kLeafFxAhead];
+    int El = 0;
     if (active) {
-        const int b = cone_box[c];
-        n = leaf_count[b];
-        Er = rexp[b];
+#pragma unroll
+        for (int u = 0; u < kLeafFxAhead; ++u) if (ch + u * CH < n) ahead[u] = Lc[(long long)(ch + u * CH) * P];
         El = lexp[(long long)c * P + m];
-        const int4* Lc = L + leaf_off[c] + m;
-        const int4* rh = rho + leaf_start[b];
-        for (int f0 = ch; f0 < n; f0 += kFxSumFold * CH) {
-            const int f1 = min(n, f0 + kFxSumFold * CH);
+    }
+    stop[tid] = kFxMinExp;
+    if (tid == 0) smax = 0;
+    __syncthreads();
+    int mx = 0;
+    for (int i = tid; i < n; i += blockDim.x) { const double2 v = rh[i]; mx = max(mx, fx_absmax_hi(v.x, v.y)); }
+    if (mx) atomicMax(&smax, mx);
+    __syncthreads();
+    const int Er = fx_expo(smax), T = fx_rho_top(n);
+    FxSum rr{0, 0}, ii{0, 0}, im{0, 0};
+    auto add = [&](int4 l, int4 d) {
+        fx_sum_mac(rr, l.x, l.y, d.x, d.y);
+        fx_sum_mac(ii, l.z, l.w, d.z, d.w);
+        fx_sum_mac(im, l.x, l.y, d.z, d.w);
+        fx_sum_mac(im, l.z, l.w, d.x, d.y);
+    };
+    for (int c0 = 0; c0 < n; c0 += kLeafFxChunk) {
+        const int c1 = min(n, c0 + kLeafFxChunk);
+        if (c0) __syncthreads();               // the previous chunk has been read
+        for (int i = c0 + tid; i < c1; i += blockDim.x) {
+            const double2 v = rh[i];
+            sr[i - c0] = Er == kFxBad ? make_int4(0, 0, 0, 0) : fx_pack_sum(fx_from(v.x, Er, T), fx_from(v.y, Er, T));
+        }
+        __syncthreads();
+        if (active) {
+            int s = c0 + (ch + CH - c0 % CH) % CH;
+            if (c0 == 0) {
+#pragma unroll
+                for (int u = 0; u < kLeafFxAhead; ++u) if (ch + u * CH < c1) add(ahead[u], sr[ch + u * CH]);
+                s = ch + kLeafFxAhead * CH;
+            }
+            while (s < c1) {
+                const int f = min(c1, s + (kFxSumFold - kLeafFxAhead) * CH);
 #pragma unroll 4
-            for (int s = f0; s < f1; s += CH) {
-                const int4 l = Lc[(long long)s * P], d = rh[s];
-                fx_sum_mac(rr, l.x, l.y, d.x, d.y);
-                fx_sum_mac(ii, l.z, l.w, d.z, d.w);
-                fx_sum_mac(im, l.x, l.y, d.z, d.w);
-                fx_sum_mac(im, l.z, l.w, d.x, d.y);
+                for (; s < f; s += CH) add(Lc[(long long)s * P], sr[s - c0]);
+                if (s < c1) { fx_sum_fold(rr); fx_sum_fold(ii); fx_sum_fold(im); }
             }
             fx_sum_fold(rr); fx_sum_fold(ii); fx_sum_fold(im);
         }
     }
     FxSum re{rr.h - ii.h, rr.m - ii.m};
     if constexpr (CH > 1) {
-        part[threadIdx.x][0] = re; part[threadIdx.x][1] = im;
+        part[tid][0] = re; part[tid][1] = im;
         __syncthreads();
-        if (active && ch == 0)
-            for (int q = 1; q < CH; ++q) {
-                const FxSum a = part[local * per_cone + q * P + m][0], b = part[local * per_cone + q * P + m][1];
-                re.h += a.h; re.m += a.m; im.h += b.h; im.m += b.m;
-            }
     }
-    fx_sum_fold(re); fx_sum_fold(im);
-    const bool bad = Er == kFxBad || El == kFxBad;
+    long long yr = 0, yi = 0;
     int er = 0, ei = 0;
-    const int E0 = bad ? 0 : El + Er - kFxSumTop - fx_rho_top(n);
-    const long long yr = fx_sum_value(re, E0, er), yi = fx_sum_value(im, E0, ei);
-    __syncthreads();
-    if (active && ch == 0) atomicMax(&stop[local], bad ? kFxBad : max(fx_top_of(yr, er), fx_top_of(yi, ei)));
+    if (active && ch == 0) {
+        for (int k = 1; k < CH; ++k) {
+            const FxSum a = part[tid + k * P][0], b = part[tid + k * P][1];
+            re.h += a.h; re.m += a.m; im.h += b.h; im.m += b.m;
+        }
+        fx_sum_fold(re); fx_sum_fold(im);
+        const bool bad = Er == kFxBad || El == kFxBad;
+        const int E0 = bad ? 0 : El + Er - kFxSumTop - T;
+        yr = fx_sum_value(re, E0, er);
+        yi = fx_sum_value(im, E0, ei);
+        atomicMax(&stop[local], bad ? kFxBad : max(fx_top_of(yr, er), fx_top_of(yi, ei)));
+    }
     __syncthreads();
     if (active && ch == 0) {
-        const int E = stop[local] > kFxMaxExp ? kFxBad : stop[local], T = fx_top(P);
-        const long long xr = E == kFxBad ? 0 : fx_align(yr, er, E, T), xi = E == kFxBad ? 0 : fx_align(yi, ei, E, T);
+        const int E = stop[local] > kFxMaxExp ? kFxBad : stop[local], Tc = fx_top(P);
+        const long long xr = E == kFxBad ? 0 : fx_align(yr, er, E, Tc), xi = E == kFxBad ? 0 : fx_align(yi, ei, E, Tc);
         coef[(long long)(cone_base + c) * P + m] = m % Ps ? fx_pack(xr, xi) : fx_pack_raw(xr, xi);
         if (m == 0) cexp[cone_base + c] = E;
     }
@@ -162,25 +195,6 @@ __global__ void __launch_bounds__(256) k_leaf_fix(const int* __restrict__ cone_b
             E == kFxBad ? make_int4(0, 0, 0, 0) : fx_pack_sum(fx_from(v.x, E, kFxSumTop), fx_from(v.y, E, kFxSumTop));
     }
 }
-// the densities of a leaf box as limbs, one exponent per box (a block per box)
-__global__ void __launch_bounds__(64) k_rho_fx(const int* __restrict__ leaf_start, const int* __restrict__ leaf_count,
-                                               const double2* __restrict__ rho, int4* __restrict__ out, int* __restrict__ rexp) {
-    __shared__ int smax;
-    const int b = blockIdx.x, s0 = leaf_start[b], n = leaf_count[b], T = fx_rho_top(n);
-    if (threadIdx.x == 0) smax = 0;
-    __syncthreads();
-    int mx = 0;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) { const double2 v = rho[s0 + i]; mx = max(mx, fx_absmax_hi(v.x, v.y)); }
-    atomicMax(&smax, mx);
-    __syncthreads();
-    const int E = fx_expo(smax);
-    if (threadIdx.x == 0) rexp[b] = E;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const double2 v = rho[s0 + i];
-        out[s0 + i] = E == kFxBad ? make_int4(0, 0, 0, 0) : fx_pack_sum(fx_from(v.x, E, T), fx_from(v.y, E, T));
-    }
-}
-
 // complex64 leaf cones with the table streamed by the tensor memory accelerator.  A persistent
 // CTA walks its cones (blockIdx.x, + gridDim.x, ...) in pieces of at most kLtSrc sources; thread 0
 // keeps kLtStages pieces in flight, each two cp.async.bulk copies (the piece's table rows and its
@@ -635,18 +649,6 @@ __global__ void __launch_bounds__(256) k_propagate_st(int pbegin, int pend, cons
     }
 }
 
-// one interpolation term in the arithmetic type: the interpolant at the term's point times its factor
-template <int PS, int PA>
-__device__ __forceinline__ void add_term(double2& acc, const InterpX& E, const int4* __restrict__ coef, const int* __restrict__ cexp) {
-    const int4* c = coef + (long long)E.cone * (PS * PA);
-    cmac<double>(acc, fx_interp_value<PS, PA>([&](int i) { return c[i]; }, cexp[E.cone], make_longlong2(E.s, E.th)),
-                 make_double2(E.fr, E.fi));
-}
-template <int PS, int PA>
-__device__ __forceinline__ void add_term(float2& acc, const InterpE<float>& E, const float2* __restrict__ coef, const int*) {
-    cmac<float>(acc, interp_eval<float, PS, PA>(coef + (long long)E.cone * (PS * PA), E.s, E.th), make_float2(E.fr, E.fi));
-}
-
 // one warp per (leaf box, up to 32 of its targets, kIbPiece of their interpolation terms), one
 // lane per target.  The targets of a leaf box share their ancestors, hence the same cousin lists
 // in the same order: their j-th terms read the same cousin box, mostly the same cone (2.5-3
@@ -654,12 +656,13 @@ __device__ __forceinline__ void add_term(float2& acc, const InterpE<float>& E, c
 // terms), so the coefficient gathers are broadcasts.  The plan is stored box-transposed (term j of
 // the box's target t at box base + j n + t) for coalesced entry loads.  Each lane writes its
 // piece's sum to part[piece][target]; k_final_t adds the pieces in order.
-template <typename R, int PS, int PA>
+template <int PS, int PA>
 __global__ void __launch_bounds__(256) k_interp_box(const int4* __restrict__ items, int nitems, int N,
                                                     const int* __restrict__ leaf_start, const int* __restrict__ leaf_count,
-                                                    const int* __restrict__ ip_ptr, const InterpT<R>* __restrict__ ipT,
-                                                    const CoefT<R>* __restrict__ coef, const int* __restrict__ cexp,
-                                                    V2<R>* __restrict__ part) {
+                                                    const int* __restrict__ ip_ptr, const InterpE<float>* __restrict__ ipT,
+                                                    const float2* __restrict__ coef, float2* __restrict__ part) {
+    using R = float;
+    constexpr int P = PS * PA;
     const int w = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     if (w >= nitems) return;
     const int lane = threadIdx.x & 31;
@@ -667,27 +670,29 @@ __global__ void __launch_bounds__(256) k_interp_box(const int4* __restrict__ ite
     const int s = leaf_start[I.x], n = leaf_count[I.x];
     const int t = I.y + lane;
     if (t >= n) return;
-    const InterpT<R>* e = ipT + ip_ptr[s] + t;
+    const InterpE<R>* e = ipT + ip_ptr[s] + t;
     V2<R> acc; acc.x = R(0); acc.y = R(0);
     int j = I.z;
-    if constexpr (sizeof(R) == 4) {   // two terms' loads in flight before either is evaluated
-        constexpr int P = PS * PA;
-        for (; j + 1 < I.w; j += 2) {
-            const InterpE<R> E0 = e[(long long)j * n], E1 = e[(long long)(j + 1) * n];
-            V2<R> c0[P], c1[P];
-            const V2<R>* b0 = coef + (long long)E0.cone * P;
-            const V2<R>* b1 = coef + (long long)E1.cone * P;
+    for (; j + 1 < I.w; j += 2) {   // two terms' loads in flight before either is evaluated
+        const InterpE<R> E0 = e[(long long)j * n], E1 = e[(long long)(j + 1) * n];
+        V2<R> c0[P], c1[P];
+        const V2<R>* b0 = coef + (long long)E0.cone * P;
+        const V2<R>* b1 = coef + (long long)E1.cone * P;
 #pragma unroll
-            for (int q = 0; q < P; ++q) { c0[q] = b0[q]; c1[q] = b1[q]; }
-            V2<R> f; f.x = E0.fr; f.y = E0.fi;
-            cmac<R>(acc, interp_eval<R, PS, PA>(c0, E0.s, E0.th), f);
-            f.x = E1.fr; f.y = E1.fi;
-            cmac<R>(acc, interp_eval<R, PS, PA>(c1, E1.s, E1.th), f);
-        }
+        for (int q = 0; q < P; ++q) { c0[q] = b0[q]; c1[q] = b1[q]; }
+        V2<R> f; f.x = E0.fr; f.y = E0.fi;
+        cmac<R>(acc, interp_eval<R, PS, PA>(c0, E0.s, E0.th), f);
+        f.x = E1.fr; f.y = E1.fi;
+        cmac<R>(acc, interp_eval<R, PS, PA>(c1, E1.s, E1.th), f);
     }
     for (; j < I.w; ++j) {
-        const InterpT<R> E = e[(long long)j * n];
-        add_term<PS, PA>(acc, E, coef, cexp);
+        const InterpE<R> E = e[(long long)j * n];
+        V2<R> c[P];
+        const V2<R>* cb = coef + (long long)E.cone * P;
+#pragma unroll
+        for (int q = 0; q < P; ++q) c[q] = cb[q];
+        V2<R> f; f.x = E.fr; f.y = E.fi;
+        cmac<R>(acc, interp_eval<R, PS, PA>(c, E.s, E.th), f);
     }
     part[(long long)(I.z / kIbPiece) * N + s + t] = acc;
 }
@@ -697,22 +702,22 @@ __global__ void __launch_bounds__(256) k_interp_box(const int4* __restrict__ ite
 // its targets, and each warp streams its targets' table rows (coalesced) against them; a target's
 // chunk sums meet in shared memory in chunk order.  Then the target's interpolation pieces
 // (k_interp_box) are added in order and the sum goes to y at the target's original index.
-template <typename R>
 __global__ void __launch_bounds__(256) k_near_box(const int2* __restrict__ items, const int* __restrict__ leaf_start,
                                                   const int* __restrict__ leaf_count, const int* __restrict__ near_src_off,
                                                   const int* __restrict__ near_src, const int* __restrict__ near_rowlen,
-                                                  const long long* __restrict__ near_off, const V2<R>* __restrict__ near,
-                                                  const V2<R>* __restrict__ rho, const int* __restrict__ ip_ptr,
-                                                  const V2<R>* __restrict__ part, int N, const long long* __restrict__ sorting,
+                                                  const long long* __restrict__ near_off, const float2* __restrict__ near,
+                                                  const float2* __restrict__ rho, const int* __restrict__ ip_ptr,
+                                                  const float2* __restrict__ part, int N, const long long* __restrict__ sorting,
                                                   double2* __restrict__ y) {
+    using R = float;
     static_assert(kNearTargets == 4 * 8, "eight warps of four targets");
-    __shared__ V2<R> srho[kNearChunk];
-    __shared__ V2<R> sacc[kNearTargets];
+    __shared__ float2 srho[kNearChunk];
+    __shared__ float2 sacc[kNearTargets];
     const int2 I = items[blockIdx.x];   // leaf box, first target
     const int b = I.x, s = leaf_start[b], n = min(kNearTargets, leaf_count[b] - I.y);
     const int rl = near_rowlen[b];
     const int* src = near_src + near_src_off[b];
-    const V2<R>* rows = near + near_off[b] + (long long)I.y * rl;
+    const float2* rows = near + near_off[b] + (long long)I.y * rl;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x < kNearTargets) { sacc[threadIdx.x].x = R(0); sacc[threadIdx.x].y = R(0); }
     for (int c0 = 0; c0 < rl; c0 += kNearChunk) {
@@ -723,13 +728,13 @@ __global__ void __launch_bounds__(256) k_near_box(const int2* __restrict__ items
         // warp w: targets 4 w .. 4 w + 3 together (four independent row loads per density read)
         const int t0 = 4 * warp;
         if (t0 < n) {
-            V2<R> acc[4];
+            float2 acc[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u) { acc[u].x = R(0); acc[u].y = R(0); }
-            const V2<R>* row = rows + (long long)t0 * rl + c0;
+            const float2* row = rows + (long long)t0 * rl + c0;
 #pragma unroll 2
             for (int e = lane; e < cn; e += 32) {
-                const V2<R> r = srho[e];
+                const float2 r = srho[e];
 #pragma unroll
                 for (int u = 0; u < 4; ++u)
                     if (t0 + u < n) cmac<R>(acc[u], row[(long long)u * rl + e], r);
@@ -744,10 +749,10 @@ __global__ void __launch_bounds__(256) k_near_box(const int2* __restrict__ items
     __syncthreads();
     if (threadIdx.x < n) {
         const int i = s + I.y + threadIdx.x;
-        V2<R> acc = sacc[threadIdx.x];
+        float2 acc = sacc[threadIdx.x];
         if (part) {
             const int npc = (ip_ptr[i + 1] - ip_ptr[i] + kIbPiece - 1) / kIbPiece;
-            for (int q = 0; q < npc; ++q) { const V2<R> a = part[(long long)q * N + i]; acc.x += a.x; acc.y += a.y; }
+            for (int q = 0; q < npc; ++q) { const float2 a = part[(long long)q * N + i]; acc.x += a.x; acc.y += a.y; }
         }
         const long long o = sorting[i];
         double2 v = y[o];
@@ -760,21 +765,22 @@ __device__ __forceinline__ InterpX interp_fx(const InterpE<double>& E) {
     return InterpX{E.cone, E.pad, fx_weight(E.s), fx_weight(E.th), E.fr, E.fi};
 }
 // the interpolation plan of each leaf box transposed: term j of the box's target t moves from
-// ip_ptr[i] + j to ip_ptr[box's first target] + j n + t (every target of a box has as many terms)
-template <typename R>
+// ip_ptr[i] + j to ip_ptr[box's first target] + j n + t (every target of a box has as many terms);
+// complex64, and the FP64 form array by array
 __global__ void k_interp_transpose(int N, const int* __restrict__ point_leaf, const int* __restrict__ leaf_start,
                                    const int* __restrict__ leaf_count, const int* __restrict__ ip_ptr,
-                                   const InterpE<double>* __restrict__ in, InterpT<R>* __restrict__ out) {
+                                   const InterpE<double>* __restrict__ in, InterpE<float>* __restrict__ out, PlanX px) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= N) return;
     const int b = point_leaf[i], s = leaf_start[b], n = leaf_count[b], t = i - s;
     const int base = ip_ptr[s], nt = ip_ptr[i + 1] - ip_ptr[i];
     for (int j = 0; j < nt; ++j) {
         const InterpE<double> E = in[ip_ptr[i] + j];
-        InterpT<R> o{};
-        if constexpr (sizeof(R) == 8) o = interp_fx(E);
-        else { o.cone = E.cone; o.s = (R)E.s; o.th = (R)E.th; o.fr = (R)E.fr; o.fi = (R)E.fi; }
-        out[base + (long long)j * n + t] = o;
+        const long long o = base + (long long)j * n + t;
+        out[o] = InterpE<float>{E.cone, (float)E.s, (float)E.th, (float)E.fr, (float)E.fi};
+        px.child[o] = E.cone;
+        px.st[o] = make_longlong2(fx_weight(E.s), fx_weight(E.th));
+        px.w[o] = make_double2(E.fr, E.fi);
     }
 }
 __global__ void k_interp_fx(const InterpE<double>* __restrict__ in, long long n, InterpX* __restrict__ out) {
@@ -786,47 +792,172 @@ __global__ void k_fx_weights(const double* __restrict__ in, int n, int2* __restr
     if (i < n) { const FxLimb t = fx_split(fx_weight(in[i])); out[i] = make_int2(t.h, t.l); }
 }
 
-// one warp per Morton-sorted target; near row layout [target][neighbour sources], and
+// complex64: one warp per Morton-sorted target; near row layout [target][neighbour sources], and
 // near_src[near_src_off[b] + e] the Morton index of entry e's source in leaf box b's rows, so the
-// lanes stride over one flat row with independent loads.  With `part`, the interpolation terms were
-// summed by k_interp_box: the target's pieces are added in order instead.
-template <typename R, int PS, int PA>
+// lanes stride over one flat row with independent loads.
+template <int PS, int PA>
 __global__ void __launch_bounds__(256) k_final_t(int N, const int* __restrict__ point_leaf, const int* __restrict__ leaf_start,
                                                  const int* __restrict__ near_src_off, const int* __restrict__ near_src,
                                                  const int* __restrict__ near_rowlen,
-                                                 const long long* __restrict__ near_off, const V2<R>* __restrict__ near,
-                                                 const V2<R>* __restrict__ rho, const int* __restrict__ ip_ptr,
-                                                 const InterpT<R>* __restrict__ ip, const CoefT<R>* __restrict__ coef,
-                                                 const int* __restrict__ cexp, const long long* __restrict__ sorting,
-                                                 double2* __restrict__ y, const V2<R>* __restrict__ part) {
+                                                 const long long* __restrict__ near_off, const float2* __restrict__ near,
+                                                 const float2* __restrict__ rho, const int* __restrict__ ip_ptr,
+                                                 const InterpE<float>* __restrict__ ip, const float2* __restrict__ coef,
+                                                 const long long* __restrict__ sorting, double2* __restrict__ y) {
+    constexpr int P = PS * PA;
     const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (i >= N) return;
     const int b = point_leaf[i];
     const int t = i - leaf_start[b];
     const int rl = near_rowlen[b];
-    const V2<R>* row = near + near_off[b] + (long long)t * rl;
+    const float2* row = near + near_off[b] + (long long)t * rl;
     const int* src = near_src + near_src_off[b];
-    V2<R> acc; acc.x = R(0); acc.y = R(0);
+    float2 acc = make_float2(0.f, 0.f);
 #pragma unroll 4
-    for (int e = lane; e < rl; e += 32) cmac<R>(acc, row[e], rho[src[e]]);
-    if (!part) {
-        for (int e = ip_ptr[i] + lane; e < ip_ptr[i + 1]; e += 32) {
-            const InterpT<R> E = ip[e];
-            add_term<PS, PA>(acc, E, coef, cexp);
-        }
+    for (int e = lane; e < rl; e += 32) cmac<float>(acc, row[e], rho[src[e]]);
+    for (int e = ip_ptr[i] + lane; e < ip_ptr[i + 1]; e += 32) {
+        const InterpE<float> E = ip[e];
+        cmac<float>(acc, interp_eval<float, PS, PA>(coef + (long long)E.cone * P, E.s, E.th), make_float2(E.fr, E.fi));
     }
-    acc.x = warp_sum_r<R>(acc.x);
-    acc.y = warp_sum_r<R>(acc.y);
+    acc.x = warp_sum_r<float>(acc.x);
+    acc.y = warp_sum_r<float>(acc.y);
     if (lane == 0) {
-        if (part) {
-            const int npc = (ip_ptr[i + 1] - ip_ptr[i] + kIbPiece - 1) / kIbPiece;
-            for (int q = 0; q < npc; ++q) { const V2<R> a = part[(long long)q * N + i]; acc.x += a.x; acc.y += a.y; }
-        }
         const long long o = sorting[i];
         double2 v = y[o];
         v.x += (double)acc.x; v.y += (double)acc.y;
         y[o] = v;
+    }
+}
+
+// FP64 in fixed point (fixpoint.cuh): near field and interpolation of a leaf box's targets, a block per
+// (box, up to kFinTargets targets) with one record (FinItem).  Interpolation: a thread per (target, term),
+// the targets fastest: the box's targets share their cousin lists, so their j-th terms read the same
+// cousin box and mostly the same cone (broadcast gathers), and the plan is stored in that order; each
+// thread keeps the sum of its target's terms, the threads of a target add up in shared memory.  Near
+// field: the neighbour boxes' densities, loaded while the interpolation runs, are brought to one exponent
+// in shared memory; a warp takes a target's table row with its lanes over the sources, and the lanes'
+// integer sums add up by shuffles.  Bound by latency at small sizes, by the wide multiply-adds else.
+// Kite k = 500 / 2000: 55 / 260 us with FP64 multiply-adds, 35 / 114 us so; 4 blocks an SM against 3:
+// 39 / 119, against 2: 41 / 150.
+template <int PS, int PA>
+__global__ void __launch_bounds__(256, 4) k_final_fx(const FinItem* __restrict__ items, const int* __restrict__ near_src,
+                                                  const int4* __restrict__ near, const int* __restrict__ nexp,
+                                                  const double2* __restrict__ rho, PlanX ip, const int4* __restrict__ coef,
+                                                  const int* __restrict__ cexp, const long long* __restrict__ sorting,
+                                                  double2* __restrict__ y) {
+    constexpr int P = PS * PA, NS = kNearChunk / 2;
+    constexpr int T = kFxSumTop;               // a lane sums at most NS / 32 products
+    __shared__ int4 srho[NS];
+    __shared__ double2 snear[kFinTargets], part[256];
+    __shared__ int smax;
+    const FinItem I = items[blockIdx.x];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, cnt = I.cnt, rl = I.rl;
+    const int* src = near_src + I.src;
+    if (tid == 0) smax = 0;
+    if (tid < cnt) snear[tid] = make_double2(0.0, 0.0);
+    double2 d0 = make_double2(0.0, 0.0);       // this thread's source of the first 256
+    if (tid < rl) d0 = rho[src[tid]];
+    // interpolation
+    const int G = 256 / cnt, g = tid / cnt, t = tid - g * cnt;
+    double2 acc = make_double2(0.0, 0.0);
+    if (g < G) {
+        long long e = I.ip + t + (long long)g * I.n;
+        int cn = 0;
+        longlong2 sn = make_longlong2(0, 0);
+        double2 fn = make_double2(0.0, 0.0);
+        if (g < I.nt) { cn = ip.child[e]; sn = ip.st[e]; fn = ip.w[e]; }
+        for (int j = g; j < I.nt; j += G) {
+            const int c = cn;
+            const longlong2 s = sn;
+            const double2 f = fn;
+            e += (long long)G * I.n;
+            if (j + G < I.nt) { cn = ip.child[e]; sn = ip.st[e]; fn = ip.w[e]; }   // in flight during this term
+            const int4* blk = coef + (long long)c * P;
+            cmac<double>(acc, fx_interp_value<PS, PA>([&](int i) { return blk[i]; }, cexp[c], s), f);
+        }
+    }
+    part[tid] = acc;
+    int mx = fx_absmax_hi(d0.x, d0.y);
+    for (int q = tid + 256; q < rl; q += 256) { const double2 v = rho[src[q]]; mx = max(mx, fx_absmax_hi(v.x, v.y)); }
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    __syncthreads();
+    if (lane == 0) atomicMax(&smax, mx);
+    // the threads of a target: four partial sums
+    double2 a4 = make_double2(0.0, 0.0);
+    const int q4 = tid / cnt, tt = tid - q4 * cnt;
+    if (q4 < 4)
+        for (int k = q4; k < G; k += 4) { const double2 v = part[k * cnt + tt]; a4.x += v.x; a4.y += v.y; }
+    __syncthreads();
+    const int E = fx_expo(smax);
+    for (int c0 = 0; c0 < rl; c0 += NS) {
+        const int cn = min(NS, rl - c0);
+        if (c0) __syncthreads();               // the previous chunk has been read
+        for (int e = tid; e < cn; e += 256) {
+            const double2 v = c0 + e < 256 ? d0 : rho[src[c0 + e]];
+            srho[e] = E == kFxBad ? make_int4(0, 0, 0, 0) : fx_pack_sum(fx_from(v.x, E, T), fx_from(v.y, E, T));
+        }
+        __syncthreads();
+        for (int q = warp; q < cnt; q += 8) {
+            const int4* row = near + I.near + (long long)q * rl + c0;
+            const int En = nexp[I.first + q];
+            FxSum rr{0, 0}, ii{0, 0}, im{0, 0};
+#pragma unroll 4
+            for (int e = lane; e < cn; e += 32) {
+                const int4 a = row[e], d = srho[e];
+                fx_sum_mac(rr, a.x, a.y, d.x, d.y);
+                fx_sum_mac(ii, a.z, a.w, d.z, d.w);
+                fx_sum_mac(im, a.x, a.y, d.z, d.w);
+                fx_sum_mac(im, a.z, a.w, d.x, d.y);
+            }
+            rr.h -= ii.h; rr.m -= ii.m;
+            fx_sum_fold(rr); fx_sum_fold(im);
+            // one shift for the warp that keeps 32 lanes' sum below 2^62
+            const int lz = min(__clzll(rr.h < 0 ? ~rr.h : rr.h), __clzll(im.h < 0 ? ~im.h : im.h));
+            const int sh = min(__reduce_min_sync(0xffffffffu, lz) - 8, kFxSumLow);
+            long long yr = sh >= 0 ? (rr.h << sh) + (rr.m >> (kFxSumLow - sh)) : rr.h >> -sh;
+            long long yi = sh >= 0 ? (im.h << sh) + (im.m >> (kFxSumLow - sh)) : im.h >> -sh;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                yr += __shfl_xor_sync(0xffffffffu, yr, o);
+                yi += __shfl_xor_sync(0xffffffffu, yi, o);
+            }
+            if (lane < 2) {
+                const int e = En + E - kFxSumTop - T + 2 * kFxSumLow - sh;
+                const double v = En == kFxBad || E == kFxBad ? __hiloint2double(0x7ff80000, 0) : fx_scaled(lane ? yi : yr, e);
+                double* o = lane ? &snear[q].y : &snear[q].x;
+                *o += v;
+            }
+        }
+    }
+    if (q4 < 4) part[tid] = a4;
+    __syncthreads();
+    if (tid < cnt) {
+        double2 v = snear[tid];
+        for (int k = 0; k < min(4, G); ++k) { v.x += part[k * cnt + tid].x; v.y += part[k * cnt + tid].y; }
+        const long long o = sorting[I.first + tid];
+        double2 w = y[o];
+        w.x += v.x; w.y += v.y;
+        y[o] = w;
+    }
+}
+// set-up: the FP64 near-field table in place as 27-bit limbs, an exponent per target row (a warp per
+// Morton-sorted target), and its complex64 copy
+__global__ void __launch_bounds__(256) k_near_fix(int N, const int* __restrict__ point_leaf, const int* __restrict__ leaf_start,
+                                                  const int* __restrict__ near_rowlen, const long long* __restrict__ near_off,
+                                                  double2* __restrict__ near, int* __restrict__ nexp, float2* __restrict__ n32) {
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (i >= N) return;
+    const int b = point_leaf[i], rl = near_rowlen[b];
+    const long long o = near_off[b] + (long long)(i - leaf_start[b]) * rl;
+    int mx = 0;
+    for (int e = lane; e < rl; e += 32) { const double2 v = near[o + e]; mx = max(mx, fx_absmax_hi(v.x, v.y)); }
+    const int E = fx_expo(__reduce_max_sync(0xffffffffu, mx));
+    if (lane == 0) nexp[i] = E;
+    for (int e = lane; e < rl; e += 32) {
+        const double2 v = near[o + e];
+        n32[o + e] = make_float2((float)v.x, (float)v.y);
+        reinterpret_cast<int4*>(near)[o + e] =
+            E == kFxBad ? make_int4(0, 0, 0, 0) : fx_pack_sum(fx_from(v.x, E, kFxSumTop), fx_from(v.y, E, kFxSumTop));
     }
 }
 
@@ -864,23 +995,19 @@ void launch_leaf_apply_t(const int* cone_box, int ncones, int cone_base, const i
                                                                        rho, P, coef);
     });
 }
-void launch_leaf_fx(const int* cone_box, int ncones, int cone_base, const int* leaf_start, const int* leaf_count,
-                    const long long* leaf_off, const int4* L, const int* lexp, const int4* rho, const int* rexp, int P, int Ps,
+int leaf_fx_cones(int P) { return 256 / P; }
+void launch_leaf_fx(const LeafItem* items, int nitems, int cone_base, const int4* L, const int* lexp, const double2* rho, int P, int Ps,
                     int4* coef, int* cexp, cudaStream_t s, int chunks) {
-    if (ncones <= 0) return;
+    if (nitems <= 0) return;
     leaf_chunks(P, chunks, [&](auto tag) {
         constexpr int CH = decltype(tag)::value;
-        const int cpb = 256 / (P * CH);
-        k_leaf_fx<CH><<<nblk_a(ncones, cpb), cpb * P * CH, 0, s>>>(cone_box, ncones, cone_base, leaf_start, leaf_count, leaf_off, L, lexp,
-                                                                  rho, rexp, P, Ps, coef, cexp);
+        const int cpb = 256 / (P * CH), split = (leaf_fx_cones(P) + cpb - 1) / cpb;
+        k_leaf_fx<CH><<<(unsigned)nitems * split, cpb * P * CH, 0, s>>>(items, split, cone_base, L, lexp, rho, P, Ps, coef, cexp);
     });
 }
 void launch_leaf_fix(const int* cone_box, int ncones, const int* leaf_count, const long long* leaf_off, int P, int4* L, int* lexp,
                      float2* l32, cudaStream_t s) {
     if (ncones > 0) k_leaf_fix<<<ncones, 256, 0, s>>>(cone_box, leaf_count, leaf_off, P, reinterpret_cast<double2*>(L), lexp, l32);
-}
-void launch_rho_fx(const int* leaf_start, const int* leaf_count, int nleaf, const double2* rho, int4* out, int* rexp, cudaStream_t s) {
-    if (nleaf > 0) k_rho_fx<<<nleaf, 64, 0, s>>>(leaf_start, leaf_count, rho, out, rexp);
 }
 static std::atomic<int> g_leaf_tma_ready{0};
 cudaError_t leaf_tma_init() {
@@ -941,53 +1068,48 @@ void launch_fx_weights(const double* in, int n, int2* out, cudaStream_t s) {
 void launch_interp_fx(const InterpE<double>* in, long long n, InterpX* out, cudaStream_t s) {
     if (n > 0) k_interp_fx<<<nblk_a(n, 256), 256, 0, s>>>(in, n, out);
 }
-template <typename R>
 void launch_final_t(int N, const int* point_leaf, const int* leaf_start, const int* near_src_off, const int* near_src,
-                    const int* near_rowlen, const long long* near_off, const V2<R>* near, const V2<R>* rho,
-                    const int* ip_ptr, const InterpT<R>* ip, const CoefT<R>* coef, const int* cexp, int Ps, int Pang,
-                    const long long* sorting, double2* y, cudaStream_t s, const V2<R>* part) {
-    IFGF_DISPATCH_P(Ps, Pang, (k_final_t<R, PS, PA><<<nblk_a((long long)N * 32, 256), 256, 0, s>>>(
+                    const int* near_rowlen, const long long* near_off, const float2* near, const float2* rho, const int* ip_ptr,
+                    const InterpE<float>* ip, const float2* coef, int Ps, int Pang, const long long* sorting, double2* y,
+                    cudaStream_t s) {
+    IFGF_DISPATCH_P(Ps, Pang, (k_final_t<PS, PA><<<nblk_a((long long)N * 32, 256), 256, 0, s>>>(
                                    N, point_leaf, leaf_start, near_src_off, near_src, near_rowlen, near_off, near, rho,
-                                   ip_ptr, ip, coef, cexp, sorting, y, part)));
+                                   ip_ptr, ip, coef, sorting, y)));
 }
-template <typename R>
-void launch_interp_box(const int4* items, int nitems, int N, const int* leaf_start, const int* leaf_count, const int* ip_ptr,
-                       const InterpT<R>* ipT, const CoefT<R>* coef, const int* cexp, int Ps, int Pang, V2<R>* part, cudaStream_t s) {
+void launch_final_fx(const FinItem* items, int nitems, const int* near_src, const int4* near, const int* nexp, const double2* rho,
+                     PlanX ip, const int4* coef, const int* cexp, int Ps, int Pang, const long long* sorting, double2* y,
+                     cudaStream_t s) {
     if (nitems <= 0) return;
-    IFGF_DISPATCH_P(Ps, Pang, (k_interp_box<R, PS, PA><<<nblk_a((long long)nitems * 32, 256), 256, 0, s>>>(
-                                   items, nitems, N, leaf_start, leaf_count, ip_ptr, ipT, coef, cexp, part)));
+    IFGF_DISPATCH_P(Ps, Pang, (k_final_fx<PS, PA><<<nitems, 256, 0, s>>>(items, near_src, near, nexp, rho, ip, coef, cexp, sorting, y)));
 }
-template <typename R>
+void launch_near_fix(int N, const int* point_leaf, const int* leaf_start, const int* near_rowlen, const long long* near_off, int4* near,
+                     int* nexp, float2* n32, cudaStream_t s) {
+    if (N > 0)
+        k_near_fix<<<nblk_a((long long)N * 32, 256), 256, 0, s>>>(N, point_leaf, leaf_start, near_rowlen, near_off,
+                                                                 reinterpret_cast<double2*>(near), nexp, n32);
+}
+void launch_interp_box(const int4* items, int nitems, int N, const int* leaf_start, const int* leaf_count, const int* ip_ptr,
+                       const InterpE<float>* ipT, const float2* coef, int Ps, int Pang, float2* part, cudaStream_t s) {
+    if (nitems <= 0) return;
+    IFGF_DISPATCH_P(Ps, Pang, (k_interp_box<PS, PA><<<nblk_a((long long)nitems * 32, 256), 256, 0, s>>>(
+                                   items, nitems, N, leaf_start, leaf_count, ip_ptr, ipT, coef, part)));
+}
 void launch_near_box(const int2* items, int nitems, const int* leaf_start, const int* leaf_count, const int* near_src_off,
-                     const int* near_src, const int* near_rowlen, const long long* near_off, const V2<R>* near, const V2<R>* rho,
-                     const int* ip_ptr, const V2<R>* part, int N, const long long* sorting, double2* y, cudaStream_t s) {
+                     const int* near_src, const int* near_rowlen, const long long* near_off, const float2* near, const float2* rho,
+                     const int* ip_ptr, const float2* part, int N, const long long* sorting, double2* y, cudaStream_t s) {
     if (nitems > 0)
-        k_near_box<R><<<nitems, 256, 0, s>>>(items, leaf_start, leaf_count, near_src_off, near_src, near_rowlen, near_off, near,
-                                              rho, ip_ptr, part, N, sorting, y);
+        k_near_box<<<nitems, 256, 0, s>>>(items, leaf_start, leaf_count, near_src_off, near_src, near_rowlen, near_off, near,
+                                           rho, ip_ptr, part, N, sorting, y);
 }
-template <typename R>
 void launch_interp_transpose(int N, const int* point_leaf, const int* leaf_start, const int* leaf_count, const int* ip_ptr,
-                             const InterpE<double>* in, InterpT<R>* out, cudaStream_t s) {
-    if (N > 0) k_interp_transpose<R><<<nblk_a(N, 256), 256, 0, s>>>(N, point_leaf, leaf_start, leaf_count, ip_ptr, in, out);
+                             const InterpE<double>* in, InterpE<float>* out, PlanX px, cudaStream_t s) {
+    if (N > 0) k_interp_transpose<<<nblk_a(N, 256), 256, 0, s>>>(N, point_leaf, leaf_start, leaf_count, ip_ptr, in, out, px);
 }
 void launch_d2f(const double2* a, long long n, float2* b, cudaStream_t s) {
     if (n > 0) k_d2f<<<nblk_a(n, 256), 256, 0, s>>>(a, n, b);
 }
 
-#define IFGF_INSTANTIATE(R)                                                                                          \
-    template void launch_intensities_t<R>(const double2*, const double*, const long long*, int, V2<R>*, cudaStream_t); \
-    template void launch_final_t<R>(int, const int*, const int*, const int*, const int*, const int*,                   \
-                                    const long long*, const V2<R>*, const V2<R>*, const int*, const InterpT<R>*,       \
-                                    const CoefT<R>*, const int*, int, int, const long long*, double2*, cudaStream_t,   \
-                                    const V2<R>*);                                                                     \
-    template void launch_interp_box<R>(const int4*, int, int, const int*, const int*, const int*, const InterpT<R>*,   \
-                                       const CoefT<R>*, const int*, int, int, V2<R>*, cudaStream_t);                   \
-    template void launch_interp_transpose<R>(int, const int*, const int*, const int*, const int*,                      \
-                                             const InterpE<double>*, InterpT<R>*, cudaStream_t);                       \
-    template void launch_near_box<R>(const int2*, int, const int*, const int*, const int*, const int*, const int*,     \
-                                     const long long*, const V2<R>*, const V2<R>*, const int*, const V2<R>*, int,      \
-                                     const long long*, double2*, cudaStream_t);
-IFGF_INSTANTIATE(double)
-IFGF_INSTANTIATE(float)
+template void launch_intensities_t<double>(const double2*, const double*, const long long*, int, double2*, cudaStream_t);
+template void launch_intensities_t<float>(const double2*, const double*, const long long*, int, float2*, cudaStream_t);
 
 }  // namespace ifgf

@@ -125,9 +125,9 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int NPEND>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(NPEND) : "memory"); }
 
-// right-hand sides per lane: two for the complex64 form (a warp covers a 64-wide batch, so
-// every table entry is read once per batch), one for FP64 (register budget)
-template <typename R> struct Rpl { static constexpr int v = sizeof(R) == 4 ? 2 : 1; };
+// right-hand sides per lane of the complex64 kernels: two (a warp covers a 64-wide batch, so every table
+// entry is read once per batch)
+constexpr int kRpl = 2;
 
 // ------------------------------------------------------------------ leaf cones
 // complex64: warp = one leaf cone x 32*RPL right-hand sides, P accumulators per (lane, RHS).  The cone's
@@ -674,15 +674,16 @@ __global__ void __launch_bounds__(32 * kPropBkWarps) k_prop_bk(int pbegin, int p
 }
 
 // ------------------------------------------------------------------ near field + interpolation
-// warp = one Morton-sorted target x 32*RPL right-hand sides; y accumulated at the original index
-template <typename R, int PS, int PA, int RPL>
+// complex64: warp = one Morton-sorted target x 32*RPL right-hand sides; y accumulated at the original index
+template <int PS, int PA, int RPL>
 __global__ void __launch_bounds__(256) k_final_b(int N, const int* __restrict__ point_leaf, const int* __restrict__ leaf_start,
                                                  const int* __restrict__ leaf_count, const int* __restrict__ nbr_ptr,
                                                  const int* __restrict__ nbr_box, const int* __restrict__ near_rowlen,
-                                                 const long long* __restrict__ near_off, const V2<R>* __restrict__ near,
-                                                 const V2<R>* __restrict__ rho, const int* __restrict__ ip_ptr,
-                                                 const InterpE<R>* __restrict__ ip, const V2<R>* __restrict__ coef,
+                                                 const long long* __restrict__ near_off, const float2* __restrict__ near,
+                                                 const float2* __restrict__ rho, const int* __restrict__ ip_ptr,
+                                                 const InterpE<float>* __restrict__ ip, const float2* __restrict__ coef,
                                                  const long long* __restrict__ sorting, int B, double2* __restrict__ yt) {
+    using R = float;
     constexpr int P = PS * PA;
     const int i = blockIdx.x * 8 + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
@@ -751,6 +752,56 @@ __global__ void __launch_bounds__(256) k_final_b(int N, const int* __restrict__ 
         v.x += (double)acc[k].x; v.y += (double)acc[k].y;
         *yo = v;
     }
+}
+
+// FP64 in fixed point (fixpoint.cuh): warp = one Morton-sorted target x 32 right-hand sides.  The
+// neighbour boxes' densities have an exponent per box, so each box's integer sum is added up in FP64.
+__global__ void __launch_bounds__(256) k_near_bx(int N, const int* __restrict__ point_leaf, const int* __restrict__ leaf_start,
+                                                 const int* __restrict__ leaf_count, const int* __restrict__ nbr_ptr,
+                                                 const int* __restrict__ nbr_box, const int* __restrict__ near_rowlen,
+                                                 const long long* __restrict__ near_off, const int4* __restrict__ near,
+                                                 const int* __restrict__ nexp, const int4* __restrict__ rho,
+                                                 const int* __restrict__ rexp, const long long* __restrict__ sorting, int B,
+                                                 double2* __restrict__ yt) {
+    const int i = blockIdx.x * 8 + (threadIdx.x >> 5);
+    const int r = blockIdx.y * 32 + (threadIdx.x & 31);
+    if (i >= N || r >= B) return;
+    const int b = point_leaf[i], En = nexp[i];
+    const int4* row = near + near_off[b] + (long long)(i - leaf_start[b]) * near_rowlen[b];
+    double2 acc = make_double2(0.0, 0.0);
+    for (int q = nbr_ptr[b]; q < nbr_ptr[b + 1]; ++q) {
+        const int bb = nbr_box[q], c = leaf_count[bb];
+        const int4* rh = rho + (long long)leaf_start[bb] * B + r;
+        const int Er = rexp[(long long)bb * B + r];
+        FxSum rr{0, 0}, ii{0, 0}, im{0, 0};
+        for (int f0 = 0; f0 < c; f0 += kFxSumFold) {
+            const int f1 = min(c, f0 + kFxSumFold);
+#pragma unroll 4
+            for (int s = f0; s < f1; ++s) {
+                const int4 a = row[s], d = rh[(long long)s * B];
+                fx_sum_mac(rr, a.x, a.y, d.x, d.y);
+                fx_sum_mac(ii, a.z, a.w, d.z, d.w);
+                fx_sum_mac(im, a.x, a.y, d.z, d.w);
+                fx_sum_mac(im, a.z, a.w, d.x, d.y);
+            }
+            fx_sum_fold(rr); fx_sum_fold(ii); fx_sum_fold(im);
+        }
+        row += c;
+        rr.h -= ii.h; rr.m -= ii.m;
+        fx_sum_fold(rr);
+        if (En == kFxBad || Er == kFxBad) {
+            acc.x = acc.y = __hiloint2double(0x7ff80000, 0);
+        } else {
+            const int E0 = En + Er - kFxSumTop - fx_rho_top(c);
+            int er, ei;
+            const long long yr = fx_sum_value(rr, E0, er), yi = fx_sum_value(im, E0, ei);
+            acc.x += fx_scaled(yr, er); acc.y += fx_scaled(yi, ei);
+        }
+    }
+    double2* yo = yt + sorting[i] * B + r;
+    double2 v = *yo;
+    v.x += acc.x; v.y += acc.y;
+    *yo = v;
 }
 
 // ------------------------------------------------------------------ interpolation grouped by cone
@@ -922,7 +973,7 @@ void launch_leaf_b(const int* cone_box, int ncones, int cone_base, const int* le
                    const long long* leaf_off, const float2* L, const float2* rho, int Ps, int Pang, int B, float2* coef,
                    cudaStream_t s) {
     if (ncones <= 0) return;
-    constexpr int RPL = Rpl<float>::v;
+    constexpr int RPL = kRpl;
     const dim3 grid(nblk_b(ncones, kLeafWarps), nblk_b(B, 32 * RPL));
     IFGF_DISPATCH_P(Ps, Pang, (k_leaf_b<PS * PA, RPL><<<grid, kLeafWarps * 32, 0, s>>>(
                                    cone_box, ncones, cone_base, leaf_start, leaf_count, leaf_off, L, rho, B, coef)));
@@ -948,7 +999,7 @@ void launch_leaf_bx(const int* cone_box, int ncones, int cone_base, const int* l
 void launch_prop_b(int pbegin, int pend, const long long* pp_ptr, const int* pp_nchild, const PropB<float>* pb, int Ps, int Pang,
                    const float* Gsep, int B, float2* coef, cudaStream_t s) {
     if (pend <= pbegin) return;
-    constexpr int RPL = Rpl<float>::v;
+    constexpr int RPL = kRpl;
     IFGF_DISPATCH_P(Ps, Pang, {
         constexpr int WPB = PropBlock<PS * PA, RPL>::W;
         const dim3 grid(nblk_b(pend - pbegin, WPB), nblk_b(B, 32 * RPL));
@@ -992,16 +1043,22 @@ bool launch_prop_bk(int pbegin, int pend, const long long* pp_ptr, const int* pp
     k_prop_bk<5, 5><<<pend - pbegin, 32 * kPropBkWarps, 0, s>>>(pbegin, pend, pp_ptr, pp_nchild, pb, Gsep, B, coef, err);
     return true;
 }
-template <typename R>
 void launch_final_b(int N, const int* point_leaf, const int* leaf_start, const int* leaf_count, const int* nbr_ptr,
-                    const int* nbr_box, const int* near_rowlen, const long long* near_off, const V2<R>* near,
-                    const V2<R>* rho, const int* ip_ptr, const InterpE<R>* ip, const V2<R>* coef, int Ps, int Pang,
+                    const int* nbr_box, const int* near_rowlen, const long long* near_off, const float2* near,
+                    const float2* rho, const int* ip_ptr, const InterpE<float>* ip, const float2* coef, int Ps, int Pang,
                     const long long* sorting, int B, double2* yt, cudaStream_t s) {
-    constexpr int RPL = Rpl<R>::v;
+    constexpr int RPL = kRpl;
     const dim3 grid(nblk_b(N, 8), nblk_b(B, 32 * RPL));
-    IFGF_DISPATCH_P(Ps, Pang, (k_final_b<R, PS, PA, RPL><<<grid, 256, 0, s>>>(N, point_leaf, leaf_start, leaf_count,
-                                                                             nbr_ptr, nbr_box, near_rowlen, near_off, near,
-                                                                             rho, ip_ptr, ip, coef, sorting, B, yt)));
+    IFGF_DISPATCH_P(Ps, Pang, (k_final_b<PS, PA, RPL><<<grid, 256, 0, s>>>(N, point_leaf, leaf_start, leaf_count,
+                                                                          nbr_ptr, nbr_box, near_rowlen, near_off, near,
+                                                                          rho, ip_ptr, ip, coef, sorting, B, yt)));
+}
+void launch_near_bx(int N, const int* point_leaf, const int* leaf_start, const int* leaf_count, const int* nbr_ptr, const int* nbr_box,
+                    const int* near_rowlen, const long long* near_off, const int4* near, const int* nexp, const int4* rho,
+                    const int* rexp, const long long* sorting, int B, double2* yt, cudaStream_t s) {
+    if (N > 0 && B > 0)
+        k_near_bx<<<dim3(nblk_b(N, 8), nblk_b(B, 32)), 256, 0, s>>>(N, point_leaf, leaf_start, leaf_count, nbr_ptr, nbr_box, near_rowlen,
+                                                                   near_off, near, nexp, rho, rexp, sorting, B, yt);
 }
 void launch_bdot(const double2* V, long long ldc, int ncols, const double2* w, long long N, int B, double2* part,
                  double2* h, double2* Hcol, int add, int sqrt_row, cudaStream_t s) {
@@ -1018,12 +1075,5 @@ void launch_bupdate(const double2* V, long long ldc, int ncols, const double2* h
 void launch_bscale(const double2* w, const double2* hn, long long N, int B, double2* out, cudaStream_t s) {
     k_bscale<<<nblk_b(N * B, 256), 256, 0, s>>>(w, hn, N * B, B, out);
 }
-
-#define IFGF_BATCH_INSTANTIATE(R)                                                                                       \
-    template void launch_final_b<R>(int, const int*, const int*, const int*, const int*, const int*, const int*,        \
-                                    const long long*, const V2<R>*, const V2<R>*, const int*, const InterpE<R>*,        \
-                                    const V2<R>*, int, int, const long long*, int, double2*, cudaStream_t);
-IFGF_BATCH_INSTANTIATE(double)
-IFGF_BATCH_INSTANTIATE(float)
 
 }  // namespace ifgf

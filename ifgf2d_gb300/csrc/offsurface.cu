@@ -17,6 +17,7 @@ struct EvalWork {
     DBuf<double> tx, ty;
     DBuf<int> leaf_cone_box;
     DBuf<long long> leaf_off;
+    DBuf<LeafItem> leaf_items;
     DBuf<LeafNode> nodes;
     DBuf<int4> leafL;
     DBuf<int> lexp;
@@ -115,6 +116,7 @@ extern "C" int ifgf2d_eval_offsurface_setup(ifgf2d_ctx* ctx, long long m, const 
         CK(W.nodes.alloc((size_t)ncl * P));
         CK(build_leaf_nodes(E, W.nodes.p, s));
         CK(W.leaf_cone_box.upload(LD.cone_box)); CK(W.leaf_off.upload(loff));
+        CK(W.leaf_items.upload(leaf_fx_items(LD.cone_box, E.leaf_start, E.leaf_count, loff, P)));
         CK(W.leafL.alloc(loff[ncl]));
         launch_leaf_setup(W.leaf_cone_box.p, ncl, ctx->leaf_start.p, ctx->leaf_count.p, W.leaf_off.p, W.nodes.p, ctx->xs_s.p,
                           ctx->ys_s.p, ctx->nxs_s.p, ctx->nys_s.p, ctx->T.Ps, ctx->T.Pang, ctx->k, ctx->form, ctx->eta, ctx->Gsep.p,
@@ -167,9 +169,8 @@ extern "C" int ifgf2d_eval_offsurface(ifgf2d_ctx* ctx, const double* density, do
     CK(cudaMemcpyAsync(ctx->vin.p, density, sizeof(double2) * N, cudaMemcpyHostToDevice, s));
     launch_intensities(ctx->vin.p, ctx->wq.p, ctx->sorting.p, N, ctx->rho.p, s);
     const TreeLevel& LD = E.L[D];
-    launch_rho_fx(ctx->leaf_start.p, ctx->leaf_count.p, (int)ctx->T.leaf_start.size(), ctx->rho.p, ctx->rhox.p, ctx->rexp.p, s);
-    launch_leaf_fx(W.leaf_cone_box.p, (int)LD.cone_nonrel.size(), LD.cone_base, ctx->leaf_start.p, ctx->leaf_count.p, W.leaf_off.p,
-                   W.leafL.p, W.lexp.p, ctx->rhox.p, ctx->rexp.p, P, E.Ps, W.coef.p, W.cexp.p, s);
+    launch_leaf_fx(W.leaf_items.p, (int)W.leaf_items.n, LD.cone_base, W.leafL.p, W.lexp.p, ctx->rho.p, P, E.Ps, W.coef.p,
+                   W.cexp.p, s);
     for (int l = D; l >= 3; --l) {
         const TreeLevel& Lp = E.L[l - 1];
         launch_propagate_fx(Lp.cone_base, Lp.cone_base + (int)Lp.cone_nonrel.size(), W.pp.view(), W.stage.level(l), E.Ps, E.Pang,

@@ -300,8 +300,8 @@ int ifgf2d_apply_timed(ifgf2d_ctx* ctx, const void* d_x, void* d_y, int mode, do
 #define IFGF2D_BATCH_TC_LEAF_FP32 4     /* leaf-cone sums, three TF32 terms per operand (6 products) */
 #define IFGF2D_BATCH_BULK_PROPAGATION 8 /* FP32 FMA propagation, child coefficients staged by TMA bulk copies */
 #define IFGF2D_BATCH_GROUPED_INTERP 16  /* complex64 interpolation grouped by cone per leaf box */
-#define IFGF2D_SINGLE_INTERP_BY_BOX_FP64 32  /* single vector, FP64: interpolation by leaf box, a lane per target */
-#define IFGF2D_SINGLE_INTERP_BY_BOX_C64 64   /* single vector, complex64: the same */
+#define IFGF2D_SINGLE_INTERP_BY_BOX_FP64 32  /* single vector, FP64: accepted; the FP64 form always works by leaf box */
+#define IFGF2D_SINGLE_INTERP_BY_BOX_C64 64   /* single vector, complex64: interpolation by leaf box, a lane per target */
 int ifgf2d_tuning_size(void);
 int ifgf2d_autotune(ifgf2d_ctx* ctx, int reps, int* choices);
 int ifgf2d_get_tuning(const ifgf2d_ctx* ctx, int* choices);

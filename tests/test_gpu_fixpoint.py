@@ -69,3 +69,40 @@ def test_gpu_fixpoint_zero_isolated_and_nonfinite(lib, oracle):
         fm.apply_device(v, out)
         torch.cuda.synchronize()
         assert not bool(torch.isfinite(torch.view_as_real(out)).all(dim=1).any())
+
+
+@pytest.mark.parametrize("Ps,Pang,npatch,nlevels", [(5, 5, 300, 4), (3, 3, 110, 0), (7, 7, 64, 0)])
+def test_gpu_fixpoint_near_and_leaf_sums(lib, oracle, Ps, Pang, npatch, nlevels):
+    """Leaf boxes beyond one staged chunk of sources (256) and near rows beyond one (512) on a shallow
+    tree; boxes of a few sources on a deep one.  The far sums against the oracle's to the tables' rounding,
+    batches of 1, 33 and 64 against the single vector to the bound above."""
+    import torch
+    k = 60.0
+    fm = lib.ForwardMap(0.02, [lib.Kite()], (), 1.0, k, Np=16, Ps=Ps, Pang=Pang, patches_per_curve=npatch, formulation="combined")
+    fm.precomps_and_setup(k, nlevels)
+    om = oracle.OracleForwardMap([oracle.curve_kite()], 16, 0.02, 1.0, k, patches_per_curve=npatch, formulation="combined")
+    om.precompute(k)
+    om.setup_ifgf(k, fm.nlevels, Ps, Pang)
+    n = fm.total_num_unknowns_
+    g = np.random.default_rng(npatch)
+    X = np.stack([_f32(g, n) for _ in range(64)], axis=1)
+    X[:, 3] = 0
+    X[:, 5] *= 2.0 ** -600
+    far, faro = fm.ifgf_far(X[:, 0]), om.ifgf_far(X[:, 0])
+    assert np.linalg.norm(far - faro) < 1e-11 * np.linalg.norm(faro)
+    Y = np.stack([fm.compute_Ax_acc(X[:, r]) for r in range(64)], axis=1)
+    for B in (1, 33, 64):
+        Yb = fm.apply_batch(X[:, :B])
+        s = 2.0 ** np.array([600.0 if r == 5 else 0.0 for r in range(B)])
+        assert np.all(np.linalg.norm((Yb - Y[:, :B]) * s, axis=0) <= 4e-15 * np.linalg.norm(Y[:, :B] * s, axis=0)), B
+    x = torch.from_numpy(np.ascontiguousarray(X.T)).cuda()
+    y, yn = torch.empty_like(x), torch.empty_like(x)
+    torch.cuda.synchronize()
+    fm.apply_batch_device(x, y, 64)
+    x[7, n // 2] = complex(np.nan, 0.0)           # a column's NaN stays in it
+    torch.cuda.synchronize()
+    fm.apply_batch_device(x, yn, 64)
+    torch.cuda.synchronize()
+    fin = torch.isfinite(torch.view_as_real(yn)).all(dim=2)
+    keep = torch.arange(64, device="cuda") != 7
+    assert not bool(fin[7].any()) and bool(fin[keep].all()) and torch.equal(yn[keep], y[keep])
