@@ -8,11 +8,16 @@ three regions (see hankel.cuh):
   x >= XC          Hankel asymptotic expansion (A&S 9.2.5-9.2.10), P and Q as polynomials
                    in 1/x^2 with coefficients (nu, m) / 2^m.
 
+green_tables.inc holds the fixed-point evaluator's tables (see green_fx.cuh): P and Q of
+H_nu = sqrt(2 / (pi x)) e^{i(x - pi/4 - nu pi/2)} (P_nu + i Q_nu) as polynomials of degree 6 in the
+position t in [-1/2, 1/2) within dyadic pieces of w = 1/x <= 1, and sin / cos of pi z / 2.
+
 All coefficients are computed here with mpmath at 50 digits and written as C hex-float
-literals.  Run:  python gen_hankel_tables.py  (writes hankel_tables.inc next to itself).
+literals and integers.  Run:  python gen_hankel_tables.py  (writes both files next to itself).
 """
 import os
 import mpmath as mp
+import numpy as np
 
 mp.mp.dps = 50
 
@@ -67,7 +72,74 @@ def asym_coeffs(nu):
     return P[:NASY], Q[:NASY]
 
 
+GX_BITS = [6, 5, 4, 4, 3, 2, 1, 0]      # log2 of the pieces of octave o: x in (2^o, 2^(o+1)]; one more for x > 2^8
+GX_Q3 = 54                               # scale of the 32-bit coefficient of t^3
+MAGIC = 0x4B400000                       # bits of 1.5 * 2^23
+
+
+def phase_free(nu, w):
+    if w == 0:
+        return mp.mpc(1, 0)
+    x = 1 / w
+    return mp.sqrt(mp.pi * x / 2) * mp.exp(-1j * (x - mp.pi / 4 - nu * mp.pi / 2)) * mp.hankel1(nu, x)
+
+
+def piece_monomials(nu, a, b, deg=6):
+    n = deg + 1
+    c = cheb_fit(lambda w: phase_free(nu, w), a, b, deg + 6)
+    assert mp.fsum(abs(x) for x in c[n:]) < mp.mpf(2) ** -61
+    T = [[mp.mpf(1)], [mp.mpf(0), mp.mpf(1)]]
+    for k in range(2, n):
+        p = [mp.mpf(0)] + [2 * x for x in T[-1]]
+        for i, x in enumerate(T[-2]):
+            p[i] -= x
+        T.append(p)
+    m = [mp.fsum(c[k] * T[k][i] for k in range(n) if i < len(T[k])) * 2 ** i for i in range(n)]
+    return m
+
+
+def green_tables():
+    out = ["// Generated by gen_hankel_tables.py -- do not edit."]
+    pieces = []
+    for o, nb in enumerate(GX_BITS):
+        lo = mp.mpf(2) ** -(o + 1)
+        pieces += [(lo * (1 + mp.mpf(i) / 2 ** nb), lo * (1 + mp.mpf(i + 1) / 2 ** nb)) for i in range(2 ** nb)]
+    pieces.append((mp.mpf(0), mp.mpf(2) ** -len(GX_BITS)))
+    out.append(f"#define GX_PIECES {len(pieces)}")
+    out.append(f"#define GX_Q3 {GX_Q3}")
+
+    def q(v, s):
+        return int(mp.nint(v * mp.mpf(2) ** s))
+
+    def w64(v):
+        v &= (1 << 64) - 1
+        return [v & 0xFFFFFFFF, v >> 32]
+
+    def f32(v):
+        return int(np.float32(float(v)).view(np.uint32))
+
+    rows = []
+    for a, b in pieces:
+        m = [piece_monomials(nu, a, b) for nu in (0, 1)]
+        poly = [[x.real for x in m[0]], [x.imag for x in m[0]], [x.real for x in m[1]], [x.imag for x in m[1]]]
+        r = []
+        for p in poly:
+            r += w64(q(p[0], 62)) + w64(q(p[1], 62))
+        for p in poly:
+            r += w64(q(p[2], 62))
+        for p in poly:
+            c3, f = q(p[3], GX_Q3), [x * mp.mpf(2) ** GX_Q3 for x in p[4:7]]
+            assert abs(c3) < 2 ** 31 and abs(f[0]) / 2 + abs(f[1]) / 4 + abs(f[2]) / 8 < 2 ** 22
+            r += [(c3 - MAGIC) & 0xFFFFFFFF] + [f32(x) for x in f]
+        rows.append(r)
+    out.append("// [piece][10]: (c0, c1) of P0, Q0, P1, Q1; c2 of (P0, Q0), (P1, Q1); (c3, c4, c5, c6) of P0, Q0, P1, Q1")
+    out.append(f"GX_TABLE unsigned gx_table[GX_PIECES * 40] = {{" + ", ".join(f"0x{x:x}u" for r in rows for x in r) + "};")
+    return out
+
+
 def main():
+    with open(os.path.join(os.path.dirname(os.path.abspath(__file__)), "green_tables.inc"), "w") as f:
+        f.write("\n".join(green_tables()) + "\n")
     out = []
     out.append("// Generated by gen_hankel_tables.py -- do not edit.")
     out.append(f"#define HK_XA {XA!r}")

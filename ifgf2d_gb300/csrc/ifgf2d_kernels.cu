@@ -11,7 +11,7 @@
 //   final        near field + all-level interpolation + un-permute
 //                                                             BoxTree.h:614-683, 876-937, 1063-1069
 #include "ifgf2d_kernels.cuh"
-#include "hankel.cuh"
+#include "green_fx.cuh"
 
 namespace ifgf {
 
@@ -184,13 +184,16 @@ __global__ void k_sing_apply(const double2* __restrict__ x, const double2* __res
 // ------------------------------------------------------------------ apply: direct far sum
 // Tiled all-pairs sum, one thread per target, sources staged in shared memory 128 at a time.
 // A tile whose patch range holds neither the target's patch nor a patch the target is
-// near-singular to runs without exclusion tests.
+// near-singular to runs without exclusion tests.  The Green values come from green_fx.cuh, which spreads
+// them over the integer and FP64 pipes (about 1000 cycles of each a warp); on the FP64 pipe alone a value
+// took about 130 operations of 64 cycles.  16385 targets of 8192 sources at k = 500: 30.6 -> 3.9 ms.
+// The tables of the set-up keep green_form: their complex64 copies stay what they were bit for bit.
 constexpr int kTile = 128;
 __global__ void __launch_bounds__(kTile) k_direct_far(const double* __restrict__ tx, const double* __restrict__ ty, int nt,
                              const int* __restrict__ t_patch, const int* __restrict__ t_nsp_ptr, const int* __restrict__ t_nsp,
                              const double* __restrict__ sx, const double* __restrict__ sy, const double* __restrict__ snx,
                              const double* __restrict__ sny, const int* __restrict__ s_patch,
-                             const double2* __restrict__ rho, int ns, double k, int form, double eta,
+                             const double2* __restrict__ rho, int ns, const __grid_constant__ GreenFx K,
                              double2* __restrict__ y, int accumulate) {
     __shared__ double shx[kTile], shy[kTile], shnx[kTile], shny[kTile];
     __shared__ double2 shr[kTile];
@@ -217,13 +220,13 @@ __global__ void __launch_bounds__(kTile) k_direct_far(const double* __restrict__
         bool check = s_patch && (pi >= pa && pi <= pb);
         for (int q = 0; q < nex; ++q) check |= (ex[q] >= pa && ex[q] <= pb);
         if (!check) {
-            for (int j = 0; j < n; ++j) cfma(acc, green_form(form, xi - shx[j], yi - shy[j], shnx[j], shny[j], k, eta), shr[j]);
+            for (int j = 0; j < n; ++j) cfma(acc, green(K, xi - shx[j], yi - shy[j], shnx[j], shny[j]), shr[j]);
         } else {
             for (int j = 0; j < n; ++j) {
                 const int pj = shp[j];
                 bool skip = (pj == pi);
                 for (int q = 0; q < nex; ++q) skip |= (ex[q] == pj);
-                if (!skip) cfma(acc, green_form(form, xi - shx[j], yi - shy[j], shnx[j], shny[j], k, eta), shr[j]);
+                if (!skip) cfma(acc, green(K, xi - shx[j], yi - shy[j], shnx[j], shny[j]), shr[j]);
             }
         }
     }
@@ -235,13 +238,13 @@ __global__ void __launch_bounds__(kTile) k_direct_far(const double* __restrict__
 // The same sum with one 128-thread block per target, for target counts that would leave most
 // SMs idle with one thread per target (N = 200: 2 blocks).  Thread t takes sources t, t + 128, ...;
 // the partial sums combine in a fixed order (warp butterfly, then warps 0..3), so the result
-// does not depend on scheduling.
+// does not depend on scheduling.  N = 200 at k = 10, with three callers: 21.7 -> 8.4 us by green_fx.cuh.
 constexpr int kDirectSplitBelow = 2 * 152 * kTile;
 __global__ void __launch_bounds__(kTile) k_direct_far_split(const double* __restrict__ tx, const double* __restrict__ ty,
                              const int* __restrict__ t_patch, const int* __restrict__ t_nsp_ptr, const int* __restrict__ t_nsp,
                              const double* __restrict__ sx, const double* __restrict__ sy, const double* __restrict__ snx,
                              const double* __restrict__ sny, const int* __restrict__ s_patch,
-                             const double2* __restrict__ rho, int ns, double k, int form, double eta,
+                             const double2* __restrict__ rho, int ns, const __grid_constant__ GreenFx K,
                              double2* __restrict__ y, int accumulate) {
     __shared__ double2 part[kTile / 32];
     const int i = blockIdx.x;
@@ -257,7 +260,7 @@ __global__ void __launch_bounds__(kTile) k_direct_far_split(const double* __rest
             skip = (pj == pi);
             for (int q = 0; q < nex; ++q) skip |= (ex[q] == pj);
         }
-        if (!skip) cfma(acc, green_form(form, xi - sx[j], yi - sy[j], snx ? snx[j] : 0.0, sny ? sny[j] : 0.0, k, eta), rho[j]);
+        if (!skip) cfma(acc, green(K, xi - sx[j], yi - sy[j], snx ? snx[j] : 0.0, sny ? sny[j] : 0.0), rho[j]);
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -502,12 +505,13 @@ void launch_direct_far(const double* tx, const double* ty, int nt, const int* t_
                        const double* sx, const double* sy, const double* snx, const double* sny, const int* s_patch,
                        const double2* rho, int ns, double k, int form, double eta, double2* y, int accumulate, cudaStream_t s) {
     if (nt <= 0) return;
+    const GreenFx K = green_fx(form, k, eta);
     if (nt < kDirectSplitBelow)
-        k_direct_far_split<<<nt, kTile, 0, s>>>(tx, ty, t_patch, t_nsp_ptr, t_nsp, sx, sy, snx, sny, s_patch, rho, ns, k, form, eta,
-                                                y, accumulate);
+        k_direct_far_split<<<nt, kTile, 0, s>>>(tx, ty, t_patch, t_nsp_ptr, t_nsp, sx, sy, snx, sny, s_patch, rho, ns, K, y,
+                                                accumulate);
     else
-        k_direct_far<<<nblk(nt, kTile), kTile, 0, s>>>(tx, ty, nt, t_patch, t_nsp_ptr, t_nsp, sx, sy, snx, sny, s_patch, rho, ns, k,
-                                                       form, eta, y, accumulate);
+        k_direct_far<<<nblk(nt, kTile), kTile, 0, s>>>(tx, ty, nt, t_patch, t_nsp_ptr, t_nsp, sx, sy, snx, sny, s_patch, rho, ns, K,
+                                                       y, accumulate);
 }
 cudaError_t preload_direct_kernels() {
     cudaFuncAttributes a;

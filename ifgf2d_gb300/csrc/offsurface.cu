@@ -8,7 +8,7 @@
 //   * the cone interpolants of the boxes in its interaction lists, level by level,
 // which covers every source once.  Targets may lie anywhere, also outside the root box.
 #include "context.hpp"
-#include "hankel.cuh"
+#include "green_fx.cuh"
 #include "fixpoint.cuh"
 
 struct EvalWork {
@@ -47,7 +47,7 @@ __global__ void __launch_bounds__(256) k_eval_targets(long long M, const double*
                                                       const int* __restrict__ leaf_start, const int* __restrict__ leaf_count,
                                                       const double* __restrict__ xs, const double* __restrict__ ys,
                                                       const double* __restrict__ nxs, const double* __restrict__ nys,
-                                                      const double2* __restrict__ rho, double k, int form, double eta,
+                                                      const double2* __restrict__ rho, const __grid_constant__ GreenFx K,
                                                       const int* __restrict__ ip_ptr, const InterpX* __restrict__ ip,
                                                       const int4* __restrict__ coef, const int* __restrict__ cexp,
                                                       double2* __restrict__ out) {
@@ -62,7 +62,7 @@ __global__ void __launch_bounds__(256) k_eval_targets(long long M, const double*
         const int s0 = leaf_start[b], n = leaf_count[b];
         for (int s = lane; s < n; s += 32) {
             const int j = s0 + s;
-            const double2 g = green_form(form, x - xs[j], y - ys[j], nxs[j], nys[j], k, eta);
+            const double2 g = green(K, x - xs[j], y - ys[j], nxs[j], nys[j]);
             cmac<double>(acc, g, rho[j]);
         }
     }
@@ -84,7 +84,7 @@ void launch_eval_targets(long long M, const double* tx, const double* ty, const 
     if (M <= 0) return;
     const unsigned grid = (unsigned)((M * 32 + 255) / 256);
     IFGF_DISPATCH_P(Ps, Pang, (k_eval_targets<PS, PA><<<grid, 256, 0, s>>>(M, tx, ty, nb_ptr, nb_box, leaf_start, leaf_count, xs,
-                                                                          ys, nxs, nys, rho, k, form, eta, ip_ptr, ip, coef,
+                                                                          ys, nxs, nys, rho, green_fx(form, k, eta), ip_ptr, ip, coef,
                                                                           cexp, out)));
 }
 
