@@ -220,6 +220,7 @@ struct ifgf2d_ctx {
     DBuf<int> leaf_cone_box;
     DBuf<long long> leaf_off;
     DBuf<LeafItem> leaf_items;      // work items of the FP64 leaf sums
+    DBuf<int4> leaf_cones;          // the complex64 leaf sums' cones
     DBuf<LeafNode> leaf_nodes_d;
     DBuf<int4> leafL;               // the FP64 form's leaf-cone tables: fixed-point limbs, with
     DBuf<int> lexp;                 // one exponent per cone and coefficient (FP64 values until set-up fixes them)
@@ -240,14 +241,11 @@ struct ifgf2d_ctx {
     DBuf<PropE<float>> pp32;
     DBuf<InterpE<float>> ip32;
     DBuf<float> Gsep32;
-    // interpolation by leaf box: work items, the plan box-transposed in both precisions, and the
-    // complex64 pieces' sums per target
-    DBuf<int4> ib_items;
-    DBuf<int2> nb_items;            // near field by leaf box (k_near_box): (box, first of up to 32 targets)
+    // near field and interpolation by leaf box: work items (k_final_fx, k_final_q), the plan
+    // box-transposed in both precisions
     PlanBuf ipT;
-    DBuf<FinItem> fx_items;         // work items of k_final_fx
+    DBuf<FinItem> fx_items, fin32_items;
     DBuf<InterpE<float>> ip32T;
-    DBuf<float2> ib_part32;
     // work vectors
     DBuf<double2> rho, vin, vout;
     std::unique_ptr<GmresWork> gw;
@@ -292,11 +290,19 @@ static inline bool all_finite(const double* v, long long n) {
 }
 
 namespace ifgf {
-// the work items of launch_leaf_fx: runs of up to leaf_fx_cones cones of one box
-inline std::vector<LeafItem> leaf_fx_items(const std::vector<int>& cone_box, const std::vector<int>& start, const std::vector<int>& count,
+// per leaf cone: table offset (two ints), first source, sources
+inline std::vector<int4> leaf_cone_list(const std::vector<int>& cone_box, const std::vector<int>& start, const std::vector<int>& count,
+                                        const std::vector<long long>& off) {
+    std::vector<int4> d(cone_box.size());
+    for (size_t c = 0; c < d.size(); ++c)
+        d[c] = make_int4((int)off[c], (int)(off[c] >> 32), start[cone_box[c]], count[cone_box[c]]);
+    return d;
+}
+// the work items of the FP64 leaf sums: runs of up to leaf_item_cones cones of one box
+inline std::vector<LeafItem> leaf_item_list(const std::vector<int>& cone_box, const std::vector<int>& start, const std::vector<int>& count,
                                            const std::vector<long long>& off, int P) {
     std::vector<LeafItem> items;
-    const int nc = (int)cone_box.size(), most = leaf_fx_cones(P);
+    const int nc = (int)cone_box.size(), most = leaf_item_cones(P);
     for (int c = 0; c < nc;) {
         int e = c + 1;
         while (e < nc && e - c < most && cone_box[e] == cone_box[c]) ++e;

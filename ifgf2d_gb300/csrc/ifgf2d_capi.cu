@@ -508,7 +508,8 @@ static int setup_cones(ifgf2d_ctx* ctx, double k, int nlevels, const SetupExtra*
     std::vector<long long> loff(ncl + 1, 0);
     for (int c = 0; c < ncl; ++c) loff[c + 1] = loff[c] + (long long)P * T.leaf_count[LD.cone_box[c]];
     CK(ctx->leaf_cone_box.upload(LD.cone_box)); CK(ctx->leaf_off.upload(loff));
-    CK(ctx->leaf_items.upload(leaf_fx_items(LD.cone_box, T.leaf_start, T.leaf_count, loff, P)));
+    CK(ctx->leaf_cones.upload(leaf_cone_list(LD.cone_box, T.leaf_start, T.leaf_count, loff)));
+    CK(ctx->leaf_items.upload(leaf_item_list(LD.cone_box, T.leaf_start, T.leaf_count, loff, P)));
     CK(ctx->leafL.alloc(loff[ncl]));
     CK(ctx->leaf_nodes_d.alloc((size_t)ncl * P));
     CK(ctx->pp.alloc((size_t)T.pp_total)); CK(ctx->pp32.alloc((size_t)T.pp_total));
@@ -549,45 +550,40 @@ static int setup_interp(ifgf2d_ctx* ctx, int nlevels, DBuf<int>& perr) {
         launch_interp_fx(ip.p, (long long)T.ip.size(), ctx->ipx.p, ctx->stream);
         CK(cudaGetLastError());
     }
-    {   // interpolation by leaf box: per box, chunks of 32 targets x pieces of kIbPiece terms
-        std::vector<int4> items;
-        std::vector<int2> nitems;
-        std::vector<FinItem> fitems;
+    {   // near field and interpolation by leaf box: equal shares of each box's targets
+        std::vector<FinItem> fitems, qitems;
         long long near_at = 0;      // the box's near-field block, and its list of sources
         int src_at = 0;
-        int maxpc = 0;
         for (int b = 0; b < nleaf; ++b) {
             const int s0 = T.leaf_start[b], n = T.leaf_count[b];
             int rl = 0;
             for (int q = T.nbr_ptr[b]; q < T.nbr_ptr[b + 1]; ++q) rl += T.leaf_count[T.nbr_box[q]];
-            if (n <= 0) { src_at += rl; continue; }
-            for (int c0 = 0; c0 < n; c0 += kNearTargets) nitems.push_back(make_int2(b, c0));
-            const int nf = (n + kFinTargets - 1) / kFinTargets;      // equal shares
-            for (int q = 0; q < nf; ++q) {
-                const int c0 = (int)((long long)n * q / nf);
-                FinItem it{};
-                it.near = near_at + (long long)c0 * rl;
-                it.first = s0 + c0; it.cnt = (int)((long long)n * (q + 1) / nf) - c0; it.n = n;
-                it.ip = T.ip_ptr[s0] + c0; it.nt = T.ip_ptr[s0 + 1] - T.ip_ptr[s0];
-                it.rl = rl; it.src = src_at;
-                fitems.push_back(it);
+            const int nt = n > 0 ? T.ip_ptr[s0 + 1] - T.ip_ptr[s0] : 0;   // the same for every target of the box
+            auto share = [&](std::vector<FinItem>& items, int most) {
+                const int nf = (n + most - 1) / most;
+                for (int q = 0; q < nf; ++q) {
+                    const int c0 = (int)((long long)n * q / nf);
+                    FinItem it{};
+                    it.near = near_at + (long long)c0 * rl;
+                    it.first = s0 + c0; it.cnt = (int)((long long)n * (q + 1) / nf) - c0; it.n = n;
+                    it.ip = T.ip_ptr[s0] + c0; it.nt = nt;
+                    it.rl = rl; it.src = src_at;
+                    items.push_back(it);
+                }
+            };
+            if (n > 0) {
+                share(fitems, kFinTargets);
+                share(qitems, fin_targets(nt));
             }
             near_at += (long long)n * rl;
             src_at += rl;
-            const int nt = T.ip_ptr[s0 + 1] - T.ip_ptr[s0];   // the same for every target of the box
-            const int npc = (nt + kIbPiece - 1) / kIbPiece;
-            maxpc = std::max(maxpc, npc);
-            for (int c0 = 0; c0 < n; c0 += 32)
-                for (int q = 0; q < npc; ++q) items.push_back(make_int4(b, c0, q * kIbPiece, std::min(nt, (q + 1) * kIbPiece)));
         }
-        CK(ctx->ib_items.upload(items));
-        CK(ctx->nb_items.upload(nitems));
         CK(ctx->fx_items.upload(fitems));
+        CK(ctx->fin32_items.upload(qitems));
         CK(ctx->ipT.alloc(T.ip.size())); CK(ctx->ip32T.alloc(T.ip.size()));
         launch_interp_transpose((int)N, ctx->point_leaf.p, ctx->leaf_start.p, ctx->leaf_count.p, ctx->ip_ptr.p, ip.p, ctx->ip32T.p,
                                 ctx->ipT.view(), ctx->stream);
         CK(cudaGetLastError());
-        CK(ctx->ib_part32.alloc((size_t)std::max(maxpc, 1) * N));
     }
     CK(ctx->coef.alloc((size_t)T.total_cones * P));
     CK(ctx->cexp.alloc((size_t)T.total_cones));
@@ -656,8 +652,7 @@ static int check_kerr(ifgf2d_ctx* ctx) {
 // ------------------------------------------------------------------ apply
 // y += near field + cousin interpolants of every target (BoxTree.h:1049-1069), from the Morton-ordered
 // intensities.  FP64: k_final_fx, by leaf box.  complex64, by target: k_final_t, a warp per target; by
-// leaf box: the interpolation by k_interp_box (pieces per target), then the near field by k_near_box,
-// which adds the pieces in order.
+// leaf box: k_final_q.
 template <typename R>
 static void launch_interp_final(ifgf2d_ctx* ctx, const CoefT<R>* coef, double2* y, bool by_box) {
     const Tree& T = ctx->T;
@@ -665,20 +660,13 @@ static void launch_interp_final(ifgf2d_ctx* ctx, const CoefT<R>* coef, double2* 
     if constexpr (sizeof(R) == 8) {
         launch_final_fx(ctx->fx_items.p, (int)ctx->fx_items.n, ctx->near_src.p, ctx->near.p, ctx->nexp.p, ctx->rho.p, ctx->ipT.view(),
                         coef, ctx->cexp.p, T.Ps, T.Pang, ctx->sorting.p, y, ctx->stream);
-    } else if (!by_box || ctx->nb_items.n == 0) {
+    } else if (!by_box) {
         launch_final_t(N, ctx->point_leaf.p, ctx->leaf_start.p, ctx->near_src_off.p, ctx->near_src.p, ctx->near_rowlen.p,
                        ctx->near_off.p, ctx->near32.p, ctx->rho32.p, ctx->ip_ptr.p, ctx->ip32.p, coef, T.Ps, T.Pang, ctx->sorting.p, y,
                        ctx->stream);
     } else {
-        const float2* part = nullptr;
-        if (ctx->ib_items.n > 0) {
-            launch_interp_box(ctx->ib_items.p, (int)ctx->ib_items.n, N, ctx->leaf_start.p, ctx->leaf_count.p, ctx->ip_ptr.p,
-                              ctx->ip32T.p, coef, T.Ps, T.Pang, ctx->ib_part32.p, ctx->stream);
-            part = ctx->ib_part32.p;
-        }
-        launch_near_box(ctx->nb_items.p, (int)ctx->nb_items.n, ctx->leaf_start.p, ctx->leaf_count.p, ctx->near_src_off.p,
-                        ctx->near_src.p, ctx->near_rowlen.p, ctx->near_off.p, ctx->near32.p, ctx->rho32.p, ctx->ip_ptr.p, part, N,
-                        ctx->sorting.p, y, ctx->stream);
+        launch_final_q(ctx->fin32_items.p, (int)ctx->fin32_items.n, ctx->near_src.p, ctx->near32.p, ctx->rho32.p, ctx->ip32T.p, coef,
+                       T.Ps, T.Pang, ctx->sorting.p, y, ctx->stream);
     }
 }
 
@@ -693,8 +681,7 @@ static void launch_leaf(ifgf2d_ctx* ctx, CoefT<R>* coef, int shape) {
         if (shape == 0 && launch_leaf_tma(ctx->leaf_cone_box.p, ncl, LD.cone_base, ctx->leaf_start.p, ctx->leaf_count.p, ctx->leaf_off.p,
                                           ctx->leafL32.p, ctx->rho32.p, T.P, coef, ctx->kerr.p, ctx->nsm, ctx->stream))
             return;
-        launch_leaf_apply_t(ctx->leaf_cone_box.p, ncl, LD.cone_base, ctx->leaf_start.p, ctx->leaf_count.p, ctx->leaf_off.p,
-                            ctx->leafL32.p, ctx->rho32.p, T.P, coef, ctx->stream, shape);
+        launch_leaf_apply_t(ctx->leaf_cones.p, ncl, LD.cone_base, ctx->leafL32.p, ctx->rho32.p, T.P, coef, ctx->stream, shape);
     } else {
         launch_leaf_fx(ctx->leaf_items.p, (int)ctx->leaf_items.n, LD.cone_base, ctx->leafL.p, ctx->lexp.p, ctx->rho.p, T.P, T.Ps, coef, ctx->cexp.p,
                        ctx->stream, shape);

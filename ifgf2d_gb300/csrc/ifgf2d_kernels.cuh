@@ -104,15 +104,15 @@ void launch_direct_far(const double* tx, const double* ty, int ntarget, const in
 // precision-templated IFGF apply (ifgf_apply.cu); R = double (plain) or float (mixed)
 template <typename R>
 void launch_intensities_t(const double2* x, const double* wq, const long long* perm, int N, V2<R>* rho, cudaStream_t s);
-void launch_leaf_apply_t(const int* cone_box, int ncones, int cone_base, const int* leaf_start, const int* leaf_count,
-                         const long long* leaf_off, const float2* L, const float2* rho, int P, float2* coef, cudaStream_t s,
-                         int chunks = 5);
-// the FP64 form in fixed point (fixpoint.cuh): the table and its exponents [cone][coefficient] from
-// launch_leaf_fix (in place of the FP64 table; l32, when not null, receives the complex64 copy); an item
-// is up to leaf_fx_cones cones of one leaf box: the table offset of the first, its local index, how many,
-// and the box's sources
+// leaf cones; chunks: the threads that share a coefficient's sum.  complex64: per cone its table offset
+// (two ints), first source and sources.  An item of the FP64 form is up to leaf_item_cones cones of one
+// leaf box: the table offset of the first, its local index, how many, and the box's sources.
 struct LeafItem { long long off; int cone, cones, first, n; };
-int leaf_fx_cones(int P);
+int leaf_item_cones(int P);
+void launch_leaf_apply_t(const int4* cones, int ncones, int cone_base, const float2* L, const float2* rho, int P, float2* coef,
+                         cudaStream_t s, int chunks = 5);
+// the FP64 form in fixed point (fixpoint.cuh): the table and its exponents [cone][coefficient] from
+// launch_leaf_fix (in place of the FP64 table; l32, when not null, receives the complex64 copy)
 void launch_leaf_fx(const LeafItem* items, int nitems, int cone_base, const int4* L, const int* lexp, const double2* rho, int P, int Ps,
                     int4* coef, int* cexp, cudaStream_t s, int chunks = 2);
 void launch_leaf_fix(const int* cone_box, int ncones, const int* leaf_count, const long long* leaf_off, int P, int4* L, int* lexp,
@@ -159,17 +159,15 @@ void launch_final_fx(const FinItem* items, int nitems, const int* near_src, cons
                      cudaStream_t s);
 void launch_near_fix(int N, const int* point_leaf, const int* leaf_start, const int* near_rowlen, const long long* near_off, int4* near,
                      int* nexp, float2* n32, cudaStream_t s);
-// complex64 interpolation by leaf box (k_interp_box): items[w] = (leaf box, first target, first term, end
-// term), pieces of kIbPiece terms; part[piece * N + target] receives each piece's sum
-constexpr int kIbPiece = 8;
-void launch_interp_box(const int4* items, int nitems, int N, const int* leaf_start, const int* leaf_count, const int* ip_ptr,
-                       const InterpE<float>* ipT, const float2* coef, int Ps, int Pang, float2* part, cudaStream_t s);
-// complex64 near field by leaf box (k_near_box): items[w] = (leaf box, first of up to 32 targets); adds
-// the near field, then the target's interpolation pieces (when part is not null), into y
-constexpr int kNearChunk = 1024, kNearTargets = 32;
-void launch_near_box(const int2* items, int nitems, const int* leaf_start, const int* leaf_count, const int* near_src_off,
-                     const int* near_src, const int* near_rowlen, const long long* near_off, const float2* near, const float2* rho,
-                     const int* ip_ptr, const float2* part, int N, const long long* sorting, double2* y, cudaStream_t s);
+// the complex64 form: pieces of kIbPiece terms, near-field sums by kNearChunk sources, fin_targets of a
+// box's targets (nt terms each) to an item
+constexpr int kIbPiece = 8, kNearChunk = 1024, kFinTargetsMax = 32, kFinParts = 1024;
+inline int fin_targets(int nt) {
+    const int npc = (nt + kIbPiece - 1) / kIbPiece, t = npc ? kFinParts / npc : kFinTargetsMax;
+    return t < 1 ? 1 : t > kFinTargetsMax ? kFinTargetsMax : t;
+}
+void launch_final_q(const FinItem* items, int nitems, const int* near_src, const float2* near, const float2* rho,
+                    const InterpE<float>* ipT, const float2* coef, int Ps, int Pang, const long long* sorting, double2* y, cudaStream_t s);
 // the interpolation plan box-transposed (term j of box target t at the box's first entry + j n + t), in
 // complex64 and as px (child the cone, w the factor)
 void launch_interp_transpose(int N, const int* point_leaf, const int* leaf_start, const int* leaf_count, const int* ip_ptr,

@@ -31,15 +31,17 @@ __global__ void k_intensities_t(const double2* __restrict__ x, const double* __r
     rho[i] = r;
 }
 
-// thread = (leaf cone, source chunk, coefficient).  CH threads share one (cone, coefficient):
-// chunk ch takes the sources s = ch, ch + CH, ...; the CH partial sums meet in shared memory.
-// Boxes hold 10-100 points, so splitting the source walk shortens the latency chain of the
-// longest boxes by CH.
+// complex64 leaf cones, thread = (cone, source chunk, coefficient).  CH threads share one (cone,
+// coefficient): chunk ch takes the sources s = ch, ch + CH, ..., by turns into two sums; the CH partial sums
+// meet in shared memory.  Boxes hold 10-100 points, so splitting the source walk shortens the latency
+// chain of the longest boxes by CH.  cones: a cone's table offset (two ints), first source and sources, one
+// load ahead of the table's.  Bound by the loads in flight: 2048 threads an SM with four of the table's
+// each.  Kite k = 500 / 2000 (72 / 600 MB): 24 / 119 us; 28 / 129 with the box looked up first and two in
+// flight.  Six loads ahead in 61 registers, half the threads: 30 / 147.
 template <int CH>
-__global__ void __launch_bounds__(256) k_leaf_apply_t(const int* __restrict__ cone_box, int ncones, int cone_base,
-                                                      const int* __restrict__ leaf_start, const int* __restrict__ leaf_count,
-                                                      const long long* __restrict__ leaf_off, const float2* __restrict__ L,
-                                                      const float2* __restrict__ rho, int P, float2* __restrict__ coef) {
+__global__ void __launch_bounds__(256, 8) k_leaf_apply_t(const int4* __restrict__ cones, int ncones, int cone_base,
+                                                      const float2* __restrict__ L, const float2* __restrict__ rho, int P,
+                                                      float2* __restrict__ coef) {
     __shared__ float2 part[256];
     const int per_cone = P * CH;
     const int cpb = blockDim.x / per_cone;
@@ -49,11 +51,12 @@ __global__ void __launch_bounds__(256) k_leaf_apply_t(const int* __restrict__ co
     const bool active = local < cpb && c < ncones;
     float2 a0 = make_float2(0.f, 0.f), a1 = a0;
     if (active) {
-        const int b = cone_box[c];
-        const int n = leaf_count[b], s0 = leaf_start[b];
-        const float2* Lc = L + leaf_off[c] + m;
-        const float2* rh = rho + s0;
+        const int4 D = cones[c];
+        const int n = D.w;
+        const float2* Lc = L + ((long long)D.y << 32 | (unsigned)D.x) + m;
+        const float2* rh = rho + D.z;
         int s = ch;
+#pragma unroll 2
         for (; s + CH < n; s += 2 * CH) {
             const float2 l0 = Lc[(long long)s * P], l1 = Lc[(long long)(s + CH) * P];
             const float2 r0 = rh[s], r1 = rh[s + CH];
@@ -73,7 +76,7 @@ __global__ void __launch_bounds__(256) k_leaf_apply_t(const int* __restrict__ co
 
 // The FP64 form of the same in fixed point (fixpoint.cuh): table and densities as 27-bit limbs, 12 wide
 // multiply-adds an entry where FP64 took 4 of the FP64 pipe's operations.  A block takes up to
-// kLeafFxCones / CH cones of one leaf box (items: table offset, first cone, cones, first source,
+// 256 / (P CH) cones of one leaf box (items: table offset, first cone, cones, first source,
 // sources): it brings the box's densities to their exponent in shared memory once, while its threads'
 // first table entries are in flight; the chunks' integer sums meet in shared memory; then the cone's
 // coefficients, whose entries have an exponent per coefficient, are brought to the cone's exponent.
@@ -649,114 +652,88 @@ __global__ void __launch_bounds__(256) k_propagate_st(int pbegin, int pend, cons
     }
 }
 
-// one warp per (leaf box, up to 32 of its targets, kIbPiece of their interpolation terms), one
-// lane per target.  The targets of a leaf box share their ancestors, hence the same cousin lists
-// in the same order: their j-th terms read the same cousin box, mostly the same cone (2.5-3
-// distinct cones per warp step on the kite trees, against up to 32 when a warp walks one target's
-// terms), so the coefficient gathers are broadcasts.  The plan is stored box-transposed (term j of
-// the box's target t at box base + j n + t) for coalesced entry loads.  Each lane writes its
-// piece's sum to part[piece][target]; k_final_t adds the pieces in order.
+// complex64: near field and interpolation of a leaf box's targets, a block per (box, share of its targets)
+// with one record (FinItem).  Near field: the neighbour boxes' densities are staged in shared memory
+// kNearChunk at a time, each warp streams two targets' table rows against them; a target's chunk sums add
+// up in chunk order.  Interpolation: a thread takes kIbPiece terms of a target, the targets fastest.  The
+// targets of a box share their ancestors, hence the same cousin lists in the same order: their j-th terms
+// read the same cousin box, mostly the same cone (2.5-3 distinct cones in 32 targets on the kite trees), so
+// the gathers are broadcasts; the plan is stored in that order.  The warps take the row pairs and then 32
+// pieces at a time from one counter, so that none waits at a barrier between the two; the pieces' sums are
+// added in order to the near sum.  Bound by the latency of the plan's and the coefficients' loads; a term's
+// plan entry is loaded during the term before.  Kite k = 100 / 500 / 2000: 25 / 37 / 64 us as two
+// kernels, 12 / 18 / 53 so; without the counter 12 / 21 / 55; two or four blocks an SM: 14 / 21 / 55 or slower.
 template <int PS, int PA>
-__global__ void __launch_bounds__(256) k_interp_box(const int4* __restrict__ items, int nitems, int N,
-                                                    const int* __restrict__ leaf_start, const int* __restrict__ leaf_count,
-                                                    const int* __restrict__ ip_ptr, const InterpE<float>* __restrict__ ipT,
-                                                    const float2* __restrict__ coef, float2* __restrict__ part) {
-    using R = float;
+__global__ void __launch_bounds__(256, 3) k_final_q(const FinItem* __restrict__ items, const int* __restrict__ near_src,
+                                                 const float2* __restrict__ near, const float2* __restrict__ rho,
+                                                 const InterpE<float>* __restrict__ ipT, const float2* __restrict__ coef,
+                                                 const long long* __restrict__ sorting, double2* __restrict__ y) {
     constexpr int P = PS * PA;
-    const int w = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-    if (w >= nitems) return;
-    const int lane = threadIdx.x & 31;
-    const int4 I = items[w];   // leaf box, first target, terms [z, w)
-    const int s = leaf_start[I.x], n = leaf_count[I.x];
-    const int t = I.y + lane;
-    if (t >= n) return;
-    const InterpE<R>* e = ipT + ip_ptr[s] + t;
-    V2<R> acc; acc.x = R(0); acc.y = R(0);
-    int j = I.z;
-    for (; j + 1 < I.w; j += 2) {   // two terms' loads in flight before either is evaluated
-        const InterpE<R> E0 = e[(long long)j * n], E1 = e[(long long)(j + 1) * n];
-        V2<R> c0[P], c1[P];
-        const V2<R>* b0 = coef + (long long)E0.cone * P;
-        const V2<R>* b1 = coef + (long long)E1.cone * P;
-#pragma unroll
-        for (int q = 0; q < P; ++q) { c0[q] = b0[q]; c1[q] = b1[q]; }
-        V2<R> f; f.x = E0.fr; f.y = E0.fi;
-        cmac<R>(acc, interp_eval<R, PS, PA>(c0, E0.s, E0.th), f);
-        f.x = E1.fr; f.y = E1.fi;
-        cmac<R>(acc, interp_eval<R, PS, PA>(c1, E1.s, E1.th), f);
-    }
-    for (; j < I.w; ++j) {
-        const InterpE<R> E = e[(long long)j * n];
-        V2<R> c[P];
-        const V2<R>* cb = coef + (long long)E.cone * P;
-#pragma unroll
-        for (int q = 0; q < P; ++q) c[q] = cb[q];
-        V2<R> f; f.x = E.fr; f.y = E.fi;
-        cmac<R>(acc, interp_eval<R, PS, PA>(c, E.s, E.th), f);
-    }
-    part[(long long)(I.z / kIbPiece) * N + s + t] = acc;
-}
-
-// near field by leaf box: one block per (leaf box, up to 32 of its targets).  The box's
-// neighbour densities rho[src[e]] are staged in shared memory kNearChunk at a time, once for all
-// its targets, and each warp streams its targets' table rows (coalesced) against them; a target's
-// chunk sums meet in shared memory in chunk order.  Then the target's interpolation pieces
-// (k_interp_box) are added in order and the sum goes to y at the target's original index.
-__global__ void __launch_bounds__(256) k_near_box(const int2* __restrict__ items, const int* __restrict__ leaf_start,
-                                                  const int* __restrict__ leaf_count, const int* __restrict__ near_src_off,
-                                                  const int* __restrict__ near_src, const int* __restrict__ near_rowlen,
-                                                  const long long* __restrict__ near_off, const float2* __restrict__ near,
-                                                  const float2* __restrict__ rho, const int* __restrict__ ip_ptr,
-                                                  const float2* __restrict__ part, int N, const long long* __restrict__ sorting,
-                                                  double2* __restrict__ y) {
-    using R = float;
-    static_assert(kNearTargets == 4 * 8, "eight warps of four targets");
     __shared__ float2 srho[kNearChunk];
-    __shared__ float2 sacc[kNearTargets];
-    const int2 I = items[blockIdx.x];   // leaf box, first target
-    const int b = I.x, s = leaf_start[b], n = min(kNearTargets, leaf_count[b] - I.y);
-    const int rl = near_rowlen[b];
-    const int* src = near_src + near_src_off[b];
-    const float2* rows = near + near_off[b] + (long long)I.y * rl;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (threadIdx.x < kNearTargets) { sacc[threadIdx.x].x = R(0); sacc[threadIdx.x].y = R(0); }
-    for (int c0 = 0; c0 < rl; c0 += kNearChunk) {
-        const int cn = min(kNearChunk, rl - c0);
-        __syncthreads();   // the previous chunk has been read
-        for (int e = threadIdx.x; e < cn; e += blockDim.x) srho[e] = rho[src[c0 + e]];
+    __shared__ float2 sacc[kFinTargetsMax], part[kFinParts];
+    __shared__ int next;
+    const FinItem I = items[blockIdx.x];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, cnt = I.cnt, rl = I.rl;
+    const int* src = near_src + I.src;
+    if (tid == 0) next = 0;
+    if (tid < cnt) sacc[tid] = make_float2(0.f, 0.f);
+    auto rows = [&](int q, int c0, int cn) {   // targets q and q + 1 against the staged densities
+        const float2* r0 = near + I.near + (long long)q * rl + c0;
+        const float2* r1 = q + 1 < cnt ? r0 + rl : r0;
+        float2 a = make_float2(0.f, 0.f), b = a;
+#pragma unroll 4
+        for (int e = lane; e < cn; e += 32) {
+            const float2 u = r0[e], v = r1[e], r = srho[e];
+            cmac<float>(a, u, r); cmac<float>(b, v, r);
+        }
+        a.x = warp_sum_r<float>(a.x); a.y = warp_sum_r<float>(a.y);
+        b.x = warp_sum_r<float>(b.x); b.y = warp_sum_r<float>(b.y);
+        if (lane == 0) {
+            sacc[q].x += a.x; sacc[q].y += a.y;
+            if (q + 1 < cnt) { sacc[q + 1].x += b.x; sacc[q + 1].y += b.y; }
+        }
+    };
+    const int npc = (I.nt + kIbPiece - 1) / kIbPiece, pairs = rl > 0 ? (cnt + 1) / 2 : 0;
+    int c0 = 0, cn;
+    for (;; c0 += kNearChunk) {
+        cn = min(kNearChunk, rl - c0);
+        for (int e = tid; e < cn; e += 256) srho[e] = rho[src[c0 + e]];
         __syncthreads();
-        // warp w: targets 4 w .. 4 w + 3 together (four independent row loads per density read)
-        const int t0 = 4 * warp;
-        if (t0 < n) {
-            float2 acc[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) { acc[u].x = R(0); acc[u].y = R(0); }
-            const float2* row = rows + (long long)t0 * rl + c0;
-#pragma unroll 2
-            for (int e = lane; e < cn; e += 32) {
-                const float2 r = srho[e];
-#pragma unroll
-                for (int u = 0; u < 4; ++u)
-                    if (t0 + u < n) cmac<R>(acc[u], row[(long long)u * rl + e], r);
+        if (c0 + kNearChunk >= rl) break;
+        for (int q = 2 * warp; q < cnt; q += 16) rows(q, c0, cn);
+        __syncthreads();                       // the chunk has been read
+    }
+    // the last chunk's rows and the pieces, each warp the next when it is done with one
+    for (;;) {
+        int u = 0;
+        if (lane == 0) u = atomicAdd(&next, 1);
+        u = __shfl_sync(0xffffffffu, u, 0);
+        if (u < pairs) { rows(2 * u, c0, cn); continue; }
+        if ((u - pairs) * 32 >= npc * cnt) break;
+        const int w = (u - pairs) * 32 + lane, pc = w / cnt, t = w - pc * cnt;
+        if (pc < npc) {
+            const InterpE<float>* e = ipT + I.ip + t;
+            const int z = min(I.nt, (pc + 1) * kIbPiece);
+            float2 acc = make_float2(0.f, 0.f);
+            InterpE<float> En = e[(long long)(pc * kIbPiece) * I.n];
+            for (int j = pc * kIbPiece; j < z; ++j) {
+                const InterpE<float> E = En;
+                if (j + 1 < z) En = e[(long long)(j + 1) * I.n];             // in flight during this term
+                cmac<float>(acc, interp_eval<float, PS, PA>(coef + (long long)E.cone * P, E.s, E.th), make_float2(E.fr, E.fi));
             }
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const R ax = warp_sum_r<R>(acc[u].x), ay = warp_sum_r<R>(acc[u].y);
-                if (lane == 0 && t0 + u < n) { sacc[t0 + u].x += ax; sacc[t0 + u].y += ay; }
-            }
+            part[w] = acc;
         }
     }
     __syncthreads();
-    if (threadIdx.x < n) {
-        const int i = s + I.y + threadIdx.x;
-        float2 acc = sacc[threadIdx.x];
-        if (part) {
-            const int npc = (ip_ptr[i + 1] - ip_ptr[i] + kIbPiece - 1) / kIbPiece;
-            for (int q = 0; q < npc; ++q) { const float2 a = part[(long long)q * N + i]; acc.x += a.x; acc.y += a.y; }
-        }
-        const long long o = sorting[i];
+    float2 sum = make_float2(0.f, 0.f);
+    if (tid < cnt) {
+        sum = sacc[tid];
+        for (int q = 0; q < npc; ++q) { const float2 v = part[q * cnt + tid]; sum.x += v.x; sum.y += v.y; }
+    }
+    if (tid < cnt) {
+        const long long o = sorting[I.first + tid];
         double2 v = y[o];
-        v.x += (double)acc.x; v.y += (double)acc.y;
+        v.x += (double)sum.x; v.y += (double)sum.y;
         y[o] = v;
     }
 }
@@ -985,23 +962,22 @@ static void leaf_chunks(int P, int chunks, Go&& go) {
     else if (chunks == 1 || 256 / (P * 5) < 1) go(std::integral_constant<int, 1>{});
     else go(std::integral_constant<int, 5>{});
 }
-void launch_leaf_apply_t(const int* cone_box, int ncones, int cone_base, const int* leaf_start, const int* leaf_count,
-                         const long long* leaf_off, const float2* L, const float2* rho, int P, float2* coef, cudaStream_t s, int chunks) {
+int leaf_item_cones(int P) { return 256 / P; }
+void launch_leaf_apply_t(const int4* cones, int ncones, int cone_base, const float2* L, const float2* rho, int P, float2* coef,
+                         cudaStream_t s, int chunks) {
     if (ncones <= 0) return;
     leaf_chunks(P, chunks, [&](auto tag) {
         constexpr int CH = decltype(tag)::value;
         const int cpb = 256 / (P * CH);
-        k_leaf_apply_t<CH><<<nblk_a(ncones, cpb), cpb * P * CH, 0, s>>>(cone_box, ncones, cone_base, leaf_start, leaf_count, leaf_off, L,
-                                                                       rho, P, coef);
+        k_leaf_apply_t<CH><<<nblk_a(ncones, cpb), cpb * P * CH, 0, s>>>(cones, ncones, cone_base, L, rho, P, coef);
     });
 }
-int leaf_fx_cones(int P) { return 256 / P; }
 void launch_leaf_fx(const LeafItem* items, int nitems, int cone_base, const int4* L, const int* lexp, const double2* rho, int P, int Ps,
                     int4* coef, int* cexp, cudaStream_t s, int chunks) {
     if (nitems <= 0) return;
     leaf_chunks(P, chunks, [&](auto tag) {
         constexpr int CH = decltype(tag)::value;
-        const int cpb = 256 / (P * CH), split = (leaf_fx_cones(P) + cpb - 1) / cpb;
+        const int cpb = 256 / (P * CH), split = (leaf_item_cones(P) + cpb - 1) / cpb;
         k_leaf_fx<CH><<<(unsigned)nitems * split, cpb * P * CH, 0, s>>>(items, split, cone_base, L, lexp, rho, P, Ps, coef, cexp);
     });
 }
@@ -1088,18 +1064,10 @@ void launch_near_fix(int N, const int* point_leaf, const int* leaf_start, const 
         k_near_fix<<<nblk_a((long long)N * 32, 256), 256, 0, s>>>(N, point_leaf, leaf_start, near_rowlen, near_off,
                                                                  reinterpret_cast<double2*>(near), nexp, n32);
 }
-void launch_interp_box(const int4* items, int nitems, int N, const int* leaf_start, const int* leaf_count, const int* ip_ptr,
-                       const InterpE<float>* ipT, const float2* coef, int Ps, int Pang, float2* part, cudaStream_t s) {
+void launch_final_q(const FinItem* items, int nitems, const int* near_src, const float2* near, const float2* rho,
+                    const InterpE<float>* ipT, const float2* coef, int Ps, int Pang, const long long* sorting, double2* y, cudaStream_t s) {
     if (nitems <= 0) return;
-    IFGF_DISPATCH_P(Ps, Pang, (k_interp_box<PS, PA><<<nblk_a((long long)nitems * 32, 256), 256, 0, s>>>(
-                                   items, nitems, N, leaf_start, leaf_count, ip_ptr, ipT, coef, part)));
-}
-void launch_near_box(const int2* items, int nitems, const int* leaf_start, const int* leaf_count, const int* near_src_off,
-                     const int* near_src, const int* near_rowlen, const long long* near_off, const float2* near, const float2* rho,
-                     const int* ip_ptr, const float2* part, int N, const long long* sorting, double2* y, cudaStream_t s) {
-    if (nitems > 0)
-        k_near_box<<<nitems, 256, 0, s>>>(items, leaf_start, leaf_count, near_src_off, near_src, near_rowlen, near_off, near,
-                                           rho, ip_ptr, part, N, sorting, y);
+    IFGF_DISPATCH_P(Ps, Pang, (k_final_q<PS, PA><<<(unsigned)nitems, 256, 0, s>>>(items, near_src, near, rho, ipT, coef, sorting, y)));
 }
 void launch_interp_transpose(int N, const int* point_leaf, const int* leaf_start, const int* leaf_count, const int* ip_ptr,
                              const InterpE<double>* in, InterpE<float>* out, PlanX px, cudaStream_t s) {

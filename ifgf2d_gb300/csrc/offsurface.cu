@@ -116,7 +116,7 @@ extern "C" int ifgf2d_eval_offsurface_setup(ifgf2d_ctx* ctx, long long m, const 
         CK(W.nodes.alloc((size_t)ncl * P));
         CK(build_leaf_nodes(E, W.nodes.p, s));
         CK(W.leaf_cone_box.upload(LD.cone_box)); CK(W.leaf_off.upload(loff));
-        CK(W.leaf_items.upload(leaf_fx_items(LD.cone_box, E.leaf_start, E.leaf_count, loff, P)));
+        CK(W.leaf_items.upload(leaf_item_list(LD.cone_box, E.leaf_start, E.leaf_count, loff, P)));
         CK(W.leafL.alloc(loff[ncl]));
         launch_leaf_setup(W.leaf_cone_box.p, ncl, ctx->leaf_start.p, ctx->leaf_count.p, W.leaf_off.p, W.nodes.p, ctx->xs_s.p,
                           ctx->ys_s.p, ctx->nxs_s.p, ctx->nys_s.p, ctx->T.Ps, ctx->T.Pang, ctx->k, ctx->form, ctx->eta, ctx->Gsep.p,
