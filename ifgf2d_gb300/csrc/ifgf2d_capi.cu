@@ -1029,8 +1029,7 @@ static int gmres_core(ifgf2d_ctx* ctx, const double2* b, double2* x, int mode, d
             cudaGraphDestroy(graph);
             return fail(ctx, IFGF2D_ERR_CUDA, std::string("building the GMRES cycle graph: ") + cudaGetErrorString(e));
         }
-        launch_copy_col(G.V.p, N, G.jdev.p, G.vin.p, G.nrm2.p, s);
-        int rc;
+        int rc;                                              // vin holds v_j
         if (pk) {
             // flexible GMRES: z_j = M(v_j) into Z[:, j], then w = A z_j
             if (pk == 1) {
@@ -1056,8 +1055,8 @@ static int gmres_core(ifgf2d_ctx* ctx, const double2* b, double2* x, int mode, d
         // the complex64 inner solves of the refinement take one Gram-Schmidt pass, as the batched
         // ones do: each correction is checked by the FP64 residual, and a short one costs one more
         // refinement pass, not a wrong answer
-        launch_arnoldi_step(G.V.p, N, m, G.jdev.p, G.w.p, G.h.p, G.H.p, G.nrm2.p, G.part.p, s,
-                            mode == IFGF2D_APPLY_IFGF_MIXED ? 1 : 2, &L, cond, true);
+        launch_arnoldi_step(G.V.p, N, m, G.jdev.p, G.w.p, G.vin.p, G.H.p, G.nrm2.p, G.part.p, s,
+                            mode == IFGF2D_APPLY_IFGF_MIXED ? 1 : 2, L, cond);
         cudaGraph_t body = nullptr;
         const cudaError_t ec = cudaStreamEndCapture(s, &body);
         if (rc != IFGF2D_OK || ec != cudaSuccess) {
@@ -1101,6 +1100,7 @@ static int gmres_core(ifgf2d_ctx* ctx, const double2* b, double2* x, int mode, d
         launch_scale(w, make_double2(1.0 / beta, 0.0), N, V, s);
         CK(cudaMemsetAsync(G.H.p, 0, sizeof(double2) * ldh * m, s));
         launch_lsq_init(L, G.jdev.p, beta, r0n, tol, (int)std::min<long long>(limit, 1 << 30), s);
+        launch_copy_col(V, N, G.jdev.p, G.vin.p, G.nrm2.p, s);
         CK(cudaGraphLaunch(G.exec[gi], s));
         launch_lsq_solve(L, ldh, G.y.p, s);
         launch_multi_axpy_dyn(pk ? G.Z.p : V, N, G.lsst.p + 1, G.y.p, N, x, s);   // x += V y, or Z y (flexible)

@@ -344,7 +344,7 @@ __global__ void k_copy_col(const double2* __restrict__ V, long long n, const int
     if (i == 0 && nrm2) *nrm2 = 0.0;
 }
 // h[c] = V[:, c]^H w for c <= *jp in two deterministic stages: blocks (row chunk, column)
-// write partial sums, then one thread per column adds its chunks in order.  The grid spans
+// write partial sums, then every block of k_cgs_update_dyn adds a column's chunks in order.  The grid spans
 // every column and row chunk, so even the first iterations keep all SMs busy.
 constexpr int kDotChunk = 2048;
 __global__ void __launch_bounds__(256) k_multidot_part(const double2* __restrict__ V, long long ldv, const int* __restrict__ jp,
@@ -370,14 +370,6 @@ __global__ void __launch_bounds__(256) k_multidot_part(const double2* __restrict
         for (int q = 0; q < (int)(blockDim.x >> 5); ++q) { a += sr[q]; b += si[q]; }
         part[(long long)col * gridDim.x + chunk] = make_double2(a, b);
     }
-}
-__global__ void k_multidot_fin(const double2* __restrict__ part, int nchunk, const int* __restrict__ jp, int ncol,
-                               double2* __restrict__ h) {
-    const int col = blockIdx.x * blockDim.x + threadIdx.x;
-    if (col >= ncol || col > *jp) return;
-    double a = 0.0, b = 0.0;
-    for (int q = 0; q < nchunk; ++q) { const double2 v = part[(long long)col * nchunk + q]; a += v.x; b += v.y; }
-    h[col] = make_double2(a, b);
 }
 // Z[:, *jp] = z (flexible GMRES keeps the preconditioned vectors)
 __global__ void k_store_col(const double2* __restrict__ z, long long n, const int* __restrict__ jp, double2* __restrict__ Z) {
@@ -406,19 +398,35 @@ __global__ void k_multidot_dyn(const double2* __restrict__ V, long long ldv, con
         if (threadIdx.x == 0) h[j] = make_double2(re, im);
     }
 }
-// w -= V[:, 0..j] h: 64 rows per block, four threads per row split the columns (j = part mod 4);
-// block 0 also writes (add = 0) or adds (add = 1) h into the Hessenberg column j.
+// w -= V[:, 0..j] h: 64 rows per block, four threads per row split the columns (j = part mod 4).  h, the
+// columns' partial dots added up, is summed by every block for itself, 256 columns at a time (a launch
+// of its own for it cost 2.3 us an orthogonalisation pass); block 0 also writes (add = 0) or adds (add = 1)
+// it into the Hessenberg column j.
 __global__ void __launch_bounds__(256) k_cgs_update_dyn(const double2* __restrict__ V, long long ldv, const int* __restrict__ jp,
-                                                        const double2* __restrict__ h, long long n, double2* __restrict__ w,
+                                                        const double2* __restrict__ dots, int nchunk, long long n, double2* __restrict__ w,
                                                         double2* __restrict__ H, int ldh, int add, double* __restrict__ nrm2) {
-    __shared__ double2 part[4][64];
+    __shared__ double2 part[4][64], h[256];
     __shared__ double npart[2];
     const int r = threadIdx.x & 63, q = threadIdx.x >> 6;
     const long long i = (long long)blockIdx.x * 64 + r;
     const int j = *jp;
     double2 acc = make_double2(0.0, 0.0);
-    if (i < n)
-        for (int c = q; c <= j; c += 4) cfma(acc, V[(long long)c * ldv + i], h[c]);
+    for (int c0 = 0; c0 <= j; c0 += 256) {
+        const int col = c0 + threadIdx.x;
+        if (c0) __syncthreads();               // the previous columns have been used
+        if (col <= j) {
+            double a = 0.0, b = 0.0;
+            for (int k = 0; k < nchunk; ++k) { const double2 v = dots[(long long)col * nchunk + k]; a += v.x; b += v.y; }
+            h[threadIdx.x] = make_double2(a, b);
+            if (blockIdx.x == 0) {
+                double2* e = H + (long long)j * ldh + col;
+                if (add) { e->x += a; e->y += b; } else *e = make_double2(a, b);
+            }
+        }
+        __syncthreads();
+        if (i < n)
+            for (int c = q; c < min(256, j + 1 - c0); c += 4) cfma(acc, V[(long long)(c0 + c) * ldv + i], h[c]);
+    }
     part[q][r] = acc;
     __syncthreads();
     double sq = 0.0;
@@ -435,24 +443,19 @@ __global__ void __launch_bounds__(256) k_cgs_update_dyn(const double2* __restric
     }
     __syncthreads();
     if (nrm2 && threadIdx.x == 0) atomicAdd(nrm2, npart[0] + npart[1]);
-    if (blockIdx.x == 0)
-        for (int c = threadIdx.x; c <= j; c += blockDim.x) {
-            double2* col = H + (long long)j * ldh;
-            if (add) { col[c].x += h[c].x; col[c].y += h[c].y; } else col[c] = h[c];
-        }
 }
-// h_{j+1,j} = ||w|| from the accumulated square; V[:, j+1] = w / h_{j+1,j}; block 0 stores
-// h_{j+1,j} in the Hessenberg matrix (j is advanced by the next kernel)
+// h_{j+1,j} = ||w|| from the accumulated square; V[:, j+1] = w / h_{j+1,j}, also into vin, the next
+// iteration's vector; block 0 stores h_{j+1,j} in the Hessenberg matrix (j is advanced by the next kernel)
 __global__ void k_scale_next(const double2* __restrict__ w, const double* __restrict__ nrm2, long long n,
-                             double2* __restrict__ V, const int* __restrict__ jp, double2* __restrict__ H, int ldh) {
+                             double2* __restrict__ V, const int* __restrict__ jp, double2* __restrict__ H, int ldh,
+                             double2* __restrict__ vin) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const int j = *jp;
     const double hn = sqrt(fmax(*nrm2, 0.0));
     const double a = hn != 0.0 ? 1.0 / hn : 0.0;
-    if (i < n) V[(long long)(j + 1) * n + i] = make_double2(w[i].x * a, w[i].y * a);
+    if (i < n) vin[i] = V[(long long)(j + 1) * n + i] = make_double2(w[i].x * a, w[i].y * a);
     if (i == 0) H[(long long)j * ldh + j + 1] = make_double2(hn, 0.0);
 }
-__global__ void k_advance(int* __restrict__ jp) { if (threadIdx.x == 0 && blockIdx.x == 0) *jp += 1; }
 
 // dependent FP64 FMA chains, 8 independent chains per thread
 __global__ void k_fp64_peak(double* out, int iters, double a, double b) {
@@ -538,20 +541,17 @@ void launch_sub(const double2* a, const double2* b, long long n, double2* out, c
     k_sub<<<nblk(n, 256), 256, 0, s>>>(a, b, n, out);
 }
 int arnoldi_part_size(long long n, int m) { return (int)(((n + kDotChunk - 1) / kDotChunk) * (m + 1)); }
-void launch_arnoldi_step(double2* V, long long n, int m, int* jp, double2* w, double2* h, double2* H, double* nrm2,
-                         double2* part, cudaStream_t s, int passes, const LsqDev* lsq, cudaGraphConditionalHandle cond,
-                         bool use_cond) {
-    // w holds A v_j on entry (the apply ran between k_copy_col and this call)
+void launch_arnoldi_step(double2* V, long long n, int m, int* jp, double2* w, double2* vin, double2* H, double* nrm2,
+                         double2* part, cudaStream_t s, int passes, LsqDev lsq, cudaGraphConditionalHandle cond) {
+    // w holds A v_j on entry, vin v_j
     const int ldh = m + 1;
     for (int pass = 0; pass < passes; ++pass) {   // classical Gram-Schmidt; the last pass sums ||w||^2
         const int nchunk = (int)((n + kDotChunk - 1) / kDotChunk);
         k_multidot_part<<<dim3(nchunk, m + 1), 256, 0, s>>>(V, n, jp, w, n, part);
-        k_multidot_fin<<<nblk(m + 1, 128), 128, 0, s>>>(part, nchunk, jp, m + 1, h);
-        k_cgs_update_dyn<<<nblk(n, 64), 256, 0, s>>>(V, n, jp, h, n, w, H, ldh, pass, pass == passes - 1 ? nrm2 : nullptr);
+        k_cgs_update_dyn<<<nblk(n, 64), 256, 0, s>>>(V, n, jp, part, nchunk, n, w, H, ldh, pass, pass == passes - 1 ? nrm2 : nullptr);
     }
-    k_scale_next<<<nblk(n, 256), 256, 0, s>>>(w, nrm2, n, V, jp, H, ldh);
-    if (lsq) launch_lsq_givens(H, ldh, jp, *lsq, cond, use_cond, s);
-    else k_advance<<<1, 32, 0, s>>>(jp);
+    k_scale_next<<<nblk(n, 256), 256, 0, s>>>(w, nrm2, n, V, jp, H, ldh, vin);
+    launch_lsq_givens(H, ldh, jp, lsq, cond, true, nrm2, s);
 }
 void launch_store_col(const double2* z, long long n, const int* jp, double2* Z, cudaStream_t s) {
     k_store_col<<<nblk(n, 256), 256, 0, s>>>(z, n, jp, Z);

@@ -297,8 +297,8 @@ struct LsqBatchDev {
 void launch_lsq_init(LsqDev L, int* jp, double beta, double r0n, double tol, int limit, cudaStream_t s);
 // after the Arnoldi step of column j = *jp: rotate it into R, update g and the estimate
 // |g_{j+1}| / ||r0||, stop on convergence, the limit or a breakdown, j += 1; with use_cond, set
-// the condition of the graph while-loop around the iteration (0 ends the cycle)
-void launch_lsq_givens(const double2* H, int ldh, int* jp, LsqDev L, cudaGraphConditionalHandle cond, bool use_cond,
+// the condition of the graph while-loop around the iteration (0 ends the cycle); *nrm2 = 0
+void launch_lsq_givens(const double2* H, int ldh, int* jp, LsqDev L, cudaGraphConditionalHandle cond, bool use_cond, double* nrm2,
                        cudaStream_t s);
 // y = R^{-1} g over the cycle's columns (st[1])
 void launch_lsq_solve(LsqDev L, int ldh, double2* y, cudaStream_t s);
@@ -338,12 +338,10 @@ void launch_seg_axpy(const SegDesc& S, const double2* V, int ncols, const double
 
 // one Arnoldi step after w = A v_j, with j read from *jp (for a captured iteration graph):
 // classical Gram-Schmidt against V[:, 0..j], `passes` times (2: CGS2), into the Hessenberg
-// column j, ||w||^2 into *nrm2 (zeroed by launch_copy_col), h_{j+1,j} and
-// V[:, j+1] = w / h_{j+1,j}; then, with lsq, the Givens step of launch_lsq_givens (which
-// advances j), else j += 1
-void launch_arnoldi_step(double2* V, long long n, int m, int* jp, double2* w, double2* h, double2* H, double* nrm2,
-                         double2* part, cudaStream_t s, int passes = 2, const LsqDev* lsq = nullptr,
-                         cudaGraphConditionalHandle cond = 0, bool use_cond = false);
+// column j, ||w||^2 into *nrm2 (zeroed by launch_copy_col and the Givens step), h_{j+1,j} and
+// V[:, j+1] = w / h_{j+1,j}, also into vin; then the Givens step of launch_lsq_givens, which advances j
+void launch_arnoldi_step(double2* V, long long n, int m, int* jp, double2* w, double2* vin, double2* H, double* nrm2,
+                         double2* part, cudaStream_t s, int passes, LsqDev lsq, cudaGraphConditionalHandle cond);
 // size (double2 entries) of the partial-sum buffer launch_arnoldi_step needs
 int arnoldi_part_size(long long n, int m);
 // Z[:, *jp] = z
