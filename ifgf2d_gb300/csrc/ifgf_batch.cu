@@ -321,7 +321,11 @@ __global__ void __launch_bounds__(NT * MS) k_leaf_bx(const int* __restrict__ con
 
 // ------------------------------------------------------------------ propagation
 // complex64: warp = one parent cone x 32*RPL right-hand sides.  Node values accumulate in the lane's own
-// shared-memory columns; the values -> coefficients map then runs in the lane's registers.
+// shared-memory columns; the values -> coefficients map then runs in the lane's registers.  The parent's
+// terms (at most 4 P, uniform over the warp) come into shared memory with one round of copies, and a term is
+// read during the one before: read one by one from global memory, a term ahead, their latency was what three
+// warps a scheduler waited for.  Kite k = 2000, 64 right-hand sides, all levels: 2438 -> 1897 us (issue 56 ->
+// 72 % of the slots; bound by the FP32 multiply-adds).  Prefetching the next child's rows: slower by 10 %.
 template <int P, int RPL>
 struct PropBlock {
     static constexpr int bytes_per_warp = P * 32 * RPL * (int)sizeof(float2);
@@ -334,12 +338,19 @@ __global__ void __launch_bounds__(WPB * 32) k_prop_b(int pbegin, int pend, const
     using R = float;
     constexpr int P = PS * PA;
     __shared__ V2<R> sv[WPB][P][32 * RPL];
+    __shared__ PropB<R> plan[WPB][4 * P];
     __shared__ R sG[PS * PS + PA * PA];
     for (int i = threadIdx.x; i < PS * PS + PA * PA; i += blockDim.x) sG[i] = Gsep[i];
     __syncthreads();
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int pc = pbegin + blockIdx.x * WPB + w;
     if (pc >= pend) return;
+    // the parent's terms, all on their way at once
+    const long long e0 = pp_ptr[pc];
+    const int ne = pp_nchild[pc] * P;
+    for (int i = lane; i < ne * (int)sizeof(PropB<R>) / 8; i += 32)
+        cp_async_el<8>(reinterpret_cast<char*>(plan[w]) + 8 * i, reinterpret_cast<const char*>(pb + e0) + 8 * i);
+    cp_async_commit();
     int rr[RPL];
     bool act[RPL];
 #pragma unroll
@@ -352,15 +363,15 @@ __global__ void __launch_bounds__(WPB * 32) k_prop_b(int pbegin, int pend, const
     for (int q = 0; q < P; ++q)
 #pragma unroll
         for (int k = 0; k < RPL; ++k) { sv[w][q][32 * k + lane].x = R(0); sv[w][q][32 * k + lane].y = R(0); }
-    const long long e0 = pp_ptr[pc];
-    const int ne = pp_nchild[pc] * P;
     V2<R> cc[RPL][P];
     int cur = -1;
+    cp_async_wait<0>();
+    __syncwarp();
     PropB<R> En{};
-    if (ne > 0) En = pb[e0];
+    if (ne > 0) En = plan[w][0];
     for (int e = 0; e < ne; ++e) {
         const PropB<R> E = En;
-        if (e + 1 < ne) En = pb[e0 + e + 1];   // next term in flight during this one
+        if (e + 1 < ne) En = plan[w][e + 1];
         if (E.child_cone != cur) {             // warp-uniform: E is the same for every lane
             cur = E.child_cone;
             const V2<R>* src = coef + (long long)cur * P * B;
@@ -808,13 +819,16 @@ __global__ void __launch_bounds__(256) k_near_bx(int N, const int* __restrict__ 
 // Two warps = one work item (up to kInterpGrpTargets targets of one leaf box), 32 right-hand
 // sides each.  The item's terms are sorted by cone, so each cone's 25 x B coefficient block is
 // loaded once for every target of the item that reads it (k_final_b loads it once per target);
-// per-target sums accumulate in shared memory, then are added into yt.
+// per-target sums accumulate in shared memory, then are added into yt.  The terms come in tiles of
+// kInterpGrpTile by cp.async: k = 500 / 2000, 64 right-hand sides, 117 / 353 -> 99 / 334 us.
+constexpr int kInterpGrpTile = 64;
 template <int PS, int PA>
 __global__ void __launch_bounds__(64) k_interp_grp(const int4* __restrict__ items, int nitems, const InterpG* __restrict__ terms,
                                                    const float2* __restrict__ coef, const long long* __restrict__ sorting, int B,
                                                    double2* __restrict__ yt) {
     constexpr int P = PS * PA;
     __shared__ float2 acc[kInterpGrpTargets][64];
+    __shared__ InterpG tile[2][kInterpGrpTile];
     const int it = blockIdx.x;
     if (it >= nitems) return;
     const int4 I = items[it];   // terms [x, y), targets [z, z + w)
@@ -822,13 +836,26 @@ __global__ void __launch_bounds__(64) k_interp_grp(const int4* __restrict__ item
     const bool act = r < B;
     const int rr = act ? r : 0;
     for (int t = 0; t < I.w; ++t) acc[t][r] = make_float2(0.f, 0.f);   // each thread its own column
+    auto fetch = [&](int e0, int b) {           // terms [e0, e0 + kInterpGrpTile) into tile b
+        const int n8 = min(kInterpGrpTile, I.y - e0) * ((int)sizeof(InterpG) / 8);
+        for (int i = r; i < n8; i += 64)
+            cp_async_el<8>(reinterpret_cast<char*>(tile[b]) + 8 * i, reinterpret_cast<const char*>(terms + e0) + 8 * i);
+        cp_async_commit();
+    };
     float2 cc[P];
     int cur = -1;
     InterpG En{};
-    if (I.x < I.y) En = terms[I.x];
+    if (I.x < I.y) fetch(I.x, 0);
     for (int e = I.x; e < I.y; ++e) {
+        const int q = (e - I.x) % kInterpGrpTile, b = (e - I.x) / kInterpGrpTile & 1;
+        if (q == 0) {                           // the tile has arrived, the other one has been used
+            cp_async_wait<0>();
+            __syncthreads();
+            if (e + kInterpGrpTile < I.y) fetch(e + kInterpGrpTile, b ^ 1);
+            En = tile[b][0];
+        }
         const InterpG E = En;
-        if (e + 1 < I.y) En = terms[e + 1];     // next term in flight during this one
+        if (q + 1 < kInterpGrpTile) En = tile[b][q + 1];     // the next term's, before this one's sums
         if (E.cone != cur) {                    // uniform over the block
             cur = E.cone;
             const float2* src = coef + (long long)cur * P * B;
