@@ -212,10 +212,14 @@ void far_b(ifgf2d_ctx* ctx, int B, double2* yt) {
         launch_prop_b(p0, p1, ctx->pp_ptr.p, ctx->pp_nchild.p, pb, T.Ps, T.Pang, ctx->Gsep32.p, B, coef, s);
     }
     const bool grouped = (ctx->tune_batch_tc & kBatchGroupedInterp) && B <= 64 && T.Ps == 5 && T.Pang == 5;
-    launch_final_b((int)ctx->D.N, ctx->point_leaf.p, ctx->leaf_start.p, ctx->leaf_count.p, ctx->nbr_ptr.p, ctx->nbr_box.p,
-                   ctx->near_rowlen.p, ctx->near_off.p, ctx->near32.p, rho, ctx->ip_ptr.p, grouped ? nullptr : ctx->ip32.p, coef,
-                          T.Ps, T.Pang, ctx->sorting.p, B, yt, s);
-    if (grouped) launch_interp_grp(W.ig_items.p, (int)W.ig_items.n, W.ig_terms.p, coef, T.Ps, T.Pang, ctx->sorting.p, B, yt, s);
+    if (grouped) {
+        launch_near_b(ctx->fin32_items.p, (int)ctx->fin32_items.n, ctx->near_src.p, ctx->near32.p, rho, ctx->sorting.p, B, yt, s);
+        launch_interp_grp(W.ig_items.p, (int)W.ig_items.n, W.ig_terms.p, coef, T.Ps, T.Pang, ctx->sorting.p, B, yt, s);
+    } else {
+        launch_final_b((int)ctx->D.N, ctx->point_leaf.p, ctx->leaf_start.p, ctx->leaf_count.p, ctx->nbr_ptr.p, ctx->nbr_box.p,
+                       ctx->near_rowlen.p, ctx->near_off.p, ctx->near32.p, rho, ctx->ip_ptr.p, ctx->ip32.p, coef, T.Ps, T.Pang,
+                       ctx->sorting.p, B, yt, s);
+    }
 }
 // the same in FP64: the cone sums in fixed point (fixpoint.cuh)
 void far_bx(ifgf2d_ctx* ctx, int B, double2* yt) {

@@ -255,6 +255,8 @@ void launch_final_b(int N, const int* point_leaf, const int* leaf_start, const i
                     const float2* rho, const int* ip_ptr, const InterpE<float>* ip, const float2* coef, int Ps, int Pang,
                     const long long* sorting, int B, double2* yt, cudaStream_t s);
 // the FP64 near field in fixed point (tables as launch_final_fx's, densities as launch_leaf_bx's)
+void launch_near_b(const FinItem* items, int nitems, const int* near_src, const float2* near, const float2* rho,
+                   const long long* sorting, int B, double2* yt, cudaStream_t s);
 void launch_near_bx(int N, const int* point_leaf, const int* leaf_start, const int* leaf_count, const int* nbr_ptr, const int* nbr_box,
                     const int* near_rowlen, const long long* near_off, const int4* near, const int* nexp, const int4* rho,
                     const int* rexp, const long long* sorting, int B, double2* yt, cudaStream_t s);

@@ -112,14 +112,15 @@ __global__ void __launch_bounds__(256) k_sing_b(const double2* __restrict__ xt, 
 }
 
 // ------------------------------------------------------------------ asynchronous copies
-// cp.async (global -> shared without a register round trip) of one 8- or 16-byte element
+// cp.async (global -> shared without a register round trip) of one 4-, 8- or 16-byte element
 template <int BYTES>
 __device__ __forceinline__ void cp_async_el(void* smem, const void* gmem) {
+    static_assert(BYTES == 4 || BYTES == 8 || BYTES == 16, "the element sizes of cp.async");
     const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
     if (BYTES == 16)
         asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem) : "memory");
     else
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sa), "l"(gmem) : "memory");
+        asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n" ::"r"(sa), "l"(gmem), "n"(BYTES) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int NPEND>
@@ -338,7 +339,7 @@ __global__ void __launch_bounds__(WPB * 32) k_prop_b(int pbegin, int pend, const
     using R = float;
     constexpr int P = PS * PA;
     __shared__ V2<R> sv[WPB][P][32 * RPL];
-    __shared__ PropB<R> plan[WPB][4 * P];
+    __shared__ alignas(16) PropB<R> plan[WPB][4 * P];
     __shared__ R sG[PS * PS + PA * PA];
     for (int i = threadIdx.x; i < PS * PS + PA * PA; i += blockDim.x) sG[i] = Gsep[i];
     __syncthreads();
@@ -739,7 +740,7 @@ __global__ void __launch_bounds__(256) k_final_b(int N, const int* __restrict__ 
         }
         sg += c;
     }
-    for (int e = ip ? ip_ptr[i] : 0; ip && e < ip_ptr[i + 1]; ++e) {   // ip null: near field only
+    for (int e = ip_ptr[i]; e < ip_ptr[i + 1]; ++e) {
         const InterpE<R> E = ip[e];
         R Ts[PS], Tt[PA];
         cheb_row<R, PS>(E.s, Ts);
@@ -762,6 +763,81 @@ __global__ void __launch_bounds__(256) k_final_b(int N, const int* __restrict__ 
         double2 v = *yo;
         v.x += (double)acc[k].x; v.y += (double)acc[k].y;
         *yo = v;
+    }
+}
+
+// complex64 near field alone (the interpolation is grouped, k_interp_grp): an item is up to 32 targets of
+// one leaf box, a warp four of them x 32 RPL right-hand sides, so that a source's density row serves four
+// targets.  The four table rows and the source list come through shared memory, kNearTile sources at a
+// time, by the warp's own copies.  Each target's sum runs over its row in order, as in k_final_b.  Bound by
+// the latency of the density rows: eight sources' are in flight (four: twice the time; the next eight in
+// registers as well: 128 registers, 5 % slower at k = 2000).  Kite k = 500 / 2000, 64 right-hand sides: 102 /
+// 384 us with a warp per target, 54 / 202 us so.
+constexpr int kNearTile = 32;
+template <int RPL>
+__global__ void __launch_bounds__(256) k_near_b(const FinItem* __restrict__ items, const int* __restrict__ near_src,
+                                                const float2* __restrict__ near, const float2* __restrict__ rho,
+                                                const long long* __restrict__ sorting, int B, double2* __restrict__ yt) {
+    __shared__ float4 rows[8][2][kNearTile][2];       // [source][targets 0, 1 | 2, 3]
+    __shared__ int srcs[8][2][kNearTile];
+    const FinItem I = items[blockIdx.x];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, t0 = 4 * w;
+    if (t0 >= I.cnt) return;
+    const int nt = min(4, I.cnt - t0);
+    const float2* row = near + I.near + (long long)t0 * I.rl;
+    auto fetch = [&](int c0, int b) {
+        const int e = c0 + lane;
+        if (e < I.rl) {
+            cp_async_el<4>(&srcs[w][b][lane], near_src + I.src + e);
+            float2* to = reinterpret_cast<float2*>(rows[w][b][lane]);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) cp_async_el<8>(to + u, row + (long long)(u < nt ? u : 0) * I.rl + e);
+        }
+        cp_async_commit();
+    };
+    int rr[RPL];
+    bool act[RPL];
+    float2 acc[4][RPL];
+#pragma unroll
+    for (int k = 0; k < RPL; ++k) {
+        const int r = blockIdx.y * 32 * RPL + 32 * k + lane;
+        act[k] = r < B;
+        rr[k] = act[k] ? r : 0;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) acc[u][k] = make_float2(0.f, 0.f);
+    }
+    if (I.rl > 0) fetch(0, 0);
+    for (int c0 = 0, b = 0; c0 < I.rl; c0 += kNearTile, b ^= 1) {
+        cp_async_wait<0>();
+        __syncwarp();                                 // the tile is there, the other one has been used
+        if (c0 + kNearTile < I.rl) fetch(c0 + kNearTile, b ^ 1);
+        const int n = min(kNearTile, I.rl - c0);
+#pragma unroll 8
+        for (int e = 0; e < n; ++e) {
+            const float2* rh = rho + (long long)srcs[w][b][e] * B;
+            const float4 v01 = rows[w][b][e][0], v23 = rows[w][b][e][1];
+#pragma unroll
+            for (int k = 0; k < RPL; ++k) {
+                const float2 d = rh[rr[k]];
+                cmac<float>(acc[0][k], make_float2(v01.x, v01.y), d);
+                cmac<float>(acc[1][k], make_float2(v01.z, v01.w), d);
+                cmac<float>(acc[2][k], make_float2(v23.x, v23.y), d);
+                cmac<float>(acc[3][k], make_float2(v23.z, v23.w), d);
+            }
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        if (u >= nt) break;
+        const long long o = sorting[I.first + t0 + u];
+#pragma unroll
+        for (int k = 0; k < RPL; ++k) {
+            if (!act[k]) continue;
+            double2* yo = yt + o * B + rr[k];
+            double2 v = *yo;
+            v.x += (double)acc[u][k].x; v.y += (double)acc[u][k].y;
+            *yo = v;
+        }
     }
 }
 
@@ -828,7 +904,7 @@ __global__ void __launch_bounds__(64) k_interp_grp(const int4* __restrict__ item
                                                    double2* __restrict__ yt) {
     constexpr int P = PS * PA;
     __shared__ float2 acc[kInterpGrpTargets][64];
-    __shared__ InterpG tile[2][kInterpGrpTile];
+    __shared__ alignas(16) InterpG tile[2][kInterpGrpTile];
     const int it = blockIdx.x;
     if (it >= nitems) return;
     const int4 I = items[it];   // terms [x, y), targets [z, z + w)
@@ -1079,6 +1155,11 @@ void launch_final_b(int N, const int* point_leaf, const int* leaf_start, const i
     IFGF_DISPATCH_P(Ps, Pang, (k_final_b<PS, PA, RPL><<<grid, 256, 0, s>>>(N, point_leaf, leaf_start, leaf_count,
                                                                           nbr_ptr, nbr_box, near_rowlen, near_off, near,
                                                                           rho, ip_ptr, ip, coef, sorting, B, yt)));
+}
+void launch_near_b(const FinItem* items, int nitems, const int* near_src, const float2* near, const float2* rho,
+                   const long long* sorting, int B, double2* yt, cudaStream_t s) {
+    if (nitems > 0 && B > 0)
+        k_near_b<kRpl><<<dim3(nitems, nblk_b(B, 32 * kRpl)), 256, 0, s>>>(items, near_src, near, rho, sorting, B, yt);
 }
 void launch_near_bx(int N, const int* point_leaf, const int* leaf_start, const int* leaf_count, const int* nbr_ptr, const int* nbr_box,
                     const int* near_rowlen, const long long* near_off, const int4* near, const int* nexp, const int4* rho,
