@@ -278,18 +278,28 @@ int check_mode(ifgf2d_ctx* ctx, int mode) {
     return IFGF2D_OK;
 }
 
-// column-major device matrices, any nrhs
+// column-major device matrices, any nrhs.  A pass of the FP64 batch gives a warp's 32 lanes a right-hand
+// side each and takes the same time for 1 as for 32, so up to kFewColumns go one by one.  A pass and one
+// column by itself, us: kite k = 100 730 and 65, k = 250 1370 and 120, k = 500 2800 and 190, k = 2000 14660 and
+// 795; they meet at 12 columns at k = 100 and 250, at 15 and 18 at k = 500 and 2000.  complex64 keeps the pass:
+// its sums have another order there.
+constexpr int kFewColumns = 11;
 int apply_cm(ifgf2d_ctx* ctx, const double2* x, double2* y, int nrhs, int mode) {
     const long long N = ctx->D.N;
-    if (mode == IFGF2D_APPLY_DIRECT) {
-        for (int r = 0; r < nrhs; ++r) {
+    auto singly = [&](int r0, int r1) -> int {
+        for (int r = r0; r < r1; ++r) {
             int rc = apply_single(ctx, x + (long long)r * N, y + (long long)r * N, mode);
             if (rc != IFGF2D_OK) return rc;
         }
         return IFGF2D_OK;
-    }
+    };
+    if (mode == IFGF2D_APPLY_DIRECT) return singly(0, nrhs);
     for (int r0 = 0; r0 < nrhs; r0 += kMaxBatch) {
         const int B = std::min(kMaxBatch, nrhs - r0);
+        if (mode == IFGF2D_APPLY_IFGF && B <= kFewColumns) {
+            if (int rc = singly(r0, r0 + B)) return rc;
+            continue;
+        }
         int rc = ensure_apply(ctx, B, mode == IFGF2D_APPLY_IFGF_MIXED);
         if (rc != IFGF2D_OK) return rc;
         BatchWork& W = *ctx->bw;

@@ -28,3 +28,17 @@ def test_gpu_mixed_by_box(lib, Ps, Pang, k, npatch, nlevels):
             out[by_box, chunks] = fm.compute_Ax_acc(x, mixed=True)
             assert np.linalg.norm(out[by_box, chunks] - y) < 2e-6 * np.linalg.norm(y)
     assert np.array_equal(out[True, 5], (fm.set_tuning(table), fm.compute_Ax_acc(x, mixed=True))[1])
+
+
+@pytest.mark.parametrize("nrhs", [1, 11, 12, 64 + 11, 64 + 12])
+def test_gpu_batch_few_columns(lib, nrhs):
+    """FP64 batches up to 11 columns, and remainders of that size, go column by column: on either side of the
+    line each column is the single vector's, to the rounding of both (4e-15, as test_gpu_fixpoint.py)."""
+    fm = lib.ForwardMap(0.02, [lib.Kite()], (), 1.0, 60.0, Np=16, patches_per_curve=64, formulation="combined")
+    fm.precomps_and_setup(60.0, 0)
+    g = np.random.default_rng(nrhs)
+    X = g.standard_normal((fm.total_num_unknowns_, nrhs)) + 1j * g.standard_normal((fm.total_num_unknowns_, nrhs))
+    Y = fm.apply_batch(X)
+    for r in range(nrhs):
+        y = fm.compute_Ax_acc(X[:, r])
+        assert np.linalg.norm(Y[:, r] - y) <= 4e-15 * np.linalg.norm(y)
