@@ -1,16 +1,17 @@
-// ifgf_apply.cu -- per-apply IFGF kernels, templated on the arithmetic type.
+// ifgf_apply.cu -- per-apply IFGF kernels, in two forms.
 //
-// R = double: the plain form (complex128 tables; cone coefficients and interpolation in block fixed
-//             point of FP64 accuracy, fixpoint.cuh, the rest FP64 arithmetic).
-// R = float : the mixed form (complex64 copies of the same FP64-computed tables, FP32
-//             arithmetic; the rectangular-polar correction stays FP64).
+// FP64 (..._fx): tables, cone coefficients and sums in block fixed point of FP64 accuracy
+//                (fixpoint.cuh), the factor ratios in FP64.
+// complex64    : complex64 copies of the same FP64-computed tables, FP32 arithmetic; the
+//                rectangular-polar correction stays FP64.
 //
-//   k_intensities  density * quadrature weight, Morton permutation   ForwardMap.tpp:425-435, BoxTree.h:954-963
-//   k_leaf_apply   leaf cone coefficients (one thread per cone x coefficient)      BoxTree.h:685-762
-//   k_propagate    child -> parent coefficients (one thread per cone x node),
-//                  separable values->coefficients map                             BoxTree.h:767-868, Interpolator.h:81-120
-//   k_final        near field + every level's cousin interpolants, one warp per target,
-//                  result added to y at the target's original index               BoxTree.h:614-683, 876-937, 1063-1069
+//   k_intensities_t                density * quadrature weight, Morton permutation  ForwardMap.tpp:425-435, BoxTree.h:954-963
+//   k_leaf_fx, k_leaf_apply_t      leaf cone coefficients                          BoxTree.h:685-762
+//   k_propagate_fx, k_propagate_t  child -> parent coefficients, separable
+//                                  values->coefficients map                        BoxTree.h:767-868, Interpolator.h:81-120
+//   k_final_fx, k_final_q          near field + every level's cousin interpolants by leaf box (k_final_t by
+//                                  target), added to y at the target's original index
+//                                                                                  BoxTree.h:614-683, 876-937, 1063-1069
 #include "fixpoint.cuh"
 #include "tcgen05.cuh"
 #include <type_traits>
@@ -35,11 +36,13 @@ __global__ void k_intensities_t(const double2* __restrict__ x, const double* __r
 // coefficient): chunk ch takes the sources s = ch, ch + CH, ..., by turns into two sums; the CH partial sums
 // meet in shared memory.  Boxes hold 10-100 points, so splitting the source walk shortens the latency
 // chain of the longest boxes by CH.  cones: a cone's table offset (two ints), first source and sources, one
-// load ahead of the table's.  Bound by the loads in flight: 2048 threads an SM with four of the table's
-// each.  Kite k = 500 / 2000 (72 / 600 MB): 24 / 119 us; 28 / 129 with the box looked up first and two in
-// flight.  Six loads ahead in 61 registers, half the threads: 30 / 147.
+// load ahead of the table's.  Bound by the loads in flight: 1536 threads an SM, each with the next four table
+// entries on their way while it uses four; the table, read once, is marked to leave the caches first.  Kite
+// k = 500 / 2000 (72 / 600 MB): 22 / 113 us; 24 / 119 with 2048 threads and four loads at a time, 28 / 129 with
+// two and the box looked up first.  Six loads at a time in 61 registers, half the threads: 30 / 147.
+constexpr int kLeafAhead = 4;                  // even: the two sums take the entries by turns
 template <int CH>
-__global__ void __launch_bounds__(256, 8) k_leaf_apply_t(const int4* __restrict__ cones, int ncones, int cone_base,
+__global__ void __launch_bounds__(256, 6) k_leaf_apply_t(const int4* __restrict__ cones, int ncones, int cone_base,
                                                       const float2* __restrict__ L, const float2* __restrict__ rho, int P,
                                                       float2* __restrict__ coef) {
     __shared__ float2 part[256];
@@ -55,14 +58,22 @@ __global__ void __launch_bounds__(256, 8) k_leaf_apply_t(const int4* __restrict_
         const int n = D.w;
         const float2* Lc = L + ((long long)D.y << 32 | (unsigned)D.x) + m;
         const float2* rh = rho + D.z;
+        float2 l[kLeafAhead];
         int s = ch;
-#pragma unroll 2
-        for (; s + CH < n; s += 2 * CH) {
-            const float2 l0 = Lc[(long long)s * P], l1 = Lc[(long long)(s + CH) * P];
-            const float2 r0 = rh[s], r1 = rh[s + CH];
-            cmac<float>(a0, l0, r0); cmac<float>(a1, l1, r1);
+#pragma unroll
+        for (int u = 0; u < kLeafAhead; ++u) if (s + u * CH < n) l[u] = __ldcs(&Lc[(long long)(s + u * CH) * P]);
+        while (s < n) {
+            float2 now[kLeafAhead];
+            const int next = s + kLeafAhead * CH;
+#pragma unroll
+            for (int u = 0; u < kLeafAhead; ++u) {             // the next entries on their way before these are used
+                now[u] = l[u];
+                if (next + u * CH < n) l[u] = __ldcs(&Lc[(long long)(next + u * CH) * P]);
+            }
+#pragma unroll
+            for (int u = 0; u < kLeafAhead; ++u) if (s + u * CH < n) cmac<float>(u % 2 ? a1 : a0, now[u], rh[s + u * CH]);
+            s = next;
         }
-        if (s < n) cmac<float>(a0, Lc[(long long)s * P], rh[s]);
         a0.x += a1.x; a0.y += a1.y;
     }
     part[threadIdx.x] = a0;
@@ -80,11 +91,13 @@ __global__ void __launch_bounds__(256, 8) k_leaf_apply_t(const int4* __restrict_
 // sources): it brings the box's densities to their exponent in shared memory once, while its threads'
 // first table entries are in flight; the chunks' integer sums meet in shared memory; then the cone's
 // coefficients, whose entries have an exponent per coefficient, are brought to the cone's exponent.
-// Bound by the table's loads in flight (4 ahead of the barriers, then 4 a step, 3 blocks an SM).  Kite
-// k = 500 / 2000, 145 MB / 1.2 GB of table: 145 / 830 us with FP64 multiply-adds, 53 / 281 us so (2.9 / 4.3
-// TB/s).  CH = 2 keeps blocks of 5 cones, which amortises the conversion; 5 takes 67 / 350 us, 1 takes
-// 65 / 272; 8 loads ahead or 4 or 5 blocks an SM: within 3 % or slower.
-constexpr int kLeafFxAhead = 4, kLeafFxChunk = 256;
+// Bound by the table's loads in flight: a thread has the next three entries on their way while it uses
+// three, and three are ahead of the barriers; the table, read once, is marked to leave the caches first.
+// Kite k = 500 / 2000, 145 MB / 1.2 GB of table: 90 / 580 us with FP64 multiply-adds, 43 / 221 us so (3.4 / 5.4
+// TB/s); without the next entries on their way 53 / 281; two or five at a time 49 / 246, 43 / 227; registers
+// for 4 blocks an SM 49 / 262.  CH = 2 keeps blocks of 5 cones, which amortises the conversion; without the
+// look-ahead 5 took 67 / 350 us, 1 took 65 / 272.
+constexpr int kLeafFxAhead = 3, kLeafFxChunk = 256;
 template <int CH>
 __global__ void __launch_bounds__(256) k_leaf_fx(const LeafItem* __restrict__ items, int split, int cone_base,
                                                  const int4* __restrict__ L, const int* __restrict__ lexp,
@@ -106,7 +119,7 @@ __global__ void __launch_bounds__(256) k_leaf_fx(const LeafItem* __restrict__ it
     int El = 0;
     if (active) {
 #pragma unroll
-        for (int u = 0; u < kLeafFxAhead; ++u) if (ch + u * CH < n) ahead[u] = Lc[(long long)(ch + u * CH) * P];
+        for (int u = 0; u < kLeafFxAhead; ++u) if (ch + u * CH < n) ahead[u] = __ldcs(&Lc[(long long)(ch + u * CH) * P]);
         El = lexp[(long long)c * P + m];
     }
     stop[tid] = kFxMinExp;
@@ -133,17 +146,24 @@ __global__ void __launch_bounds__(256) k_leaf_fx(const LeafItem* __restrict__ it
         }
         __syncthreads();
         if (active) {
-            int s = c0 + (ch + CH - c0 % CH) % CH;
-            if (c0 == 0) {
+            int s = c0 + (ch + CH - c0 % CH) % CH, terms = 0;
+            if (c0) {
 #pragma unroll
-                for (int u = 0; u < kLeafFxAhead; ++u) if (ch + u * CH < c1) add(ahead[u], sr[ch + u * CH]);
-                s = ch + kLeafFxAhead * CH;
+                for (int u = 0; u < kLeafFxAhead; ++u) if (s + u * CH < n) ahead[u] = __ldcs(&Lc[(long long)(s + u * CH) * P]);
             }
             while (s < c1) {
-                const int f = min(c1, s + (kFxSumFold - kLeafFxAhead) * CH);
-#pragma unroll 4
-                for (; s < f; s += CH) add(Lc[(long long)s * P], sr[s - c0]);
-                if (s < c1) { fx_sum_fold(rr); fx_sum_fold(ii); fx_sum_fold(im); }
+                int4 now[kLeafFxAhead];
+                const int next = s + kLeafFxAhead * CH;
+#pragma unroll
+                for (int u = 0; u < kLeafFxAhead; ++u) {      // the next entries on their way before these are used
+                    now[u] = ahead[u];
+                    if (next + u * CH < c1) ahead[u] = __ldcs(&Lc[(long long)(next + u * CH) * P]);
+                }
+#pragma unroll
+                for (int u = 0; u < kLeafFxAhead; ++u) if (s + u * CH < c1) add(now[u], sr[s + u * CH - c0]);
+                s = next;
+                terms += kLeafFxAhead;
+                if (terms + kLeafFxAhead > kFxSumFold) { fx_sum_fold(rr); fx_sum_fold(ii); fx_sum_fold(im); terms = 0; }
             }
             fx_sum_fold(rr); fx_sum_fold(ii); fx_sum_fold(im);
         }
