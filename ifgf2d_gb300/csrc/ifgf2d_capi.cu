@@ -797,9 +797,9 @@ extern "C" int ifgf2d_apply_timed(ifgf2d_ctx* ctx, const void* d_x, void* d_y, i
 }
 
 // ------------------------------------------------------------------ launch-shape autotuner
-// Times every launch shape of the leaf kernel (source chunks 1, 2, 5, 10) and of each level's
-// propagation (2, 4 or the most cones per block) on this context's own tables, both
-// precisions, and keeps the fastest (median of `reps` CUDA-event timings).  choices (may be
+// Times every launch shape of the leaf kernels (source chunks 1, 2, 5, 10) and of each level's complex64
+// propagation (2, 4 or the most cones per block) on this context's own tables,
+// and keeps the fastest (median of `reps` CUDA-event timings).  choices (may be
 // NULL) receives the table: leaf FP64, leaf complex64, then kTuneLevels propagation entries
 // per precision, then the batched complex64 kernels on the tcgen05 tensor cores (bit 0 leaf
 // cones in 3xTF32, bit 1 propagation, bit 2 leaf cones with three TF32 terms per operand; FP32

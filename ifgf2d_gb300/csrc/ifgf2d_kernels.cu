@@ -6,10 +6,7 @@
 //   sing_apply   singular / near-singular correction        ForwardMap.tpp:481-515
 //   intensities  density * quadrature weight (+ Morton perm) ForwardMap.tpp:425-435, BoxTree.h:954-963
 //   direct_far   O(N^2) far sum with exclusions             ForwardMap.tpp:438-478
-//   leaf_apply   leaf cone coefficients                      BoxTree.h:685-762
-//   propagate    child -> parent cone coefficients           BoxTree.h:767-868
-//   final        near field + all-level interpolation + un-permute
-//                                                             BoxTree.h:614-683, 876-937, 1063-1069
+// The cone and near-field sums are in ifgf_apply.cu (one vector) and ifgf_batch.cu.
 #include "ifgf2d_kernels.cuh"
 #include "green_fx.cuh"
 

@@ -17,8 +17,9 @@
 //              cone's coefficients are loaded once                 BoxTree.h:767-868, Interpolator.h:81-120
 //   k_prop_bx, k_interp_bx  the FP64 propagation and interpolation
 //              in fixed point (fixpoint.cuh)
-//   k_final_b  near field (+ complex64 cousin interpolation) per
-//              target                                              BoxTree.h:614-683, 876-937
+//   k_near_b, k_interp_grp  near field by four targets, cousin
+//              interpolation grouped by cone; k_final_b both by
+//              target; k_near_bx the FP64 near field               BoxTree.h:614-683, 876-937
 //
 // plus the batched GMRES vector kernels (per-RHS dot products, CGS updates, scaling).
 #include "fixpoint.cuh"

@@ -284,11 +284,12 @@ int ifgf2d_apply_timed(ifgf2d_ctx* ctx, const void* d_x, void* d_y, int mode, do
 
 /* Launch-shape autotuner (no counterpart in the reference): times every launch shape of the
  * leaf-cone kernel (source chunks per coefficient 1, 2, 5, 10; complex64 also 0, the table
- * streamed through shared memory by TMA bulk copies), of each level's propagation (2, 4 or the
- * most cones per block, or 1: child blocks staged in shared memory) and of the single-vector
- * interpolation (by target or by leaf box) on this context's own tables, in both precisions, and
- * keeps the fastest.  The table has ifgf2d_tuning_size() ints: leaf FP64, leaf complex64, then
- * per precision one propagation entry per level (0 = the most cones per block), then a bit
+ * streamed through shared memory by TMA bulk copies) in both precisions, of each level's complex64
+ * propagation (2, 4 or the most cones per block, or 1: child blocks staged in shared memory) and of
+ * the complex64 single-vector interpolation (by target or by leaf box) on this context's own tables,
+ * and keeps the fastest.  The table has ifgf2d_tuning_size() ints: leaf FP64, leaf complex64, then
+ * per precision one propagation entry per level (0 = the most cones per block; the FP64 entries are
+ * accepted, its kernel has one shape), then a bit
  * mask of kernel choices: the batched complex64 kernels that run in 3xTF32 on the tcgen05
  * tensor cores (IFGF2D_BATCH_TC_*; FP32 FMA otherwise), the other batched choices and the
  * single-vector interpolation by leaf box (IFGF2D_SINGLE_INTERP_BY_BOX_*); the default is
