@@ -10,7 +10,7 @@ three regions (see hankel.cuh):
 
 green_tables.inc holds the fixed-point evaluator's tables (see green_fx.cuh): P and Q of
 H_nu = sqrt(2 / (pi x)) e^{i(x - pi/4 - nu pi/2)} (P_nu + i Q_nu) as polynomials of degree 6 in the
-position t in [-1/2, 1/2) within dyadic pieces of w = 1/x <= 1, and sin / cos of pi z / 2.
+position t in [-1/2, 1/2) within dyadic pieces of w = 1/x <= 1, as an array of 16-byte elements.
 
 All coefficients are computed here with mpmath at 50 digits and written as C hex-float
 literals and integers.  Run:  python gen_hankel_tables.py  (writes both files next to itself).
@@ -133,7 +133,7 @@ def green_tables():
             r += [(c3 - MAGIC) & 0xFFFFFFFF] + [f32(x) for x in f]
         rows.append(r)
     out.append("// [piece][10]: (c0, c1) of P0, Q0, P1, Q1; c2 of (P0, Q0), (P1, Q1); (c3, c4, c5, c6) of P0, Q0, P1, Q1")
-    out.append(f"GX_TABLE unsigned gx_table[GX_PIECES * 40] = {{" + ", ".join(f"0x{x:x}u" for r in rows for x in r) + "};")
+    out.append(f"GX_TABLE gx_table[GX_PIECES * 10] = {{" + ", ".join(f"0x{x:x}u" for r in rows for x in r) + "};")
     return out
 
 

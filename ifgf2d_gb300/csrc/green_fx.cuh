@@ -21,10 +21,14 @@
 #include "fixpoint.cuh"
 #include "hankel.cuh"
 
-#define GX_TABLE __device__ const
-#include "green_tables.inc"
-
 namespace ifgf {
+
+namespace gx {
+// 16 bytes of the table, one load; the table's element, so that its alignment is the loads'
+struct alignas(16) Four { unsigned x, y, z, w; };
+#define GX_TABLE __device__ const Four
+#include "green_tables.inc"
+}  // namespace gx
 
 struct GreenFx {
     unsigned long long kinv, kap_hi;   // 1/k = kinv 2^(kinv_e - 64); k / (2 pi) = (kap_hi 2^32 + kap_lo) 2^(kap_e - 96)
@@ -203,8 +207,8 @@ __host__ __device__ __forceinline__ void cos_sin(unsigned long long f, long long
     S = quad & 2 ? -b : b;
 }
 
-struct alignas(16) Four { unsigned x, y, z, w; };
 __host__ __device__ __forceinline__ Four load(const Four* p) {
+    static_assert(alignof(Four) == sizeof(uint4), "read as a uint4");
 #ifdef __CUDA_ARCH__
     const uint4 v = __ldg(reinterpret_cast<const uint4*>(p));
     return Four{v.x, v.y, v.z, v.w};
@@ -295,7 +299,7 @@ static __device__ __noinline__ double2 green_slow(int form, double dx, double dy
 __device__ __forceinline__ double2 green(const GreenFx& K, double dx, double dy, double nx, double ny) {
     const double d2 = dx * dx + dy * dy;
     if ((unsigned)__double2hiint(d2) - K.lo >= K.span) return green_slow(K.form, dx, dy, nx, ny, K.k, K.eta0);
-    return gx::value(K, reinterpret_cast<const gx::Four*>(gx_table), d2, K.form == 2 ? dx * nx + dy * ny : 0.0);
+    return gx::value(K, gx::gx_table, d2, K.form == 2 ? dx * nx + dy * ny : 0.0);
 }
 
 }  // namespace ifgf
