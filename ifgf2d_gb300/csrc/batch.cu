@@ -24,6 +24,7 @@ struct TermsXBuf {
         if (e == cudaSuccess) e = rows.alloc(n * batch_x_rows(Ps, Pang));
         return e;
     }
+    void release() { id.release(); w.release(); rows.release(); }
     TermsX view() const { return TermsX{id.p, w.p, rows.p}; }
 };
 
@@ -65,6 +66,19 @@ struct BatchWork {
     DBuf<double2> Z;
     DBuf<float2> ug;
     int zcap = 0, zm = 0;
+
+    // the vectors and coefficients of the applies, whose size goes with cap
+    void release_columns() {
+        xt.release(); yt.release(); rho64.release(); coef64.release(); rho32.release(); coef32.release();
+        xt32.release(); cexp64.release(); rhox.release(); rexp.release();
+        cap = 0;
+    }
+    // everything an apply needs
+    void release_apply() {
+        release_columns();
+        px64.release(); ig64.release(); ig64_items.release();
+        pb32.release(); W32.release(); t5err.release(); leaf_items.release(); ig_items.release(); ig_terms.release();
+    }
 };
 
 void ifgf::free_batch(ifgf2d_ctx* ctx) {
@@ -111,14 +125,12 @@ void grouped_interp_plan(const Tree& T, std::vector<int4>& items, std::vector<Te
     }, 64);
 }
 
-int ensure_apply(ifgf2d_ctx* ctx, int B, bool mixed) {
-    if (!ctx->bw) ctx->bw = new BatchWork;
+int grow_apply(ifgf2d_ctx* ctx, int B, bool mixed) {
     BatchWork& W = *ctx->bw;
     const long long N = ctx->D.N;
     const size_t ncoef = (size_t)ctx->T.total_cones * ctx->T.P;
     if (W.cap < B) {
-        W.xt.release(); W.yt.release(); W.rho64.release(); W.coef64.release(); W.rho32.release(); W.coef32.release();
-        W.xt32.release(); W.cexp64.release(); W.rhox.release(); W.rexp.release();
+        W.release_columns();
         CK(W.xt.alloc((size_t)N * B)); CK(W.yt.alloc((size_t)N * B));
         W.cap = B;
     }
@@ -156,6 +168,7 @@ int ensure_apply(ifgf2d_ctx* ctx, int B, bool mixed) {
         if (!W.W32.p) {
             CK(W.W32.alloc(ctx->W.n));
             launch_d2f(ctx->W.p, (long long)ctx->W.n, W.W32.p, ctx->stream);
+            CK(cudaGetLastError());
         }
     } else {
         if (!W.rho64.p) { CK(W.rho64.alloc((size_t)N * W.cap)); CK(W.coef64.alloc(ncoef * W.cap)); }
@@ -180,6 +193,14 @@ int ensure_apply(ifgf2d_ctx* ctx, int B, bool mixed) {
         }
     }
     return IFGF2D_OK;
+}
+// The workspace of a batched apply.  A buffer's presence stands for its whole group's, filled: one that
+// could not be had or filled takes all of them with it, and the next call starts anew.
+int ensure_apply(ifgf2d_ctx* ctx, int B, bool mixed) {
+    if (!ctx->bw) ctx->bw = new BatchWork;
+    const int rc = grow_apply(ctx, B, mixed);
+    if (rc != IFGF2D_OK) ctx->bw->release_apply();
+    return rc;
 }
 
 // yt += the far field: complex64
@@ -318,6 +339,7 @@ int ensure_solve(ifgf2d_ctx* ctx, int B, int m) {
     const long long N = ctx->D.N;
     if (W.scap < B || W.m != m) {
         const size_t nb = (size_t)N * B;
+        W.scap = W.zcap = 0;                   // until every buffer is there
         CK(W.V.alloc(nb * (m + 1))); CK(W.w.alloc(nb)); CK(W.t.alloc(nb));
         CK(W.b.alloc(nb)); CK(W.x.alloc(nb)); CK(W.r.alloc(nb)); CK(W.d.alloc(nb));
         CK(W.h.alloc((size_t)(m + 1) * B)); CK(W.H.alloc((size_t)m * (m + 1) * B));
@@ -361,6 +383,7 @@ int gmres_batch(ifgf2d_ctx* ctx, const double2* b, double2* x, int B, int mode, 
     if (rc != IFGF2D_OK) return rc;
     BatchWork& W = *ctx->bw;
     if (spec && (W.zcap < W.scap || W.zm != m)) {   // flexible: the preconditioned columns Z
+        W.zcap = 0;
         CK(W.Z.alloc((size_t)N * W.scap * m));
         CK(W.ug.alloc((size_t)spectral_grid_size(spec) * W.scap));
         W.zcap = W.scap; W.zm = m;
@@ -511,7 +534,7 @@ int solve_il(ifgf2d_ctx* ctx, int B, int mode, double tol, int restart, int max_
             // only the columns still short of the tolerance: the batched applies cost in
             // proportion to their columns, frozen ones included
             const size_t nc = (size_t)N * Bc;
-            if (W.cb.n < nc) {
+            if (std::min({W.cb.n, W.cx.n, W.cr.n, W.cd.n, W.ct.n}) < nc) {
                 CK(W.cb.alloc((size_t)N * B)); CK(W.cx.alloc((size_t)N * B)); CK(W.cr.alloc((size_t)N * B));
                 CK(W.cd.alloc((size_t)N * B)); CK(W.ct.alloc((size_t)N * B));
             }
@@ -563,7 +586,7 @@ extern "C" int ifgf2d_apply_batch(ifgf2d_ctx* ctx, const double* x, double* y, i
     const int chunk = std::min(nrhs, kMaxBatch);
     if (!ctx->bw) ctx->bw = new BatchWork;
     BatchWork& W = *ctx->bw;
-    if (W.xcm.n < (size_t)N * chunk) { CK(W.xcm.alloc((size_t)N * chunk)); CK(W.ycm.alloc((size_t)N * chunk)); }
+    if (std::min(W.xcm.n, W.ycm.n) < (size_t)N * chunk) { CK(W.xcm.alloc((size_t)N * chunk)); CK(W.ycm.alloc((size_t)N * chunk)); }
     for (int r0 = 0; r0 < nrhs; r0 += chunk) {
         const int B = std::min(chunk, nrhs - r0);
         const size_t bytes = sizeof(double2) * (size_t)N * B;
@@ -599,7 +622,7 @@ int solve_batch(ifgf2d_ctx* ctx, const double* rhs, double* x, int nrhs, int mod
     if (mode == IFGF2D_APPLY_IFGF_MIXED && (rc = ensure_apply(ctx, chunk, false))) return rc;
     if ((rc = ensure_solve(ctx, chunk, (int)std::min<long long>(restart, N)))) return rc;
     BatchWork& W = *ctx->bw;
-    if (W.xcm.n < (size_t)N * chunk) { CK(W.xcm.alloc((size_t)N * chunk)); CK(W.ycm.alloc((size_t)N * chunk)); }
+    if (std::min(W.xcm.n, W.ycm.n) < (size_t)N * chunk) { CK(W.xcm.alloc((size_t)N * chunk)); CK(W.ycm.alloc((size_t)N * chunk)); }
     cudaStream_t s = ctx->stream;
     for (int r0 = 0; r0 < nrhs; r0 += chunk) {
         const int B = std::min(chunk, nrhs - r0);

@@ -76,21 +76,28 @@ struct DBuf {
         n = 0;
         owner = nullptr;
     }
+    // on failure the buffer is empty and the runtime's error is cleared, so that a later call may try again
     cudaError_t alloc(size_t cnt) {
         release();
-        n = cnt;
         if (cnt == 0) return cudaSuccess;
-        if (cudaStream_t s = alloc_stream()) {
-            owner = s;
-            return cudaMallocAsync((void**)&p, cnt * sizeof(T), s);
+        const cudaStream_t s = alloc_stream();
+        const cudaError_t e = s ? cudaMallocAsync((void**)&p, cnt * sizeof(T), s) : cudaMalloc((void**)&p, cnt * sizeof(T));
+        if (e != cudaSuccess) {
+            p = nullptr;
+            cudaGetLastError();
+            return e;
         }
-        return cudaMalloc((void**)&p, cnt * sizeof(T));
+        n = cnt;
+        owner = s;
+        return cudaSuccess;
     }
     cudaError_t upload(const T* src, size_t cnt) {
         cudaError_t e = alloc(cnt);
         if (e != cudaSuccess || cnt == 0) return e;
-        if (owner) return cudaMemcpyAsync(p, src, cnt * sizeof(T), cudaMemcpyHostToDevice, owner);
-        return cudaMemcpy(p, src, cnt * sizeof(T), cudaMemcpyHostToDevice);
+        e = owner ? cudaMemcpyAsync(p, src, cnt * sizeof(T), cudaMemcpyHostToDevice, owner)
+                  : cudaMemcpy(p, src, cnt * sizeof(T), cudaMemcpyHostToDevice);
+        if (e != cudaSuccess) release();
+        return e;
     }
     cudaError_t upload(const std::vector<T>& v) { return upload(v.data(), v.size()); }
 };

@@ -345,7 +345,7 @@ int group_workspace(ifgf2d_group* G, int m) {
     ifgf2d_ctx* ctx = G->g;
     const long long N = ctx->D.N;
     const int B = G->n;
-    if (!G->seg_of.p) {
+    if (!(G->seg_of.p && G->seg_chunk_ptr.p && G->chunk_lo.p)) {
         std::vector<int> seg(N), sc(B + 1, 0);
         std::vector<long long> lo;
         for (int s = 0; s < B; ++s) {
@@ -361,6 +361,7 @@ int group_workspace(ifgf2d_group* G, int m) {
     if (G->m != m) {
         G->drop_graphs();
         const size_t ldh = (size_t)m + 1;
+        G->m = 0;                              // until every buffer is there
         CK(G->V.alloc((size_t)N * ldh)); CK(G->w.alloc(N)); CK(G->vin.alloc(N)); CK(G->t.alloc(N));
         CK(G->H.alloc(ldh * m * B)); CK(G->hh.alloc(ldh * B)); CK(G->part.alloc(ldh * G->nchunk));
         CK(G->Y.alloc((size_t)m * B)); CK(G->hn.alloc(B)); CK(G->jdev.alloc(1)); CK(G->act.alloc(m));
@@ -406,7 +407,7 @@ int group_gmres(ifgf2d_group* G, const double2* b, double2* x, int mode, const s
     const SegDesc S = seg_desc(G);
     const LsqBatchDev L{G->lsR.p, G->lsg.p, G->lsgc.p, G->lsgs.p, G->lsst.p, G->lssc.p, m, B};
     const int gi = (mode == IFGF2D_APPLY_IFGF_MIXED ? 1 : 0) + (spec ? 2 : 0);
-    if (spec && G->Z.n != (size_t)N * m) { CK(G->Z.alloc((size_t)N * m)); CK(G->zt.alloc(N)); }
+    if (spec && (G->Z.n != (size_t)N * m || !G->zt.p)) { CK(G->Z.alloc((size_t)N * m)); CK(G->zt.alloc(N)); }
     if (!G->exec[gi]) {
         cudaGraph_t graph;
         CK(cudaGraphCreate(&graph, 0));
@@ -519,7 +520,7 @@ int group_solve(ifgf2d_group* G, const double* rhs, double* xout, int mode, doub
     AllocStream guard(ctx->stream);
     cudaStream_t s = ctx->stream;
     if (int rc = group_workspace(G, (int)std::max<long long>(1, std::min<long long>(restart, N)))) return rc;
-    if (G->b.n != (size_t)N) { CK(G->b.alloc(N)); CK(G->x.alloc(N)); CK(G->r.alloc(N)); CK(G->d.alloc(N)); }
+    if (!(G->b.p && G->x.p && G->r.p && G->d.p)) { CK(G->b.alloc(N)); CK(G->x.alloc(N)); CK(G->r.alloc(N)); CK(G->d.alloc(N)); }
     CK(cudaMemcpyAsync(G->b.p, rhs, sizeof(double2) * N, cudaMemcpyHostToDevice, s));
     std::vector<int> iters(B, 0);
     std::vector<double> est(B, 0.0);

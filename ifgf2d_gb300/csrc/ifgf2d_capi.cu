@@ -998,6 +998,7 @@ static int gmres_core(ifgf2d_ctx* ctx, const double2* b, double2* x, int mode, d
     GmresWork& G = *ctx->gw;
     if (G.n != N || G.m != m) {
         G.drop_graphs();
+        G.n = 0;                               // until every buffer is there
         CK(G.V.alloc((size_t)N * (m + 1))); CK(G.w.alloc(N)); CK(G.h.alloc(m + 2)); CK(G.t.alloc(N)); CK(G.vin.alloc(N));
         CK(G.H.alloc((size_t)ldh * m)); CK(G.y.alloc(m)); CK(G.nrm2.alloc(1)); CK(G.jdev.alloc(1));
         CK(G.part.alloc((size_t)arnoldi_part_size(N, m)));
@@ -1007,8 +1008,8 @@ static int gmres_core(ifgf2d_ctx* ctx, const double2* b, double2* x, int mode, d
         G.n = N; G.m = m;
     }
     const int pk = P ? P->kind() : 0;
-    if (pk && !G.Z.p) { CK(G.Z.alloc((size_t)N * m)); CK(G.zt.alloc(N)); }
-    if (pk == 3 && !G.zt2.p) { CK(G.zt2.alloc(N)); CK(G.zt3.alloc(N)); }
+    if (pk && !(G.Z.p && G.zt.p)) { CK(G.Z.alloc((size_t)N * m)); CK(G.zt.alloc(N)); }
+    if (pk == 3 && !(G.zt2.p && G.zt3.p)) { CK(G.zt2.alloc(N)); CK(G.zt3.alloc(N)); }
     const LsqDev L{G.lsR.p, G.lsg.p, G.lsgc.p, G.lsgs.p, G.lsst.p, G.lssc.p, m};
     const int gi = mode + 3 * pk;
     if (!G.exec[gi]) {
