@@ -303,7 +303,8 @@ int check_mode(ifgf2d_ctx* ctx, int mode) {
 // side each and takes the same time for 1 as for 32, so up to kFewColumns go one by one.  A pass and one
 // column by itself, us: kite k = 100 730 and 65, k = 250 1370 and 120, k = 500 2800 and 190, k = 2000 14660 and
 // 795; they meet at 12 columns at k = 100 and 250, at 15 and 18 at k = 500 and 2000.  complex64 keeps the pass:
-// its sums have another order there.
+// its sums have another order there.  So do matrices that overlap: a pass reads its columns before it writes
+// any, a column by itself writes y while it reads x.
 constexpr int kFewColumns = 11;
 int apply_cm(ifgf2d_ctx* ctx, const double2* x, double2* y, int nrhs, int mode) {
     const long long N = ctx->D.N;
@@ -317,7 +318,9 @@ int apply_cm(ifgf2d_ctx* ctx, const double2* x, double2* y, int nrhs, int mode) 
     if (mode == IFGF2D_APPLY_DIRECT) return singly(0, nrhs);
     for (int r0 = 0; r0 < nrhs; r0 += kMaxBatch) {
         const int B = std::min(kMaxBatch, nrhs - r0);
-        if (mode == IFGF2D_APPLY_IFGF && B <= kFewColumns) {
+        const double2 *xc = x + (long long)r0 * N, *yc = y + (long long)r0 * N;
+        const bool apart = xc + (long long)B * N <= yc || yc + (long long)B * N <= xc;
+        if (mode == IFGF2D_APPLY_IFGF && B <= kFewColumns && apart) {
             if (int rc = singly(r0, r0 + B)) return rc;
             continue;
         }

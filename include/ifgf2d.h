@@ -153,7 +153,8 @@ int ifgf2d_solve(ifgf2d_ctx* ctx, const double* rhs, double* x, int mode, double
 #define IFGF2D_MAX_BATCH 64
 int ifgf2d_apply_batch(ifgf2d_ctx* ctx, const double* x, double* y, int nrhs, int mode);
 /* the same on device-resident matrices (cudaMalloc'ed, N * nrhs complex each); asynchronous on
- * the context's stream */
+ * the context's stream.  The IFGF modes read a chunk's columns before they write any of its results, so
+ * y may be x or overlap it within a chunk. */
 int ifgf2d_apply_batch_device(ifgf2d_ctx* ctx, const void* d_x, void* d_y, int nrhs, int mode);
 /* ifgf2d_solve for every column of rhs: GMRES runs for all right-hand sides in lock step with
  * the batched operator, each with its own Krylov basis, Hessenberg matrix, rotations and stop
