@@ -12,8 +12,9 @@
 //     three wide multiply-adds into two 64-bit accumulators, exact and free of overflow.
 // Every value is held to 2^-56 of its block's largest and every weight to 2^-59, an eighth of the
 // FP64 rounding unit of the largest value; the sums round once.  So the results are nearer to the
-// exact ones than FP64 arithmetic's.  Blocks that hold a NaN or an infinity, or values above 2^1000,
-// carry the exponent kFxBad and evaluate to NaN.
+// exact ones than FP64 arithmetic's.  Exponents cover FP64's whole range, subnormal numbers included;
+// blocks that hold a NaN or an infinity, or whose values pass FP64's range, carry the exponent kFxBad and
+// evaluate to NaN.
 #pragma once
 #include "ifgf_device.cuh"
 
@@ -21,9 +22,10 @@ namespace ifgf {
 
 constexpr int kFxLow = 29;                    // bits of the low limb
 constexpr int kFxOne = 2 * kFxLow;            // fraction bits of a weight
-constexpr int kFxMinExp = -940;               // smallest block exponent: values below 2^(kFxMinExp - T) vanish
-constexpr int kFxMaxExp = 1000;               // larger (or non-finite) values make the block kFxBad
+constexpr int kFxMinExp = -1022;              // smallest block exponent: its values' unit is below FP64's smallest number
+constexpr int kFxMaxExp = 1024;               // larger (or non-finite) values make the block kFxBad
 constexpr int kFxBad = 0x7fffffff;
+constexpr int kFxNear0 = -960, kFxNear1 = 1010;   // exponents whose blocks' values are normal numbers
 __host__ __device__ constexpr int fx_top(int P) { return P <= 36 ? 55 : 54; }
 
 // limbs of a 64-bit integer, |value| < 2^60: the low one balanced (what is stored), or as the bits
@@ -58,8 +60,8 @@ __host__ __device__ constexpr int fx_rows4(int Ps, int Pang) { return (Ps + Pang
 
 // a block's exponent from the largest high word of its values' magnitudes: |value| < 2^E
 __device__ __forceinline__ int fx_expo(int maxhi) {
-    const int e = (maxhi >> 20) - 1022;
-    return e > kFxMaxExp ? kFxBad : max(e, kFxMinExp);
+    const int e = (maxhi >> 20) - 1022;        // kFxMinExp at least
+    return e > kFxMaxExp ? kFxBad : e;
 }
 __device__ __forceinline__ int fx_absmax_hi(double a, double b) {
     return max(__double2hiint(a) & 0x7fffffff, __double2hiint(b) & 0x7fffffff);
@@ -74,13 +76,24 @@ __device__ __forceinline__ long long fx_from(double v, int E, int T) {
     const long long x = s > 60 ? 0ll : ((mant << 3) + (1ll << (s - 1))) >> s;
     return hi < 0 ? -x : x;
 }
-// x 2^(E - T) as a double (x an integer below 2^62 in magnitude)
-__device__ __forceinline__ double fx_value(long long x, int E, int T) {
-    const double d = (double)x;
-    int hi = __double2hiint(d);
-    hi = x != 0 ? (int)((unsigned)hi + ((unsigned)(E - T) << 20)) : 0;
-    hi = E == kFxBad ? 0x7ff80000 : hi;        // NaN
-    return __hiloint2double(hi, __double2loint(d));
+// d 2^e for d = 0 or 1 <= |d| < 2^63, rounded once: subnormal or infinite where FP64's range ends
+__device__ __forceinline__ double fx_ldexp(double d, int e) {
+    const int a = min(max(e, -1000), 1000), b = min(max(e - a, -1022), 1023);
+    return d * __hiloint2double((1023 + a) << 20, 0) * __hiloint2double((1023 + b) << 20, 0);
+}
+// (x, y) 2^(E - T) as doubles (x and y integers below 2^62 in magnitude)
+__device__ __forceinline__ double2 fx_value(long long x, long long y, int E, int T) {
+    double a = (double)x, b = (double)y;
+    if ((unsigned)(E - kFxNear0) <= (unsigned)(kFxNear1 - kFxNear0)) {
+        const unsigned sh = (unsigned)(E - T) << 20;
+        a = __hiloint2double(x != 0 ? (int)((unsigned)__double2hiint(a) + sh) : 0, __double2loint(a));
+        b = __hiloint2double(y != 0 ? (int)((unsigned)__double2hiint(b) + sh) : 0, __double2loint(b));
+    } else {
+        const double nan = __hiloint2double(0x7ff80000, 0);
+        a = E == kFxBad ? nan : fx_ldexp(a, E - T);
+        b = E == kFxBad ? nan : fx_ldexp(b, E - T);
+    }
+    return make_double2(a, b);
 }
 
 // T_1..T_{n-1} of a weight (T_0 = 1 is left out), t[i] holding T_{i+1}:
@@ -144,7 +157,7 @@ __device__ __forceinline__ double2 fx_interp_value(Load&& c, int E, longlong2 st
     fx_cheb<PA>(st.y, Tt);
     long long re, im;
     fx_interp<PS, PA>(Ts, Tt, c, re, im);
-    return make_double2(fx_value(re, E, fx_top(PS * PA)), fx_value(im, E, fx_top(PS * PA)));
+    return fx_value(re, im, E, fx_top(PS * PA));
 }
 // ---- table sums (leaf cones): sum_s L[s] rho[s] of complex values, the table entries and the densities
 // both as integers of kFxSumTop bits in two 27-bit limbs, X = h 2^27 + l, |l| <= 2^26 (the left-out
@@ -181,13 +194,12 @@ __device__ __forceinline__ long long fx_align(long long y, int e, int E, int T) 
     const int sh = e - E + T;
     return sh >= 0 ? y << sh : (sh < -62 ? 0ll : (y + (1ll << (-sh - 1))) >> -sh);
 }
-// y 2^e as a double, 0 or infinity outside its range
+// y 2^e as a double, rounded once more where it is subnormal, infinite past the range
 __device__ __forceinline__ double fx_scaled(long long y, int e) {
     const double d = (double)y;
     const int hi = __double2hiint(d), x = ((hi >> 20) & 0x7ff) + e;
-    if (y == 0 || x <= 0) return 0.0;
-    return x >= 0x7ff ? __hiloint2double((hi & 0x80000000) | 0x7ff00000, 0)
-                      : __hiloint2double((hi & 0x800fffff) | (x << 20), __double2loint(d));
+    if (y == 0 || (unsigned)(x - 1) >= 0x7feu) return fx_ldexp(d, e);
+    return __hiloint2double((hi & 0x800fffff) | (x << 20), __double2loint(d));
 }
 // the exponent that y 2^e stays below
 __device__ __forceinline__ int fx_top_of(long long y, int e) { return y ? e + 64 - __clzll(y < 0 ? -y : y) : kFxMinExp; }

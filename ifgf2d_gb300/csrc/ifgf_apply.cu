@@ -93,13 +93,14 @@ __global__ void __launch_bounds__(256, 6) k_leaf_apply_t(const int4* __restrict_
 // coefficients, whose entries have an exponent per coefficient, are brought to the cone's exponent.
 // Bound by the table's loads in flight: a thread has the next three entries on their way while it uses
 // three, and three are ahead of the barriers; the table, read once, is marked to leave the caches first.
-// Kite k = 500 / 2000, 145 MB / 1.2 GB of table: 90 / 580 us with FP64 multiply-adds, 43 / 221 us so (3.4 / 5.4
-// TB/s); without the next entries on their way 53 / 281; two or five at a time 49 / 246, 43 / 227; registers
-// for 4 blocks an SM 49 / 262.  CH = 2 keeps blocks of 5 cones, which amortises the conversion; without the
+// Kite k = 500 / 2000, 145 MB / 1.2 GB of table: 90 / 580 us with FP64 multiply-adds, 41 / 219 us so (3.5 / 5.5
+// TB/s); without the next entries on their way 53 / 281; two or five at a time 49 / 246, 43 / 227.  CH = 2 is
+// held to the 64 registers that let 4 blocks share an SM: left alone it takes 68, and the apply 6 / 35 us
+// longer.  CH = 2 keeps blocks of 5 cones, which amortises the conversion; without the
 // look-ahead 5 took 67 / 350 us, 1 took 65 / 272.
 constexpr int kLeafFxAhead = 3, kLeafFxChunk = 256;
 template <int CH>
-__global__ void __launch_bounds__(256) k_leaf_fx(const LeafItem* __restrict__ items, int split, int cone_base,
+__global__ void __launch_bounds__(256, CH == 2 ? 4 : 0) k_leaf_fx(const LeafItem* __restrict__ items, int split, int cone_base,
                                                  const int4* __restrict__ L, const int* __restrict__ lexp,
                                                  const double2* __restrict__ rho, int P, int Ps, int4* __restrict__ coef,
                                                  int* __restrict__ cexp) {

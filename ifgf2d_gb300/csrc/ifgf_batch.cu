@@ -478,7 +478,7 @@ __device__ __forceinline__ void terms_x(StageX<PS, PA>& S, TermsX terms, long lo
             long long re, im;
             fx_interp<PS, PA>(t, t + PS - 1, [&](int q) { return cc[q]; }, re, im);
             const double2 w = S.w[i];
-            add(id.y, make_double2(fx_value(re, E, T), fx_value(im, E, T)), w);
+            add(id.y, fx_value(re, im, E, T), w);
         }
     }
 }
