@@ -251,7 +251,8 @@ void far_bx(ifgf2d_ctx* ctx, int B, double2* yt) {
     BatchWork& W = *ctx->bw;
     launch_rho_bx(ctx->leaf_start.p, ctx->leaf_count.p, (int)T.leaf_start.size(), W.rho64.p, B, W.rhox.p, W.rexp.p, s);
     launch_leaf_bx(ctx->leaf_cone_box.p, (int)LD.cone_nonrel.size(), LD.cone_base, ctx->leaf_start.p, ctx->leaf_count.p,
-                   ctx->leaf_off.p, ctx->leafL.p, ctx->lexp.p, W.rhox.p, W.rexp.p, T.Ps, T.Pang, B, W.coef64.p, W.cexp64.p, s);
+                   ctx->leaf_off.p, ctx->leafL.p, ctx->lexp.p, W.rhox.p, W.rexp.p, T.Ps, T.Pang, B, ctx->leaf_most, W.coef64.p,
+                   W.cexp64.p, s);
     for (int l = Dl; l >= 3; --l) {
         const TreeLevel& Lp = T.L[l - 1];
         launch_prop_bx(Lp.cone_base, Lp.cone_base + (int)Lp.cone_nonrel.size(), ctx->pp_ptr.p, W.px64.view(), T.Ps, T.Pang, ctx->GsepX.p,

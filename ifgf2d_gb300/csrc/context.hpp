@@ -227,6 +227,7 @@ struct ifgf2d_ctx {
     DBuf<int> leaf_cone_box;
     DBuf<long long> leaf_off;
     DBuf<LeafItem> leaf_items;      // work items of the FP64 leaf sums
+    int leaf_most = 0;              // sources of the largest leaf box
     DBuf<int4> leaf_cones;          // the complex64 leaf sums' cones
     DBuf<LeafNode> leaf_nodes_d;
     DBuf<int4> leafL;               // the FP64 form's leaf-cone tables: fixed-point limbs, with

@@ -162,10 +162,9 @@ __device__ __forceinline__ double2 fx_interp_value(Load&& c, int E, longlong2 st
 // ---- table sums (leaf cones): sum_s L[s] rho[s] of complex values, the table entries and the densities
 // both as integers of kFxSumTop bits in two 27-bit limbs, X = h 2^27 + l, |l| <= 2^26 (the left-out
 // products l l stay below 2^-56 of the largest).  The entries of one coefficient share an exponent, the
-// densities of one leaf box another; a box of more than 128 points gives its densities fewer bits, so
-// that no sum overflows.
-constexpr int kFxSumLow = 27, kFxSumTop = 54, kFxSumFold = 64;
-__device__ __forceinline__ int fx_rho_top(int n) { return kFxSumTop - max(0, 32 - __clz(max(n - 1, 0)) - 7); }
+// densities of one leaf box another.  kFxSumMost terms fit the 64-bit sums; larger boxes are summed in
+// parts of at most so many.
+constexpr int kFxSumLow = 27, kFxSumTop = 54, kFxSumFold = 64, kFxSumMost = 128;
 __device__ __forceinline__ int4 fx_pack_sum(long long re, long long im) {
     const int rh = (int)((re + (1ll << (kFxSumLow - 1))) >> kFxSumLow), ih = (int)((im + (1ll << (kFxSumLow - 1))) >> kFxSumLow);
     return make_int4(rh, (int)((unsigned)re - ((unsigned)rh << kFxSumLow)), ih, (int)((unsigned)im - ((unsigned)ih << kFxSumLow)));
@@ -177,17 +176,24 @@ __device__ __forceinline__ void fx_sum_mac(FxSum& s, int ah, int al, int bh, int
     s.m = fx_wide(al, bh, s.m);
     s.h = fx_wide(ah, bh, s.h);
 }
-__device__ __forceinline__ void fx_sum_fold(FxSum& s) {
-    s.h += s.m >> kFxSumLow;
-    s.m &= (1ll << kFxSumLow) - 1;
+__device__ __forceinline__ void fx_sum_fold(FxSum& s, int K = 0) {
+    s.h += s.m >> (kFxSumLow + K);
+    s.m &= (1ll << (kFxSumLow + K)) - 1;
 }
-// a folded sum of blocks with exponent E (table plus density, minus their bits) as y 2^e, |y| < 2^62 with
-// at most the sum's own bits lost
-__device__ __forceinline__ long long fx_sum_value(FxSum s, int E, int& e) {
-    const int lz = __clzll(s.h < 0 ? ~s.h : s.h);
-    const int sh = min(max(lz - 3, 0), kFxSumLow);
-    e = E + 2 * kFxSumLow - sh;
-    return (s.h << sh) + (s.m >> (kFxSumLow - sh));
+// The parts of a sum of n > kFxSumMost terms add up without loss in units of 2^K, K = fx_sum_wide(n): h of 2^K,
+// m of 2^-kFxSumLow
+__device__ __forceinline__ int fx_sum_wide(int n) { return max(0, 32 - __clz(max(n - 1, 0)) - 7); }
+__device__ __forceinline__ void fx_sum_part(FxSum& s, FxSum part, int K) {
+    s.h += part.h >> K;
+    s.m += ((part.h & ((1ll << K) - 1)) << kFxSumLow) + part.m;
+}
+// a folded sum's value, or such parts' (K > 0), of blocks with exponent E (table plus density, minus their bits) as
+// y 2^e, |y| < 2^62 with at most the sum's own bits lost
+__device__ __forceinline__ long long fx_sum_value(FxSum s, int E, int& e, int K = 0) {
+    const int low = kFxSumLow + K, lz = __clzll(s.h < 0 ? ~s.h : s.h);
+    const int sh = min(max(lz - 3, 0), low);
+    e = E + 2 * kFxSumLow + K - sh;
+    return (s.h << sh) + (s.m >> (low - sh));
 }
 // y 2^e as the integer of a block with exponent E and T bits, rounded
 __device__ __forceinline__ long long fx_align(long long y, int e, int E, int T) {

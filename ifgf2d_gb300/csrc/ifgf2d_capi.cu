@@ -510,6 +510,7 @@ static int setup_cones(ifgf2d_ctx* ctx, double k, int nlevels, const SetupExtra*
     CK(ctx->leaf_cone_box.upload(LD.cone_box)); CK(ctx->leaf_off.upload(loff));
     CK(ctx->leaf_cones.upload(leaf_cone_list(LD.cone_box, T.leaf_start, T.leaf_count, loff)));
     CK(ctx->leaf_items.upload(leaf_item_list(LD.cone_box, T.leaf_start, T.leaf_count, loff, P)));
+    ctx->leaf_most = T.leaf_count.empty() ? 0 : *std::max_element(T.leaf_count.begin(), T.leaf_count.end());
     CK(ctx->leafL.alloc(loff[ncl]));
     CK(ctx->leaf_nodes_d.alloc((size_t)ncl * P));
     CK(ctx->pp.alloc((size_t)T.pp_total)); CK(ctx->pp32.alloc((size_t)T.pp_total));

@@ -203,12 +203,13 @@ void launch_sing_b(const double2* xt, const float2* xt32, const double2* W, cons
 void launch_leaf_b(const int* cone_box, int ncones, int cone_base, const int* leaf_start, const int* leaf_count,
                    const long long* leaf_off, const float2* L, const float2* rho, int Ps, int Pang, int B, float2* coef,
                    cudaStream_t s);
-// the FP64 form in fixed point: table as launch_leaf_fx's, densities and exponents [box][B] from launch_rho_bx
+// the FP64 form in fixed point: table as launch_leaf_fx's, densities and exponents [box][B] from launch_rho_bx;
+// most: the sources of the largest leaf box
 void launch_rho_bx(const int* leaf_start, const int* leaf_count, int nleaf, const double2* rho, int B, int4* out, int* rexp,
                    cudaStream_t s);
 void launch_leaf_bx(const int* cone_box, int ncones, int cone_base, const int* leaf_start, const int* leaf_count,
                     const long long* leaf_off, const int4* L, const int* lexp, const int4* rho, const int* rexp, int Ps, int Pang, int B,
-                    int4* coef, int* cexp, cudaStream_t s);
+                    int most, int4* coef, int* cexp, cudaStream_t s);
 void launch_prop_b(int pbegin, int pend, const long long* pp_ptr, const int* pp_nchild, const PropB<float>* pb, int Ps, int Pang,
                    const float* Gsep, int B, float2* coef, cudaStream_t s);
 // the FP64 form in fixed point (fixpoint.cuh): coefficients [cone][P][B] as limbs with one exponent per

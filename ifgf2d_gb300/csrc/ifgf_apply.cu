@@ -93,27 +93,33 @@ __global__ void __launch_bounds__(256, 6) k_leaf_apply_t(const int4* __restrict_
 // coefficients, whose entries have an exponent per coefficient, are brought to the cone's exponent.
 // Bound by the table's loads in flight: a thread has the next three entries on their way while it uses
 // three, and three are ahead of the barriers; the table, read once, is marked to leave the caches first.
-// Kite k = 500 / 2000, 145 MB / 1.2 GB of table: 90 / 580 us with FP64 multiply-adds, 41 / 219 us so (3.5 / 5.5
-// TB/s); without the next entries on their way 53 / 281; two or five at a time 49 / 246, 43 / 227.  CH = 2 is
-// held to the 64 registers that let 4 blocks share an SM: left alone it takes 68, and the apply 6 / 35 us
+// Kite k = 500 / 2000, 145 MB / 1.2 GB of table: 90 / 580 us with FP64 multiply-adds, 43 / 229 us so (3.4 / 5.2
+// TB/s); without the next entries on their way 53 / 281; two or five at a time 49 / 246, 43 / 227.  The kernel is
+// held to the 64 registers that let 4 blocks share an SM: left alone it took 68, and the apply 6 / 35 us
 // longer.  CH = 2 keeps blocks of 5 cones, which amortises the conversion; without the
 // look-ahead 5 took 67 / 350 us, 1 took 65 / 272.
-constexpr int kLeafFxAhead = 3, kLeafFxChunk = 256;
+// BIG, a box of more than kFxSumMost sources: a thread's sums of a chunk go to parts in shared memory that
+// add up without loss.
+constexpr int kLeafFxAhead = 3;
 template <int CH>
-__global__ void __launch_bounds__(256, CH == 2 ? 4 : 0) k_leaf_fx(const LeafItem* __restrict__ items, int split, int cone_base,
-                                                 const int4* __restrict__ L, const int* __restrict__ lexp,
-                                                 const double2* __restrict__ rho, int P, int Ps, int4* __restrict__ coef,
-                                                 int* __restrict__ cexp) {
-    __shared__ int4 sr[kLeafFxChunk];
-    __shared__ FxSum part[CH > 1 ? 256 : 1][2];
-    __shared__ int stop[256], smax;
-    const LeafItem I = items[blockIdx.x / split];
+struct LeafFx {
+    static constexpr int chunk = CH > 1 ? 256 : 128;   // sources staged at a time, at most kFxSumMost a thread
+    int4 sr[chunk];
+    FxSum part[256][2];
+    int stop[256], smax;
+};
+template <int CH, bool BIG>
+__device__ __forceinline__ void leaf_fx(LeafFx<CH>& S, const LeafItem& I, int split, int cone_base, const int4* __restrict__ L,
+                                        const int* __restrict__ lexp, const double2* __restrict__ rho, int P, int Ps,
+                                        int4* __restrict__ coef, int* __restrict__ cexp) {
+    constexpr int CHUNK = LeafFx<CH>::chunk;
+    static_assert(CHUNK <= CH * kFxSumMost, "a thread's share of a chunk fits its sums");
     const int per_cone = P * CH, cpb = blockDim.x / per_cone, tid = threadIdx.x;
     const int local = tid / per_cone, r = tid - local * per_cone;
     const int ch = CH > 1 ? r / P : 0, m = r - ch * P;
     const int q = (blockIdx.x % split) * cpb + local;         // cone of the item
     const bool active = q < I.cones;
-    const int n = I.n, c = I.cone + q;
+    const int n = I.n, c = I.cone + q, K = BIG ? fx_sum_wide(n) : 0;
     const int4* Lc = L + I.off + (long long)q * n * P + m;
     const double2* rh = rho + I.first;
     int4 ahead[kLeafFxAhead];
@@ -123,14 +129,16 @@ __global__ void __launch_bounds__(256, CH == 2 ? 4 : 0) k_leaf_fx(const LeafItem
         for (int u = 0; u < kLeafFxAhead; ++u) if (ch + u * CH < n) ahead[u] = __ldcs(&Lc[(long long)(ch + u * CH) * P]);
         El = lexp[(long long)c * P + m];
     }
-    stop[tid] = kFxMinExp;
-    if (tid == 0) smax = 0;
+    S.stop[tid] = kFxMinExp;
+    if (BIG) S.part[tid][0] = S.part[tid][1] = FxSum{0, 0};
+    if (tid == 0) S.smax = 0;
     __syncthreads();
     int mx = 0;
     for (int i = tid; i < n; i += blockDim.x) { const double2 v = rh[i]; mx = max(mx, fx_absmax_hi(v.x, v.y)); }
-    if (mx) atomicMax(&smax, mx);
+    if (mx) atomicMax(&S.smax, mx);
     __syncthreads();
-    const int Er = fx_expo(smax), T = fx_rho_top(n);
+    const int Er = fx_expo(S.smax);
+    constexpr int T = kFxSumTop;
     FxSum rr{0, 0}, ii{0, 0}, im{0, 0};
     auto add = [&](int4 l, int4 d) {
         fx_sum_mac(rr, l.x, l.y, d.x, d.y);
@@ -138,12 +146,12 @@ __global__ void __launch_bounds__(256, CH == 2 ? 4 : 0) k_leaf_fx(const LeafItem
         fx_sum_mac(im, l.x, l.y, d.z, d.w);
         fx_sum_mac(im, l.z, l.w, d.x, d.y);
     };
-    for (int c0 = 0; c0 < n; c0 += kLeafFxChunk) {
-        const int c1 = min(n, c0 + kLeafFxChunk);
+    for (int c0 = 0; c0 < (BIG ? n : 1); c0 += CHUNK) {
+        const int c1 = BIG ? min(n, c0 + CHUNK) : n;
         if (c0) __syncthreads();               // the previous chunk has been read
         for (int i = c0 + tid; i < c1; i += blockDim.x) {
             const double2 v = rh[i];
-            sr[i - c0] = Er == kFxBad ? make_int4(0, 0, 0, 0) : fx_pack_sum(fx_from(v.x, Er, T), fx_from(v.y, Er, T));
+            S.sr[i - c0] = Er == kFxBad ? make_int4(0, 0, 0, 0) : fx_pack_sum(fx_from(v.x, Er, T), fx_from(v.y, Er, T));
         }
         __syncthreads();
         if (active) {
@@ -161,40 +169,56 @@ __global__ void __launch_bounds__(256, CH == 2 ? 4 : 0) k_leaf_fx(const LeafItem
                     if (next + u * CH < c1) ahead[u] = __ldcs(&Lc[(long long)(next + u * CH) * P]);
                 }
 #pragma unroll
-                for (int u = 0; u < kLeafFxAhead; ++u) if (s + u * CH < c1) add(now[u], sr[s + u * CH - c0]);
+                for (int u = 0; u < kLeafFxAhead; ++u) if (s + u * CH < c1) add(now[u], S.sr[s + u * CH - c0]);
                 s = next;
                 terms += kLeafFxAhead;
                 if (terms + kLeafFxAhead > kFxSumFold) { fx_sum_fold(rr); fx_sum_fold(ii); fx_sum_fold(im); terms = 0; }
             }
             fx_sum_fold(rr); fx_sum_fold(ii); fx_sum_fold(im);
+            if (BIG) {
+                fx_sum_part(S.part[tid][0], FxSum{rr.h - ii.h, rr.m - ii.m}, K);
+                fx_sum_part(S.part[tid][1], im, K);
+                rr = ii = im = FxSum{0, 0};
+            }
         }
     }
     FxSum re{rr.h - ii.h, rr.m - ii.m};
+    if (BIG) { re = S.part[tid][0]; im = S.part[tid][1]; }
     if constexpr (CH > 1) {
-        part[tid][0] = re; part[tid][1] = im;
+        if (!BIG) { S.part[tid][0] = re; S.part[tid][1] = im; }
         __syncthreads();
     }
     long long yr = 0, yi = 0;
     int er = 0, ei = 0;
     if (active && ch == 0) {
         for (int k = 1; k < CH; ++k) {
-            const FxSum a = part[tid + k * P][0], b = part[tid + k * P][1];
+            const FxSum a = S.part[tid + k * P][0], b = S.part[tid + k * P][1];
             re.h += a.h; re.m += a.m; im.h += b.h; im.m += b.m;
         }
-        fx_sum_fold(re); fx_sum_fold(im);
+        fx_sum_fold(re, K); fx_sum_fold(im, K);
         const bool bad = Er == kFxBad || El == kFxBad;
         const int E0 = bad ? 0 : El + Er - kFxSumTop - T;
-        yr = fx_sum_value(re, E0, er);
-        yi = fx_sum_value(im, E0, ei);
-        atomicMax(&stop[local], bad ? kFxBad : max(fx_top_of(yr, er), fx_top_of(yi, ei)));
+        yr = fx_sum_value(re, E0, er, K);
+        yi = fx_sum_value(im, E0, ei, K);
+        atomicMax(&S.stop[local], bad ? kFxBad : max(fx_top_of(yr, er), fx_top_of(yi, ei)));
     }
     __syncthreads();
     if (active && ch == 0) {
-        const int E = stop[local] > kFxMaxExp ? kFxBad : stop[local], Tc = fx_top(P);
+        const int E = S.stop[local] > kFxMaxExp ? kFxBad : S.stop[local], Tc = fx_top(P);
         const long long xr = E == kFxBad ? 0 : fx_align(yr, er, E, Tc), xi = E == kFxBad ? 0 : fx_align(yi, ei, E, Tc);
         coef[(long long)(cone_base + c) * P + m] = m % Ps ? fx_pack(xr, xi) : fx_pack_raw(xr, xi);
         if (m == 0) cexp[cone_base + c] = E;
     }
+}
+template <int CH>
+__global__ void __launch_bounds__(256, CH > 1 ? 4 : 0) k_leaf_fx(const LeafItem* __restrict__ items, int split, int cone_base,
+                                                 const int4* __restrict__ L, const int* __restrict__ lexp,
+                                                 const double2* __restrict__ rho, int P, int Ps, int4* __restrict__ coef,
+                                                 int* __restrict__ cexp) {
+    __shared__ LeafFx<CH> S;
+    const LeafItem I = items[blockIdx.x / split];
+    if (I.n <= kFxSumMost) leaf_fx<CH, false>(S, I, split, cone_base, L, lexp, rho, P, Ps, coef, cexp);
+    else leaf_fx<CH, true>(S, I, split, cone_base, L, lexp, rho, P, Ps, coef, cexp);
 }
 
 // set-up: a leaf cone's FP64 table in place as 27-bit limbs, an exponent per coefficient; l32 (may be

@@ -24,6 +24,7 @@
 // plus the batched GMRES vector kernels (per-RHS dot products, CGS updates, scaling).
 #include "fixpoint.cuh"
 #include "tcgen05.cuh"
+#include <type_traits>
 
 namespace ifgf {
 
@@ -218,7 +219,7 @@ __global__ void k_rho_bx(const int* __restrict__ leaf_start, const int* __restri
                          int4* __restrict__ out, int* __restrict__ rexp) {
     const int b = blockIdx.x, r = threadIdx.x;
     if (r >= B) return;
-    const int n = leaf_count[b], T = fx_rho_top(n);
+    const int n = leaf_count[b], T = kFxSumTop;
     const long long s0 = leaf_start[b];
     int mx = 0;
     for (int i = 0; i < n; ++i) { const double2 v = rho[(s0 + i) * B + r]; mx = max(mx, fx_absmax_hi(v.x, v.y)); }
@@ -233,15 +234,17 @@ __global__ void k_rho_bx(const int* __restrict__ leaf_start, const int* __restri
 // coefficients a thread: their integer sums (eight registers each) stay in registers.  The table streams
 // through shared memory kLeafBxTile sources at a time (cp.async, double-buffered), read as broadcasts.
 // Bound by the wide multiply-adds (12 an entry); kite k = 500, 64 right-hand sides 4.0 -> 1.2 ms.
+// BIG (launched for trees with a box of more than kFxSumMost sources): such a box's sums of kFxSumMost
+// sources each are added up in FP64, in the place of the coefficients.
 constexpr int kLeafBxTile = 8;
-template <int P, int MS, int NT>
+template <int P, int MS, int NT, bool BIG>
 __global__ void __launch_bounds__(NT * MS) k_leaf_bx(const int* __restrict__ cone_box, int cone_base, const int* __restrict__ leaf_start,
                                                      const int* __restrict__ leaf_count, const long long* __restrict__ leaf_off,
                                                      const int4* __restrict__ L, const int* __restrict__ lexp,
                                                      const int4* __restrict__ rho, const int* __restrict__ rexp, int B, int Ps,
                                                      int4* __restrict__ coef, int* __restrict__ cexp) {
     constexpr int PM = (P + MS - 1) / MS, TS = kLeafBxTile;
-    static_assert(kFxSumFold % TS == 0, "folds between tiles");
+    static_assert(kFxSumFold % TS == 0 && kFxSumMost % kFxSumFold == 0, "folds between tiles, parts of whole folds");
     __shared__ int4 tile[2][TS * P];
     __shared__ int stop[NT];
     const int c = blockIdx.x, lt = threadIdx.x, part = threadIdx.y, tid = part * NT + lt;
@@ -260,6 +263,8 @@ __global__ void __launch_bounds__(NT * MS) k_leaf_bx(const int* __restrict__ con
 #pragma unroll
     for (int m = 0; m < PM; ++m) re[m] = im[m] = FxSum{0, 0};
     const int4* rh = rho + (long long)leaf_start[b] * B + rr;
+    int Er = BIG ? rexp[(long long)b * B + rr] : 0;
+    double2* sums = reinterpret_cast<double2*>(coef + (long long)(cone_base + c) * P * B + r);
     const int nt = (n + TS - 1) / TS;
     int4 dn = n > 0 ? rh[0] : make_int4(0, 0, 0, 0);
     if (nt > 0) load_tile(0);
@@ -286,9 +291,50 @@ __global__ void __launch_bounds__(NT * MS) k_leaf_bx(const int* __restrict__ con
         if ((t + 1) % (kFxSumFold / TS) == 0 || t + 1 == nt)
 #pragma unroll
             for (int m = 0; m < PM; ++m) { fx_sum_fold(re[m]); fx_sum_fold(im[m]); }
+        if (BIG && n > kFxSumMost && ((t + 1) % (kFxSumMost / TS) == 0 || t + 1 == nt)) {
+#pragma unroll
+            for (int m = 0; m < PM; ++m) {
+                const int q = part * PM + m;
+                if (q < P && act) {
+                    const int El = lexp[(long long)c * P + q], E0 = Er == kFxBad || El == kFxBad ? 0 : El + Er - 2 * kFxSumTop;
+                    int ea, eb;
+                    const long long ya = fx_sum_value(re[m], E0, ea), yb = fx_sum_value(im[m], E0, eb);
+                    double2* o = sums + (long long)q * B;
+                    const double2 a = t < kFxSumMost / TS ? make_double2(0.0, 0.0) : *o;
+                    *o = make_double2(a.x + fx_scaled(ya, ea), a.y + fx_scaled(yb, eb));
+                }
+                re[m] = im[m] = FxSum{0, 0};
+            }
+        }
         __syncthreads();                        // the buffer is refilled two tiles later
     }
-    const int Er = rexp[(long long)b * B + rr], T = fx_top(P);
+    const int T = fx_top(P);
+    if (BIG && n > kFxSumMost) {
+        int mx = 0;
+        for (int m = 0; m < PM; ++m) {
+            const int q = part * PM + m;
+            if (q >= P || !act) break;
+            const double2 v = sums[(long long)q * B];
+            mx = max(mx, lexp[(long long)c * P + q] == kFxBad || Er == kFxBad ? 0x7ff00000 : fx_absmax_hi(v.x, v.y));
+        }
+        if (MS > 1) {
+            atomicMax(&stop[lt], mx);
+            __syncthreads();
+            mx = stop[lt];
+        }
+        if (!act) return;
+        const int E = fx_expo(max(mx, 0));
+        for (int m = 0; m < PM; ++m) {
+            const int q = part * PM + m;
+            if (q >= P) break;
+            const double2 v = sums[(long long)q * B];
+            const long long xr = E == kFxBad ? 0 : fx_from(v.x, E, T), xi = E == kFxBad ? 0 : fx_from(v.y, E, T);
+            reinterpret_cast<int4*>(sums)[(long long)q * B] = q % Ps ? fx_pack(xr, xi) : fx_pack_raw(xr, xi);
+        }
+        if (part == 0) cexp[(long long)(cone_base + c) * B + r] = E;
+        return;
+    }
+    if (!BIG) Er = rexp[(long long)b * B + rr];
     int top = kFxMinExp;                        // the sums in place as y = .h, e = .m of y 2^e
 #pragma unroll
     for (int m = 0; m < PM; ++m) {
@@ -296,7 +342,7 @@ __global__ void __launch_bounds__(NT * MS) k_leaf_bx(const int* __restrict__ con
         if (q >= P) continue;
         const int El = lexp[(long long)c * P + q];
         if (Er == kFxBad || El == kFxBad) { top = kFxBad; continue; }
-        const int E0 = El + Er - kFxSumTop - fx_rho_top(n);
+        const int E0 = El + Er - 2 * kFxSumTop;
         int ea, eb;
         const long long ya = fx_sum_value(re[m], E0, ea), yb = fx_sum_value(im[m], E0, eb);
         re[m].h = ya; im[m].h = yb; re[m].m = ea; im[m].m = eb;
@@ -861,30 +907,33 @@ __global__ void __launch_bounds__(256) k_near_bx(int N, const int* __restrict__ 
         const int bb = nbr_box[q], c = leaf_count[bb];
         const int4* rh = rho + (long long)leaf_start[bb] * B + r;
         const int Er = rexp[(long long)bb * B + r];
-        FxSum rr{0, 0}, ii{0, 0}, im{0, 0};
-        for (int f0 = 0; f0 < c; f0 += kFxSumFold) {
-            const int f1 = min(c, f0 + kFxSumFold);
+        for (int p0 = 0; p0 < c; p0 += kFxSumMost) {            // the sum of the box, or of kFxSumMost of its sources
+            const int p1 = min(c, p0 + kFxSumMost);
+            FxSum rr{0, 0}, ii{0, 0}, im{0, 0};
+            for (int f0 = p0; f0 < p1; f0 += kFxSumFold) {
+                const int f1 = min(p1, f0 + kFxSumFold);
 #pragma unroll 4
-            for (int s = f0; s < f1; ++s) {
-                const int4 a = row[s], d = rh[(long long)s * B];
-                fx_sum_mac(rr, a.x, a.y, d.x, d.y);
-                fx_sum_mac(ii, a.z, a.w, d.z, d.w);
-                fx_sum_mac(im, a.x, a.y, d.z, d.w);
-                fx_sum_mac(im, a.z, a.w, d.x, d.y);
+                for (int s = f0; s < f1; ++s) {
+                    const int4 a = row[s], d = rh[(long long)s * B];
+                    fx_sum_mac(rr, a.x, a.y, d.x, d.y);
+                    fx_sum_mac(ii, a.z, a.w, d.z, d.w);
+                    fx_sum_mac(im, a.x, a.y, d.z, d.w);
+                    fx_sum_mac(im, a.z, a.w, d.x, d.y);
+                }
+                fx_sum_fold(rr); fx_sum_fold(ii); fx_sum_fold(im);
             }
-            fx_sum_fold(rr); fx_sum_fold(ii); fx_sum_fold(im);
+            rr.h -= ii.h; rr.m -= ii.m;
+            fx_sum_fold(rr);
+            if (En == kFxBad || Er == kFxBad) {
+                acc.x = acc.y = __hiloint2double(0x7ff80000, 0);
+            } else {
+                const int E0 = En + Er - 2 * kFxSumTop;
+                int er, ei;
+                const long long yr = fx_sum_value(rr, E0, er), yi = fx_sum_value(im, E0, ei);
+                acc.x += fx_scaled(yr, er); acc.y += fx_scaled(yi, ei);
+            }
         }
         row += c;
-        rr.h -= ii.h; rr.m -= ii.m;
-        fx_sum_fold(rr);
-        if (En == kFxBad || Er == kFxBad) {
-            acc.x = acc.y = __hiloint2double(0x7ff80000, 0);
-        } else {
-            const int E0 = En + Er - kFxSumTop - fx_rho_top(c);
-            int er, ei;
-            const long long yr = fx_sum_value(rr, E0, er), yi = fx_sum_value(im, E0, ei);
-            acc.x += fx_scaled(yr, er); acc.y += fx_scaled(yi, ei);
-        }
     }
     double2* yo = yt + sorting[i] * B + r;
     double2 v = *yo;
@@ -1088,16 +1137,19 @@ void launch_rho_bx(const int* leaf_start, const int* leaf_count, int nleaf, cons
 }
 void launch_leaf_bx(const int* cone_box, int ncones, int cone_base, const int* leaf_start, const int* leaf_count,
                     const long long* leaf_off, const int4* L, const int* lexp, const int4* rho, const int* rexp, int Ps, int Pang, int B,
-                    int4* coef, int* cexp, cudaStream_t s) {
+                    int most, int4* coef, int* cexp, cudaStream_t s) {
     if (ncones <= 0 || B <= 0) return;
     IFGF_DISPATCH_P(Ps, Pang, {
         constexpr int P = PS * PA, MS = (P + 12) / 13;   // at most 13 coefficients (104 registers of sums) a thread
-        if (B <= 32)
-            k_leaf_bx<P, MS, 32><<<dim3(ncones, 1), dim3(32, MS), 0, s>>>(cone_box, cone_base, leaf_start, leaf_count, leaf_off, L, lexp,
-                                                                         rho, rexp, B, Ps, coef, cexp);
-        else
-            k_leaf_bx<P, MS, 64><<<dim3(ncones, nblk_b(B, 64)), dim3(64, MS), 0, s>>>(cone_box, cone_base, leaf_start, leaf_count, leaf_off,
-                                                                                     L, lexp, rho, rexp, B, Ps, coef, cexp);
+        auto go = [&](auto nt, auto big) {
+            constexpr int NT = decltype(nt)::value;
+            k_leaf_bx<P, MS, NT, decltype(big)::value><<<dim3(ncones, nblk_b(B, NT)), dim3(NT, MS), 0, s>>>(
+                cone_box, cone_base, leaf_start, leaf_count, leaf_off, L, lexp, rho, rexp, B, Ps, coef, cexp);
+        };
+        using N32 = std::integral_constant<int, 32>;
+        using N64 = std::integral_constant<int, 64>;
+        if (most <= kFxSumMost) B <= 32 ? go(N32{}, std::false_type{}) : go(N64{}, std::false_type{});
+        else B <= 32 ? go(N32{}, std::true_type{}) : go(N64{}, std::true_type{});
     });
 }
 void launch_prop_b(int pbegin, int pend, const long long* pp_ptr, const int* pp_nchild, const PropB<float>* pb, int Ps, int Pang,

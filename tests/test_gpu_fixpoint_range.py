@@ -31,3 +31,38 @@ def test_gpu_densities_near_the_ends_of_the_range(lib, Ps, Pang):
         assert np.linalg.norm(z - y) <= 1e-15 * np.linalg.norm(y), q
         v = fm.propagate_acc(tx, ty, X[:, 0] * 2.0 ** float(q)) * 2.0 ** float(-q)
         assert np.linalg.norm(v - u) <= 1e-15 * np.linalg.norm(u), q
+
+
+def _weights(npatch, Np=16):
+    """the kite's quadrature weights: Fejer's first rule on equal parts of the parameter, times the arc length"""
+    th = np.pi * (2 * np.arange(Np) + 1) / (2 * Np)
+    w = 2 / Np * (1 - 2 * sum(np.cos(2 * m * th) / (4 * m * m - 1) for m in range(1, Np // 2 + 1)))
+    t = (np.pi / npatch) * (2 * np.arange(npatch)[:, None] + 1 + np.cos(th)[None, :])
+    return ((np.pi / npatch) * w[None, :] * np.hypot(-np.sin(t) - 1.3 * np.sin(2 * t), 1.5 * np.cos(t))).ravel()
+
+
+@pytest.mark.parametrize("npatch,nlevels", [(1024, 3), (512, 4)])
+def test_gpu_small_densities_beside_a_large_one_in_a_large_box(lib, npatch, nlevels):
+    """Leaf boxes of several hundred to a thousand points: one intensity of 1 and, around it, others of 5 units
+    of 2^-53.  Densities keep 54 bits in a box of any size, so the small ones are held exactly; coefficients
+    and results are rounded at 2^-53 of the large one's field, some 2e-2 of the small ones' few hundred."""
+    fm = _map(lib, k=20.0, npatch=npatch, nlevels=nlevels)
+    n = fm.total_num_unknowns_
+    w = _weights(npatch)
+    j = n // 5
+    d = np.hypot(fm.xs_ - fm.xs_[j], fm.ys_ - fm.ys_[j])
+    spike, small = np.zeros(n, complex), np.zeros(n, complex)
+    spike[j] = 1.0
+    small[(d < 0.3) & (d > 0)] = 5 * 2.0 ** -53
+    far = d > 1.6                                       # beyond the neighbour boxes
+
+    def check(a, b, c):
+        assert np.linalg.norm((c - a - b)[far]) < 0.1 * np.linalg.norm(b[far])
+
+    check(fm.ifgf_far(spike), fm.ifgf_far(small), fm.ifgf_far(spike + small))
+    for nrhs in (13, 40):
+        X = np.zeros((n, nrhs), complex)
+        X[:, 0], X[:, 5], X[:, nrhs - 1] = spike / w, small / w, (spike + small) / w
+        Y = fm.apply_batch(X)
+        check(Y[:, 0], Y[:, 5], Y[:, nrhs - 1])
+        assert not Y[:, 1].any()
