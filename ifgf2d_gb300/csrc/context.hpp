@@ -191,7 +191,10 @@ struct ifgf2d_ctx {
     // launch shapes per precision (0 FP64, 1 complex64): leaf-kernel source chunks, and cones
     // per block of each level's propagation (0 = the most that fit 256 threads); set by
     // ifgf2d_autotune / ifgf2d_set_tuning
-    int tune_leaf[2] = {2, 5};      // complex64 also 0: the table streamed by TMA bulk copies (k_leaf_tma)
+    // (FP64: by the set-up, leaf_fx_chunks, until then; complex64 also 0: the table streamed by TMA bulk
+    // copies, k_leaf_tma)
+    int tune_leaf[2] = {2, 5};
+    bool leaf_tuned = false;
     int tune_prop[2][kTuneLevels] = {};
     // kernel choices (bit mask): batched complex64 kernels on the tcgen05 tensor cores in 3xTF32
     // (else FP32 FMA), the batched grouped interpolation, the single-vector interpolation by box
@@ -319,6 +322,12 @@ inline std::vector<LeafItem> leaf_item_list(const std::vector<int>& cone_box, co
     }
     return items;
 }
+// threads that share a coefficient's sum in the FP64 leaf sums: 2, but 5 for trees of so few leaf cones (32 an
+// SM, 1.6 times what 4 blocks of 5 cones an SM hold) that the length of a thread's walk is what counts.  us with 2 and
+// 5 threads: 202 cones of boxes of 80, 330 and 660 sources 20 / 14, 104 / 51 and 205 / 96; 1040 to 4456 cones of 140 to 570
+// sources 65 / 35, 135 / 72, 260 / 212, 180 / 152; 2310 and 4866 of 33 sources 22 / 20 and 30 / 30; 10924 and 45614 (kite
+// k = 500 and 2000) 43 / 57 and 229 / 307.
+inline int leaf_fx_chunks(int cones) { return cones <= 32 * 152 ? 5 : 2; }
 // What a group of obstacles (group.cu) changes in the device part of the IFGF set-up: (k, eta)
 // per leaf box and per leaf cone (device arrays), and the leaf-cone nodes and the propagation
 // plan, both built member by member.

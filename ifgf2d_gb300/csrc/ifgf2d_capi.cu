@@ -510,6 +510,7 @@ static int setup_cones(ifgf2d_ctx* ctx, double k, int nlevels, const SetupExtra*
     CK(ctx->leaf_cone_box.upload(LD.cone_box)); CK(ctx->leaf_off.upload(loff));
     CK(ctx->leaf_cones.upload(leaf_cone_list(LD.cone_box, T.leaf_start, T.leaf_count, loff)));
     CK(ctx->leaf_items.upload(leaf_item_list(LD.cone_box, T.leaf_start, T.leaf_count, loff, P)));
+    if (!ctx->leaf_tuned) ctx->tune_leaf[0] = leaf_fx_chunks(ncl);
     ctx->leaf_most = T.leaf_count.empty() ? 0 : *std::max_element(T.leaf_count.begin(), T.leaf_count.end());
     CK(ctx->leafL.alloc(loff[ncl]));
     CK(ctx->leaf_nodes_d.alloc((size_t)ncl * P));
@@ -819,6 +820,7 @@ extern "C" int ifgf2d_get_tuning(const ifgf2d_ctx* ctx, int* choices) {
 }
 extern "C" int ifgf2d_set_tuning(ifgf2d_ctx* ctx, const int* c) {
     if (!ctx || !c) return IFGF2D_ERR_ARG;
+    if (c[0] != ctx->tune_leaf[0]) ctx->leaf_tuned = true;
     ctx->tune_leaf[0] = c[0]; ctx->tune_leaf[1] = c[1];
     for (int p = 0; p < 2; ++p)
         for (int l = 0; l < kTuneLevels; ++l) ctx->tune_prop[p][l] = c[2 + p * kTuneLevels + l];
@@ -850,6 +852,7 @@ static int tune_precision(ifgf2d_ctx* ctx, int reps, CoefT<R>* coef) {
         if (ms < best) { best = ms; bestc = ch; }
     }
     ctx->tune_leaf[pr] = bestc;
+    if (pr == 0) ctx->leaf_tuned = true;
     for (int l = Dl; l >= 3 && l < kTuneLevels && sizeof(R) == 4; --l) {   // the FP64 kernel has one shape
         best = 1e30f; int bestp = 0;
         for (int cpb : {2, 4, 0, kPropStaged}) {

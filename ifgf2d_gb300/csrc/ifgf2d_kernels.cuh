@@ -114,7 +114,7 @@ void launch_leaf_apply_t(const int4* cones, int ncones, int cone_base, const flo
 // the FP64 form in fixed point (fixpoint.cuh): the table and its exponents [cone][coefficient] from
 // launch_leaf_fix (in place of the FP64 table; l32, when not null, receives the complex64 copy)
 void launch_leaf_fx(const LeafItem* items, int nitems, int cone_base, const int4* L, const int* lexp, const double2* rho, int P, int Ps,
-                    int4* coef, int* cexp, cudaStream_t s, int chunks = 2);
+                    int4* coef, int* cexp, cudaStream_t s, int chunks);
 void launch_leaf_fix(const int* cone_box, int ncones, const int* leaf_count, const long long* leaf_off, int P, int4* L, int* lexp,
                      float2* l32, cudaStream_t s);
 // complex64 leaf cones with the table streamed through shared memory by TMA bulk copies

@@ -18,6 +18,7 @@ struct EvalWork {
     DBuf<int> leaf_cone_box;
     DBuf<long long> leaf_off;
     DBuf<LeafItem> leaf_items;
+    int leaf_chunks = 2;
     DBuf<LeafNode> nodes;
     DBuf<int4> leafL;
     DBuf<int> lexp;
@@ -117,6 +118,7 @@ extern "C" int ifgf2d_eval_offsurface_setup(ifgf2d_ctx* ctx, long long m, const 
         CK(build_leaf_nodes(E, W.nodes.p, s));
         CK(W.leaf_cone_box.upload(LD.cone_box)); CK(W.leaf_off.upload(loff));
         CK(W.leaf_items.upload(leaf_item_list(LD.cone_box, E.leaf_start, E.leaf_count, loff, P)));
+        W.leaf_chunks = leaf_fx_chunks(ncl);
         CK(W.leafL.alloc(loff[ncl]));
         launch_leaf_setup(W.leaf_cone_box.p, ncl, ctx->leaf_start.p, ctx->leaf_count.p, W.leaf_off.p, W.nodes.p, ctx->xs_s.p,
                           ctx->ys_s.p, ctx->nxs_s.p, ctx->nys_s.p, ctx->T.Ps, ctx->T.Pang, ctx->k, ctx->form, ctx->eta, ctx->Gsep.p,
@@ -170,7 +172,7 @@ extern "C" int ifgf2d_eval_offsurface(ifgf2d_ctx* ctx, const double* density, do
     launch_intensities(ctx->vin.p, ctx->wq.p, ctx->sorting.p, N, ctx->rho.p, s);
     const TreeLevel& LD = E.L[D];
     launch_leaf_fx(W.leaf_items.p, (int)W.leaf_items.n, LD.cone_base, W.leafL.p, W.lexp.p, ctx->rho.p, P, E.Ps, W.coef.p,
-                   W.cexp.p, s);
+                   W.cexp.p, s, W.leaf_chunks);
     for (int l = D; l >= 3; --l) {
         const TreeLevel& Lp = E.L[l - 1];
         launch_propagate_fx(Lp.cone_base, Lp.cone_base + (int)Lp.cone_nonrel.size(), W.pp.view(), W.stage.level(l), E.Ps, E.Pang,

@@ -294,7 +294,9 @@ int ifgf2d_apply_timed(ifgf2d_ctx* ctx, const void* d_x, void* d_y, int mode, do
  * mask of kernel choices: the batched complex64 kernels that run in 3xTF32 on the tcgen05
  * tensor cores (IFGF2D_BATCH_TC_*; FP32 FMA otherwise), the other batched choices and the
  * single-vector interpolation by leaf box (IFGF2D_SINGLE_INTERP_BY_BOX_*); the default is
- * IFGF2D_BATCH_TC_LEAF | IFGF2D_BATCH_GROUPED_INTERP | IFGF2D_SINGLE_INTERP_BY_BOX_C64.
+ * IFGF2D_BATCH_TC_LEAF | IFGF2D_BATCH_GROUPED_INTERP | IFGF2D_SINGLE_INTERP_BY_BOX_C64,
+ * and for the FP64 leaf sums a number of chunks that every set-up derives from its leaf cones until the
+ * autotuner or set_tuning changes it.
  * get / set read and restore it (e.g. from an on-disk cache); applies use the context's
  * current table. */
 #define IFGF2D_BATCH_TC_LEAF 1          /* leaf-cone sums, 3xTF32 (two TF32 terms per operand) */

@@ -66,3 +66,21 @@ def test_gpu_small_densities_beside_a_large_one_in_a_large_box(lib, npatch, nlev
         Y = fm.apply_batch(X)
         check(Y[:, 0], Y[:, 5], Y[:, nrhs - 1])
         assert not Y[:, 1].any()
+
+
+@pytest.mark.parametrize("k,npatch,nlevels,chunks", [(20.0, 256, 3, 5), (500.0, 512, 0, 2)])
+def test_gpu_leaf_shapes(lib, k, npatch, nlevels, chunks):
+    """The set-up takes five threads a coefficient for few leaf cones and two for many; integer sums are the
+    same in every shape.  A shape that was set stays over the next set-up."""
+    fm = _map(lib, k=k, npatch=npatch, nlevels=nlevels)
+    g = np.random.default_rng(npatch)
+    x = g.standard_normal(fm.total_num_unknowns_) + 1j * g.standard_normal(fm.total_num_unknowns_)
+    y = fm.compute_Ax_acc(x)
+    t = fm.get_tuning()
+    assert t[0] == chunks
+    for c in (1, 2, 5, 10):
+        t[0] = c
+        fm.set_tuning(t)
+        fm.precomps_and_setup(k, nlevels)
+        assert fm.get_tuning()[0] == c
+        assert np.array_equal(fm.compute_Ax_acc(x), y)
