@@ -124,8 +124,9 @@ __device__ __forceinline__ void hankel01(double x, double2& h0, double2& h1) {
 }
 
 // Single-layer kernel (i/4) H0(k r), 0 for r < 1e-14 (ForwardMap/GreenFunctions.hpp:87-108)
-__device__ __forceinline__ double2 green_sl(double dx, double dy, double k) {
-    const double r = sqrt(dx * dx + dy * dy);
+// at |d|^2 = d2
+__device__ __forceinline__ double2 green_sl(double d2, double k) {
+    const double r = sqrt(d2);
     if (r < 1e-14) return make_double2(0.0, 0.0);
     const double2 h = hankel1<0>(k * r);
     return make_double2(-0.25 * h.y, 0.25 * h.x);
@@ -133,18 +134,20 @@ __device__ __forceinline__ double2 green_sl(double dx, double dy, double k) {
 
 // Combined-field kernel without the jump term, target minus source d = x - y, unit normal n
 // at the source y:  dPhi/dn_y - i eta Phi = (ik/4) H1(kr) (d.n)/r + (eta/4) H0(kr); 0 for r < 1e-14.
-__device__ __forceinline__ double2 green_cfie(double dx, double dy, double nx, double ny, double k, double eta) {
-    const double r = sqrt(dx * dx + dy * dy);
+// d2 = |d|^2, dn = d.n, k4 = k/4, eta4 = eta/4
+__device__ __forceinline__ double2 green_cfie(double d2, double dn, double k, double k4, double eta4) {
+    const double r = sqrt(d2);
     if (r < 1e-14) return make_double2(0.0, 0.0);
     double2 h0, h1;
     hankel01(k * r, h0, h1);
-    const double c = 0.25 * k * (dx * nx + dy * ny) / r;   // (ik/4)(d.n)/r = i c
-    return make_double2(-c * h1.y + 0.25 * eta * h0.x, c * h1.x + 0.25 * eta * h0.y);
+    const double c = k4 * dn / r;              // (ik/4)(d.n)/r = i c
+    return make_double2(-c * h1.y + eta4 * h0.x, c * h1.x + eta4 * h0.y);
 }
 
 // kernel of the chosen formulation (eta unused for the single layer)
 __device__ __forceinline__ double2 green_form(int form, double dx, double dy, double nx, double ny, double k, double eta) {
-    return form == 2 ? green_cfie(dx, dy, nx, ny, k, eta) : green_sl(dx, dy, k);
+    const double d2 = dx * dx + dy * dy;
+    return form == 2 ? green_cfie(d2, dx * nx + dy * ny, k, 0.25 * k, 0.25 * eta) : green_sl(d2, k);
 }
 
 // e^{ikr}/sqrt(r) (GreenFunctions.hpp:125-131)
