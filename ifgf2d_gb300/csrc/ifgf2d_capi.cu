@@ -1060,7 +1060,7 @@ static int gmres_core(ifgf2d_ctx* ctx, const double2* b, double2* x, int mode, d
         // the complex64 inner solves of the refinement take one Gram-Schmidt pass, as the batched
         // ones do: each correction is checked by the FP64 residual, and a short one costs one more
         // refinement pass, not a wrong answer
-        launch_arnoldi_step(G.V.p, N, m, G.jdev.p, G.w.p, G.vin.p, G.H.p, G.nrm2.p, G.part.p, s,
+        launch_arnoldi_step(G.V.p, N, m, G.jdev.p, G.w.p, G.vin.p, G.h.p, G.H.p, G.nrm2.p, G.part.p, s,
                             mode == IFGF2D_APPLY_IFGF_MIXED ? 1 : 2, L, cond);
         cudaGraph_t body = nullptr;
         const cudaError_t ec = cudaStreamEndCapture(s, &body);

@@ -341,9 +341,8 @@ __global__ void k_copy_col(const double2* __restrict__ V, long long n, const int
     if (i == 0 && nrm2) *nrm2 = 0.0;
 }
 // h[c] = V[:, c]^H w for c <= *jp in two deterministic stages: blocks (row chunk, column)
-// write partial sums, then every block of k_cgs_update_dyn adds a column's chunks in order.  The grid spans
-// every column and row chunk, so even the first iterations keep all SMs busy.
-constexpr int kDotChunk = 2048;
+// write partial sums, then every block of k_cgs_update_dyn, or k_multidot_fin, adds a column's chunks in order.
+// The grid spans every column and row chunk, so even the first iterations keep all SMs busy.
 __global__ void __launch_bounds__(256) k_multidot_part(const double2* __restrict__ V, long long ldv, const int* __restrict__ jp,
                                                        const double2* __restrict__ w, long long n, double2* __restrict__ part) {
     const int col = blockIdx.y;
@@ -367,6 +366,14 @@ __global__ void __launch_bounds__(256) k_multidot_part(const double2* __restrict
         for (int q = 0; q < (int)(blockDim.x >> 5); ++q) { a += sr[q]; b += si[q]; }
         part[(long long)col * gridDim.x + chunk] = make_double2(a, b);
     }
+}
+__global__ void k_multidot_fin(const double2* __restrict__ part, int nchunk, const int* __restrict__ jp, int ncol,
+                               double2* __restrict__ h) {
+    const int col = blockIdx.x * blockDim.x + threadIdx.x;
+    if (col >= ncol || col > *jp) return;
+    double a = 0.0, b = 0.0;
+    for (int q = 0; q < nchunk; ++q) { const double2 v = part[(long long)col * nchunk + q]; a += v.x; b += v.y; }
+    h[col] = make_double2(a, b);
 }
 // Z[:, *jp] = z (flexible GMRES keeps the preconditioned vectors)
 __global__ void k_store_col(const double2* __restrict__ z, long long n, const int* __restrict__ jp, double2* __restrict__ Z) {
@@ -396,8 +403,8 @@ __global__ void k_multidot_dyn(const double2* __restrict__ V, long long ldv, con
     }
 }
 // w -= V[:, 0..j] h: 64 rows per block, four threads per row split the columns (j = part mod 4).  h, the
-// columns' partial dots added up, is summed by every block for itself, 256 columns at a time (a launch
-// of its own for it cost 2.3 us an orthogonalisation pass); block 0 also writes (add = 0) or adds (add = 1)
+// columns' nchunk partial dots added up, is summed by every block for itself, 256 columns at a time (few
+// chunks: a launch of its own cost 2.3 us an orthogonalisation pass); block 0 also writes (add = 0) or adds (add = 1)
 // it into the Hessenberg column j.
 __global__ void __launch_bounds__(256) k_cgs_update_dyn(const double2* __restrict__ V, long long ldv, const int* __restrict__ jp,
                                                         const double2* __restrict__ dots, int nchunk, long long n, double2* __restrict__ w,
@@ -537,15 +544,17 @@ void launch_scale(const double2* w, double2 a, long long n, double2* out, cudaSt
 void launch_sub(const double2* a, const double2* b, long long n, double2* out, cudaStream_t s) {
     k_sub<<<nblk(n, 256), 256, 0, s>>>(a, b, n, out);
 }
-int arnoldi_part_size(long long n, int m) { return (int)(((n + kDotChunk - 1) / kDotChunk) * (m + 1)); }
-void launch_arnoldi_step(double2* V, long long n, int m, int* jp, double2* w, double2* vin, double2* H, double* nrm2,
+int arnoldi_part_size(long long n, int m) { return (int)(dot_chunks(n) * (m + 1)); }
+void launch_arnoldi_step(double2* V, long long n, int m, int* jp, double2* w, double2* vin, double2* h, double2* H, double* nrm2,
                          double2* part, cudaStream_t s, int passes, LsqDev lsq, cudaGraphConditionalHandle cond) {
     // w holds A v_j on entry, vin v_j
     const int ldh = m + 1;
     for (int pass = 0; pass < passes; ++pass) {   // classical Gram-Schmidt; the last pass sums ||w||^2
-        const int nchunk = (int)((n + kDotChunk - 1) / kDotChunk);
+        const int nchunk = (int)dot_chunks(n), terms = (int)dot_block_terms(n);
         k_multidot_part<<<dim3(nchunk, m + 1), 256, 0, s>>>(V, n, jp, w, n, part);
-        k_cgs_update_dyn<<<nblk(n, 64), 256, 0, s>>>(V, n, jp, part, nchunk, n, w, H, ldh, pass, pass == passes - 1 ? nrm2 : nullptr);
+        if (terms < nchunk) k_multidot_fin<<<nblk(m + 1, 128), 128, 0, s>>>(part, nchunk, jp, m + 1, h);
+        k_cgs_update_dyn<<<nblk(n, 64), 256, 0, s>>>(V, n, jp, terms < nchunk ? h : part, terms, n, w, H, ldh, pass,
+                                                     pass == passes - 1 ? nrm2 : nullptr);
     }
     k_scale_next<<<nblk(n, 256), 256, 0, s>>>(w, nrm2, n, V, jp, H, ldh, vin);
     launch_lsq_givens(H, ldh, jp, lsq, cond, true, nrm2, s);

@@ -342,9 +342,18 @@ void launch_seg_axpy(const SegDesc& S, const double2* V, int ncols, const double
 // one Arnoldi step after w = A v_j, with j read from *jp (for a captured iteration graph):
 // classical Gram-Schmidt against V[:, 0..j], `passes` times (2: CGS2), into the Hessenberg
 // column j, ||w||^2 into *nrm2 (zeroed by launch_copy_col and the Givens step), h_{j+1,j} and
-// V[:, j+1] = w / h_{j+1,j}, also into vin; then the Givens step of launch_lsq_givens, which advances j
-void launch_arnoldi_step(double2* V, long long n, int m, int* jp, double2* w, double2* vin, double2* H, double* nrm2,
+// V[:, j+1] = w / h_{j+1,j}, also into vin; then the Givens step of launch_lsq_givens, which advances j.
+// h: m + 1 entries of scratch
+void launch_arnoldi_step(double2* V, long long n, int m, int* jp, double2* w, double2* vin, double2* h, double2* H, double* nrm2,
                          double2* part, cudaStream_t s, int passes, LsqDev lsq, cudaGraphConditionalHandle cond);
+// Its dot products are sums over chunks of kDotChunk rows.  Every block of the update (64 rows) adds up to
+// kDotBlockChunks chunks of each column for itself; a longer vector's are added up once by a kernel of their own,
+// as that work of the blocks together grows with the square of the length.  An iteration's time beyond the
+// apply, us over 20 / 80 columns, by the blocks and by a kernel of its own: N = 81920 86 / 158 and 80 / 144,
+// 131072 130 / 262 and 112 / 219, 524288 873 / 1706 and 396 / 820; at 65536 63 / 117 by the blocks.
+constexpr int kDotChunk = 2048, kDotBlockChunks = 32;
+constexpr long long dot_chunks(long long n) { return (n + kDotChunk - 1) / kDotChunk; }
+constexpr long long dot_block_terms(long long n) { return dot_chunks(n) <= kDotBlockChunks ? dot_chunks(n) : 1; }
 // size (double2 entries) of the partial-sum buffer launch_arnoldi_step needs
 int arnoldi_part_size(long long n, int m);
 // Z[:, *jp] = z

@@ -27,3 +27,13 @@ using namespace ifgf::gx;
 using Element = std::remove_all_extents_t<decltype(gx_table)>;
 static_assert(alignof(Element) >= 16 && sizeof(Element) % 16 == 0, "16-byte loads");
 """)
+
+
+def test_orthogonalisation_work_grows_with_the_length(tmp_path):
+    """Each block of the Gram-Schmidt update (64 rows) adds a bounded number of partial dots of a column."""
+    _compiles(tmp_path, """
+#include "ifgf2d_kernels.cuh"
+using namespace ifgf;
+static_assert(dot_block_terms(200) == 1 && dot_block_terms(65536) == 32, "few chunks: by the blocks");
+static_assert(dot_block_terms(65537) == 1 && dot_block_terms(1 << 19) == 1 && dot_block_terms(1ll << 32) == 1, "more: added up once");
+""")
