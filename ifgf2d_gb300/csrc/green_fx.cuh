@@ -13,8 +13,9 @@
 //      holds them to 2^-61; the terms from t^4 on fit FP32, the t^3 one 32 bits.
 //   4. i H1 and H0 share the phase: g = A e^{i(x - pi/4)} (c (P1 + i Q1) + eta/4 (P0 + i Q0)), the
 //      bracket with one binary exponent, the larger of the two coefficients'.
-// The errors are a few 2^-57 of |g| beside those of the FP64 operations that are left (|d|^2, d . n, the
-// products by A), against x times the rounding of k r and more before.  Arguments x <= 1, x >= 2^30, r < 1e-14 and non-finite values take green_form.
+// The errors are a few 2^-57 of |g| and x 2^-58 in the phase (r is an integer in units of 2^-58 of a power of
+// two: 1e-15 at x = 300, 5e-13 at 10^5) beside those of the FP64 operations that are left (|d|^2, d . n, the
+// products by A), against x 2^-53, the rounding of k r, and more before.  Arguments x <= 1, x >= 2^30, r < 1e-14 and non-finite values take green_form.
 #pragma once
 #include <cmath>
 #include <cstring>

@@ -84,3 +84,30 @@ def test_gpu_leaf_shapes(lib, k, npatch, nlevels, chunks):
         fm.precomps_and_setup(k, nlevels)
         assert fm.get_tuning()[0] == c
         assert np.array_equal(fm.compute_Ax_acc(x), y)
+
+
+def test_gpu_parts_of_a_falling_density(lib, oracle):
+    """A density that falls by 1e-30 along the curve, quarter by quarter: the far field of each quarter alone has
+    the oracle's digits (1e-11, the tables' rounding, as in test_gpu_fixpoint.py), however small the quarter is,
+    single vector and batch; the whole is the sum of the quarters to the rounding of the largest."""
+    k, npatch = 60.0, 64
+    fm = _map(lib, k=k, npatch=npatch)
+    om = oracle.OracleForwardMap([oracle.curve_kite()], 16, 0.02, 1.0, k, patches_per_curve=npatch, formulation="combined")
+    om.precompute(k)
+    om.setup_ifgf(k, fm.nlevels)
+    n = fm.total_num_unknowns_
+    g = np.random.default_rng(5)
+    x = (g.standard_normal(n) + 1j * g.standard_normal(n)) * np.exp(-np.linspace(0.0, 69.0, n))
+    parts = np.zeros((n, 13), complex)
+    for q in range(4):
+        parts[q * n // 4:(q + 1) * n // 4, 3 * q] = x[q * n // 4:(q + 1) * n // 4]
+    Y = fm.apply_batch(parts)
+    whole = fm.compute_Ax_acc(x)
+    for q in range(4):
+        p = parts[:, 3 * q]
+        far, faro = fm.ifgf_far(p), om.ifgf_far(p)
+        assert np.linalg.norm(far - faro) < 1e-11 * np.linalg.norm(faro), q
+        y = fm.compute_Ax_acc(p)
+        assert np.linalg.norm(Y[:, 3 * q] - y) <= 4e-15 * np.linalg.norm(y), q
+        whole = whole - y
+    assert np.linalg.norm(whole) < 4e-15 * np.linalg.norm(Y[:, 0])
