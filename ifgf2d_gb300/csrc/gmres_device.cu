@@ -144,7 +144,7 @@ __device__ void rotate_column(const double2* h, int j, double2* col, const doubl
     xj.x = __shfl_sync(0xffffffffu, e.x, 31); xj.y = __shfl_sync(0xffffffffu, e.y, 31);
 }
 __global__ void k_lsq_givens(const double2* __restrict__ H, int ldh, int* __restrict__ jp, LsqDev L,
-                             cudaGraphConditionalHandle cond, int use_cond, double* __restrict__ nrm2) {
+                             cudaGraphConditionalHandle cond, double* __restrict__ nrm2) {
     const int j = *jp;
     const double2* h = H + (long long)j * ldh;
     double2* col = L.R + (long long)j * ldh;
@@ -154,7 +154,7 @@ __global__ void k_lsq_givens(const double2* __restrict__ H, int ldh, int* __rest
     if (nrm2) *nrm2 = 0.0;     // the next iteration's update adds to it
     int* st = L.st;
     if (st[0] || j >= L.m) {   // a stopped cycle stays stopped
-        if (use_cond) cudaGraphSetConditional(cond, 0);
+        cudaGraphSetConditional(cond, 0);
         return;
     }
     double hn = 0.0;
@@ -167,7 +167,7 @@ __global__ void k_lsq_givens(const double2* __restrict__ H, int ldh, int* __rest
     st[1] = j + 1;
     if (stop) st[0] = 1;
     *jp = j + 1;
-    if (use_cond) cudaGraphSetConditional(cond, (stop || j + 1 >= L.m) ? 0u : 1u);
+    cudaGraphSetConditional(cond, (stop || j + 1 >= L.m) ? 0u : 1u);
 }
 
 // y = R^{-1} g over the first st[1] columns, one warp, 32 columns at a time from the last.  A lane holds one
@@ -439,9 +439,9 @@ inline unsigned nblocks(long long n, int b) { return (unsigned)((n + b - 1) / b)
 void launch_lsq_init(LsqDev L, int* jp, double beta, double r0n, double tol, int limit, cudaStream_t s) {
     k_lsq_init<<<1, 128, 0, s>>>(L, jp, beta, r0n, tol, limit);
 }
-void launch_lsq_givens(const double2* H, int ldh, int* jp, LsqDev L, cudaGraphConditionalHandle cond, bool use_cond, double* nrm2,
+void launch_lsq_givens(const double2* H, int ldh, int* jp, LsqDev L, cudaGraphConditionalHandle cond, double* nrm2,
                        cudaStream_t s) {
-    k_lsq_givens<<<1, 32, 0, s>>>(H, ldh, jp, L, cond, use_cond ? 1 : 0, nrm2);
+    k_lsq_givens<<<1, 32, 0, s>>>(H, ldh, jp, L, cond, nrm2);
 }
 void launch_lsq_solve(LsqDev L, int ldh, double2* y, cudaStream_t s) { k_lsq_solve<<<1, 32, 0, s>>>(L, ldh, y); }
 void launch_multi_axpy_dyn(const double2* V, long long ldv, const int* ncols, const double2* y, long long n, double2* w,

@@ -179,7 +179,8 @@ __host__ __device__ __forceinline__ unsigned long long root4(unsigned long long 
     return ((unsigned long long)Y0 << 39) + (unsigned long long)(((long long)(int)Y0 * c) >> 21);
 }
 
-// 2^62 (cos, sin) of f 2^-64 turns
+// 2^62 (cos, sin) of f 2^-64 turns: the power series of cos and sin of pi z / 2 in u = z^2, coefficients (-1)^j (pi /
+// 2)^(2 j) / (2 j)! and (-1)^j (pi / 2)^(2 j + 1) / (2 j + 1)! times 2^62, in the FP32 tails 2^50 (j >= 6) and 2^47 (j >= 5)
 __host__ __device__ __forceinline__ void cos_sin(unsigned long long f, long long& C, long long& S) {
     const unsigned long long g = f + (1ull << 61);
     const int quad = (int)(g >> 62);

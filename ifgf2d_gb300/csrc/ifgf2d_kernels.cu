@@ -380,28 +380,6 @@ __global__ void k_store_col(const double2* __restrict__ z, long long n, const in
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) Z[(long long)(*jp) * n + i] = z[i];
 }
-__global__ void k_multidot_dyn(const double2* __restrict__ V, long long ldv, const int* __restrict__ jp,
-                               const double2* __restrict__ w, long long n, double2* __restrict__ h) {
-    const int j = blockIdx.x;
-    if (j > *jp) return;
-    const double2* v = V + (long long)j * ldv;
-    double re = 0.0, im = 0.0;
-    for (long long i = threadIdx.x; i < n; i += blockDim.x) {
-        const double2 a = v[i], b = w[i];
-        re = fma(a.x, b.x, fma(a.y, b.y, re));
-        im = fma(a.x, b.y, fma(-a.y, b.x, im));
-    }
-    __shared__ double sr[32], si[32];
-    re = warp_sum(re); im = warp_sum(im);
-    if ((threadIdx.x & 31) == 0) { sr[threadIdx.x >> 5] = re; si[threadIdx.x >> 5] = im; }
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        const int nw = blockDim.x >> 5;
-        re = threadIdx.x < nw ? sr[threadIdx.x] : 0.0; im = threadIdx.x < nw ? si[threadIdx.x] : 0.0;
-        re = warp_sum(re); im = warp_sum(im);
-        if (threadIdx.x == 0) h[j] = make_double2(re, im);
-    }
-}
 // w -= V[:, 0..j] h: 64 rows per block, four threads per row split the columns (j = part mod 4).  h, the
 // columns' nchunk partial dots added up, is summed by every block for itself, 256 columns at a time (few
 // chunks: a launch of its own cost 2.3 us an orthogonalisation pass); block 0 also writes (add = 0) or adds (add = 1)
@@ -557,7 +535,7 @@ void launch_arnoldi_step(double2* V, long long n, int m, int* jp, double2* w, do
                                                      pass == passes - 1 ? nrm2 : nullptr);
     }
     k_scale_next<<<nblk(n, 256), 256, 0, s>>>(w, nrm2, n, V, jp, H, ldh, vin);
-    launch_lsq_givens(H, ldh, jp, lsq, cond, true, nrm2, s);
+    launch_lsq_givens(H, ldh, jp, lsq, cond, nrm2, s);
 }
 void launch_store_col(const double2* z, long long n, const int* jp, double2* Z, cudaStream_t s) {
     k_store_col<<<nblk(n, 256), 256, 0, s>>>(z, n, jp, Z);

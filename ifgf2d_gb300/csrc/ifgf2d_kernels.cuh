@@ -299,9 +299,9 @@ struct LsqBatchDev {
 // a restart cycle starts: g = beta e_1, j = 0, limit iterations allowed
 void launch_lsq_init(LsqDev L, int* jp, double beta, double r0n, double tol, int limit, cudaStream_t s);
 // after the Arnoldi step of column j = *jp: rotate it into R, update g and the estimate
-// |g_{j+1}| / ||r0||, stop on convergence, the limit or a breakdown, j += 1; with use_cond, set
+// |g_{j+1}| / ||r0||, stop on convergence, the limit or a breakdown, j += 1; set
 // the condition of the graph while-loop around the iteration (0 ends the cycle); *nrm2 = 0
-void launch_lsq_givens(const double2* H, int ldh, int* jp, LsqDev L, cudaGraphConditionalHandle cond, bool use_cond, double* nrm2,
+void launch_lsq_givens(const double2* H, int ldh, int* jp, LsqDev L, cudaGraphConditionalHandle cond, double* nrm2,
                        cudaStream_t s);
 // y = R^{-1} g over the cycle's columns (st[1])
 void launch_lsq_solve(LsqDev L, int ldh, double2* y, cudaStream_t s);

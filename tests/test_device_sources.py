@@ -3,7 +3,10 @@
 Each check is a small translation unit over the library's own headers that nvcc must accept.
 """
 import os
+import re
 import subprocess
+
+import pytest
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
@@ -37,3 +40,20 @@ using namespace ifgf;
 static_assert(dot_block_terms(200) == 1 && dot_block_terms(65536) == 32, "few chunks: by the blocks");
 static_assert(dot_block_terms(65537) == 1 && dot_block_terms(1 << 19) == 1 && dot_block_terms(1ll << 32) == 1, "more: added up once");
 """)
+
+
+def test_cosine_and_sine_coefficients():
+    """The constants of cos_sin are the power series it names."""
+    mp = pytest.importorskip("mpmath")
+    mp.mp.dps = 40
+    text = open(os.path.join(ROOT, "ifgf2d_gb300", "csrc", "green_fx.cuh")).read()
+    body = re.search(r"void cos_sin\(.*?\n}\n", text, re.S)[0]
+    cos, sin = body.split("const int v5")
+    for part, odd, tail, scale in ((cos, 0, 6, 50), (sin, 1, 5, 47)):
+        c = [(-1) ** j * (mp.pi / 2) ** (2 * j + odd) / mp.factorial(2 * j + odd) for j in range(tail + 5)]
+        for j in range(tail):
+            assert f"0x{int(mp.nint(abs(c[j]) * 2 ** 62)):x}ll" in part, j
+        assert str(int(mp.nint(abs(c[tail]) * 2 ** scale))) in part
+        floats = [float(v) for v in re.findall(r"-?\d+\.\d+(?=[f)])", part)]
+        for j in range(tail + 1, tail + 4 + odd):
+            assert min(abs(v - float(c[j] * 2 ** scale)) for v in floats) < 1e-6 * abs(float(c[j] * 2 ** scale)), j
