@@ -322,12 +322,13 @@ inline std::vector<LeafItem> leaf_item_list(const std::vector<int>& cone_box, co
     }
     return items;
 }
-// threads that share a coefficient's sum in the FP64 leaf sums: 2, but 5 for trees of so few leaf cones (32 an
-// SM, 1.6 times what 4 blocks of 5 cones an SM hold) that the length of a thread's walk is what counts.  us with 2 and
-// 5 threads: 202 cones of boxes of 80, 330 and 660 sources 20 / 14, 104 / 51 and 205 / 96; 1040 to 4456 cones of 140 to 570
-// sources 65 / 35, 135 / 72, 260 / 212, 180 / 152; 2310 and 4866 of 33 sources 22 / 20 and 30 / 30; 10924 and 45614 (kite
-// k = 500 and 2000) 43 / 57 and 229 / 307.
-inline int leaf_fx_chunks(int cones) { return cones <= 32 * 152 ? 5 : 2; }
+// threads that share a coefficient's sum in the FP64 leaf sums: 2, but 5 for trees of few leaf cones (up to 12 an
+// SM, where 4 blocks of 5 would fit), as the length of a thread's walk is what counts there.  us of the leaf sums with 2
+// and 5 threads: 202 cones of boxes of 80, 330 and 660 sources 20 / 14, 104 / 51 and 205 / 96; 1040 to 1784 cones of 140 to
+// 570 sources 65 / 35, 135 / 72, 260 / 212; 10924 and 45614 cones (kite k = 500 and 2000) 43 / 57 and 229 / 307.  Whole
+// applies of three callers: kite k = 60 and 80 (below the line) 19.2 / 18.2 and 22.5 / 21.6, k = 100 and 150 (above it)
+// 26.3 / 27.8 and 34.7 / 38.0.
+inline int leaf_fx_chunks(int cones) { return cones <= 12 * 152 ? 5 : 2; }
 // What a group of obstacles (group.cu) changes in the device part of the IFGF set-up: (k, eta)
 // per leaf box and per leaf cone (device arrays), and the leaf-cone nodes and the propagation
 // plan, both built member by member.

@@ -300,7 +300,7 @@ __host__ __device__ __forceinline__ double2 value(const GreenFx& K, const Four* 
 // k = 0.5: 643 and 402 ms, combined and single layer; out of line, with these formed again, 662 and 411).
 __device__ __forceinline__ double2 green(const GreenFx& K, double dx, double dy, double nx, double ny) {
     const double d2 = dx * dx + dy * dy;
-    if ((unsigned)__double2hiint(d2) - K.lo >= K.span) {
+    if (__builtin_expect((unsigned)__double2hiint(d2) - K.lo >= K.span, 0)) {
         if (K.form != 2) return green_sl(d2, K.k);
         return green_cfie(d2, dx * nx + dy * ny, K.k, K.k4, K.eta4);
     }

@@ -235,9 +235,11 @@ __global__ void __launch_bounds__(kTile) k_direct_far(const double* __restrict__
 // The same sum with one 128-thread block per target, for target counts that would leave most
 // SMs idle with one thread per target (N = 200: 2 blocks).  Thread t takes sources t, t + 128, ...;
 // the partial sums combine in a fixed order (warp butterfly, then warps 0..3), so the result
-// does not depend on scheduling.  N = 200 at k = 10, with three callers: 21.7 -> 8.4 us by green_fx.cuh.
+// does not depend on scheduling.  N = 200 at k = 10, with three callers: 21.7 -> 8.4 us by green_fx.cuh.  Six blocks an SM
+// are asked for so that the compiler takes 80 registers: with the 68 it takes by itself the value's chain is 6 % longer
+// at N = 200 to 400, with 96 (five blocks) the sum 8 % at N = 1664.
 constexpr int kDirectSplitBelow = 2 * 152 * kTile;
-__global__ void __launch_bounds__(kTile) k_direct_far_split(const double* __restrict__ tx, const double* __restrict__ ty,
+__global__ void __launch_bounds__(kTile, 6) k_direct_far_split(const double* __restrict__ tx, const double* __restrict__ ty,
                              const int* __restrict__ t_patch, const int* __restrict__ t_nsp_ptr, const int* __restrict__ t_nsp,
                              const double* __restrict__ sx, const double* __restrict__ sy, const double* __restrict__ snx,
                              const double* __restrict__ sny, const int* __restrict__ s_patch,
