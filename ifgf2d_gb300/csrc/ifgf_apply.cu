@@ -435,9 +435,9 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // term interpolates in integers (about 160 wide multiply-adds) and takes 6 FP64 operations for its
 // conversion and factor ratio, against 60 with FP64 interpolation.  The node values get their cone's
 // common exponent, the values->coefficients map runs in integers again, and the coefficients are
-// normalised to the top bits of the cone's largest.  Kite, all levels: k = 500 290 -> 100 us, k = 2000
-// 1287 -> 399 us (the FP64 kernel before it ran at 91-95 % of the FP64 pipe).  What bounds it: the wide
-// multiply-adds and 64-bit shifts take two issue slots each; some 45 % of the slots issue.  Measured
+// normalised to the top bits of the cone's largest.  Kite, all levels: k = 500 290 -> 96 us, k = 2000
+// 1287 -> 381 us (the FP64 kernel before it ran at 91-95 % of the FP64 pipe).  What bounds it: the wide
+// multiply-adds and 64-bit shifts take two issue slots each; some 41 % of the slots issue.  Measured
 // slower: a thread per node gathering from L1 (110 us), a warp per parent cone (131 us: 25 of 32
 // lanes), persistent blocks that fetch ahead (111-125 us).
 template <int PS, int PA>
@@ -859,8 +859,8 @@ __global__ void __launch_bounds__(256) k_final_t(int N, const int* __restrict__ 
 // field: the neighbour boxes' densities, loaded while the interpolation runs, are brought to one exponent
 // in shared memory; a warp takes a target's table row with its lanes over the sources, and the lanes'
 // integer sums add up by shuffles.  Bound by latency at small sizes, by the wide multiply-adds else.
-// Kite k = 500 / 2000: 55 / 260 us with FP64 multiply-adds, 35 / 114 us so; 4 blocks an SM against 3:
-// 39 / 119, against 2: 41 / 150.
+// Kite k = 500 / 2000: 55 / 260 us with FP64 multiply-adds, 33 / 105 us so.  When it took 35 / 114 with 4 blocks
+// an SM, 3 took 39 / 119 and 2 41 / 150.
 template <int PS, int PA>
 __global__ void __launch_bounds__(256, 4) k_final_fx(const FinItem* __restrict__ items, const int* __restrict__ near_src,
                                                   const int4* __restrict__ near, const int* __restrict__ nexp,

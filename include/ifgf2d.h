@@ -149,7 +149,9 @@ int ifgf2d_solve(ifgf2d_ctx* ctx, const double* rhs, double* x, int mode, double
  * ForwardMap.tpp:658-697).  x, y, rhs are column-major N x nrhs complex matrices (right-hand
  * side r at offset 2*N*r doubles, interleaved re/im), as an Eigen::MatrixXcd stores them.  The
  * IFGF modes process up to IFGF2D_MAX_BATCH right-hand sides per pass over the tables (larger
- * batches run in chunks); IFGF2D_APPLY_DIRECT runs one right-hand side at a time. */
+ * batches run in chunks); IFGF2D_APPLY_DIRECT runs one right-hand side at a time.  FP64 chunks of
+ * up to eleven columns take the single-vector apply column by column, so the last bits of a column may
+ * differ with the width of its batch (3e-16 of its norm). */
 #define IFGF2D_MAX_BATCH 64
 int ifgf2d_apply_batch(ifgf2d_ctx* ctx, const double* x, double* y, int nrhs, int mode);
 /* the same on device-resident matrices (cudaMalloc'ed, N * nrhs complex each); asynchronous on
