@@ -127,18 +127,15 @@ struct PlanStage {
     const int* level(int l) const { return list.p + at[l]; }
     cudaError_t build(const Tree& T, const long long* pp_ptr, PlanX pp, cudaStream_t s) {
         at.assign(T.nlevels + 1, 0);
-        size_t total = 0;
+        StageLevels L;
+        if (T.nlevels > StageLevels::most) return cudaErrorInvalidValue;
         for (int l = T.nlevels - 1; l >= 3; --l) {
-            at[l] = total;
-            total += stage_plan_size((int)T.L[l - 1].cone_nonrel.size(), T.Ps, T.Pang);
-        }
-        cudaError_t e = list.alloc(total);
-        for (int l = T.nlevels - 1; l >= 3 && e == cudaSuccess; --l) {
             const TreeLevel& Lp = T.L[l - 1];
-            launch_stage_plan(Lp.cone_base, Lp.cone_base + (int)Lp.cone_nonrel.size(), pp_ptr, pp, T.Ps, T.Pang, list.p + at[l], s);
-            e = cudaGetLastError();
+            at[l] = L.add(Lp.cone_base, Lp.cone_base + (int)Lp.cone_nonrel.size(), T.Ps, T.Pang);
         }
-        return e;
+        if (const cudaError_t e = list.alloc(L.size(T.Ps, T.Pang)); e != cudaSuccess) return e;
+        launch_stage_plan(L, pp_ptr, pp, T.Ps, T.Pang, list.p, s);
+        return cudaGetLastError();
     }
 };
 

@@ -497,8 +497,6 @@ static int setup_cones(ifgf2d_ctx* ctx, double k, int nlevels, const SetupExtra*
         CK(ctx->GsepX.alloc(Gs.size()));
         std::vector<float> Gs32(Gs.begin(), Gs.end());
         CK(ctx->Gsep32.upload(Gs32));
-        launch_fx_weights(ctx->Gsep.p, (int)Gs.size(), ctx->GsepX.p, ctx->stream);
-        CK(cudaGetLastError());
     }
     // The uploads come before the kernels that follow them: a copy from pageable host memory
     // queued behind a running kernel holds the host until the kernel ends.  The leaf-cone nodes'
@@ -526,12 +524,15 @@ static int setup_cones(ifgf2d_ctx* ctx, double k, int nlevels, const SetupExtra*
     if (ex) CK(ex->build_plan(ctx->pp.view(), ctx->pp32.p, perr.p, ctx->stream));
     else if (by_level) CK(by_level->gather(ctx->pp.view(), ctx->pp32.p, perr.p, ctx->stream));
     else CK(build_prop_plan(T, ctx->pp.view(), ctx->pp32.p, perr.p, ctx->stream));
-    CK(ctx->pp_stage.build(T, ctx->pp_ptr.p, ctx->pp.view(), ctx->stream));
     // leaf-cone tables
     launch_leaf_setup(ctx->leaf_cone_box.p, ncl, ctx->leaf_start.p, ctx->leaf_count.p, ctx->leaf_off.p, ctx->leaf_nodes_d.p,
                       ctx->xs_s.p, ctx->ys_s.p, ctx->nxs_s.p, ctx->nys_s.p, T.Ps, T.Pang, k, ctx->form, ctx->eta, ctx->Gsep.p,
                       reinterpret_cast<double2*>(ctx->leafL.p), ctx->stream, ex ? ex->keta_leafcone : nullptr);
     CK(cudaGetLastError());
+    // what only the applies need, behind the tables: between the uploads above the first of these held the host
+    // 0.2 ms, as a copy from pageable memory waits for the kernel before it
+    launch_fx_weights(ctx->Gsep.p, (int)ctx->Gsep.n, ctx->GsepX.p, ctx->stream);
+    CK(ctx->pp_stage.build(T, ctx->pp_ptr.p, ctx->pp.view(), ctx->stream));
     return IFGF2D_OK;
 }
 
@@ -541,19 +542,8 @@ static int setup_interp(ifgf2d_ctx* ctx, int nlevels, DBuf<int>& perr) {
     const long long N = D.N;
     const int P = T.P;
     const int nleaf = (int)T.leaf_start.size();
-    DBuf<InterpEntryD> ip;
-    {   // interpolation plan: the entries come from the host tree
-        static_assert(sizeof(InterpEntry) == sizeof(InterpEntryD), "host and device plan layouts differ");
-        CK(ip.upload(reinterpret_cast<const InterpEntryD*>(T.ip.data()), T.ip.size()));
-        CK(ctx->ip_ptr.upload(T.ip_ptr));
-        CK(ctx->ip32.alloc(T.ip.size()));
-        CK(ctx->ipx.alloc(T.ip.size()));
-        launch_interp_to_c64(ip.p, (long long)T.ip.size(), ctx->ip32.p, ctx->stream);
-        launch_interp_fx(ip.p, (long long)T.ip.size(), ctx->ipx.p, ctx->stream);
-        CK(cudaGetLastError());
-    }
+    std::vector<FinItem> fitems, qitems;
     {   // near field and interpolation by leaf box: equal shares of each box's targets
-        std::vector<FinItem> fitems, qitems;
         long long near_at = 0;      // the box's near-field block, and its list of sources
         int src_at = 0;
         for (int b = 0; b < nleaf; ++b) {
@@ -580,8 +570,18 @@ static int setup_interp(ifgf2d_ctx* ctx, int nlevels, DBuf<int>& perr) {
             near_at += (long long)n * rl;
             src_at += rl;
         }
+    }
+    DBuf<InterpEntryD> ip;
+    {   // interpolation plan: the entries come from the host tree
+        static_assert(sizeof(InterpEntry) == sizeof(InterpEntryD), "host and device plan layouts differ");
+        CK(ip.upload(reinterpret_cast<const InterpEntryD*>(T.ip.data()), T.ip.size()));
+        CK(ctx->ip_ptr.upload(T.ip_ptr));
         CK(ctx->fx_items.upload(fitems));
         CK(ctx->fin32_items.upload(qitems));
+        CK(ctx->ip32.alloc(T.ip.size()));
+        CK(ctx->ipx.alloc(T.ip.size()));
+        launch_interp_to_c64(ip.p, (long long)T.ip.size(), ctx->ip32.p, ctx->stream);
+        launch_interp_fx(ip.p, (long long)T.ip.size(), ctx->ipx.p, ctx->stream);
         CK(ctx->ipT.alloc(T.ip.size())); CK(ctx->ip32T.alloc(T.ip.size()));
         launch_interp_transpose((int)N, ctx->point_leaf.p, ctx->leaf_start.p, ctx->leaf_count.p, ctx->ip_ptr.p, ip.p, ctx->ip32T.p,
                                 ctx->ipT.view(), ctx->stream);

@@ -131,10 +131,15 @@ constexpr int kPropStaged = 1;
 void launch_propagate_t(int pbegin, int pend, const long long* pp_ptr, const int* pp_nchild, const PropE<float>* pp, int Ps,
                         int Pang, const float* Gsep, float2* coef, cudaStream_t s, int cones_per_block = 0);
 // the FP64 form in fixed point: GsepX the separable map's entries as limbs, cexp the cones' exponents,
-// stage the records of the level's groups of parents (stage_plan_size ints for ncones parents), which
-// launch_stage_plan fills together with pp.slot
-size_t stage_plan_size(int ncones, int Ps, int Pang);
-void launch_stage_plan(int pbegin, int pend, const long long* pp_ptr, PlanX pp, int Ps, int Pang, int* stage, cudaStream_t s);
+// stage the records of the level's groups of parents, which launch_stage_plan fills for all levels together
+// with pp.slot
+struct StageLevels {
+    static constexpr int most = 24;             // the deepest tree
+    int n = 0, begin[most] = {}, end[most] = {}, group[most + 1] = {};     // parents, first group of each level
+    size_t add(int b, int e, int Ps, int Pang);       // one more level, parents [b, e): where its records start
+    size_t size(int Ps, int Pang) const;              // ints of all records
+};
+void launch_stage_plan(const StageLevels& L, const long long* pp_ptr, PlanX pp, int Ps, int Pang, int* stage, cudaStream_t s);
 void launch_propagate_fx(int pbegin, int pend, PlanX pp, const int* stage, int Ps, int Pang, const int2* GsepX, int4* coef, int* cexp,
                          cudaStream_t s);
 // n doubles in [-1, 1] as fixed-point limbs; the interpolation plan with (s, theta) as weights

@@ -531,16 +531,19 @@ __global__ void __launch_bounds__(kPropFxThreads) k_propagate_fx(int pbegin, int
 }
 
 // set-up of k_propagate_fx: a group's record with the first PropFx::slots of its distinct child cones
-// in ascending order, and per term its slot (PropFx::slots: not staged)
+// in ascending order, and per term its slot (PropFx::slots: not staged).  All levels in one launch: a level by
+// itself takes the latency of one group's searches, 24 to 29 us at k = 500 however few its groups.
 template <int P>
-__global__ void __launch_bounds__(kPropFxThreads) k_stage_plan(int pbegin, int pend, const long long* __restrict__ pp_ptr, PlanX pp,
-                                                               int* __restrict__ stage) {
+__global__ void __launch_bounds__(kPropFxThreads) k_stage_plan(const __grid_constant__ StageLevels L, const long long* __restrict__ pp_ptr,
+                                                               PlanX pp, int* __restrict__ stage) {
     using F = PropFx<P>;
     constexpr int CPB = F::cones, CAP = F::slots, NT = kPropFxThreads;
     __shared__ int kid[F::terms], uniq[F::terms];
     __shared__ int nu;
     const int tid = threadIdx.x;
-    const int c0 = pbegin + blockIdx.x * CPB, nc = min(CPB, pend - c0);
+    int l = 0;
+    while (l + 1 < L.n && (int)blockIdx.x >= L.group[l + 1]) ++l;
+    const int c0 = L.begin[l] + ((int)blockIdx.x - L.group[l]) * CPB, nc = min(CPB, L.end[l] - c0);
     const long long e0 = pp_ptr[c0];
     const int nt = min((int)(pp_ptr[c0 + nc] - e0), F::terms);
     if (tid == 0) nu = 0;
@@ -1067,15 +1070,23 @@ void launch_propagate_t(int pbegin, int pend, const long long* pp_ptr, const int
                                                                                                      pp_nchild, pp, Gsep, coef);
     });
 }
-size_t stage_plan_size(int ncones, int Ps, int Pang) {
-    size_t n = 0;
-    IFGF_DISPATCH_P(Ps, Pang, n = (size_t)((ncones + PropFx<PS * PA>::cones - 1) / PropFx<PS * PA>::cones) * PropFx<PS * PA>::record;);
-    return n;
+size_t StageLevels::add(int b, int e, int Ps, int Pang) {
+    int groups = 0, record = 0;
+    IFGF_DISPATCH_P(Ps, Pang, { groups = (int)nblk_a(e - b, PropFx<PS * PA>::cones); record = PropFx<PS * PA>::record; });
+    begin[n] = b; end[n] = e;
+    const size_t at = (size_t)group[n] * record;
+    group[n + 1] = group[n] + groups;
+    ++n;
+    return at;
 }
-void launch_stage_plan(int pbegin, int pend, const long long* pp_ptr, PlanX pp, int Ps, int Pang, int* stage, cudaStream_t s) {
-    if (pend <= pbegin) return;
-    IFGF_DISPATCH_P(Ps, Pang, (k_stage_plan<PS * PA><<<nblk_a(pend - pbegin, PropFx<PS * PA>::cones), kPropFxThreads, 0, s>>>(
-                                   pbegin, pend, pp_ptr, pp, stage)));
+size_t StageLevels::size(int Ps, int Pang) const {
+    size_t record = 0;
+    IFGF_DISPATCH_P(Ps, Pang, record = PropFx<PS * PA>::record;);
+    return (size_t)group[n] * record;
+}
+void launch_stage_plan(const StageLevels& L, const long long* pp_ptr, PlanX pp, int Ps, int Pang, int* stage, cudaStream_t s) {
+    if (L.group[L.n] <= 0) return;
+    IFGF_DISPATCH_P(Ps, Pang, (k_stage_plan<PS * PA><<<L.group[L.n], kPropFxThreads, 0, s>>>(L, pp_ptr, pp, stage)));
 }
 void launch_propagate_fx(int pbegin, int pend, PlanX pp, const int* stage, int Ps, int Pang, const int2* GsepX, int4* coef, int* cexp,
                          cudaStream_t s) {
