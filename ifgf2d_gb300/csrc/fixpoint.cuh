@@ -81,17 +81,21 @@ __device__ __forceinline__ double fx_ldexp(double d, int e) {
     const int a = min(max(e, -1000), 1000), b = min(max(e - a, -1022), 1023);
     return d * __hiloint2double((1023 + a) << 20, 0) * __hiloint2double((1023 + b) << 20, 0);
 }
+// what a block's exponent E does to its values: added to a double's high word, if near (else by fx_ldexp)
+struct FxScale { unsigned add; int e; bool near; };
+__device__ __forceinline__ FxScale fx_scale(int E, int T) {
+    return FxScale{(unsigned)(E - T) << 20, E == kFxBad ? kFxBad : E - T, (unsigned)(E - kFxNear0) <= (unsigned)(kFxNear1 - kFxNear0)};
+}
 // (x, y) 2^(E - T) as doubles (x and y integers below 2^62 in magnitude)
-__device__ __forceinline__ double2 fx_value(long long x, long long y, int E, int T) {
+__device__ __forceinline__ double2 fx_value(long long x, long long y, FxScale s) {
     double a = (double)x, b = (double)y;
-    if ((unsigned)(E - kFxNear0) <= (unsigned)(kFxNear1 - kFxNear0)) {
-        const unsigned sh = (unsigned)(E - T) << 20;
-        a = __hiloint2double(x != 0 ? (int)((unsigned)__double2hiint(a) + sh) : 0, __double2loint(a));
-        b = __hiloint2double(y != 0 ? (int)((unsigned)__double2hiint(b) + sh) : 0, __double2loint(b));
+    if (s.near) {
+        a = __hiloint2double(x != 0 ? (int)((unsigned)__double2hiint(a) + s.add) : 0, __double2loint(a));
+        b = __hiloint2double(y != 0 ? (int)((unsigned)__double2hiint(b) + s.add) : 0, __double2loint(b));
     } else {
         const double nan = __hiloint2double(0x7ff80000, 0);
-        a = E == kFxBad ? nan : fx_ldexp(a, E - T);
-        b = E == kFxBad ? nan : fx_ldexp(b, E - T);
+        a = s.e == kFxBad ? nan : fx_ldexp(a, s.e);
+        b = s.e == kFxBad ? nan : fx_ldexp(b, s.e);
     }
     return make_double2(a, b);
 }
@@ -157,7 +161,7 @@ __device__ __forceinline__ double2 fx_interp_value(Load&& c, int E, longlong2 st
     fx_cheb<PA>(st.y, Tt);
     long long re, im;
     fx_interp<PS, PA>(Ts, Tt, c, re, im);
-    return fx_value(re, im, E, fx_top(PS * PA));
+    return fx_value(re, im, fx_scale(E, fx_top(PS * PA)));
 }
 // ---- table sums (leaf cones): sum_s L[s] rho[s] of complex values, the table entries and the densities
 // both as integers of kFxSumTop bits in two 27-bit limbs, X = h 2^27 + l, |l| <= 2^26 (the left-out

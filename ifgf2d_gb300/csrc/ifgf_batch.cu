@@ -237,8 +237,12 @@ __global__ void k_rho_bx(const int* __restrict__ leaf_start, const int* __restri
 // BIG (launched for trees with a box of more than kFxSumMost sources): such a box's sums of kFxSumMost
 // sources each are added up in FP64, in the place of the coefficients.
 constexpr int kLeafBxTile = 8;
+// With 6 x 6 cones BIG's loads for all coefficients at once took 237 registers and one block an SM; one at a time and held
+// to two blocks, 64 right-hand sides of kite k = 200 take 3.33 ms instead of 3.65.  The other orders keep two and
+// three blocks without, and lose 3 % with it.
 template <int P, int MS, int NT, bool BIG>
-__global__ void __launch_bounds__(NT * MS) k_leaf_bx(const int* __restrict__ cone_box, int cone_base, const int* __restrict__ leaf_start,
+__global__ void __launch_bounds__(NT * MS, BIG && P == 36 ? 65536 / (NT * MS * 160) : 0)
+                                           k_leaf_bx(const int* __restrict__ cone_box, int cone_base, const int* __restrict__ leaf_start,
                                                      const int* __restrict__ leaf_count, const long long* __restrict__ leaf_off,
                                                      const int4* __restrict__ L, const int* __restrict__ lexp,
                                                      const int4* __restrict__ rho, const int* __restrict__ rexp, int B, int Ps,
@@ -304,6 +308,7 @@ __global__ void __launch_bounds__(NT * MS) k_leaf_bx(const int* __restrict__ con
                     *o = make_double2(a.x + fx_scaled(ya, ea), a.y + fx_scaled(yb, eb));
                 }
                 re[m] = im[m] = FxSum{0, 0};
+                if (P == 36) asm volatile("" ::: "memory");   // one coefficient's loads at a time
             }
         }
         __syncthreads();                        // the buffer is refilled two tiles later
@@ -494,7 +499,8 @@ __device__ __forceinline__ void terms_x(StageX<PS, PA>& S, TermsX terms, long lo
                                         const int* __restrict__ cexp, int B, int rr, Add&& add) {
     constexpr int P = PS * PA, N4 = fx_rows4(PS, PA), T = fx_top(P);
     int4 cc[P];
-    int cur = -1, E = 0;
+    int cur = -1;
+    FxScale scale{};
     for (int c0 = 0; c0 < n; c0 += kTermsChunk) {
         const int cnt = min(kTermsChunk, n - c0);
         __syncthreads();                       // the previous chunk has been read
@@ -513,7 +519,7 @@ __device__ __forceinline__ void terms_x(StageX<PS, PA>& S, TermsX terms, long lo
                 const int4* src = coef + (long long)cur * P * B + rr;
 #pragma unroll
                 for (int q = 0; q < P; ++q) cc[q] = src[(long long)q * B];
-                E = cexp[(long long)cur * B + rr];
+                scale = fx_scale(cexp[(long long)cur * B + rr], T);
             }
             FxLimb t[2 * N4];
 #pragma unroll
@@ -524,7 +530,7 @@ __device__ __forceinline__ void terms_x(StageX<PS, PA>& S, TermsX terms, long lo
             long long re, im;
             fx_interp<PS, PA>(t, t + PS - 1, [&](int q) { return cc[q]; }, re, im);
             const double2 w = S.w[i];
-            add(id.y, fx_value(re, im, E, T), w);
+            add(id.y, fx_value(re, im, scale), w);
         }
     }
 }
