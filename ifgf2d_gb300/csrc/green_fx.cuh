@@ -15,7 +15,8 @@
 //      bracket with one binary exponent, the larger of the two coefficients'.
 // The errors are a few 2^-57 of |g| and x 2^-58 in the phase (r is an integer in units of 2^-58 of a power of
 // two: 1e-15 at x = 300, 5e-13 at 10^5) beside those of the FP64 operations that are left (|d|^2, d . n, the
-// products by A), against x 2^-53, the rounding of k r, and more before.  Arguments x <= 1, x >= 2^30, r < 1e-14 and non-finite values take green_form.
+// products by A), against x 2^-53, the rounding of k r, and more before.  Arguments x <= 1, x >= 2^30, r < 1e-14
+// and non-finite values take the FP64 form.
 #pragma once
 #include <cmath>
 #include <cstring>
